@@ -39,7 +39,7 @@ static constexpr int BM = 128;  // weight rows per CTA (UMMA M)
 static constexpr int BK = 64;   // k elements per stage (128 B rows, SWIZZLE_128B)
 template <int BN>
 struct TcCfg {
-  static constexpr int STAGES = BN <= 128 ? 6 : 4;  // 6 x (16+16) KiB at BN=128; 4 x 48 KiB at BN=256
+  static constexpr int STAGES = BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : BN <= 128 ? 7 : 4;  // what 227 KiB hold (4 x 48 KiB at BN=256)
 };
 
 // ------------------------------------------------------------------ PTX wrappers
@@ -52,11 +52,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// bounded wait: a protocol bug must trap (loud failure), never hang the GPU
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-  uint32_t done = 0;
-  long long t0 = clock64();
-  while (true) {
+// Waits for the phase of this parity.  After the limit (about a second) it sets *dead, and from then on no wait of the CTA waits: the
+// producers stop, the epilogue stores values that are not numbers, the CTA lets copies in flight land and returns.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
+  for (int i = 0; i < 4000000; ++i) {
+    uint32_t done = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -64,9 +64,22 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (done) return;
-    if (clock64() - t0 > 4000000000ll) __trap();  // ~2 s
+    if (done) return true;
+    if ((i & 63) == 63 && *dead) return false;
   }
+  *dead = 1;
+  return false;
+}
+__device__ __forceinline__ void dead_drain(const volatile int* dead) {
+  if (*dead)
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+}
+// one lane of the converged warp; under a branch on it the compiler emits tcgen05 and TMA instructions once (under a branch on the
+// lane number each of them goes through code for any set of active lanes)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
@@ -101,6 +114,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mark_bad(uint32_t (&r)[16]) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) r[j] = 0x7fc00000u;
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -166,6 +183,9 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
                                                             const __grid_constant__ CUtensorMap map_x, TcArgs g) {
   pdl_trigger();  // let the next kernel's CTAs get scheduled; they wait in their own pdl_wait()
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int dead_s;
+  volatile int* const dead = &dead_s;
+  if (threadIdx.x == 0) dead_s = 0;  // (a barrier follows before any wait)
   constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -223,8 +243,12 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
   };
 
+  // The loops of both roles carry stage, parity and descriptors from step to step, and the MMA loop runs on the whole warp with one
+  // elected lane.  With a division by the stage count, a clock read per wait and descriptors built per product a step took 0.27 us
+  // whatever the tile's width (76 steps at K = 4864: 22.8 us on an idle chip); now 0.18 us (15.4 us).  The products of a step
+  // themselves take 0.025 us at 16 tokens, 0.27 us at 256.
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // Weights never depend on the previous kernel: start streaming them BEFORE waiting for
       // it (programmatic dependent launch), so HBM stays busy across the kernel boundary.
       const int pre = g.w_static ? min(nkb, TC_STAGES) : 0;
@@ -235,33 +259,37 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       pdl_wait();  // activations are produced by the previous kernel
       for (int i = 0; i < pre; ++i)
         tma_load_2d(smem0 + i * STAGE_BYTES + A_BYTES, &map_x, full_bar(i), (kb0 + i) * BK, tok_base);
+      int s = pre == TC_STAGES ? 0 : pre;
+      uint32_t ph = pre == TC_STAGES ? 0 : 1;  // the first pass over the ring waits for nothing
       for (int i = pre; i < nkb; ++i) {
-        const int s = i % TC_STAGES;
-        const uint32_t ph = (i / TC_STAGES) & 1;
-        mbar_wait(empty_bar(s), ph ^ 1);
+        if (!mbar_wait(empty_bar(s), ph, dead)) break;
         mbar_expect_tx(full_bar(s), STAGE_BYTES);
         load_w(i, s);
         tma_load_2d(smem0 + s * STAGE_BYTES + A_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, tok_base);
+        if (++s == TC_STAGES) s = 0, ph ^= 1;
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, BN);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % TC_STAGES;
-        const uint32_t ph = (i / TC_STAGES) & 1;
-        mbar_wait(full_bar(s), ph);
-        tc_fence_after();
-        const uint32_t sa = smem0 + s * STAGE_BYTES, sb = sa + A_BYTES;
+    constexpr uint32_t idesc = make_idesc(BM, BN);
+    const uint64_t ad0 = make_desc(smem0), bd0 = make_desc(smem0 + A_BYTES);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int i = 0; i < nkb; ++i) {
+      mbar_wait(full_bar(s), ph, dead);
+      tc_fence_after();
+      const uint64_t step = (uint64_t)(s * (STAGE_BYTES >> 4));
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          // advance 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
-          umma_bf16(tmem_base, make_desc(sa + k * 32), make_desc(sb + k * 32), idesc, (i | k) != 0);
-        }
+        for (int k = 0; k < BK / 16; ++k)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
+          umma_bf16(tmem_base, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (i | k) != 0);
         umma_commit(empty_bar(s));  // frees the smem stage once the MMAs have read it
       }
-      umma_commit(tmem_full_bar);  // accumulator complete
+      __syncwarp();
+      if (++s == TC_STAGES) s = 0, ph ^= 1;
     }
+    if (elect_one()) umma_commit(tmem_full_bar);  // accumulator complete
+    __syncwarp();
   }
 
   // ================= epilogue =================
@@ -278,15 +306,17 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       const int qd = warp & 3;
       pdl_wait();  // `out` may still be read (residual) by the previous kernel
       if (nkb > 0) {
-        mbar_wait(tmem_full_bar, 0);
+        mbar_wait(tmem_full_bar, 0, dead);
         tc_fence_after();
       }
+      const bool bad = *dead;
       const int lane_row = qd * 32 + lane;
 #pragma unroll
       for (int c0 = 0; c0 < BN; c0 += 16) {
         uint32_t r[16];
         if (nkb > 0) {
           tmem_ld16(tmem_base + ((uint32_t)(qd * 32) << 16) + c0, r);
+          if (bad) mark_bad(r);
         } else {
 #pragma unroll
           for (int j = 0; j < 16; ++j) r[j] = 0u;
@@ -362,6 +392,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
     __syncthreads();
     if (warp == 1) {
+      dead_drain(dead);
       tc_fence_after();
       tmem_dealloc(tmem_base, TMEM_COLS);
     }
@@ -376,15 +407,17 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   if (epi_warp) {
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
     if (nkb > 0) {
-      mbar_wait(tmem_full_bar, 0);
+      mbar_wait(tmem_full_bar, 0, dead);
       tc_fence_after();
     }
+    const bool bad = *dead;
     const int lane_row = qd * 32 + lane;  // TMEM lane = row inside the 128-row tile
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 16) {
       uint32_t r[16];
       if (nkb > 0) {
         tmem_ld16(tmem_base + ((uint32_t)(qd * 32) << 16) + c0, r);
+        if (bad) mark_bad(r);
       } else {
 #pragma unroll
         for (int j = 0; j < 16; ++j) r[j] = 0u;
@@ -495,6 +528,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   }
   __syncthreads();
   if (warp == 1) {
+    dead_drain(dead);
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
@@ -528,6 +562,9 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
                                                                    int token_tiles) {
   pdl_trigger();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int dead_s;
+  volatile int* const dead = &dead_s;
+  if (threadIdx.x == 0) dead_s = 0;  // (a barrier follows before any wait)
   constexpr int A_BYTES = BM * BK * 2;
   constexpr uint32_t TMEM_COLS = 512;  // two accumulators
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -575,17 +612,17 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 1;
+      bool go = true;
       pdl_wait();  // activations come from the previous kernel (these launches run for 30-300 us: no early weight prefetch)
-      for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      for (int t = blockIdx.x; t < total && go; t += gridDim.x) {
         int tile, ttile, si, row0;
         tile_geom(t, tile, ttile, si, row0);
         const CUtensorMap* map_w = g.dual ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % P_STAGES;
-          const uint32_t ph = (it / P_STAGES) & 1;
-          mbar_wait(empty_bar(s), ph ^ 1);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(go = mbar_wait(empty_bar(s), ph, dead))) break;
           mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
           const uint32_t sa = smem0 + s * P_STAGE_BYTES;
           if (g.dual) {
@@ -595,31 +632,35 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
             tma_load_2d(sa, map_w, full_bar(s), kb * BK, row0);
           }
           tma_load_2d(sa + A_BYTES, &map_x, full_bar(s), kb * BK, ttile * PBN);
+          if (++s == P_STAGES) s = 0, ph ^= 1;
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, PBN);
-      uint32_t it = 0;
-      int j = 0;
-      for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
-        const int buf = j & 1;
-        mbar_wait(tempty_bar(buf), (((uint32_t)j >> 1) & 1) ^ 1);  // epilogue has drained this accumulator
+    constexpr uint32_t idesc = make_idesc(BM, PBN);
+    const uint64_t ad0 = make_desc(smem0), bd0 = make_desc(smem0 + A_BYTES);
+    int s = 0, j = 0;
+    uint32_t ph = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+      const int buf = j & 1;
+      mbar_wait(tempty_bar(buf), (((uint32_t)j >> 1) & 1) ^ 1, dead);  // epilogue has drained this accumulator
+      tc_fence_after();
+      const uint32_t acc = tmem_base + (uint32_t)buf * PBN;
+      for (int kb = 0; kb < nkb; ++kb) {
+        mbar_wait(full_bar(s), ph, dead);
         tc_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)buf * PBN;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int s = it % P_STAGES;
-          const uint32_t ph = (it / P_STAGES) & 1;
-          mbar_wait(full_bar(s), ph);
-          tc_fence_after();
-          const uint32_t sa = smem0 + s * P_STAGE_BYTES, sb = sa + A_BYTES;
+        const uint64_t step = (uint64_t)(s * (P_STAGE_BYTES >> 4));
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_bf16(acc, make_desc(sa + k * 32), make_desc(sb + k * 32), idesc, (kb | k) != 0);
+          for (int k = 0; k < BK / 16; ++k) umma_bf16(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
           umma_commit(empty_bar(s));
         }
-        umma_commit(tfull_bar(buf));
+        __syncwarp();
+        if (++s == P_STAGES) s = 0, ph ^= 1;
       }
+      if (elect_one()) umma_commit(tfull_bar(buf));
+      __syncwarp();
     }
   } else {
     // ---- epilogue warps 2-9: two warps per TMEM lane quarter, each draining half of the columns (r02: with four warps the
@@ -642,8 +683,9 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       const int col0 = g.dual ? 0 : g.seg[si].col0;
       const int tok_base = ttile * PBN;
       const int buf = j & 1;
-      mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1);
+      mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
       tc_fence_after();
+      const bool bad = *dead;
       const uint32_t acc = tmem_base + (uint32_t)buf * PBN + ((uint32_t)(qd * 32) << 16);
       const int n_tok_all = min(PBN, g.M - tok_base);
 #pragma unroll 1
@@ -654,6 +696,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       for (int c0 = cw; c0 < cw + P_HALF / 2; c0 += 16) {
         uint32_t r[16];
         tmem_ld16(acc + h0 + c0, r);
+        if (bad) mark_bad(r);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           const unsigned short hb = __bfloat16_as_ushort(f2bf(__uint_as_float(r[q])));
@@ -723,6 +766,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   }
   __syncthreads();
   if (warp == 1) {
+    dead_drain(dead);
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
