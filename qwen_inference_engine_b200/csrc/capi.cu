@@ -205,24 +205,14 @@ static int scratch(void** p, size_t* cap, size_t need) {
 
 int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st) {
   if (M < 1 || N < 64 || (N % 8) || K < 1) return fail(QIE_EINVAL, "matmul_fast: need M>=1, N>=64, N%%8==0");
-  static thread_local void* ws = nullptr;
-  static thread_local size_t ws_cap = 0;
-  static thread_local int* counters = nullptr;
-  if (!counters) {
-    CU(cudaMalloc(&counters, 8192 * sizeof(int)));
-    CU(cudaMemset(counters, 0, 8192 * sizeof(int)));
-  }
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  int rc = scratch(&ws, &ws_cap, std::max<size_t>((size_t)32 << 20, (size_t)M * K * 4 * 4));
-  if (rc) return rc;
-  TensorMap2D wmap, xmap;
+  TensorMap2D wmap;
   CU(make_tensor_map_2d(&wmap, (const bf16*)B, K, N, 128));
-  CU(make_tensor_map_2d(&xmap, (const bf16*)A, M, N, tc_token_tile(M)));
   TcGemm t{};
   t.w[0] = &wmap;
-  t.x = &xmap;
+  t.x = (const bf16*)A;
   t.rows[0] = K;
   t.nseg = 1;
   t.M = M;
@@ -230,11 +220,6 @@ int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, in
   t.epi = EPI_STORE;
   t.out = (bf16*)C;
   t.ld_out = K;
-  t.ws = (float*)ws;
-  t.ws_bytes = ws_cap;
-  t.max_splits = (int)std::max<size_t>(1, ws_cap / ((size_t)M * K * sizeof(float)));
-  t.counters = counters;
-  t.n_counters = 8192;
   t.w_static = 0;  // B may have been written by the caller's previous kernel
   CU(launch_gemm_tcgen05(t, sms, (cudaStream_t)st, nullptr));
   return QIE_OK;
@@ -403,7 +388,7 @@ static void engine_free(qie_engine* e) {
   if (!e->blob_owned) e->blob = nullptr;
   void* dev[] = {e->blob, e->cos_d, e->sin_d, e->kv.pool, e->block_table_d, e->ids_d, e->pos_d, e->slot_d,
                  e->sampled_d, e->rowstep_d, e->x, e->xn, e->q, e->k, e->v, e->att, e->h, e->logits, e->qkv,
-                 e->gemm_ws, e->attn_ws_o, e->attn_ws_ml, e->gemm_counters, e->mega_layers_d, e->mega_cand_d,
+                 e->attn_ws_o, e->attn_ws_ml, e->mega_layers_d, e->mega_cand_d,
                  e->mega_bar_d, e->mega_prof_d, e->mega_wmaps_d[0], e->mega_wmaps_d[1], e->tp_buf, e->tp_cand, e->tp_xbuf, e->x2,
                  e->mega_wmaps_tp_d[0], e->mega_wmaps_tp_d[1], e->mega_kvmap_d, e->mega_hmap_d, e->gemv_part_d};
   for (int r = 0; r < MEGA_MAX_TP; ++r)
@@ -635,10 +620,6 @@ static int engine_finish_setup(qie_engine* e) {
       CU(make_tensor_map_2d(&m.down, w.down, (int)H, (int)I, 128));
     }
     CU(make_tensor_map_2d(&e->lm_head_map, e->lm_head, c.vocab, (int)H, 128));
-    e->gemm_ws_bytes = std::max<size_t>((size_t)64 << 20, R * 2 * I * sizeof(float) * 2);
-    CU(cudaMalloc(&e->gemm_ws, e->gemm_ws_bytes));
-    CU(cudaMalloc(&e->gemm_counters, 8192 * sizeof(int)));
-    CU(cudaMemsetAsync(e->gemm_counters, 0, 8192 * sizeof(int), e->stream));
     CU(cudaMalloc(&e->attn_ws_o, (size_t)e->attn_max_splits * R * Dq * sizeof(float)));
     CU(cudaMalloc(&e->attn_ws_ml, (size_t)e->attn_max_splits * R * c.n_q * 2 * sizeof(float)));
   }

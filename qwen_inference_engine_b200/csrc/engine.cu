@@ -95,28 +95,18 @@ static cudaError_t gemm_rows(qie_engine* e, int kind, GemmArgs g, int n_rows, si
 // tcgen05 GEMM launch (fast numerics, rows > 8). x: [n, K] activations.
 static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K, int nseg, const TensorMap2D* const* w,
                            const int* rows, int epi, bf16* out, int ld_out) {
-  TensorMap2D xmap;
-  cudaError_t r = make_tensor_map_2d(&xmap, x, n, K, tc_token_tile(n));
-  if (r != cudaSuccess) return r;
   TcGemm t{};
-  int cols = 0;
   for (int i = 0; i < nseg; ++i) {
     t.w[i] = w[i];
     t.rows[i] = rows[i];
-    cols += rows[i];
   }
-  t.x = &xmap;
+  t.x = x;
   t.nseg = nseg;
   t.M = n;
   t.K = K;
   t.epi = epi;
   t.out = out;
   t.ld_out = ld_out;
-  t.ws = e->gemm_ws;
-  t.ws_bytes = e->gemm_ws_bytes;
-  t.max_splits = (int)std::max<size_t>(1, e->gemm_ws_bytes / ((size_t)n * cols * sizeof(float)));
-  t.counters = e->gemm_counters;
-  t.n_counters = 8192;
   t.w_static = 1;
   int nl = 0;
   qie_engine::ProfRec pr{kind, nullptr, nullptr};
@@ -125,7 +115,7 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
     cudaEventCreate(&pr.b);
     cudaEventRecord(pr.a, e->stream);
   }
-  r = launch_gemm_tcgen05(t, e->num_sms, e->stream, &nl);
+  cudaError_t r = launch_gemm_tcgen05(t, e->num_sms, e->stream, &nl);
   if (r != cudaSuccess) return r;
   if (e->prof_on) {
     cudaEventRecord(pr.b, e->stream);

@@ -115,9 +115,6 @@ struct RopeTable {
 struct TcProjector {
   bool use = false;
   bf16 *ab = nullptr, *cb = nullptr;
-  float* ws = nullptr;
-  size_t ws_bytes = 0;
-  int* counters = nullptr;
   void* maps = nullptr;  // std::map<const bf16*, TensorMap2D>*: weight descriptors by pointer
   cudaError_t alloc(size_t rows, size_t max_k, size_t max_n, cudaStream_t st);
   void release();

@@ -182,10 +182,6 @@ cudaError_t TcProjector::alloc(size_t rows, size_t max_k, size_t max_n, cudaStre
   cudaError_t r;
   if ((r = cudaMalloc(&ab, rows * max_k * sizeof(bf16))) != cudaSuccess) return r;
   if ((r = cudaMalloc(&cb, rows * max_n * sizeof(bf16))) != cudaSuccess) return r;
-  ws_bytes = (size_t)64 << 20;
-  if ((r = cudaMalloc(&ws, ws_bytes)) != cudaSuccess) return r;
-  if ((r = cudaMalloc(&counters, 8192 * sizeof(int))) != cudaSuccess) return r;
-  if ((r = cudaMemsetAsync(counters, 0, 8192 * sizeof(int), st)) != cudaSuccess) return r;
   maps = new std::map<const bf16*, TensorMap2D>();
   const char* v = getenv("QIE_NG_TC");
   use = !(v && v[0] == '0');
@@ -195,10 +191,10 @@ cudaError_t TcProjector::alloc(size_t rows, size_t max_k, size_t max_n, cudaStre
 void TcProjector::release() {
   delete static_cast<std::map<const bf16*, TensorMap2D>*>(maps);
   maps = nullptr;
-  void* dev[] = {ab, cb, ws, counters};
+  void* dev[] = {ab, cb};
   for (void* p : dev)
     if (p) cudaFree(p);
-  ab = cb = nullptr, ws = nullptr, counters = nullptr;
+  ab = cb = nullptr;
 }
 
 bool TcProjector::fits(int n, int K, int N, const bf16* W) const {
@@ -223,33 +219,20 @@ cudaError_t TcProjector::gemm_bf16(qie_engine* e, const bf16* A, const bf16* W, 
     if (r != cudaSuccess) return r;
     it = mp->emplace(W, wm).first;
   }
-  cudaError_t r;
-  TensorMap2D xmap;
-  // many rows but few output columns (N = 1024 at 2048 rows: 64 tiles of 128 x 256): half-size token tiles fill the SMs without
-  // the split over K and its reduction through the cluster
-  int tile = tc_token_tile(n);
-  static const bool small_on = [] { const char* v = getenv("QIE_TC_TILE128"); return !(v && v[0] == '0'); }();
-  if (small_on && tile == 256 && (long)((N + 127) / 128) * ((n + 255) / 256) * 2 <= e->num_sms) tile = 128;
-  if ((r = make_tensor_map_2d(&xmap, A, n, K, tile)) != cudaSuccess) return r;
   TcGemm t{};
   t.w[0] = &it->second;
   t.rows[0] = N;
-  t.x = &xmap;
+  t.x = A;
   t.nseg = 1;
   t.M = n;
   t.K = K;
   t.epi = EPI_STORE;
   t.out = C;
   t.ld_out = N;
-  t.ws = ws;
-  t.ws_bytes = ws_bytes;
-  t.max_splits = (int)std::max<size_t>(1, ws_bytes / ((size_t)n * N * sizeof(float)));
-  t.counters = counters;
-  t.n_counters = 8192;
-  t.token_tile = tile;
   t.w_static = 0;  // the operand comes from the kernel in front
   int nl = 0;
-  if ((r = launch_gemm_tcgen05(t, e->num_sms, st, &nl)) != cudaSuccess) return r;
+  cudaError_t r = launch_gemm_tcgen05(t, e->num_sms, st, &nl);
+  if (r != cudaSuccess) return r;
   e->launches += nl > 0 ? nl - 1 : 0;  // the caller counts one
   return cudaSuccess;
 }

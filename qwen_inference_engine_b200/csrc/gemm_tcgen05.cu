@@ -163,17 +163,18 @@ __device__ __forceinline__ float silu_fast_f(float x) {
 
 struct TcSeg {
   int rows;   // weight rows of this segment
-  int col0;   // first output column of this segment
   int tile0;  // first tile index
+  int ld;     // row stride of its output
+  bf16* out;  // its first output column
 };
 
 struct TcArgs {
   int M, K;
   int nseg, n_tiles, splits, kb_per_split, kb_total;
-  int epi, dual, w_static, ld_out;
+  int epi, dual, w_static;
+  int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
   TcSeg seg[3];
-  bf16* out;  // [M, ld_out]
 };
 
 template <int BN>
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
   constexpr int TC_STAGES = TcCfg<BN>::STAGES;
-  static_assert(TC_STAGES * STAGE_BYTES >= BN * BM * 4, "reduction tile must fit in the pipeline ring");
+  static_assert(TC_STAGES * STAGE_BYTES >= BN * (BM + 32) * 4, "reduction tile must fit in the pipeline ring");
   // 1024-byte alignment for SWIZZLE_128B (same offset in every CTA of a cluster: the dynamic
   // shared window starts at the same address in all CTAs of a kernel)
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -208,8 +209,8 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   // dual (gate/up): one tile = 64 gate rows + the same 64 up rows; segment 0 = gate map, 1 = up map
   const CUtensorMap* map_w = g.dual ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
   const int row0 = g.dual ? tile * (BM / 2) : (tile - g.seg[si].tile0) * BM;
-  const int seg_rows = g.seg[si].rows;
-  const int col0 = g.dual ? 0 : g.seg[si].col0;
+  const int seg_rows = g.seg[si].rows, ld = g.seg[si].ld;
+  bf16* const out = g.seg[si].out;
   const int kb0 = split * g.kb_per_split;
   const int kb1 = min(g.kb_total, kb0 + g.kb_per_split);
   const int nkb = max(0, kb1 - kb0);
@@ -348,7 +349,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
             const int tok = cc >> 4, part = cc & 15;
             const int w_row = row0 + part * 8;
             ok[u] = cc < total && w_row < seg_rows;
-            dst[u] = g.out + (size_t)(tok_base + tok) * g.ld_out + col0 + w_row;
+            dst[u] = out + (size_t)(tok_base + tok) * ld + w_row;
             if (ok[u]) {
               y[u] = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
               if (g.epi == EPI_RESIDUAL) x[u] = *reinterpret_cast<const uint4*>(dst[u]);
@@ -386,7 +387,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
             const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(silu_ref_f(hi2f(gs[e])))));
             o4[e] = pack2(f2bf(a0), f2bf(a1));
           }
-          *reinterpret_cast<uint4*>(g.out + (size_t)(tok_base + tok) * g.ld_out + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+          *reinterpret_cast<uint4*>(out + (size_t)(tok_base + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
         }
       }
     }
@@ -399,11 +400,16 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     return;
   }
   // red[token][lane] fp32 (conflict-free: a warp writes 32 consecutive floats per token);
-  // it reuses the pipeline ring, which is idle once tmem_full has fired.
+  // it reuses the pipeline ring, which is idle once tmem_full has fired.  CTA r of the cluster reduces rows
+  // [r * rows_per, (r + 1) * rows_per); a token's pitch is a tile's row plus rows_per values (at most 32), so that the 16-byte reads of
+  // eight neighbouring threads (the rows of a token, then the next token) fall on different banks.
   const uint32_t red = smem0;
   const bool epi_warp = warp >= 2;
   const int qd = warp & 3;  // TMEM lane quarter of this epilogue warp
   const bool via_smem = g.splits > 1 || g.dual;
+  const int tile_rows = g.dual ? BM / 2 : BM;  // output rows produced by this tile
+  const int rows_per = ((tile_rows + g.splits - 1) / g.splits + 3) & ~3;
+  const uint32_t pitch = (uint32_t)(BM + min(rows_per, 32)) * 4u;
   if (epi_warp) {
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
     if (nkb > 0) {
@@ -425,7 +431,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       if (via_smem) {
 #pragma unroll
         for (int j = 0; j < 16; ++j)
-          asm volatile("st.shared.b32 [%0], %1;" ::"r"(red + (uint32_t)((c0 + j) * BM + lane_row) * 4u), "r"(r[j]) : "memory");
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(red + (uint32_t)(c0 + j) * pitch + (uint32_t)lane_row * 4u), "r"(r[j]) : "memory");
       } else {
         // no split, single accumulator: epilogue straight from registers
         const int w_row = row0 + lane_row;
@@ -434,7 +440,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
           for (int j = 0; j < 16; ++j) {
             const int tok = tok_base + c0 + j;
             if (tok < g.M) {
-              bf16* dst = g.out + (size_t)tok * g.ld_out + col0 + w_row;
+              bf16* dst = out + (size_t)tok * ld + w_row;
               const float v = __uint_as_float(r[j]);
               if (g.epi == EPI_RESIDUAL)
                 *dst = f2bf(__fadd_rn(bf2f(*dst), bf2f(f2bf(v))));
@@ -454,14 +460,11 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     if (epi_warp) {
       const int t = threadIdx.x - 64;  // 0..127
       const int S = g.splits;
-      const int tile_rows = g.dual ? BM / 2 : BM;          // output rows produced by this tile
-      const int rows_per = (tile_rows + S - 1) / S;        // rows reduced by this CTA
       const int rbeg = split * rows_per;
-      const int rcnt = max(0, min(rows_per, tile_rows - rbeg));
+      const int groups = max(0, min(rows_per, tile_rows - rbeg)) / 4;  // (tile_rows and rows_per are multiples of 4)
       const int n_tok = min(BN, g.M - tok_base);
-      // Two outputs per thread and step, every load of the step requested before the first use: the S
-      // distributed-shared-memory reads of an output (and the residual's old value) are independent, but
-      // interleaved with their additions they went out one DSMEM round trip at a time.
+      // A thread reduces four rows of a token, one 16-byte read per split; every read of an item is requested before the first sum.
+      // With one 4-byte read per value and split the reduction of 64 tokens over 8 CTAs took 5.1 us, now 3.2.
       constexpr int MAXS = 8;  // portable cluster size
       uint32_t rb[MAXS];
 #pragma unroll
@@ -469,57 +472,61 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
         rb[sp] = red;
         if (S > 1 && sp < S) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb[sp]) : "r"(red), "r"(sp));
       }
-      const int total = rcnt * n_tok;
-      for (int o0 = t; o0 < total; o0 += 2 * 128) {
-        float v[2][MAXS], v2[2][MAXS];
-        bf16* dst[2];
-        bf16 old[2];
-        bool ok[2], in_rows[2];
+      auto ld4 = [&](int sp, uint32_t off, float (&v)[4]) {
+        if (S > 1)
+          asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(rb[sp] + off) : "memory");
+        else
+          asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(red + off) : "memory");
+      };
+      const bool vec = ld % 4 == 0 && seg_rows % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+      for (int o = t; o < groups * n_tok; o += 128) {
+        const int tok = o / groups, rr = rbeg + (o - tok * groups) * 4, w_row = row0 + rr;
+        if (w_row >= seg_rows) continue;
+        const uint32_t off = (uint32_t)tok * pitch + (uint32_t)rr * 4u;
+        float v[MAXS][4], v2[MAXS][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int o = o0 + u * 128;
-          ok[u] = o < total;
-          const int oo = ok[u] ? o : 0;
-          const int tok = oo / rcnt, rr = rbeg + oo % rcnt;
-          const uint32_t off1 = (uint32_t)(tok * BM + rr) * 4u;
-          const uint32_t off2 = off1 + (uint32_t)(BM / 2) * 4u;  // dual: the up half of the tile
-          const int w_row = row0 + rr;
-          in_rows[u] = ok[u] && w_row < seg_rows;
-          dst[u] = g.out + (size_t)(tok_base + tok) * g.ld_out + col0 + w_row;
-          if (in_rows[u] && g.epi == EPI_RESIDUAL) old[u] = *dst[u];
+        for (int sp = 0; sp < MAXS; ++sp)
+          if (sp < S) {
+            ld4(sp, off, v[sp]);
+            if (g.dual) ld4(sp, off + (uint32_t)(BM / 2) * 4u, v2[sp]);  // the up half of the tile
+          }
+        bf16* dst = out + (size_t)(tok_base + tok) * ld + w_row;
+        float old[4] = {0.f, 0.f, 0.f, 0.f};
+        if (g.epi == EPI_RESIDUAL) {
+          if (vec) {
+            const uint2 x = *reinterpret_cast<const uint2*>(dst);
+            old[0] = lo2f(x.x), old[1] = hi2f(x.x), old[2] = lo2f(x.y), old[3] = hi2f(x.y);
+          } else {
 #pragma unroll
-          for (int sp = 0; sp < MAXS; ++sp) {
-            v[u][sp] = 0.f;
-            v2[u][sp] = 0.f;
-            if (ok[u] && sp < S) {
-              if (S > 1) {
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[u][sp]) : "r"(rb[sp] + off1) : "memory");
-                if (g.dual) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v2[u][sp]) : "r"(rb[sp] + off2) : "memory");
-              } else {
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[u][sp]) : "r"(red + off1) : "memory");
-                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v2[u][sp]) : "r"(red + off2) : "memory");
-              }
-            }
+            for (int e = 0; e < 4; ++e)
+              if (w_row + e < seg_rows) old[e] = bf2f(dst[e]);
           }
         }
+        bf16 y[4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (!in_rows[u]) continue;
+        for (int e = 0; e < 4; ++e) {
           float acc = 0.f, acc2 = 0.f;
 #pragma unroll
           for (int sp = 0; sp < MAXS; ++sp)
-            if (sp < S) {  // rank order, as before
-              acc += v[u][sp];
-              acc2 += v2[u][sp];
+            if (sp < S) {  // rank order
+              acc += v[sp][e];
+              if (g.dual) acc2 += v2[sp][e];
             }
           if (g.epi == EPI_STORE) {
-            *dst[u] = f2bf(acc);
+            y[e] = f2bf(acc);
           } else if (g.epi == EPI_RESIDUAL) {
-            *dst[u] = f2bf(__fadd_rn(bf2f(old[u]), bf2f(f2bf(acc))));
+            y[e] = f2bf(__fadd_rn(old[e], bf2f(f2bf(acc))));
           } else {
             const float gt = bf2f(f2bf(acc)), up = bf2f(f2bf(acc2));
-            *dst[u] = f2bf(__fmul_rn(up, bf2f(f2bf(silu_ref_f(gt)))));
+            y[e] = f2bf(__fmul_rn(up, bf2f(f2bf(silu_ref_f(gt)))));
           }
+        }
+        if (vec) {
+          *reinterpret_cast<uint2*>(dst) = make_uint2(pack2(y[0], y[1]), pack2(y[2], y[3]));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (w_row + e < seg_rows) dst[e] = y[e];
         }
       }
     }
@@ -534,23 +541,18 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   }
 }
 
-// ------------------------------------------------------------------ persistent variant (prefill)
-// Same tiles, same math, for launches without split-K and >= 129 tokens (BN = 256): ONE CTA per SM walks the
-// output tiles (weight tile fastest, so neighbouring CTAs share a token tile in L2), the accumulator is double
-// buffered in TMEM (2 x 256 columns), and the epilogue of tile j (TMEM -> bf16 staging tile in shared memory ->
-// 16-byte global accesses) runs on warps 2-5 while warps 0/1 already stream and multiply tile j+1.  ncu on the
-// one-tile-per-CTA kernel showed the tensor pipe 32-47 % active at K = 1536: per tile ~2.5 us of prologue and
-// ~8 us of epilogue sat next to a ~7-9 us mainloop (profiles/r01c_ncu_full_prefill_kernels.csv).
-static constexpr int PBN = 256;
-// r02: four operand stages instead of three (ncu: tensor pipe 37-61 % active with L2 at 15-32 % of its peak -- the mainloop
-// waited for TMA, 3 x 512 MMA cycles of lookahead do not cover the load latency); the room comes from a half-size
-// staging tile: the epilogue drains and stores the accumulator in two halves of 128 tokens.
-// (measured dead end: a 128-token tile variant -- 6 stages of 32 KiB -- for the launches whose 256-token tiles quantise badly
-// over the SMs, e.g. o_proj / down_proj of the 1.5B shape, 192 tiles = 65 % of two waves: 15.5 -> 16.3 ms, 7B 62.8 -> 70.9 ms;
-// the half-size tiles lose more per flop than the fuller waves give back.  Only the 0.5B shape gained, 8.5 -> 8.1 ms.)
-static constexpr int P_STAGES = 4;
-static constexpr int P_STAGE_BYTES = BM * BK * 2 + PBN * BK * 2;  // 48 KiB
-static constexpr int P_HALF = PBN / 2;
+// ------------------------------------------------------------------ persistent variant
+// Same tiles, same math, for launches without split-K: ONE CTA per SM walks the output tiles (weight tile fastest, so neighbouring
+// CTAs share a token tile in L2), the accumulator is double buffered in TMEM (2 x 256 columns), and the epilogue of tile j (TMEM ->
+// bf16 staging tile in shared memory -> 16-byte global accesses, 128 tokens at a time) runs on warps 2-9 while warps 0/1 already
+// stream and multiply tile j+1.  ncu on the one-tile-per-CTA kernel showed the tensor pipe 32-47 % active at K = 1536: per tile
+// ~2.5 us of prologue and ~8 us of epilogue sat next to a ~7-9 us mainloop (profiles/r01c_ncu_full_prefill_kernels.csv).
+// A tile has g.bn tokens, any multiple of 16 (pick_tile): with 256 always, 4096 tokens x 1536 outputs were 192 tiles on 148 SMs, two
+// waves filled to 65 %.  The ring takes the stages that fit: 4 of 48 KiB at 256 tokens, 10 of 18 KiB at 16.
+static constexpr int PBN = 256;                   // TMEM columns of an accumulator
+static constexpr int P_HALF = 128;                // tokens of the staging tile
+static constexpr int P_RING = 4 * (BM * BK * 2 + PBN * BK * 2);     // 192 KiB
+static constexpr int P_MAX_STAGES = 10;
 static constexpr int P_EPI = 256;                 // epilogue threads (8 warps)
 static constexpr int P_THREADS = 64 + P_EPI;      // + TMA warp + MMA warp
 static constexpr int P_STAGING = P_HALF * BM * 2;                   // bf16 [128 tokens][128 rows] = 32 KiB
@@ -568,13 +570,14 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   constexpr int A_BYTES = BM * BK * 2;
   constexpr uint32_t TMEM_COLS = 512;  // two accumulators
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t stg = smem0 + P_STAGES * P_STAGE_BYTES;
+  const int bn = g.bn, stages = g.stages, stage_bytes = A_BYTES + bn * BK * 2;
+  const uint32_t stg = smem0 + P_RING;
   const uint32_t bars = stg + P_STAGING;  // full[S], empty[S], tmem_full[2], tmem_empty[2], slot
   auto full_bar = [&](int s) { return bars + 8u * s; };
-  auto empty_bar = [&](int s) { return bars + 8u * (P_STAGES + s); };
-  auto tfull_bar = [&](int b) { return bars + 8u * (2 * P_STAGES + b); };
-  auto tempty_bar = [&](int b) { return bars + 8u * (2 * P_STAGES + 2 + b); };
-  const uint32_t slot = bars + 8u * (2 * P_STAGES + 4);
+  auto empty_bar = [&](int s) { return bars + 8u * (P_MAX_STAGES + s); };
+  auto tfull_bar = [&](int b) { return bars + 8u * (2 * P_MAX_STAGES + b); };
+  auto tempty_bar = [&](int b) { return bars + 8u * (2 * P_MAX_STAGES + 2 + b); };
+  const uint32_t slot = bars + 8u * (2 * P_MAX_STAGES + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = g.n_tiles * token_tiles;
@@ -585,7 +588,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
-    for (int s = 0; s < P_STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
     }
@@ -616,29 +619,45 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       int s = 0;
       uint32_t ph = 1;
       bool go = true;
-      pdl_wait();  // activations come from the previous kernel (these launches run for 30-300 us: no early weight prefetch)
+      auto load_w = [&](int kb, int si, int row0) {
+        const uint32_t sa = smem0 + s * stage_bytes;
+        if (g.dual) {
+          tma_load_2d(sa, &map_w0, full_bar(s), kb * BK, row0);
+          tma_load_2d(sa + A_BYTES / 2, &map_w1, full_bar(s), kb * BK, row0);
+        } else {
+          tma_load_2d(sa, si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2), full_bar(s), kb * BK, row0);
+        }
+      };
+      int tile, ttile, si, row0;
+      // the first stages' weights in front of the wait for the previous kernel, which wrote the activations
+      int pre = 0;
+      if (g.w_static && blockIdx.x < total) {
+        tile_geom(blockIdx.x, tile, ttile, si, row0);
+        for (pre = min(nkb, stages); s < pre; ++s) {
+          mbar_expect_tx(full_bar(s), stage_bytes);
+          load_w(s, si, row0);
+        }
+        s = 0;
+      }
+      pdl_wait();
       for (int t = blockIdx.x; t < total && go; t += gridDim.x) {
-        int tile, ttile, si, row0;
         tile_geom(t, tile, ttile, si, row0);
-        const CUtensorMap* map_w = g.dual ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!(go = mbar_wait(empty_bar(s), ph, dead))) break;
-          mbar_expect_tx(full_bar(s), P_STAGE_BYTES);
-          const uint32_t sa = smem0 + s * P_STAGE_BYTES;
-          if (g.dual) {
-            tma_load_2d(sa, &map_w0, full_bar(s), kb * BK, row0);
-            tma_load_2d(sa + A_BYTES / 2, &map_w1, full_bar(s), kb * BK, row0);
+          if (pre > 0) {  // (the first stages: nothing to wait for)
+            --pre;
           } else {
-            tma_load_2d(sa, map_w, full_bar(s), kb * BK, row0);
+            if (!(go = mbar_wait(empty_bar(s), ph, dead))) break;
+            mbar_expect_tx(full_bar(s), stage_bytes);
+            load_w(kb, si, row0);
           }
-          tma_load_2d(sa + A_BYTES, &map_x, full_bar(s), kb * BK, ttile * PBN);
-          if (++s == P_STAGES) s = 0, ph ^= 1;
+          tma_load_2d(smem0 + s * stage_bytes + A_BYTES, &map_x, full_bar(s), kb * BK, ttile * bn);
+          if (++s == stages) s = 0, ph ^= 1;
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    constexpr uint32_t idesc = make_idesc(BM, PBN);
+    const uint32_t idesc = make_idesc(BM, bn);
     const uint64_t ad0 = make_desc(smem0), bd0 = make_desc(smem0 + A_BYTES);
     int s = 0, j = 0;
     uint32_t ph = 0;
@@ -650,14 +669,14 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       for (int kb = 0; kb < nkb; ++kb) {
         mbar_wait(full_bar(s), ph, dead);
         tc_fence_after();
-        const uint64_t step = (uint64_t)(s * (P_STAGE_BYTES >> 4));
+        const uint64_t step = (uint64_t)(s * (stage_bytes >> 4));
         if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) umma_bf16(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
           umma_commit(empty_bar(s));
         }
         __syncwarp();
-        if (++s == P_STAGES) s = 0, ph ^= 1;
+        if (++s == stages) s = 0, ph ^= 1;
       }
       if (elect_one()) umma_commit(tfull_bar(buf));
       __syncwarp();
@@ -679,21 +698,20 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
       int tile, ttile, si, row0;
       tile_geom(t, tile, ttile, si, row0);
-      const int seg_rows = g.seg[si].rows;
-      const int col0 = g.dual ? 0 : g.seg[si].col0;
-      const int tok_base = ttile * PBN;
+      const int seg_rows = g.seg[si].rows, ld = g.seg[si].ld;
+      bf16* const out = g.seg[si].out;
+      const int tok_base = ttile * bn;
       const int buf = j & 1;
       mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
       tc_fence_after();
       const bool bad = *dead;
       const uint32_t acc = tmem_base + (uint32_t)buf * PBN + ((uint32_t)(qd * 32) << 16);
-      const int n_tok_all = min(PBN, g.M - tok_base);
+      const int n_tok_all = min(bn, g.M - tok_base);
 #pragma unroll 1
-      for (int hf = 0; hf < 2; ++hf) {  // tokens [128 hf, 128 hf + 128) of the tile through the 32 KiB staging tile
-      const int h0 = hf * P_HALF;
-      const int cw = ((warp - 2) >> 2) * (P_HALF / 2);  // this warp's columns of the half: [cw, cw + 64)
+      for (int h0 = 0; h0 < bn; h0 += P_HALF) {  // tokens [h0, h0 + 128) of the tile through the 32 KiB staging tile
+      const int width = min(P_HALF, bn - h0);
 #pragma unroll 4
-      for (int c0 = cw; c0 < cw + P_HALF / 2; c0 += 16) {
+      for (int c0 = ((warp - 2) >> 2) * 16; c0 < width; c0 += 32) {  // every other 16 columns: the quarter's second warp has the rest
         uint32_t r[16];
         tmem_ld16(acc + h0 + c0, r);
         if (bad) mark_bad(r);
@@ -705,7 +723,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       }
       tc_fence_before();
       asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (hf == 1 && tq == 0) mbar_arrive_local(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
+      if (h0 + P_HALF >= bn && tq == 0) mbar_arrive_local(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
       const int n_tok = max(0, min(P_HALF, n_tok_all - h0));
       if (!g.dual) {
         const int totalc = n_tok * (BM / 8);
@@ -719,7 +737,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
             const int tok = cc >> 4, part = cc & 15;
             const int w_row = row0 + part * 8;
             ok[u] = cc < totalc && w_row < seg_rows;
-            dst[u] = g.out + (size_t)(tok_base + h0 + tok) * g.ld_out + col0 + w_row;
+            dst[u] = out + (size_t)(tok_base + h0 + tok) * ld + w_row;
             if (ok[u]) {
               if (g.epi == EPI_RESIDUAL) x[u] = *reinterpret_cast<const uint4*>(dst[u]);
               y[u] = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
@@ -756,12 +774,11 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
             const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(silu_fast_f(hi2f(gs[e])))));
             o4[e] = pack2(f2bf(a0), f2bf(a1));
           }
-          *reinterpret_cast<uint4*>(g.out + (size_t)(tok_base + h0 + tok) * g.ld_out + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+          *reinterpret_cast<uint4*>(out + (size_t)(tok_base + h0 + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
         }
       }
-      if (hf == 0) asm volatile("bar.sync 2, 256;" ::: "memory");  // the staging tile is rewritten by the second half
+      asm volatile("bar.sync 2, 256;" ::: "memory");  // the staging tile is rewritten by the next tokens
       }
-      asm volatile("bar.sync 2, 256;" ::: "memory");  // the staging tile is rewritten by the next tile
     }
   }
   __syncthreads();
@@ -854,7 +871,7 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
 }
 
 template <int BN>
-static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, int token_tiles, cudaStream_t st) {
+static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int STAGE_BYTES = BM * BK * 2 + BN * BK * 2;
   constexpr size_t smem = (size_t)TcCfg<BN>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
@@ -889,10 +906,50 @@ static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, int token_tiles, 
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN>, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(t.x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN>, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g);
 }
 
-int tc_token_tile(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256; }
+struct TcTile {
+  int bn, splits;
+  bool persist;
+};
+// Tokens of a tile and splits over K.  Measured on B200 in graphs of the same launch, weights in L2 (us):
+//  * One wave of CTAs: the smallest of 16 ... 128 tokens whose tiles all fit on the SMs.  A k-block takes the same time at any width up
+//    to 128, narrower tiles fill and drain faster: 896 x 896, 1000 tokens: 64 7.1, 128 7.8, 256 9.5 (a split over 5 CTAs: 50.8).
+//  * More tiles than that: the persistent kernel.  256 tokens, unless a width with fuller waves takes less than 0.9 of waves x width
+//    (1536 outputs at 4096 rows: 107 -> 86 with 176; a few per cent less on paper were none: 8960 outputs 82.7 with 256, 85.5 with
+//    224).  Below 160 tokens the loop, not the tensor core, sets a tile's time, so of those the narrowest wins, whose ring holds most
+//    k-blocks: 151936 x 896 for one row 79 -> 47.
+//  * Few tiles and a long K: a cluster of 2, 4 or 8 CTAs splits K (never in the reference's order).  Its reduction costs about
+//    1.1 us + (0.1, 0.055, 0.045) us x tokens, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
+//    clusters have to run at once (`most` clusters of a size fit; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
+//    against 27 with 4).
+static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool may_split) {
+  auto ctas = [&](int bn) { return (long)tiles * ((M + bn - 1) / bn); };
+  TcTile best{16, 1, false};
+  while (best.bn < 256 && ctas(best.bn) > num_sms) best.bn *= 2;
+  if (best.bn < 256) {
+    if (!may_split) return best;
+    float cost = 0.19f * nkb;
+    static const int most[3] = {64, 28, 14};
+    static const float per_token[3] = {0.1f, 0.055f, 0.045f};
+    for (int i = 0; i < 3; ++i)
+      for (int bn = 16; bn <= 128; bn *= 2) {
+        const int s = 2 << i;
+        if (nkb < 2 * s || ctas(bn) > most[i] || (bn > 16 && bn / 2 >= M)) continue;
+        const float c = 0.19f * ((nkb + s - 1) / s) + 1.1f + per_token[i] * bn;
+        if (c < cost) cost = c, best.bn = bn, best.splits = s;
+      }
+    return best;
+  }
+  if (!vec) return best;  // outputs that 16-byte stores cannot reach: one tile per CTA
+  best.persist = true;
+  auto waves = [&](int bn) { return (ctas(bn) + num_sms - 1) / num_sms * std::max(bn, 160); };
+  long cost = waves(256) * 9 / 10;
+  for (int bn = 16; bn < 256; bn += 16)
+    if (waves(bn) < cost) cost = waves(bn), best.bn = bn;
+  return best;
+}
 
 cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, int* launches) {
   if (t.M < 1 || t.K < BK || (t.K % 8) || t.nseg < 1 || t.nseg > 3) return cudaErrorInvalidValue;
@@ -903,66 +960,49 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.epi = t.epi;
   g.dual = t.epi == EPI_SILU_MUL;
   g.w_static = t.w_static;
-  g.ld_out = t.ld_out;
-  g.out = t.out;
   int tiles = 0, cols = 0;
   if (g.dual) {
     // segments = (gate, up) with equal row counts; the weight maps must have 64-row boxes
     if (t.nseg != 2 || t.rows[0] != t.rows[1]) return cudaErrorInvalidValue;
-    g.seg[0].rows = t.rows[0];
-    g.seg[0].col0 = 0;
-    g.seg[0].tile0 = 0;
+    g.seg[0] = TcSeg{t.rows[0], 0, t.ld_out, t.out};
     g.nseg = 1;
     tiles = (t.rows[0] + BM / 2 - 1) / (BM / 2);
-    cols = t.rows[0];
   } else {
     for (int i = 0; i < t.nseg; ++i) {
-      g.seg[i].rows = t.rows[i];
-      g.seg[i].col0 = cols;
-      g.seg[i].tile0 = tiles;
+      g.seg[i] = TcSeg{t.rows[i], tiles, t.ld_out, t.out + cols};
       tiles += (t.rows[i] + BM - 1) / BM;
       cols += t.rows[i];
     }
   }
-  (void)cols;
   g.n_tiles = tiles;
   g.kb_total = (t.K + BK - 1) / BK;
-  const int BN = t.token_tile ? t.token_tile : tc_token_tile(t.M);
-  if (BN != 16 && BN != 32 && BN != 64 && BN != 128 && BN != 256) return cudaErrorInvalidValue;
-  const int token_tiles = (t.M + BN - 1) / BN;
-  // split-K (= cluster size along grid.y) so that roughly one CTA lands on every SM; every
-  // slice keeps >= 2 k-blocks; cluster size <= 8 (the portable maximum)
-  int splits = 1;
-  const int ctas = tiles * token_tiles;
-  if (ctas * 2 <= num_sms) {
-    splits = num_sms / ctas;
-    splits = std::min(splits, std::max(1, g.kb_total / 2));
-    splits = std::min(splits, std::min(8, std::max(1, t.max_splits)));  // portable cluster size
-  }
-  g.kb_per_split = (g.kb_total + splits - 1) / splits;
-  splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
-  g.splits = splits;
-  {
-    bool vec = (t.ld_out % 8 == 0) && ((reinterpret_cast<uintptr_t>(t.out) & 15) == 0);
-    for (int i = 0; i < t.nseg; ++i) vec = vec && (t.rows[i] % 8 == 0);
-    g.staged = splits == 1 && vec;
-  }
-  cudaError_t e;
-  static const bool persist_on = [] { const char* v = getenv("QIE_TC_PERSIST"); return !(v && v[0] == '0'); }();
-  if (persist_on && g.staged && BN == PBN && tiles * token_tiles > num_sms / 2) {
-    // prefill-sized launches: persistent tile loop, epilogue overlapped with the next tile's mainloop
-    constexpr size_t smem = (size_t)P_STAGES * P_STAGE_BYTES + P_STAGING + 1024 /*align*/ + 256 /*barriers*/;
+  bool vec = true;  // the epilogue through a staging tile stores 16 bytes
+  for (int i = 0; i < g.nseg; ++i)
+    vec = vec && g.seg[i].rows % 8 == 0 && g.seg[i].ld % 8 == 0 && (reinterpret_cast<uintptr_t>(g.seg[i].out) & 15) == 0;
+  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, vec, true);
+  const int token_tiles = (t.M + tl.bn - 1) / tl.bn;
+  g.kb_per_split = (g.kb_total + tl.splits - 1) / tl.splits;
+  g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
+  g.staged = g.splits == 1 && vec;
+  TensorMap2D x;
+  cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
+  if (e != cudaSuccess) return e;
+  if (launches) *launches = 1;
+  if (tl.persist) {
+    constexpr size_t smem = (size_t)P_RING + P_STAGING + 1024 /*align*/ + 256 /*barriers*/;
     static PerDeviceOnce set;
     if (set.need()) {
       e = cudaFuncSetAttribute(gemm_tcgen05_persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       set.done();
     }
+    g.bn = tl.bn;
+    g.stages = std::min(P_MAX_STAGES, P_RING / (BM * BK * 2 + tl.bn * BK * 2));
     const CUtensorMap* w0 = reinterpret_cast<const CUtensorMap*>(t.w[0]);
     const CUtensorMap* w1 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 1 ? 1 : 0]);
     const CUtensorMap* w2 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 2 ? 2 : 0]);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(std::min(num_sms, tiles * token_tiles));
+    cfg.gridDim = dim3((unsigned)std::min<long>(num_sms, (long)tiles * token_tiles));
     cfg.blockDim = dim3(P_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -971,18 +1011,15 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = g_use_pdl ? 1 : 0;
-    if (launches) *launches = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(t.x), g, token_tiles);
+    return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
   }
-  switch (BN) {
-    case 16: e = launch_bn<16>(t, g, token_tiles, st); break;
-    case 32: e = launch_bn<32>(t, g, token_tiles, st); break;
-    case 64: e = launch_bn<64>(t, g, token_tiles, st); break;
-    case 128: e = launch_bn<128>(t, g, token_tiles, st); break;
-    default: e = launch_bn<256>(t, g, token_tiles, st); break;
+  switch (tl.bn) {
+    case 16: return launch_bn<16>(t, g, x, token_tiles, st);
+    case 32: return launch_bn<32>(t, g, x, token_tiles, st);
+    case 64: return launch_bn<64>(t, g, x, token_tiles, st);
+    case 128: return launch_bn<128>(t, g, x, token_tiles, st);
+    default: return launch_bn<256>(t, g, x, token_tiles, st);
   }
-  if (launches) *launches = 1;
-  return e;
 }
 
 }  // namespace qie

@@ -143,21 +143,14 @@ cudaError_t make_tensor_map_kv(TensorMap2D* out, const bf16* pool, unsigned long
 // cache rows of one layer as a 3-D tensor {row elements, positions of a page, pages} (page stride page_elems): box = 64 elements x box_rows
 // positions of one page, 128-byte swizzle
 cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_elems, int page_size, int n_pages, size_t page_elems, int box_rows);
-int tc_token_tile(int M);
 struct TcGemm {
-  const TensorMap2D* w[3];  // weight maps, box rows = 128
-  const TensorMap2D* x;     // activation map [M, K], box rows = tc_token_tile(M)
+  const TensorMap2D* w[3];  // weight maps, box rows = 128 (EPI_SILU_MUL: 64)
+  const bf16* x;            // activations [M, K]
   int rows[3];
   int nseg, M, K, epi;
   bf16* out;     // [M, ld_out]; EPI_SILU_MUL: segments are (gate, up), out has rows[0] columns
   int ld_out;
-  float* ws;
-  size_t ws_bytes;
-  int max_splits;
-  int* counters;   // zero-initialised ints for the fused split-K reduction (nullptr: separate finalize kernel)
-  int n_counters;
-  int w_static;    // weights are not produced by a preceding kernel: prefetch them before the PDL wait
-  int token_tile;  // 0: tc_token_tile(M); else the box rows the caller built the activation map with (16, 32, 64, 128 or 256)
+  int w_static;  // weights are not produced by a preceding kernel: prefetch them before the PDL wait
 };
 cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, int* launches);
 
