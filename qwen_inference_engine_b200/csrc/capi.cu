@@ -51,17 +51,15 @@ int qie_matmul(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, 
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  for (int r0 = 0; r0 < M; r0 += 64) {
-    GemmArgs g{};
-    g.A = (const bf16*)A + (size_t)r0 * N;
-    g.lda = N;
-    g.M = std::min(64, M - r0);
-    g.K = N;
-    g.nseg = 1;
-    g.epi = EPI_STORE;
-    g.seg[0] = GemmSeg{(const bf16*)B, nullptr, (bf16*)C + (size_t)r0 * K, K, K};
-    CU(launch_gemm_ref_order(g, sms, (cudaStream_t)st));
-  }
+  GemmArgs g{};
+  g.A = (const bf16*)A;
+  g.lda = N;
+  g.M = M;
+  g.K = N;
+  g.nseg = 1;
+  g.epi = EPI_STORE;
+  g.seg[0] = GemmSeg{(const bf16*)B, nullptr, (bf16*)C, K, K};
+  CU(launch_gemm_ref_rows(g, sms, (cudaStream_t)st, 0, nullptr));  // B may have been written by the caller's previous kernel
   return QIE_OK;
 }
 int qie_qknorm(qie_bf16* x, const qie_bf16* w, int head_dim, int n_tok, int row_dim, int n_heads, qie_stream st) {

@@ -78,17 +78,12 @@ static void capture_copy(qie_engine* e, const char* tag, int layer, const bf16* 
   cudaMemcpyAsync(b.d, src, elems * sizeof(bf16), cudaMemcpyDeviceToDevice, e->stream);
 }
 
-// C[rows, *] = A * W^T in chunks of <= 64 rows (the reference-order kernel keeps one
-// fp32 fragment per 16 rows; larger M just re-streams W per chunk).
-static cudaError_t gemm_rows(qie_engine* e, int kind, GemmArgs g, int n_rows, size_t a_stride) {
-  for (int r0 = 0; r0 < n_rows; r0 += 64) {
-    GemmArgs c = g;
-    c.A = g.A + (size_t)r0 * a_stride;
-    c.M = std::min(64, n_rows - r0);
-    for (int s = 0; s < g.nseg; ++s)  // EPI_STORE_F32: `out` is a float*, twice the bf16 stride
-      c.seg[s].out = g.seg[s].out + (size_t)r0 * g.seg[s].ld_out * (g.epi == EPI_STORE_F32 ? 2 : 1);
-    QIE_TRY(kind, launch_gemm_ref_order(c, e->num_sms, e->stream));
-  }
+// C[rows, *] = A * W^T in the reference's order
+static cudaError_t gemm_rows(qie_engine* e, int kind, GemmArgs g, int n_rows) {
+  g.M = n_rows;
+  int nl = 0;
+  QIE_TRY(kind, launch_gemm_ref_rows(g, e->num_sms, e->stream, 1, &nl));
+  e->launches += nl - 1;  // QIE_TRY counts one
   return cudaSuccess;
 }
 
@@ -166,7 +161,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       g.seg[0] = GemmSeg{w.q, nullptr, e->q, Dq, Dq};
       g.seg[1] = GemmSeg{w.k, nullptr, e->k, Dkv, Dkv};
       g.seg[2] = GemmSeg{w.v, nullptr, e->v, Dkv, Dkv};
-      cudaError_t r = gemm_rows(e, KK_GEMM_QKV, g, n, H);
+      cudaError_t r = gemm_rows(e, KK_GEMM_QKV, g, n);
       if (r != cudaSuccess) return r;
     }
     {
@@ -277,7 +272,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       g.nseg = 1;
       g.epi = EPI_RESIDUAL;
       g.seg[0] = GemmSeg{w.o, nullptr, e->x, H, H};
-      cudaError_t r = gemm_rows(e, KK_GEMM_O, g, n, Dq);
+      cudaError_t r = gemm_rows(e, KK_GEMM_O, g, n);
       if (r != cudaSuccess) return r;
     }
     capture_copy(e, "x_attn", l, e->x, (size_t)n * H);
@@ -295,7 +290,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       g.nseg = 1;
       g.epi = EPI_SILU_MUL;
       g.seg[0] = GemmSeg{w.gate, w.up, e->h, I, I};
-      cudaError_t r = gemm_rows(e, KK_GEMM_GATEUP, g, n, H);
+      cudaError_t r = gemm_rows(e, KK_GEMM_GATEUP, g, n);
       if (r != cudaSuccess) return r;
     }
     capture_copy(e, "mlp_h", l, e->h, (size_t)n * I);
@@ -312,7 +307,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       g.nseg = 1;
       g.epi = EPI_RESIDUAL;
       g.seg[0] = GemmSeg{w.down, nullptr, e->x, H, H};
-      cudaError_t r = gemm_rows(e, KK_GEMM_DOWN, g, n, I);
+      cudaError_t r = gemm_rows(e, KK_GEMM_DOWN, g, n);
       if (r != cudaSuccess) return r;
     }
     capture_copy(e, "x_out", l, e->x, (size_t)n * H);
@@ -333,7 +328,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     g.nseg = 1;
     g.epi = EPI_STORE;
     g.seg[0] = GemmSeg{e->lm_head, nullptr, e->logits, c.vocab, c.vocab};
-    cudaError_t r = gemm_rows(e, KK_LM_HEAD, g, n_out, H);
+    cudaError_t r = gemm_rows(e, KK_LM_HEAD, g, n_out);
     if (r != cudaSuccess) return r;
   }
   capture_copy(e, "logits", -1, e->logits, (size_t)n_out * c.vocab);
@@ -391,7 +386,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       g.seg[0] = GemmSeg{w.q + (size_t)pl.q_row0 * H, nullptr, e->q, Dq_l, Dq_l, 0};
       g.seg[1] = GemmSeg{w.k + (size_t)pl.kv_row0 * H, nullptr, e->k, Dkv_l, Dkv_l, 0};
       g.seg[2] = GemmSeg{w.v + (size_t)pl.kv_row0 * H, nullptr, e->v, Dkv_l, Dkv_l, 0};
-      cudaError_t r = gemm_rows(e, KK_GEMM_QKV, g, n, H);
+      cudaError_t r = gemm_rows(e, KK_GEMM_QKV, g, n);
       if (r != cudaSuccess) return r;
     }
     {
@@ -439,7 +434,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       g.nseg = 1;
       g.epi = EPI_STORE_F32;
       g.seg[0] = GemmSeg{w.o + pl.q_row0, nullptr, reinterpret_cast<bf16*>(e->tp_buf), H, H, Dq};
-      cudaError_t r = gemm_rows(e, KK_GEMM_O, g, n, Dq_l);
+      cudaError_t r = gemm_rows(e, KK_GEMM_O, g, n);
       if (r != cudaSuccess) return r;
       r = tp_allreduce_f32(&e->tp, e->tp_buf, (size_t)n * H, st);
       if (r != cudaSuccess) return r;
@@ -454,7 +449,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       g.nseg = 1;
       g.epi = EPI_SILU_MUL;
       g.seg[0] = GemmSeg{w.gate + (size_t)pl.inter0 * H, w.up + (size_t)pl.inter0 * H, e->h, I_l, I_l, 0};
-      cudaError_t r = gemm_rows(e, KK_GEMM_GATEUP, g, n, H);
+      cudaError_t r = gemm_rows(e, KK_GEMM_GATEUP, g, n);
       if (r != cudaSuccess) return r;
     }
     {  // down_proj over the local intermediate columns -> all-reduce -> residual
@@ -465,7 +460,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       g.nseg = 1;
       g.epi = EPI_STORE_F32;
       g.seg[0] = GemmSeg{w.down + pl.inter0, nullptr, reinterpret_cast<bf16*>(e->tp_buf), H, H, I};
-      cudaError_t r = gemm_rows(e, KK_GEMM_DOWN, g, n, I_l);
+      cudaError_t r = gemm_rows(e, KK_GEMM_DOWN, g, n);
       if (r != cudaSuccess) return r;
       r = tp_allreduce_f32(&e->tp, e->tp_buf, (size_t)n * H, st);
       if (r != cudaSuccess) return r;
@@ -482,7 +477,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
     g.nseg = 1;
     g.epi = EPI_STORE;
     g.seg[0] = GemmSeg{e->lm_head + (size_t)pl.vocab0 * H, nullptr, e->logits, V_l, V_l, 0};
-    cudaError_t r = gemm_rows(e, KK_LM_HEAD, g, n_out, H);
+    cudaError_t r = gemm_rows(e, KK_LM_HEAD, g, n_out);
     if (r != cudaSuccess) return r;
   }
   // local arg-max (reference tie-break; vocab/tp is a multiple of 256, so the low byte of the index is

@@ -172,6 +172,7 @@ struct TcArgs {
   int M, K;
   int nseg, n_tiles, splits, kb_per_split, kb_total;
   int epi, dual, w_static;
+  int exact;       // reference-order numerics: SiLU as the reference computes it (expf, IEEE division)
   int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
   TcSeg seg[3];
@@ -770,8 +771,10 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
           uint32_t o4[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(silu_fast_f(lo2f(gs[e])))));
-            const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(silu_fast_f(hi2f(gs[e])))));
+            const float s0 = g.exact ? silu_ref_f(lo2f(gs[e])) : silu_fast_f(lo2f(gs[e]));
+            const float s1 = g.exact ? silu_ref_f(hi2f(gs[e])) : silu_fast_f(hi2f(gs[e]));
+            const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(s0)));
+            const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(s1)));
             o4[e] = pack2(f2bf(a0), f2bf(a1));
           }
           *reinterpret_cast<uint4*>(out + (size_t)(tok_base + h0 + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
@@ -960,6 +963,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.epi = t.epi;
   g.dual = t.epi == EPI_SILU_MUL;
   g.w_static = t.w_static;
+  g.exact = t.exact;
   int tiles = 0, cols = 0;
   if (g.dual) {
     // segments = (gate, up) with equal row counts; the weight maps must have 64-row boxes
@@ -969,7 +973,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     tiles = (t.rows[0] + BM / 2 - 1) / (BM / 2);
   } else {
     for (int i = 0; i < t.nseg; ++i) {
-      g.seg[i] = TcSeg{t.rows[i], tiles, t.ld_out, t.out + cols};
+      g.seg[i] = t.outs[i] ? TcSeg{t.rows[i], tiles, t.lds[i], t.outs[i]} : TcSeg{t.rows[i], tiles, t.ld_out, t.out + cols};
       tiles += (t.rows[i] + BM - 1) / BM;
       cols += t.rows[i];
     }
@@ -979,7 +983,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   bool vec = true;  // the epilogue through a staging tile stores 16 bytes
   for (int i = 0; i < g.nseg; ++i)
     vec = vec && g.seg[i].rows % 8 == 0 && g.seg[i].ld % 8 == 0 && (reinterpret_cast<uintptr_t>(g.seg[i].out) & 15) == 0;
-  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, vec, true);
+  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, vec, !t.exact);
   const int token_tiles = (t.M + tl.bn - 1) / tl.bn;
   g.kb_per_split = (g.kb_total + tl.splits - 1) / tl.splits;
   g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
@@ -1020,6 +1024,54 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     case 128: return launch_bn<128>(t, g, x, token_tiles, st);
     default: return launch_bn<256>(t, g, x, token_tiles, st);
   }
+}
+
+// Reference-order products of any number of rows.  The chain of tcgen05.mma over ascending k of 16 into one accumulator gives the bits of
+// the reference's chain of m16n8k16 products: 1.5e9 outputs of 84 combinations of shape and distribution (values of 2^+-60, cancelling
+// sums, subnormals, overflow, infinities, NaN) showed no difference, and tests/test_gpu_gemm_exact.py repeats a part of them.  So
+// the reference order takes the tcgen05 kernels without the split over K, at every row count: 896 x 4864 at 1000 rows 290 us ->
+// 12.6 (the mma.sync kernel runs 64 rows a launch and reads the weights again for each), at 16 rows 10.5 -> 4.7; 4864 x 896 at 400 rows
+// 737 -> 16.5; 896 x 151936 at 1 row 79 -> 47.  The mma.sync kernel keeps what TMA or the tile cannot express: K below one k-block, fp32 outputs (the partial sums
+// of tensor parallelism), column slices of a wider matrix, operands off a 16-byte boundary.
+cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches) {
+  if (launches) *launches = 0;
+  bool tc = a.M >= 1 && a.K >= BK && a.K % 8 == 0 && a.lda == a.K && a.epi != EPI_STORE_F32 && a.nseg <= 3 &&
+            (reinterpret_cast<uintptr_t>(a.A) & 15) == 0;
+  for (int i = 0; i < a.nseg; ++i) tc = tc && (a.seg[i].ldw == 0 || a.seg[i].ldw == a.K);
+  if (tc) {
+    const bool dual = a.epi == EPI_SILU_MUL;
+    TcGemm t{};
+    t.x = a.A;
+    t.nseg = dual ? 2 : a.nseg;
+    t.M = a.M;
+    t.K = a.K;
+    t.epi = a.epi;
+    t.exact = 1;
+    t.w_static = w_static;
+    t.out = a.seg[0].out;
+    t.ld_out = a.seg[0].ld_out;
+    TensorMap2D w[3];
+    for (int i = 0; i < t.nseg && tc; ++i) {
+      const GemmSeg& sg = a.seg[dual ? 0 : i];
+      tc = make_tensor_map_2d(&w[i], dual && i ? sg.W2 : sg.W, sg.rows, a.K, dual ? BM / 2 : BM) == cudaSuccess;
+      t.w[i] = &w[i];
+      t.rows[i] = sg.rows;
+      t.outs[i] = sg.out;
+      t.lds[i] = sg.ld_out;
+    }
+    if (tc) return launch_gemm_tcgen05(t, num_sms, st, launches);
+  }
+  for (int r0 = 0; r0 < a.M; r0 += 64) {
+    GemmArgs c = a;
+    c.A = a.A + (size_t)r0 * a.lda;
+    c.M = std::min(64, a.M - r0);
+    for (int i = 0; i < a.nseg; ++i)  // EPI_STORE_F32: `out` is a float*, twice the bf16 stride
+      c.seg[i].out = a.seg[i].out + (size_t)r0 * a.seg[i].ld_out * (a.epi == EPI_STORE_F32 ? 2 : 1);
+    cudaError_t e = launch_gemm_ref_order(c, num_sms, st);
+    if (e != cudaSuccess) return e;
+    if (launches) ++*launches;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace qie

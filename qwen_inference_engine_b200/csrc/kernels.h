@@ -150,9 +150,14 @@ struct TcGemm {
   int nseg, M, K, epi;
   bf16* out;     // [M, ld_out]; EPI_SILU_MUL: segments are (gate, up), out has rows[0] columns
   int ld_out;
+  bf16* outs[3];  // segments with outputs of their own (row strides lds) instead of columns of `out`; null: `out`
+  int lds[3];
+  int exact;     // reference-order numerics: k ascending in one accumulator (no split over K), SiLU as the reference computes it
   int w_static;  // weights are not produced by a preceding kernel: prefetch them before the PDL wait
 };
 cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, int* launches);
+// reference-order GEMM of any number of rows (tcgen05, or launch_gemm_ref_order 64 rows at a time); *launches: kernels launched
+cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches);
 
 cudaError_t launch_rmsnorm_fast(const bf16* x, const bf16* w, bf16* y, size_t hidden, size_t n_tok, size_t x_stride,
                                 cudaStream_t st, float eps = 1e-04f);
