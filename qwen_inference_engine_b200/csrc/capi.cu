@@ -157,6 +157,7 @@ int qie_attention_pagelist(const qie_bf16* const* d_k_pages, const qie_bf16* con
   a.k_pages = reinterpret_cast<const bf16* const*>(d_k_pages);
   a.v_pages = reinterpret_cast<const bf16* const*>(d_v_pages);
   a.pl_layers = n_layers;
+  a.one_seq = 1;
   CU(launch_attention_ref(a, (cudaStream_t)st));
   return QIE_OK;
 }

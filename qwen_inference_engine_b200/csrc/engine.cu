@@ -256,6 +256,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.layer = l;
       a.max_kv_len = max_kv_len;
       a.kv = e->kv;
+      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
       QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
     }
     capture_copy(e, "attn", l, e->att, (size_t)n * Dq);
@@ -424,6 +425,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       a.layer = l;
       a.max_kv_len = max_kv_len;
       a.kv = e->kv;
+      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
       QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
     }
     {  // o_proj over the local head columns -> partial sums -> all-reduce -> residual

@@ -106,8 +106,14 @@ struct AttnArgs {
   const bf16* const* k_pages = nullptr;
   const bf16* const* v_pages = nullptr;
   int pl_layers = 0;
+  int one_seq = 0;    // 1: every row is known to belong to one sequence (a prompt, a page list)
+  int tile_rows = 0;  // attention_ref_kernel: leave tiles of this many rows to attention_ref_rows_kernel where they are one sequence's; 0: none
 };
 cudaError_t launch_attention_ref(const AttnArgs& a, cudaStream_t st);
+// the same for rows of one sequence (attn_ref_rows.cu): rows a CTA takes and virtual rows (row x query head) of its tile, 0 if it does
+// not take these sizes
+int attention_ref_tile_rows(const AttnArgs& a, int num_sms, int* virtual_rows);
+cudaError_t launch_attention_ref_rows(const AttnArgs& a, int rows, int virtual_rows, cudaStream_t st);
 // K, V rows [n_tok, kv_dim] -> positions pos0 + t of a page list in the reference's layout (see AttnArgs)
 cudaError_t launch_kv_store_pagelist(bf16* const* k_pages, bf16* const* v_pages, int page_size, int n_layers, int layer, int kv_dim,
                                      const bf16* K, const bf16* V, int pos0, int n_tok, cudaStream_t st);

@@ -415,6 +415,12 @@ __global__ void __launch_bounds__(256) attention_ref_kernel(AttnArgs a) {
 
   const int h = blockIdx.x, tok = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (a.tile_rows) {
+    const int r0 = tok / a.tile_rows * a.tile_rows, r1 = min(r0 + a.tile_rows, a.n_tok);
+    bool one = true;
+    for (int i = r0 + 1; i < r1; ++i) one = one && a.slot[i] == a.slot[r0];
+    if (one) return;  // attention_ref_rows_kernel has done this row
+  }
   const int kv_len = a.pos[tok] + 1;
   const int group = a.n_q / a.kv.n_kv;
   const int kvh = h / group;
@@ -505,8 +511,20 @@ __global__ void __launch_bounds__(256) attention_ref_kernel(AttnArgs a) {
   }
 }
 
-cudaError_t launch_attention_ref(const AttnArgs& a, cudaStream_t st) {
-  if (a.n_tok == 0) return cudaSuccess;
+cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
+  if (args.n_tok == 0) return cudaSuccess;
+  AttnArgs a = args;
+  if (a.kv.hd == 64 || a.kv.hd == 128 || a.kv.hd == 256) {
+    int dev = 0, sms = 0, vr = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    a.tile_rows = attention_ref_tile_rows(a, sms, &vr);
+    if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
+      e = launch_attention_ref_rows(a, a.tile_rows, vr, st);
+      if (e != cudaSuccess || a.one_seq || a.tile_rows == 1) return e;
+    }
+  }
   int max_pages_used = (a.max_kv_len + a.kv.page_size - 1) / a.kv.page_size;
   size_t smem = (size_t)a.max_kv_len * sizeof(float) + (size_t)max_pages_used * sizeof(int);
   dim3 grid(a.n_q, a.n_tok);
