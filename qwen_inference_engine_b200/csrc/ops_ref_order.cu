@@ -753,35 +753,32 @@ __global__ void greedy_merge_kernel(const Cand* __restrict__ cands, int* __restr
 // k-th best key is found by a radix select: six 8-bit digits from the top, one 256-bin shared-memory histogram pass
 // over the row per digit (the row is 300 KB and stays in L2), then one pass collects the k keys >= the threshold, a
 // bitonic sort orders them, and thread 0 runs the reference's tail (temperature, softmax over k, XORWOW draw, CDF
-// scan) unchanged.  7 passes instead of k = 50 (x exclusion-list checks); one block of 1024 threads per row.
+// scan) unchanged.  7 passes instead of k = 50 (x exclusion-list checks); one block per row.  What the cluster kernel below does not take.
 __device__ __forceinline__ unsigned long long topk_key(uint16_t bits, int idx) {
   if (bits == 0x8000u) bits = 0;  // -0.0 == +0.0 in the reference's float compares
   const uint32_t v16 = (bits & 0x8000u) ? (uint32_t)(uint16_t)~bits : (uint32_t)(bits | 0x8000u);
   const uint32_t rev = __brev((unsigned)idx << 24);  // brev of the low byte, in the low byte
   return ((unsigned long long)v16 << 32) | ((unsigned long long)rev << 24) | (unsigned long long)(0xFFFFFFu - (unsigned)idx);
 }
-__global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab,
-                                                                    float temperature, int k, uint64_t seed, uint64_t seed_stride,
-                                                                    const int* __restrict__ step_ptr, unsigned long long subsequence) {
-  pdl_wait();
-  pdl_trigger();
+__device__ __forceinline__ bool topk_valid(uint16_t b) {  // -inf and NaN are never selected (the reference's v > best fails for both)
+  const uint16_t a = b & 0x7fffu;
+  return !(a > 0x7f80u) && b != 0xff80u;
+}
+__device__ __noinline__ void topk_select_row(const bf16* __restrict__ logits, int* __restrict__ out, int rowi, size_t vocab, float temperature, int k,
+                                             uint64_t seed, uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
   __shared__ unsigned hist[256];
   __shared__ unsigned long long sel[256];  // the selected keys, then sorted best first
   __shared__ float topk_vals[256];
   __shared__ int topk_idxs[256];
   __shared__ unsigned long long s_prefix;
   __shared__ int s_need, s_count;
-  const uint16_t* row = reinterpret_cast<const uint16_t*>(logits) + (size_t)blockIdx.x * vocab;
+  const uint16_t* row = reinterpret_cast<const uint16_t*>(logits) + (size_t)rowi * vocab;
   const int tid = threadIdx.x;
   if (!(temperature > 0.0f)) temperature = 1.0f;
   k = min(k, (int)min(vocab, (size_t)256));
-  auto valid = [](uint16_t b) {  // -inf and NaN are never selected (the reference's v > best fails for both)
-    const uint16_t a = b & 0x7fffu;
-    return !(a > 0x7f80u) && b != 0xff80u;
-  };
   // how many candidates exist at all
   unsigned mine = 0;
-  for (size_t i = tid; i < vocab; i += blockDim.x) mine += valid(row[i]) ? 1u : 0u;
+  for (size_t i = tid; i < vocab; i += blockDim.x) mine += topk_valid(row[i]) ? 1u : 0u;
   if (tid == 0) s_count = 0;
   __syncthreads();
   mine = __reduce_add_sync(0xffffffffu, mine);
@@ -789,7 +786,7 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
   __syncthreads();
   const int actual_k = min(k, s_count);
   if (actual_k <= 0) {
-    if (tid == 0) out[blockIdx.x] = -1;
+    if (tid == 0) out[rowi] = -1;
     return;
   }
   if (tid == 0) {
@@ -804,7 +801,7 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
     const int shift = 8 * d;
     for (size_t i = tid; i < vocab; i += blockDim.x) {
       const uint16_t b = row[i];
-      if (!valid(b)) continue;
+      if (!topk_valid(b)) continue;
       const unsigned long long key = topk_key(b, (int)i);
       if (d == 5 || (key >> (shift + 8)) == (prefix >> (shift + 8))) atomicAdd(&hist[(unsigned)(key >> shift) & 255u], 1u);
     }
@@ -827,7 +824,7 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
   __syncthreads();
   for (size_t i = tid; i < vocab; i += blockDim.x) {
     const uint16_t b = row[i];
-    if (!valid(b)) continue;
+    if (!topk_valid(b)) continue;
     const unsigned long long key = topk_key(b, (int)i);
     if (key >= thr) {
       const int slot = atomicAdd(&s_count, 1);
@@ -853,12 +850,12 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
   if (tid < actual_k) {
     const int idx = (int)(0xFFFFFFu - (unsigned)(sel[tid] & 0xFFFFFFull));
     topk_idxs[tid] = idx;
-    topk_vals[tid] = bf2f(logits[(size_t)blockIdx.x * vocab + idx]);
+    topk_vals[tid] = bf2f(logits[(size_t)rowi * vocab + idx]);
   }
   __syncthreads();
   if (tid == 0) {  // the reference's tail, logit_decode.cu:225-273 (as in sample_topk_kernel)
     if (actual_k == 1) {
-      out[blockIdx.x] = topk_idxs[0];
+      out[rowi] = topk_idxs[0];
       return;
     }
     float max_val = __fdiv_rn(topk_vals[0], temperature);
@@ -874,7 +871,7 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
       sum = __fadd_rn(sum, topk_vals[i]);
     }
     curandState rng;
-    unsigned long long sd = seed + (unsigned long long)blockIdx.x * seed_stride + (step_ptr ? (unsigned)step_ptr[blockIdx.x] : 0u);
+    unsigned long long sd = seed + (unsigned long long)rowi * seed_stride + (step_ptr ? (unsigned)step_ptr[rowi] : 0u);
     curand_init(sd, subsequence, 0, &rng);
     float u = __fmul_rn(curand_uniform(&rng), sum);
     float cum = 0.0f;
@@ -886,8 +883,183 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
         break;
       }
     }
-    out[blockIdx.x] = picked;
+    out[rowi] = picked;
   }
+}
+
+__global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab,
+                                                                    float temperature, int k, uint64_t seed, uint64_t seed_stride,
+                                                                    const int* __restrict__ step_ptr, unsigned long long subsequence) {
+  pdl_wait();
+  pdl_trigger();
+  topk_select_row(logits, out, blockIdx.x, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence);
+}
+
+// 1 < k <= TC_MOST: a cluster of 8 CTAs per row, each over an eighth of the row, 16 bytes a load.  The k-th largest of the threads' maxima is a
+// bound that at least k values of the slice reach; the values that reach it (about 1.1 k of them) are the slice's candidates.  The first
+// CTA gathers the candidates of all slices through distributed shared memory, finds the k-th value by bisection over its 16 bits,
+// ranks what is left by counting (all keys differ) and runs the reference's tail: quotients and exponentials by a thread each, the
+// two sums in the reference's order.  A slice with more candidates than fit (a row of equal logits) falls back to the radix select.
+// One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384; here 18.5 and 39.  The bound
+// is the latency of the steps, not memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 15.6 us, 29 here.
+constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;
+template <int TC_THREADS>
+__global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
+    sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
+                               uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
+  static_assert(TC_THREADS >= 256, "topk_select_row clears and sorts 256 entries, a thread each");
+  pdl_wait();
+  pdl_trigger();
+  __shared__ unsigned long long cand[TC_CAP];             // this slice's candidates
+  __shared__ unsigned long long all[TC_CTAS * TC_CAP];    // first CTA: everybody's
+  __shared__ unsigned long long best[TC_CAP];         // first CTA: those that reach the k-th value
+  __shared__ float vals[TC_MOST];
+  __shared__ int idxs[TC_MOST];
+  __shared__ int s_n, s_cnt, s_tot;
+  __shared__ float s_u;
+  const int tid = threadIdx.x, slice = blockIdx.x, rowi = blockIdx.y;
+  const uint16_t* row = reinterpret_cast<const uint16_t*>(logits) + (size_t)rowi * vocab;
+  if (!(temperature > 0.0f)) temperature = 1.0f;
+  k = min(k, (int)min(vocab, (size_t)TC_MOST));
+  // elements in front of the first 16-byte boundary and behind the last whole piece belong to the first slice
+  const int head = (int)min((size_t)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / 2, vocab);
+  const size_t nvec = (vocab - head) / 8, per = (nvec + TC_CTAS - 1) / TC_CTAS, v0 = min(nvec, slice * per), v1 = min(nvec, v0 + per);
+  const int tail0 = head + (int)nvec * 8, loose = slice == 0 ? head + (int)vocab - tail0 : 0;
+  // order-preserving 16 bits; 0: never selected
+  auto order16 = [](uint32_t b) -> uint32_t {
+    if (!topk_valid((uint16_t)b)) return 0u;
+    if (b == 0x8000u) b = 0;  // -0.0 == +0.0
+    return (b & 0x8000u) ? (uint32_t)(uint16_t)~b : (b | 0x8000u);
+  };
+  auto each = [&](auto&& f) {  // f(order16, bits, index) for this thread's share of the slice
+    for (size_t v = v0 + tid; v < v1; v += TC_THREADS) {
+      const uint4 q = *reinterpret_cast<const uint4*>(row + head + v * 8);
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        f(order16(w[e] & 0xffffu), w[e] & 0xffffu, head + (int)v * 8 + 2 * e);
+        f(order16(w[e] >> 16), w[e] >> 16, head + (int)v * 8 + 2 * e + 1);
+      }
+    }
+    if (tid < loose) {
+      const int i = tid < head ? tid : tail0 + tid - head;
+      f(order16(row[i]), (uint32_t)row[i], i);
+    }
+  };
+  uint32_t mx = 0;
+  each([&](uint32_t o, uint32_t, int) { mx = max(mx, o); });
+  // the largest bound that k maxima reach (1 if fewer threads have a value: then every value is a candidate)
+  uint32_t bound = 0;
+#pragma unroll 1
+  for (int bit = 15; bit >= 0; --bit) {
+    const uint32_t t = bound | (1u << bit);
+    if (__syncthreads_count(mx >= t) >= k) bound = t;
+  }
+  bound = max(bound, 1u);
+  if (tid == 0) s_n = 0;
+  __syncthreads();
+  if (mx >= bound)
+    each([&](uint32_t o, uint32_t b, int i) {
+      if (o < bound) return;
+      const int at = atomicAdd(&s_n, 1);
+      if (at < TC_CAP) cand[at] = topk_key((uint16_t)b, i);
+    });
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (slice == 0) {
+    // ---- gather
+    int n = 0;
+    bool over = false;
+    for (int c = 0; c < TC_CTAS; ++c) {
+      uint32_t an, ac;
+      int cn;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(an) : "r"(smem_u32(&s_n)), "r"(c));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ac) : "r"(smem_u32(cand)), "r"(c));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(cn) : "r"(an) : "memory");
+      over = over || cn > TC_CAP;
+      for (int i = tid; i < min(cn, TC_CAP); i += TC_THREADS)
+        asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(all[n + i]) : "r"(ac + 8u * (uint32_t)i) : "memory");
+      n += min(cn, TC_CAP);
+    }
+    __syncthreads();
+    const int actual_k = min(k, n);
+    // ---- the actual_k-th value, by bisection over its 16 bits
+    uint32_t kth = 0;
+    if (!over && actual_k > 0) {
+#pragma unroll 1
+      for (int bit = 15; bit >= 0; --bit) {
+        const uint32_t t = kth | (1u << bit);
+        if (tid == 0) s_cnt = 0;
+        __syncthreads();
+        int c = 0;
+        for (int i = tid; i < n; i += TC_THREADS) c += (uint32_t)(all[i] >> 32) >= t;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if ((tid & 31) == 0 && c) atomicAdd(&s_cnt, c);
+        __syncthreads();
+        if (s_cnt >= actual_k) kth = t;
+        __syncthreads();
+      }
+    }
+    if (tid == 0) s_tot = 0;
+    __syncthreads();
+    if (!over && actual_k > 0)
+      for (int i = tid; i < n; i += TC_THREADS)
+        if ((uint32_t)(all[i] >> 32) >= kth) {
+          const int at = atomicAdd(&s_tot, 1);
+          if (at < TC_CAP) best[at] = all[i];
+        }
+    __syncthreads();
+    const int m = s_tot;
+    if (over || m > TC_CAP) {
+      topk_select_row(logits, out, rowi, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence);
+    } else if (actual_k == 0) {
+      if (tid == 0) out[rowi] = -1;
+    } else {
+      // ---- rank by counting
+      for (int i = tid; i < m; i += TC_THREADS) {
+        const unsigned long long key = best[i];
+        int rank = 0;
+        for (int j = 0; j < m; ++j) rank += best[j] > key;
+        if (rank < actual_k) {
+          const int idx = (int)(0xFFFFFFu - (unsigned)(key & 0xFFFFFFull));
+          idxs[rank] = idx;
+          vals[rank] = __fdiv_rn(bf2f(logits[(size_t)rowi * vocab + idx]), temperature);
+        }
+      }
+      __syncthreads();
+      // ---- the reference's tail, logit_decode.cu:225-273: the best quotient is the largest (division by a positive number keeps the order)
+      if (actual_k == 1) {
+        if (tid == 0) out[rowi] = idxs[0];  // softmax over one candidate is 1; u in (0,1] always selects it
+      } else {
+        const float max_val = vals[0];
+        __syncthreads();
+        if (tid < actual_k) vals[tid] = expf(__fsub_rn(vals[tid], max_val));
+        if (tid == TC_THREADS - 1) {  // (a warp of its own)
+          curandState rng;
+          const unsigned long long sd = seed + (unsigned long long)rowi * seed_stride + (step_ptr ? (unsigned)step_ptr[rowi] : 0u);
+          curand_init(sd, subsequence, 0, &rng);
+          s_u = curand_uniform(&rng);
+        }
+        __syncthreads();
+        if (tid == 0) {
+          float sum = 0.0f, cum = 0.0f;
+          for (int i = 0; i < actual_k; ++i) sum = __fadd_rn(sum, vals[i]);
+          const float u = __fmul_rn(s_u, sum);
+          int picked = idxs[actual_k - 1];
+          for (int i = 0; i < actual_k; ++i) {
+            cum = __fadd_rn(cum, vals[i]);
+            if (u <= cum) {
+              picked = idxs[i];
+              break;
+            }
+          }
+          out[rowi] = picked;
+        }
+      }
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // nobody leaves while the first CTA reads its candidates
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature,
@@ -927,10 +1099,20 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
     (void)launch_k(greedy_merge_kernel, dim3((n_rows + 63) / 64), dim3(64), 0, st, (const Cand*)cands, out_tokens, n_rows);
     return cudaGetLastError();
   }
-  // k > 1: radix-select kernel (7 passes over the row); QIE_TOPK_SCAN=1 keeps the k-round scan of the reference (A/B knob,
-  // and the only path for vocabularies beyond 2^24 entries, which the 24-bit index field of the key cannot hold)
-  static const bool scan_env = [] { const char* v = getenv("QIE_TOPK_SCAN"); return v && v[0] == '1'; }();
-  if (k > 1 && !scan_env && vocab < (1u << 24))
+  if (k > 1 && k <= TC_MOST && vocab < (1u << 24) && n_rows <= 65535) {
+    // many rows: 256 threads, so that more clusters are on the chip at once (64 rows of 151936, k = 50: 39 us, 42 with 512); few rows:
+    // 512, for shorter passes (1 row 18.5, 22 with 256)
+    if (n_rows > 16)
+      (void)launch_k(sample_topk_cluster_kernel<256>, dim3(TC_CTAS, n_rows), dim3(256), 0, st, logits, out_tokens, vocab, temperature, k, seed,
+                     seed_stride, step_ptr, (unsigned long long)subsequence);
+    else
+      (void)launch_k(sample_topk_cluster_kernel<512>, dim3(TC_CTAS, n_rows), dim3(512), 0, st, logits, out_tokens, vocab, temperature, k, seed,
+                     seed_stride, step_ptr, (unsigned long long)subsequence);
+    return cudaGetLastError();
+  }
+  // more than TC_MOST candidates: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the
+  // 24-bit index field of the key cannot hold, and for k < 1
+  if (k > 1 && vocab < (1u << 24))
     (void)launch_k(sample_topk_select_kernel, dim3(n_rows), dim3(1024), 0, st, logits, out_tokens, vocab, temperature, k, seed, seed_stride,
                    step_ptr, (unsigned long long)subsequence);
   else

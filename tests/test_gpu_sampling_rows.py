@@ -1,0 +1,53 @@
+"""Sampling with a cluster of CTAs per row (csrc/ops_ref_order.cu, sample_topk_cluster_kernel) against the C restatement of the reference's
+sampler: rows on and off a 16-byte boundary, ties, rows that overflow the candidate lists, rows with fewer candidates than k."""
+import numpy as np
+import pytest
+import torch
+
+from util import bf16_to_f32, f32_to_bf16, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def layers():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from qwen_inference_engine_b200 import layers as L
+    return L
+
+
+def row(kind, vocab, rng):
+    x = rng.standard_normal(vocab).astype(np.float32) * 2.5
+    if kind == "ties":
+        x = np.round(x)
+    if kind == "equal":  # every value is a candidate: more than a slice's list holds
+        x[:] = 1.5
+    if kind == "few":
+        x[:] = -np.inf
+        x[rng.integers(0, vocab, size=7)] = rng.standard_normal(7)
+    if kind == "one slice":  # all large values side by side
+        x[vocab // 2:vocab // 2 + 300] += 40
+    if kind == "zeros":
+        x = np.where(x > 3, 0.0, -0.0) - (x < 0)
+    return f32_to_bf16(x)
+
+
+@pytest.mark.parametrize("kind", ["normal", "ties", "equal", "few", "one slice", "zeros"])
+@pytest.mark.parametrize("vocab,rows", [(151936, 3), (32001, 5), (1000, 2), (519, 9)])
+@pytest.mark.parametrize("k", [1, 2, 50, 128])
+def test_rows_against_the_restatement(layers, oracle, vocab, rows, kind, k):
+    rng = np.random.default_rng(vocab + k)
+    lg = np.stack([row(kind, vocab, rng) for _ in range(rows)])
+    for seed in (1234, 77):
+        got = layers.sample_topk_bf16(to_dev(lg), vocab, 0.7, k, seed)
+        for r in range(rows):
+            want = oracle.argmax_tiebreak(lg[r]) if k == 1 else oracle.sample_topk(lg[r], 0.7, k, seed)
+            assert got[r] == want, (r, seed)
+
+
+def test_nothing_to_choose(layers):
+    x = np.full((2, 4099), -np.inf, np.float32)
+    x[1, 4098] = 3
+    assert layers.sample_topk_bf16(to_dev(f32_to_bf16(x)), 4099, 1.0, 50, 1).tolist() == [-1, 4098]
+    assert np.isinf(bf16_to_f32(f32_to_bf16(x))[0]).all()
