@@ -28,6 +28,7 @@ namespace qie {
 static constexpr int PF_QT = 64;     // query rows per CTA
 static constexpr int PF_KT = 64;     // kv positions per pipeline stage
 static constexpr int PF_STAGES = 2;
+static constexpr int PF_TWO_TERM = 1024;  // positions up to which the weights are hi + lo pairs
 static constexpr int PF_MAX_PAGES = 1024;  // page ids cached in shared memory
 
 template <int HD>
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(128, 3) attn_prefill_fast_kernel(FastAttnArgs 
   const float sl2 = a.scale_log2;
   // P = hi + lo (bf16) for short contexts, where few positions average the rounding error of P;
   // beyond 1024 positions the single bf16 term is below the output's own bf16 rounding
-  const bool two_term = kv_len <= 1024;
+  const bool two_term = kv_len <= PF_TWO_TERM;
   // last visible position of rows g and g+8 of this warp
   const int lim0 = pos_first + warp * 16 + g, lim1 = lim0 + 8;
   const int warp_last = pos_first + min(warp * 16 + 15, n_rows - 1);  // beyond this nothing is visible to the warp
@@ -280,6 +281,9 @@ static cudaError_t launch_pf_hd(const FastAttnArgs& a, cudaStream_t st) {
 cudaError_t launch_attention_prefill_fast(const FastAttnArgs& a, cudaStream_t st) {
   if (a.n_tok == 0) return cudaSuccess;
   if (a.n_q % a.kv.n_kv) return cudaErrorInvalidValue;
+  // tcgen05 (attn_prompt_tc.cu), but for the shortest contexts of head_dim 64, where 64-row tiles on mma.sync are quicker (16 rows 4.7
+  // us, 5.4 there; 128 rows 6.7, 6.9; 100 rows behind 100 9.9, 8.7); head_dim 128: 16 rows 6.2, 6.3; 64 rows 6.7, 6.1
+  if ((a.kv.hd == 128 || a.max_kv_len > 128) && attention_prompt_tc_takes(a)) return launch_attention_prompt_tc(a, PF_TWO_TERM, st);
   switch (a.kv.hd) {
     case 64: return launch_pf_hd<64>(a, st);
     case 128: return launch_pf_hd<128>(a, st);

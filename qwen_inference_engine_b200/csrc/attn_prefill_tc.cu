@@ -1,16 +1,16 @@
 // attn_prefill_tc.cu -- causal prefill attention on the 5th-gen tensor cores (tcgen05 + TMEM), head_dim 128.
 //
-// Same contract as attn_prefill_fast.cu (rows = consecutive positions of one sequence, K/V already in the paged
-// pool, fast numerics), different machine mapping: a CTA owns 128 query rows of one head and walks the causal
-// range in tiles of 128 keys;
+// What attn_prompt_tc.cu does not take: pages of other than 16 positions.  Same contract as attn_prefill_fast.cu (rows = consecutive
+// positions of one sequence, K/V already in the paged pool, fast numerics), different machine mapping: a CTA owns 128 query rows of one
+// head and walks the causal range in tiles of 128 keys;
 //   S = Q K^T   : tcgen05.mma, A = Q tile, B = K tile (both K-major, 128-byte swizzle), D = 128 x 128 fp32 in TMEM
 //   softmax     : warps 0-3, thread t = query row t = TMEM lane t reads its S row with tcgen05.ld, keeps the running
 //                 max / sum, writes P (bf16) as the K-major A operand of the second product into shared memory
 //   O_t = P V   : tcgen05.mma, B = V tile as stored in the pool ([key][hd]: N-contiguous = MN-major), fresh
 //                 accumulator per tile in a second TMEM region; the softmax threads fold it into their fp32 row in
 //                 registers (o = o * corr + O_t), so TMEM is never read-modify-written
-// One elected thread of warp 4 issues the MMAs; all 160 threads copy K/V tiles with 16-byte cp.async into the
-// swizzled layout the descriptors expect (pages are 16 positions: no single TMA box covers a tile), the next tile's
+// One elected thread of the last warp issues the MMAs; all threads copy K/V tiles with 16-byte cp.async into the
+// swizzled layout the descriptors expect, the next tile's
 // copies are in flight while the current tile is multiplied.  Replaces the mma.sync kernel (141 TFLOP/s, bound by
 // ldmatrix + softmax issue between the MMAs) for head_dim 128 and >= 256 rows.
 #include <cuda.h>
@@ -115,8 +115,7 @@ __device__ __forceinline__ uint32_t tile_off(int r, int ch) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a, int lbo_sbo_swap,
-                                                                  const __grid_constant__ CUtensorMap kvm, int use_tma) {
+__global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a, int lbo_sbo_swap) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
   unsigned char* sg = smem_raw + (s0 - smem_u32(smem_raw));
   // mbarriers: S product done (two: TMEM buffer t & 1; the copy path uses the first), P V done, K tile landed (two
   // buffers), V tile landed (two)
-  const uint32_t bar_s = s0 + SM_BAR, bar_o = bar_s + 16, slot = bar_s + 24, bar_k = bar_s + 32, bar_v = bar_s + 48;
+  const uint32_t bar_s = s0 + SM_BAR, bar_o = bar_s + 16, slot = bar_s + 24;
   int* s_pages = reinterpret_cast<int*>(sg + SM_PAGES);
   float* xmax = reinterpret_cast<float*>(sg + SM_X);  // [2][128]
   float* xsum = xmax + 256;                            // [2][128]
@@ -147,10 +146,6 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     mbar_init_(bar_s, 1);
     mbar_init_(bar_s + 8, 1);
     mbar_init_(bar_o, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init_(bar_k + 8 * i, 1);
-      mbar_init_(bar_v + 8 * i, 1);
-    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == MMA_WARP) {
@@ -196,42 +191,12 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     }
     cp_async_commit();
   };
-  // K/V tiles by TMA (r02; pages of 16 positions): the 32 lanes of the MMA warp request the 2 x 8 x 2 boxes of a tile --
-  // (K | V) x 8 page chunks x 2 column halves of 64, 2 KiB each, written with the 128-byte swizzle to exactly the place
-  // tile_off() puts them -- so the eight softmax warps issue no copy instructions at all.  Chunks behind the last
-  // page of the sequence repeat that page (finite values; their keys are masked).
-  const int n_kv_pages = (kv_len - 1) / psz + 1;
-  auto tma_kv = [&](int tile, int buf, int is_v) {  // MMA warp: lanes 0-15 request the 8 page chunks x 2 column halves of K or V
-    const int pg = (lane >> 1) & 7, half = lane & 1;
-    const int pi = min(tile * (TK / 16) + pg, n_kv_pages - 1);
-    const int page = pi < MAXP ? s_pages[pi] : bt[pi];
-    const int row = (((page * a.kv.n_layers + a.layer) * 2 + is_v) * a.kv.n_kv + kvh) * psz;
-    const uint32_t dst = s0 + (is_v ? SM_V0 : SM_K0) + buf * TILE_B + half * BLK + pg * 16 * 128;
-    const uint32_t bar = (is_v ? bar_v : bar_k) + 8u * (uint32_t)buf;
-    if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)TILE_B) : "memory");
-    __syncwarp();
-    if (lane < 16)
-      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                   ::"r"(dst), "l"(&kvm), "r"(bar), "r"(half * 64), "r"(row)
-                   : "memory");
-  };
-  if (use_tma) {
-    if (warp == MMA_WARP) {
-      tma_kv(0, 0, 0);
-      tma_kv(0, 0, 1);
-      if (n_tiles > 1) tma_kv(1, 1, 0);
-    }
-  } else {
-    load_tile(0, 0);
-  }
+  load_tile(0, 0);
 
   // Where the time goes (T = 4096, 12 heads, 171 us; probe builds that skip one part each): both MMA chains 35 us,
   // the exp + bf16-pack pass 53 us (16 384 ex2 + 8 192 cvt per tile on the 16-lane XU pipe), everything else --
   // tile copies, TMEM loads, row max, O fold, P stores, barriers, CTA prologue/epilogue -- 94 us.  An MN-major V
   // descriptor costs the same as a K-major one.
-  // r02: with the cp.async copies, S in two TMEM buffers / S(t+1) issued before the softmax of tile t was a dead end (17.5 ->
-  // 18.5 ms: the softmax warps are the critical path and a second copy pass cost them more than the S latency it hid);
-  // with K/V by TMA the same schedule is free for them (the TMA path below).
   const uint32_t lbo = (lbo_sbo_swap & 1) ? 1024u : (uint32_t)BLK, sbo = (lbo_sbo_swap & 1) ? (uint32_t)BLK : 1024u;
   constexpr uint32_t ID_S = idesc_(128, 128, false), ID_O = idesc_(128, 128, true);
   const float sl2 = a.scale_log2;
@@ -322,47 +287,6 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     umma_commit_(bar_o);
   };
 
-  if (use_tma) {
-    // ---- TMA path, software pipeline: S(t+1) goes to the tensor pipe in front of the softmax of tile t (two S buffers in
-    // TMEM); K(t+2) is requested as soon as S(t) is done, V(t+1) as soon as P V(t-1) is done.  The MMA warp does all of
-    // that; the softmax warps only wait for mbarriers.
-    if (warp == MMA_WARP && lane == 0) {
-      mbar_wait_(bar_k, 0);
-      issue_s(0, 0);
-    }
-    for (int it = 0; it < n_tiles; ++it) {
-      const int buf = it & 1;
-      if (warp == MMA_WARP) {
-        if (lane == 0 && it + 1 < n_tiles) {
-          mbar_wait_(bar_k + 8u * (uint32_t)(buf ^ 1), (uint32_t)(((it + 1) >> 1) & 1));  // K(it+1) has landed
-          issue_s(it + 1, buf ^ 1);  // (everybody read S(it-1) out of that buffer in front of the last __syncthreads)
-        }
-        __syncwarp();
-        if (it + 1 < n_tiles) {  // V(it+1) takes the place of V(it-1)
-          if (it > 0) mbar_wait_(bar_o, (uint32_t)((it - 1) & 1));
-          tma_kv(it + 1, buf ^ 1, 1);
-        }
-        if (it + 2 < n_tiles) {  // K(it+2) takes the place of K(it)
-          mbar_wait_(bar_s + 8u * (uint32_t)buf, (uint32_t)((it >> 1) & 1));
-          tma_kv(it + 2, buf, 0);
-        }
-      } else {
-        if (it > 0) {  // fold the previous tile's P V product
-          mbar_wait_(bar_o, (uint32_t)((it - 1) & 1));
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          fold_o();
-        }
-        mbar_wait_(bar_s + 8u * (uint32_t)buf, (uint32_t)((it >> 1) & 1));
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        softmax_tile(it, buf);
-      }
-      __syncthreads();
-      if (warp == MMA_WARP && lane == 0) {
-        mbar_wait_(bar_v + 8u * (uint32_t)buf, (uint32_t)((it >> 1) & 1));  // V(it) has landed
-        issue_pv(it);
-      }
-    }
-  } else {
   for (int it = 0; it < n_tiles; ++it) {
     const int buf = it & 1;
     cp_async_wait<0>();  // tile it (requested one iteration ago)
@@ -386,7 +310,6 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     __syncthreads();
     // ---- O_t = P V
     if (warp == MMA_WARP && lane == 0) issue_pv(it);
-  }
   }
   if (soft) {
     mbar_wait_(bar_o, (uint32_t)((n_tiles - 1) & 1));
@@ -420,20 +343,15 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
 cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap, cudaStream_t st) {
   if (a.n_tok == 0) return cudaSuccess;
   if (a.kv.hd != HDX || a.n_q % a.kv.n_kv) return cudaErrorInvalidValue;
+  if (attention_prompt_tc_takes(a)) return launch_attention_prompt_tc(a, 0, st);
   static PerDeviceOnce set;
   if (set.need()) {
     cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
     if (e != cudaSuccess) return e;
     set.done();
   }
-  // K/V by TMA: the pool as rows of one head (256 bytes), boxes of 16 slots x 64 columns; pages of 16 positions only
-  // (QIE_ATTN_TC_TMA=0 keeps the cp.async copies: A/B knob)
-  static const bool tma_env = [] { const char* v = getenv("QIE_ATTN_TC_TMA"); return !(v && v[0] == '0'); }();
-  TensorMap2D tm{};
-  const unsigned long long rows = (unsigned long long)a.kv.n_pages * a.kv.n_layers * 2ull * a.kv.n_kv * a.kv.page_size;
-  const int use_tma = tma_env && a.kv.page_size == 16 && make_tensor_map_kv(&tm, a.kv.pool, rows, HDX, 16) == cudaSuccess;
   dim3 grid(a.n_q, (a.n_tok + TQ - 1) / TQ);
-  (void)launch_k(attn_prefill_tc_kernel, grid, dim3(NTHR), (size_t)SM_TOTAL, st, a, lbo_sbo_swap, *reinterpret_cast<const CUtensorMap*>(&tm), use_tma);
+  (void)launch_k(attn_prefill_tc_kernel, grid, dim3(NTHR), (size_t)SM_TOTAL, st, a, lbo_sbo_swap);
   return cudaGetLastError();
 }
 

@@ -235,6 +235,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.n_q = c.n_q;
       a.layer = l;
       a.n_splits = 1;
+      a.max_kv_len = max_kv_len;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.kv = e->kv;
       // head_dim 128 and at least one full 128-row query tile: tcgen05 / TMEM kernel (QIE_ATTN_TC=0 keeps mma.sync)

@@ -127,6 +127,7 @@ struct FastAttnArgs {
   const int* block_table;
   int max_pages, n_tok, n_q, layer, n_splits;
   float scale_log2;  // log2(e) / sqrt(hd)
+  int max_kv_len;    // prompts: upper bound on the positions a row sees (how the work is split)
   float* ws_o;       // [n_splits][n_tok][n_q][hd]
   float* ws_ml;      // [n_splits][n_tok][n_q][2]
   KvGeom kv;
@@ -135,6 +136,10 @@ cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st)
 // causal tiled attention for prefill rows (attn_prefill_fast.cu): rows are consecutive positions
 // pos[0]+t of one sequence (slot[0]); n_splits / ws_* unused
 cudaError_t launch_attention_prefill_fast(const FastAttnArgs& a, cudaStream_t st);
+// the same on tcgen05 / TMEM (attn_prompt_tc.cu), head_dim 64 or 128, pages of 16; tiles that see at most two_term positions keep their
+// softmax weights as bf16 hi + lo pairs
+bool attention_prompt_tc_takes(const FastAttnArgs& a);
+cudaError_t launch_attention_prompt_tc(const FastAttnArgs& a, int two_term, cudaStream_t st);
 // the same on tcgen05 / TMEM (attn_prefill_tc.cu), head_dim 128; lbo_sbo_swap: descriptor probe, 0 in production
 cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap, cudaStream_t st);
 

@@ -1,0 +1,62 @@
+"""Prompt attention on tcgen05 with 64-key tiles (csrc/attn_prompt_tc.cu) against the reference-order attention, over the edges of tiles, the
+split of the keys over a cluster and the border between the two forms of the weights.  Pool rows that no position owns hold NaN.
+
+Bounds: a rounding to bf16 (8 significant bits) is off by at most 2^-8 of the value, and both results are rounded: 2^-7 of the value.  Weights as
+bf16 hi + lo pairs are good to 2^-16, the exponentials to 2^-20: 2^-14 of the largest value covers their sum.  Single bf16 weights are off by 2^-8 of
+themselves and add up to one: 2^-8 of the largest value."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TWO_TERM = 1024
+
+
+@pytest.fixture(scope="module")
+def layers():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from qwen_inference_engine_b200 import layers as L
+    return L
+
+
+def check(layers, entry, nq, nkv, hd, first, n, spare=0, scale=1.0):
+    g = torch.Generator("cuda").manual_seed(1000 * first + n + hd)
+    total = first + n
+
+    def rand(*shape):
+        return torch.randn(*shape, generator=g, device="cuda")
+
+    pool = layers.KvPool((total + 15) // 16 + spare, 16, 2, nkv, hd, max_seqs=1)
+    pool.pool.fill_(float("nan"))
+    q, k, v = (scale * rand(n, nq * hd)).bfloat16(), rand(total, nkv * hd).bfloat16(), rand(total, nkv * hd).bfloat16()
+    at = torch.arange(total, dtype=torch.int32, device="cuda")
+    pool.store(1, k, v, at, torch.zeros_like(at))
+    pos, slot = at[first:].contiguous(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    want, got = torch.zeros_like(q), torch.full_like(q, float("nan"))
+    layers.launch_attn(q, want, pool, 1, pos, slot, nq)
+    getattr(layers, entry)(q, got, pool, 1, pos, slot, nq)
+    torch.cuda.synchronize()
+    top = v.abs().max().double()
+    d = (got.double() - want.double()).abs() - 2.0 ** -7 * want.double().abs()
+    pairs = entry.endswith("fast") * (torch.arange(n, device="cuda") + first < TWO_TERM)
+    assert torch.isfinite(got).all()
+    assert (d <= torch.where(pairs, 2.0 ** -14, 2.0 ** -8)[:, None] * top).all(), float(d.max() / top)
+
+
+@pytest.mark.parametrize("entry,nq,nkv,hd", [("launch_attn_prefill_fast", 14, 2, 64), ("launch_attn_prefill_fast", 3, 3, 64),
+                                             ("launch_attn_prefill_fast", 12, 2, 128), ("launch_attn_prefill_tc", 28, 4, 128)])
+@pytest.mark.parametrize("first,n", [(0, 1), (0, 63), (0, 64), (0, 65), (0, 129), (127, 1), (128, 130), (300, 100), (950, 200), (1500, 17), (0, 1100), (2050, 300)])
+def test_against_reference_order(layers, entry, nq, nkv, hd, first, n):
+    check(layers, entry, nq, nkv, hd, first, n)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("spare", [0, 4, 30, 200])
+def test_more_parts_than_keys(layers, hd, spare):
+    """a block table for more positions than the sequence has: parts of the cluster without a key, parts that a row does not see"""
+    check(layers, "launch_attn_prefill_fast", 4, 2, hd, 70, 90, spare)
+
+
+def test_growing_maxima(layers):
+    """scores of a few hundred: the reference maximum moves by more than an exponent's range between tiles"""
+    check(layers, "launch_attn_prefill_fast", 2, 1, 64, 0, 700, scale=40.0)
