@@ -232,12 +232,19 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
     return fail(QIE_EINVAL, "attention_decode_fast: need n_q/n_kv <= 16 and head_dim 64 or 128");
   static thread_local void *wo = nullptr, *wml = nullptr;
   static thread_local size_t wo_cap = 0, wml_cap = 0;
-  if (n_splits <= 0) n_splits = 4;
+  if (n_splits <= 0) {
+    int dev = 0, sms = 0;
+    CU(cudaGetDevice(&dev));
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    n_splits = attention_decode_splits(n_tok, kv->n_kv_heads, kv->head_dim, max_pages * kv->page_size, sms);
+  }
   n_splits = std::min(n_splits, 64);
-  int rc = scratch(&wo, &wo_cap, (size_t)n_splits * n_tok * n_q_heads * kv->head_dim * 4);
-  if (rc) return rc;
-  rc = scratch(&wml, &wml_cap, (size_t)n_splits * n_tok * n_q_heads * 2 * 4);
-  if (rc) return rc;
+  if (n_splits > FD_CLUSTER) {
+    int rc = scratch(&wo, &wo_cap, (size_t)n_splits * n_tok * n_q_heads * kv->head_dim * 4);
+    if (rc) return rc;
+    rc = scratch(&wml, &wml_cap, (size_t)n_splits * n_tok * n_q_heads * 2 * 4);
+    if (rc) return rc;
+  }
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;

@@ -133,6 +133,8 @@ struct FastAttnArgs {
   KvGeom kv;
 };
 cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st);
+constexpr int FD_CLUSTER = 8;  // splits that need no workspace
+int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms);
 // causal tiled attention for prefill rows (attn_prefill_fast.cu): rows are consecutive positions
 // pos[0]+t of one sequence (slot[0]); n_splits / ws_* unused
 cudaError_t launch_attention_prefill_fast(const FastAttnArgs& a, cudaStream_t st);
