@@ -1,9 +1,8 @@
 // gemm_tcgen05.cu -- C[M,Nout] = A[M,K] * W[Nout,K]^T on the 5th-gen tensor cores
-// (tcgen05.mma, accumulator in TMEM, operands staged by TMA), for M > 8: batched decode
-// (M = sequences) and prefill (M = prompt tokens).  Fast numerics: fp32 accumulation in
-// the tensor core's own order (+ a fixed-order split-K sum), so results match the
-// reference's wmma kernel (/root/reference/layers/src/matrix_mul.cu:165-288) within the
-// bf16 tolerance, not bit for bit; gemm_ref_order.cu stays the bit-exact path for M <= 8.
+// (tcgen05.mma, accumulator in TMEM, operands staged by TMA): batched decode
+// (M = sequences) and prefill (M = prompt tokens).  Without a split over K the results are the bits of the
+// reference's wmma kernel (/root/reference/layers/src/matrix_mul.cu:165-288; launch_gemm_ref_rows); fast numerics
+// may split K (a fixed-order sum of the splits) and match it within the bf16 tolerance.
 //
 // Swap-AB: the weight tile is the UMMA "A" operand (M = 128 weight rows = 128 TMEM lanes),
 // the activations are the "B" operand (N = BN tokens, 16..256), both K-major, 128-byte
@@ -545,18 +544,18 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 // ------------------------------------------------------------------ persistent variant
 // Same tiles, same math, for launches without split-K: ONE CTA per SM walks the output tiles (weight tile fastest, so neighbouring
 // CTAs share a token tile in L2), the accumulator is double buffered in TMEM (2 x 256 columns), and the epilogue of tile j (TMEM ->
-// bf16 staging tile in shared memory -> 16-byte global accesses, 128 tokens at a time) runs on warps 2-9 while warps 0/1 already
+// bf16 staging tile in shared memory -> global memory, 64 tokens at a time) runs on warps 2-9 while warps 0/1 already
 // stream and multiply tile j+1.  ncu on the one-tile-per-CTA kernel showed the tensor pipe 32-47 % active at K = 1536: per tile
 // ~2.5 us of prologue and ~8 us of epilogue sat next to a ~7-9 us mainloop (profiles/r01c_ncu_full_prefill_kernels.csv).
 // A tile has g.bn tokens, any multiple of 16 (pick_tile): with 256 always, 4096 tokens x 1536 outputs were 192 tiles on 148 SMs, two
 // waves filled to 65 %.  The ring takes the stages that fit: 4 of 48 KiB at 256 tokens, 10 of 18 KiB at 16.
 static constexpr int PBN = 256;                   // TMEM columns of an accumulator
-static constexpr int P_HALF = 128;                // tokens of the staging tile
+static constexpr int P_STEP = 64;                 // tokens of a staging tile (two of them)
 static constexpr int P_RING = 4 * (BM * BK * 2 + PBN * BK * 2);     // 192 KiB
 static constexpr int P_MAX_STAGES = 10;
 static constexpr int P_EPI = 256;                 // epilogue threads (8 warps)
 static constexpr int P_THREADS = 64 + P_EPI;      // + TMA warp + MMA warp
-static constexpr int P_STAGING = P_HALF * BM * 2;                   // bf16 [128 tokens][128 rows] = 32 KiB
+static constexpr int P_STAGING = 2 * P_STEP * BM * 2;               // bf16 [2][64 tokens][128 rows] = 32 KiB
 
 __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                                    const __grid_constant__ CUtensorMap map_w1,
@@ -684,7 +683,11 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     }
   } else {
     // ---- epilogue warps 2-9: two warps per TMEM lane quarter, each draining half of the columns (r02: with four warps the
-    // epilogue of a K = 1536 tile -- drain, SiLU * up, 64 KiB of stores -- took longer than the tile's mainloop)
+    // epilogue of a K = 1536 tile -- drain, SiLU * up, 64 KiB of stores -- took longer than the tile's mainloop).  64 tokens at a time
+    // go through one of two staging tiles, so one barrier a step is enough: who drains into a tile has passed the barrier behind its
+    // last readers.  Plain results leave by bulk copies, a token's 256 bytes each; residuals are requested before the drain.
+    // With two barriers per 128 tokens, 16-byte stores by all threads and residuals requested behind the barrier (us, weights in L2; cuBLAS
+    // 78): 4096 tokens, 1536 x 8960 82 -> 78; 2000: 42.7 -> 41.0; 1000: 24.6 -> 23.6; 18944 x 3584 with residual, 400: 75 -> 70.
     constexpr uint32_t PITCH = BM * 2;
     const int qd = warp & 3;
     const int lane_row = qd * 32 + lane;
@@ -694,8 +697,10 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
       return v;
     };
+    const bool bulk = !g.dual && g.epi == EPI_STORE;
+    const int copier = lane < P_STEP / 8 ? (warp - 2) * (P_STEP / 8) + lane : P_STEP;  // the token whose copy this thread issues
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
-    int j = 0;
+    int j = 0, it = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
       int tile, ttile, si, row0;
       tile_geom(t, tile, ttile, si, row0);
@@ -703,86 +708,92 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       bf16* const out = g.seg[si].out;
       const int tok_base = ttile * bn;
       const int buf = j & 1;
-      mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
-      tc_fence_after();
-      const bool bad = *dead;
       const uint32_t acc = tmem_base + (uint32_t)buf * PBN + ((uint32_t)(qd * 32) << 16);
       const int n_tok_all = min(bn, g.M - tok_base);
+      bool bad = false;
 #pragma unroll 1
-      for (int h0 = 0; h0 < bn; h0 += P_HALF) {  // tokens [h0, h0 + 128) of the tile through the 32 KiB staging tile
-      const int width = min(P_HALF, bn - h0);
-#pragma unroll 4
-      for (int c0 = ((warp - 2) >> 2) * 16; c0 < width; c0 += 32) {  // every other 16 columns: the quarter's second warp has the rest
-        uint32_t r[16];
-        tmem_ld16(acc + h0 + c0, r);
-        if (bad) mark_bad(r);
+      for (int h0 = 0; h0 < bn; h0 += P_STEP, ++it) {
+        const int width = min(P_STEP, bn - h0), n_tok = max(0, min(P_STEP, n_tok_all - h0));
+        const uint32_t st0 = stg + (uint32_t)(it & 1) * (P_STEP * PITCH);
+        constexpr int U = P_STEP * (BM / 8) / P_EPI;  // 16-byte pieces of a thread
+        uint4 x[U];
+        bool ok[U];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const unsigned short hb = __bfloat16_as_ushort(f2bf(__uint_as_float(r[q])));
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(stg + (uint32_t)(c0 + q) * PITCH + (uint32_t)lane_row * 2u), "h"(hb) : "memory");
+        for (int u = 0; u < U; ++u) {
+          const int c = tq + u * P_EPI, w_row = row0 + (c & 15) * 8;
+          ok[u] = (c >> 4) < n_tok && w_row < seg_rows;
+          if (!g.dual && g.epi == EPI_RESIDUAL && ok[u])
+            x[u] = *reinterpret_cast<const uint4*>(out + (size_t)(tok_base + h0 + (c >> 4)) * ld + w_row);
         }
-      }
-      tc_fence_before();
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (h0 + P_HALF >= bn && tq == 0) mbar_arrive_local(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
-      const int n_tok = max(0, min(P_HALF, n_tok_all - h0));
-      if (!g.dual) {
-        const int totalc = n_tok * (BM / 8);
-        for (int c = tq; c < totalc; c += 8 * P_EPI) {
-          uint4 y[8], x[8];
-          bf16* dst[8];
-          bool ok[8];
+        if (h0 == 0) {
+          mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
+          tc_fence_after();
+          bad = *dead;
+        }
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int cc = c + u * P_EPI;
-            const int tok = cc >> 4, part = cc & 15;
-            const int w_row = row0 + part * 8;
-            ok[u] = cc < totalc && w_row < seg_rows;
-            dst[u] = out + (size_t)(tok_base + h0 + tok) * ld + w_row;
-            if (ok[u]) {
-              if (g.epi == EPI_RESIDUAL) x[u] = *reinterpret_cast<const uint4*>(dst[u]);
-              y[u] = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
-            }
+        for (int c0 = ((warp - 2) >> 2) * 16; c0 < P_STEP; c0 += 32) {  // every other 16 columns: the quarter's second warp has the rest
+          if (c0 >= width) break;
+          uint32_t r[16];
+          tmem_ld16(acc + h0 + c0, r);
+          if (bad) mark_bad(r);
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            const unsigned short hb = __bfloat16_as_ushort(f2bf(__uint_as_float(r[q])));
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(st0 + (uint32_t)(c0 + q) * PITCH + (uint32_t)lane_row * 2u), "h"(hb) : "memory");
           }
+        }
+        tc_fence_before();
+        if (bulk) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the other staging tile has been read: the next step may write it
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (h0 + P_STEP >= bn && tq == 0) mbar_arrive_local(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
+        if (bulk) {
+          if (copier < n_tok) {
+            bf16* dst = out + (size_t)(tok_base + h0 + copier) * ld + row0;
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(st0 + (uint32_t)copier * PITCH),
+                         "r"(2 * min(BM, seg_rows - row0))
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        } else if (!g.dual) {
 #pragma unroll
-          for (int u = 0; u < 8; ++u) {
+          for (int u = 0; u < U; ++u) {
             if (!ok[u]) continue;
-            if (g.epi == EPI_RESIDUAL) {
-              const uint32_t xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, ys[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
-              uint32_t o4[4];
+            const int c = tq + u * P_EPI;
+            const uint4 y = lds128(st0 + (uint32_t)(c >> 4) * PITCH + (uint32_t)(c & 15) * 16u);
+            const uint32_t xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, ys[4] = {y.x, y.y, y.z, y.w};
+            uint32_t o4[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                o4[e] = pack2(f2bf(__fadd_rn(lo2f(xs[e]), lo2f(ys[e]))), f2bf(__fadd_rn(hi2f(xs[e]), hi2f(ys[e]))));
-              *reinterpret_cast<uint4*>(dst[u]) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-            } else {
-              *reinterpret_cast<uint4*>(dst[u]) = y[u];
+            for (int e = 0; e < 4; ++e)
+              o4[e] = pack2(f2bf(__fadd_rn(lo2f(xs[e]), lo2f(ys[e]))), f2bf(__fadd_rn(hi2f(xs[e]), hi2f(ys[e]))));
+            *reinterpret_cast<uint4*>(out + (size_t)(tok_base + h0 + (c >> 4)) * ld + row0 + (c & 15) * 8) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+          }
+        } else {
+          const int totalc = n_tok * (BM / 16);
+          for (int c = tq; c < totalc; c += P_EPI) {
+            const int tok = c >> 3, part = c & 7;
+            const int w_row = row0 + part * 8;
+            if (w_row >= seg_rows) continue;
+            const uint4 gt = lds128(st0 + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
+            const uint4 up = lds128(st0 + (uint32_t)tok * PITCH + (uint32_t)(BM / 2) * 2u + (uint32_t)part * 16u);
+            const uint32_t gs[4] = {gt.x, gt.y, gt.z, gt.w}, us[4] = {up.x, up.y, up.z, up.w};
+            uint32_t o4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float s0 = g.exact ? silu_ref_f(lo2f(gs[e])) : silu_fast_f(lo2f(gs[e]));
+              const float s1 = g.exact ? silu_ref_f(hi2f(gs[e])) : silu_fast_f(hi2f(gs[e]));
+              const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(s0)));
+              const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(s1)));
+              o4[e] = pack2(f2bf(a0), f2bf(a1));
             }
+            *reinterpret_cast<uint4*>(out + (size_t)(tok_base + h0 + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
           }
         }
-      } else {
-        const int totalc = n_tok * (BM / 16);
-        for (int c = tq; c < totalc; c += P_EPI) {
-          const int tok = c >> 3, part = c & 7;
-          const int w_row = row0 + part * 8;
-          if (w_row >= seg_rows) continue;
-          const uint4 gt = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
-          const uint4 up = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)(BM / 2) * 2u + (uint32_t)part * 16u);
-          const uint32_t gs[4] = {gt.x, gt.y, gt.z, gt.w}, us[4] = {up.x, up.y, up.z, up.w};
-          uint32_t o4[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float s0 = g.exact ? silu_ref_f(lo2f(gs[e])) : silu_fast_f(lo2f(gs[e]));
-            const float s1 = g.exact ? silu_ref_f(hi2f(gs[e])) : silu_fast_f(hi2f(gs[e]));
-            const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(s0)));
-            const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(s1)));
-            o4[e] = pack2(f2bf(a0), f2bf(a1));
-          }
-          *reinterpret_cast<uint4*>(out + (size_t)(tok_base + h0 + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-        }
-      }
-      asm volatile("bar.sync 2, 256;" ::: "memory");  // the staging tile is rewritten by the next tokens
       }
     }
+    if (bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // written, before the CTA gives its shared memory back
   }
   __syncthreads();
   if (warp == 1) {
