@@ -6,7 +6,8 @@
 // query tokens, walks the page list for every (token, kv position) pair and runs the softmax
 // in one thread -- O(T^2) serial work per head.  Here the T x t score matrix is tiled the
 // FlashAttention-2 way; results agree with the reference within the north-star 1e-2 bf16
-// tolerance (tests/test_gpu_fast_path.py); ops_ref_order.cu stays the bit-exact path.
+// tolerance (tests/test_gpu_fast_path.py); ops_ref_order.cu stays the bit-exact path.  attn_prompt_tc.cu takes pages of 16 positions,
+// but for contexts up to 128 of head_dim 64.
 //
 // Mapping (tensor-pipe bound for long prompts: 4*hd*T^2/2 flop per head):
 //   rows  : the chunk's query rows are consecutive positions pos[0]+t of ONE sequence; their

@@ -282,7 +282,7 @@ int attention_ref_tile_rows(const AttnArgs& a, int num_sms, int* virtual_rows) {
   int best = 0;
   for (int R = 32 / np; R >= 8 && R >= G; R /= 2) {
     const size_t s = ((size_t)a.max_kv_len * R + page_ints(a)) * sizeof(float);
-    if (s > 180 * 1024) continue;  // (above 5.7k positions: attention_ref_kernel)
+    if (s > 180 * 1024) continue;  // (8 virtual rows above 5.7k positions, 16 above 2.8k: attention_ref_kernel)
     best = R / G, *virtual_rows = R;
     if (s <= 76 * 1024 && (long)((a.n_tok + best - 1) / best) * a.kv.n_kv >= 2 * num_sms) break;
   }

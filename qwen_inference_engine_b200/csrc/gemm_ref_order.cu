@@ -1,5 +1,5 @@
-// gemm_ref_order.cu -- skinny GEMM  C[M,Nout] = A[M,K] * W[Nout,K]^T  for decode / short
-// prefill, reproducing the accumulation order of the reference's wmma kernel
+// gemm_ref_order.cu -- skinny GEMM  C[M,Nout] = A[M,K] * W[Nout,K]^T  for what the tcgen05 kernels of the reference
+// order (launch_gemm_ref_rows, gemm_tcgen05.cu) do not take, reproducing the accumulation order of the reference's wmma kernel
 // (/root/reference/layers/src/matrix_mul.cu:165-288):
 //   * activations are the A operand (row-major 16 x 16 tiles, rows >= M are zero),
 //     weight rows are the B operand ("col" = k-contiguous), exactly as the reference

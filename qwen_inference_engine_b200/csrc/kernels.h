@@ -145,7 +145,7 @@ cudaError_t launch_attention_prompt_tc(const FastAttnArgs& a, int two_term, cuda
 // the same on tcgen05 / TMEM (attn_prefill_tc.cu), head_dim 128; lbo_sbo_swap: descriptor probe, 0 in production
 cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap, cudaStream_t st);
 
-// tcgen05 GEMM (fast numerics, M > 8)
+// tcgen05 GEMM (fast numerics; without a split over K also the reference's order)
 struct TensorMap2D {
   alignas(64) unsigned char opaque[128];  // CUtensorMap
 };

@@ -396,7 +396,7 @@ cudaError_t launch_residual_add(bf16* a, const bf16* b, size_t n, cudaStream_t s
 }
 
 // ------------------------------------------------------------------ attention
-// grid (q head, token); 256 threads.  Phase 1: one warp per kv position computes the
+// What attn_ref_rows.cu does not take.  grid (q head, token); 256 threads.  Phase 1: one warp per kv position computes the
 // score with the reference's 2^k tree over head_dim.  Phase 2: max (order free), expf,
 // the reference's sequential sum, p = e/sum.  Phase 3: thread d accumulates
 // out[d] = fma(p[k], v[k][d], out[d]) for k ascending (self_attension.cu:112-137).
