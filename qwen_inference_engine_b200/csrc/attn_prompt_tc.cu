@@ -2,7 +2,8 @@
 // (fast numerics; the contract of attn_prefill_fast.cu: rows are consecutive positions of one sequence, keys and values are in the pool).
 //
 // A CTA owns 128 query rows of one head and walks the causal range in tiles of 64 keys; two CTAs share an SM.
-//   S = Q K^T  : tcgen05.mma, 128 x 64 fp32 in one of two TMEM buffers, issued two tiles ahead of its softmax
+//   S = Q K^T  : tcgen05.mma, 128 x 64 fp32 in one of two TMEM buffers, issued two tiles ahead of its softmax, behind the product that
+//                read the weights there
 //   softmax    : warps 0-3, one thread per row (= TMEM lane): 64 scores in registers, no exchange between threads.  The weights go back over
 //                the scores' columns as bf16, where the second product takes its A operand from
 //   O += P V   : accumulates in TMEM; where a maximum grew, the row's warp scales O behind its exponentials, when the product of the
@@ -197,7 +198,8 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
       issue_pv(t);
       if (t + 2 < n_tiles) {
         mbar_wait_tc(bar_k + b, ph ^ 1, dead);
-        issue_s(t + 2);  // (over the weights' columns: products run in the order of their issue)
+        mbar_wait_tc(bar_o + b, ph, dead);  // S(t + 2) goes over the weights that P V(t) reads, and only products on one accumulator are
+        issue_s(t + 2);                     // ordered by their issue.  (The weights of t + 1 are a softmax away: nothing is lost.)
       }
     }
   } else {

@@ -60,3 +60,29 @@ def test_more_parts_than_keys(layers, hd, spare):
 def test_growing_maxima(layers):
     """scores of a few hundred: the reference maximum moves by more than an exponent's range between tiles"""
     check(layers, "launch_attn_prefill_fast", 2, 1, 64, 0, 700, scale=40.0)
+
+
+@pytest.mark.parametrize("entry,nq,nkv,hd", [("launch_attn_prefill_fast", 14, 2, 64), ("launch_attn_prefill_fast", 12, 2, 128), ("launch_attn_prefill_tc", 12, 2, 128)])
+@pytest.mark.parametrize("first,n", [(0, 1500), (1200, 128)])
+def test_same_bits_every_time(layers, entry, nq, nkv, hd, first, n):
+    """scores two tiles ahead take the columns of the weights in front: whatever the products' timing, beside other work and on an idle chip, the same
+    bits (one query tile with its keys split over a cluster, and many tiles)"""
+    g = torch.Generator("cuda").manual_seed(hd + n)
+    total = first + n
+    pool = layers.KvPool((total + 15) // 16, 16, 1, nkv, hd, max_seqs=1)
+    pool.pool.normal_(generator=g)
+    q = torch.randn(n, nq * hd, generator=g, device="cuda").bfloat16()
+    pos, slot = torch.arange(first, total, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    a = torch.randn(2048, 2048, generator=g, device="cuda").bfloat16()
+    side, outs = torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for i in range(40):
+        if i % 2:
+            with torch.cuda.stream(side):
+                a @ a
+        outs.append(torch.empty_like(q))
+        getattr(layers, entry)(q, outs[-1], pool, 0, pos, slot, nq)
+        if i % 4 == 0:
+            torch.cuda.synchronize()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o.view(torch.int16), outs[0].view(torch.int16)) for o in outs[1:])
