@@ -35,11 +35,17 @@ constexpr int TQ = 128, TK = 64;
 constexpr int QBLK = TQ * 128, KBLK = TK * 128;  // [rows][64 columns] bf16 in 8-row swizzle atoms
 constexpr int NSOFT = 128, NTHR = NSOFT + 64;      // + a warp for the products, one for the copies
 constexpr int MAXP = 1024;                       // page ids in shared memory
+constexpr uint32_t TMEM_COLS = 256;              // two tiles of scores, O
 
 template <int HD>
 struct PromptSmem {
   static constexpr int TILE = HD / 64 * KBLK;    // K and V: two stages each
-  static constexpr int Q = 0, K = HD / 64 * QBLK, V = K + 2 * TILE, BAR = V + 2 * TILE, PAGES = BAR + 128, TOTAL = PAGES + MAXP * 4 + 1024;
+  static constexpr int Q = 0, K = HD / 64 * QBLK, V = K + 2 * TILE, BAR = V + 2 * TILE, PAGES = BAR + 128, END = PAGES + MAXP * 4 + 1024;
+  // A CTA allocates TMEM_COLS of an SM's 512 columns and a third one would wait for them while it keeps its cluster's other CTAs from
+  // ending: shared memory is reserved so that a third does not fit (head size 64 needs 53 of the 76 KB).  Registers alone do not promise it.
+  static constexpr int TOTAL = END > 76 * 1024 ? END : 76 * 1024;
+  static_assert(512 / TMEM_COLS == 2 && 3 * (TOTAL + 1024) > 228 * 1024, "no more CTAs on an SM than its TMEM columns allow");
+  static_assert(2 * (TOTAL + 1024 + 2 * TQ * 4 + 64) <= 228 * 1024, "two of them");
   static constexpr int PITCH = (HD + 4) * 4;     // a part's O rows
   static_assert(TQ * PITCH <= BAR, "O rows fit over the operands");
 };
@@ -118,7 +124,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == NSOFT / 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(256u) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   for (int i = tid; i < min(MAXP, n_pages); i += NTHR) s_pages[i] = bt[i];
@@ -364,7 +370,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
     if (*dead)  // copies in flight land
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
 }
 
