@@ -23,6 +23,7 @@
 //           with the second kernel, 18.0 as a cluster
 #include <algorithm>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"
@@ -279,8 +280,7 @@ __global__ void __launch_bounds__(128) attn_decode_fast_kernel(FastAttnArgs a) {
     }
   }
   if (!cluster) return;
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync_all();
   const uint32_t sp = smem_u32(part);
   for (int i = split * 128 + threadIdx.x; i < G * HD; i += 128 * a.n_splits) {
     const int r = i / HD;
@@ -305,8 +305,7 @@ __global__ void __launch_bounds__(128) attn_decode_fast_kernel(FastAttnArgs a) {
       }
     a.out[(size_t)b * a.n_q * HD + (size_t)(kvh * G) * HD + i] = f2bf(O / L);
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // nobody leaves while others read its part
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync_all();  // nobody leaves while others read its part
 }
 
 // out[b,h,:] = sum_s O_s 2^(m_s-M) / sum_s l_s 2^(m_s-M)

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"
@@ -327,8 +328,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
   }
   if (parts > 1) {
     // ---- every part sums its share of the rows over the cluster
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync_all();
     const int rows = TQ / parts, n_parts = (all_tiles + per - 1) / per;  // parts without tiles have nothing to add
     for (int i = tid; i < rows * (HD / 4); i += NTHR) {
       const int row = part * rows + i / (HD / 4), c = i % (HD / 4) * 4;
@@ -361,8 +361,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
       const float inv = 1.f / total;
       *reinterpret_cast<uint2*>(a.out + (size_t)(t0 + row) * Dq + (size_t)h * HD + c) = make_uint2(pack2f(sum.x * inv, sum.y * inv), pack2f(sum.z * inv, sum.w * inv));
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // nobody leaves while others read its rows
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync_all();  // nobody leaves while others read its rows
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -18,6 +18,7 @@
 #include <mutex>
 #include <vector>
 
+#include "cluster.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"
@@ -964,8 +965,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
       const int at = atomicAdd(&s_n, 1);
       if (at < TC_CAP) cand[at] = topk_key((uint16_t)b, i);
     });
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync_all();
   if (slice == 0) {
     // ---- gather
     int n = 0;
@@ -1058,8 +1058,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
       }
     }
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // nobody leaves while the first CTA reads its candidates
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync_all();  // nobody leaves while the first CTA reads its candidates
 }
 
 cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature,
