@@ -67,6 +67,11 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
     const int l = a.pos[row0 + i] + 1;
     max_len = max(max_len, l), min_len = min(min_len, l);
   }
+  if (max_len <= 0) {  // no row sees a position: zeros, and no page to read
+    for (int i = tid; i < n * G * HD; i += NT)
+      a.out[(size_t)(row0 + i / (G * HD)) * a.n_q * HD + (size_t)kvh * G * HD + i % (G * HD)] = f2bf(0.f);
+    return;
+  }
   if (tid < R) s_len[tid] = tid < n * G ? a.pos[row0 + tid / G] + 1 : 0;
   if (!PL) {
     const int* bt = a.block_table + (size_t)slot * a.max_pages;

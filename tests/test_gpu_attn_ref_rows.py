@@ -72,6 +72,15 @@ def test_rows_of_several_sequences(layers, nq, nkv, hd, spoil):
     assert torch.equal(got[0], got[1])
 
 
+@pytest.mark.parametrize("nq,nkv,hd", [(14, 2, 64), (12, 2, 128), (8, 2, 256)])
+def test_rows_that_see_nothing(layers, nq, nkv, hd):
+    """rows at position -1 (nothing to attend to) give zeros, in tiles of their own and beside others"""
+    rows = [(0, -1)] * 40 + [(0, i) for i in range(17)] + [(0, -1), (0, 30), (0, -1)] + [(0, -1)] * 33
+    got, _, _ = both(layers, nq, nkv, hd, 16, [40], rows, hd)
+    assert torch.equal(got[0], got[1])
+    assert not got[0][torch.tensor([p < 0 for _, p in rows], device="cuda")].any()
+
+
 @pytest.mark.parametrize("offset", [0, 2])
 @pytest.mark.parametrize("hd,n", [(64, 50), (128, 21)])
 def test_page_list(layers, hd, n, offset):
