@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 
 #include "engine.h"
@@ -35,6 +36,13 @@ extern "C" {
 const char* qie_last_error(void) { return g_err; }
 int qie_abi_version(void) { return 6; }
 
+// pointers that a kernel reads or writes n bytes at a time
+static bool aligned(size_t n, std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if (reinterpret_cast<uintptr_t>(p) % n) return false;
+  return true;
+}
+
 // ---------------------------------------------------------------- operator level
 int qie_embedding(qie_bf16* out, const qie_bf16* table, const int* ids, size_t hidden, size_t n_tok, qie_stream st) {
   CU(launch_embedding((bf16*)out, (const bf16*)table, ids, hidden, n_tok, (cudaStream_t)st));
@@ -48,6 +56,7 @@ int qie_rmsnorm(const qie_bf16* x, const qie_bf16* w, qie_bf16* y, size_t hidden
 int qie_matmul(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st) {
   // reference argument meaning (helpers.cuh:81): N = inner dim, K = output columns
   if (M < 0 || N <= 0 || K <= 0 || (N & 7)) return fail(QIE_EINVAL, "matmul: need N %% 8 == 0 (got M=%d N=%d K=%d)", M, N, K);
+  if (M > 0 && !aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul: A and B must start on a 16-byte boundary");
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -204,6 +213,7 @@ static int scratch(void** p, size_t* cap, size_t need) {
 
 int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st) {
   if (M < 1 || N < 64 || (N % 8) || K < 1) return fail(QIE_EINVAL, "matmul_fast: need M>=1, N>=64, N%%8==0");
+  if (!aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul_fast: A and B must start on a 16-byte boundary");
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -230,6 +240,7 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_decode_fast: bad layer");
   if (n_q_heads % kv->n_kv_heads || n_q_heads / kv->n_kv_heads > 16 || (kv->head_dim != 64 && kv->head_dim != 128))
     return fail(QIE_EINVAL, "attention_decode_fast: need n_q/n_kv <= 16 and head_dim 64 or 128");
+  if (n_tok > 0 && (!aligned(16, {kv->pool}) || !aligned(4, {Q}))) return fail(QIE_EINVAL, "attention_decode_fast: the pool must start on a 16-byte, Q on a 4-byte boundary");
   static thread_local void *wo = nullptr, *wml = nullptr;
   static thread_local size_t wo_cap = 0, wml_cap = 0;
   if (n_splits <= 0) {
@@ -270,6 +281,8 @@ int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16*
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_prefill_fast: bad layer");
   if (n_q_heads % kv->n_kv_heads || (kv->head_dim != 64 && kv->head_dim != 128))
     return fail(QIE_EINVAL, "attention_prefill_fast: need n_q %% n_kv == 0 and head_dim 64 or 128");
+  if (n_tok > 0 && (!aligned(16, {kv->pool, Q}) || !aligned(4, {out})))
+    return fail(QIE_EINVAL, "attention_prefill_fast: the pool and Q must start on a 16-byte, out on a 4-byte boundary");
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -293,6 +306,7 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
                              qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_prefill_tc: bad layer");
   if (n_q_heads % kv->n_kv_heads || kv->head_dim != 128) return fail(QIE_EINVAL, "attention_prefill_tc: head_dim must be 128");
+  if (n_tok > 0 && !aligned(16, {kv->pool, Q, out})) return fail(QIE_EINVAL, "attention_prefill_tc: the pool, Q and out must start on a 16-byte boundary");
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;

@@ -229,6 +229,11 @@ static cudaError_t launch_mt(const GemmArgs& g, int nw, size_t smem, cudaStream_
 cudaError_t launch_gemm_ref_order(const GemmArgs& a, int num_sms, cudaStream_t st) {
   GemmArgs g = a;
   if (g.M < 1 || g.M > 64 || g.K < 8 || (g.K & 7) || g.nseg < 1 || g.nseg > 3) return cudaErrorInvalidValue;
+  // rows are read 16 bytes at a time
+  auto off16 = [](const void* p, int ld) { return ((reinterpret_cast<uintptr_t>(p) & 15) | (ld & 7)) != 0; };
+  bool off = off16(g.A, g.lda);
+  for (int i = 0; i < g.nseg; ++i) off = off || off16(g.seg[i].W, g.seg[i].ldw) || (g.epi == EPI_SILU_MUL && off16(g.seg[i].W2, 0));
+  if (off) return cudaErrorInvalidValue;
   int u = 0;
   for (int i = 0; i < g.nseg; ++i) {
     g.unit_begin[i] = u;

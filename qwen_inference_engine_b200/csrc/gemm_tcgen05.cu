@@ -1033,7 +1033,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
 // the reference order takes the tcgen05 kernels without the split over K, at every row count: 896 x 4864 at 1000 rows 290 us ->
 // 12.6 (the mma.sync kernel runs 64 rows a launch and reads the weights again for each), at 16 rows 10.5 -> 4.7; 4864 x 896 at 400 rows
 // 737 -> 16.5; 896 x 151936 at 1 row 79 -> 47.  The mma.sync kernel keeps what TMA or the tile cannot express: K below one k-block, fp32 outputs (the partial sums
-// of tensor parallelism), column slices of a wider matrix, operands off a 16-byte boundary.
+// of tensor parallelism), column slices of a wider matrix.  Operands off a 16-byte boundary are refused: both kernels read 16 bytes at a time.
 cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches) {
   if (launches) *launches = 0;
   bool tc = a.M >= 1 && a.K >= BK && a.K % 8 == 0 && a.lda == a.K && a.epi != EPI_STORE_F32 && a.nseg <= 3 &&

@@ -181,3 +181,21 @@ def test_compat_replay_links_against_the_product_library():
         assert f" T {s}" in lib, s
     exe_syms = subprocess.run(["nm", "-DC", exe], capture_output=True, text=True).stdout
     assert " U llm(" in exe_syms and " U build_indexed_tensors" in exe_syms
+
+
+@pytest.mark.parametrize("name,args,at", [
+    ("qie_matmul", lambda p: (p[0], p[1], p[2], 4, 896, 64, None), (0, 1)),
+    ("qie_matmul_fast", lambda p: (p[0], p[1], p[2], 4, 896, 64, None), (0, 1)),
+    ("qie_attention_prefill_fast", lambda p: (p[3], 0, p[0], p[1], 4096, 4096, 4096, 8, 4, 4, None), (0, 1, 3)),
+    ("qie_attention_prefill_tc", lambda p: (p[3], 0, p[0], p[1], 4096, 4096, 4096, 8, 4, 4, 0, None), (0, 1, 3)),
+    ("qie_attention_decode_fast", lambda p: (p[3], 0, p[0], p[1], 4096, 4096, 4096, 8, 4, 4, 0, None), (0, 3))])
+def test_operands_off_their_boundary_are_refused(name, args, at):
+    """kernels that read 16 bytes at a time never see such a pointer: the call returns an error before it touches the device"""
+    from qwen_inference_engine_b200._lib import KvView
+    lib = q.lib()
+    for i in at:
+        p = [4096 * (k + 1) + 2 * (k == i) for k in range(4)]
+        view = KvView(p[3], 8, 16, 1, 2, 128)
+        p[3] = C.byref(view)
+        assert getattr(lib, name)(*args(p)) == -1
+        assert b"boundary" in lib.qie_last_error()
