@@ -124,6 +124,8 @@ def lib():
         "qie_decode_run": (i32, [vp, vp, vp, i32, i32, vp]),
         "qie_decode_step_device": (i32, [vp, vp, i32]),
         "qie_sync": (i32, [vp]),
+        "qie_kernel_status": (i32, []),
+        "qie_wait_selftest": (i32, [vp, vp]),
         "qie_capture_enable": (i32, [vp, i32]),
         "qie_capture_read": (C.c_long, [vp, C.c_char_p, i32, vp, sz]),
         "qie_launch_count": (C.c_long, [vp]),

@@ -16,7 +16,7 @@
 // What bounds it: the chain of a tile, 1500 - 1600 cycles alone on an SM: exponentials 620 (512 are the unit's floor), maximum 190, scaling O
 // 140 - 220 and waiting for its product 140, waiting for S 250, TMEM reads and writes 140.  14 heads of 64, 3000 rows: 105 us with mma.sync,
 // 45 here; 12 heads of 128, 4096 rows: 140 us (128-key tiles, O in registers, one CTA an SM), 72 here = 720 TFLOP/s.
-// Every wait has a limit; when one runs out the CTA stores values that are not numbers.
+// Every wait has a limit; when one runs out the CTA stores values that are not numbers and reports it.
 #include <cuda.h>
 
 #include <algorithm>
@@ -89,12 +89,6 @@ __device__ __forceinline__ unsigned long long twice(float x) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(v) : "f"(x));
   return v;
 }
-__device__ __forceinline__ bool elect() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-
 template <int HD>
 __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a, int two_term, int parts, const __grid_constant__ CUtensorMap kvm) {
   using SM = PromptSmem<HD>;
@@ -173,7 +167,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
     auto issue_s = [&](int t) {
       const uint64_t k = dk + (uint64_t)((t & 1) * (SM::TILE >> 4));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (elect()) {
+      if (elect_tc()) {
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk)
           umma_tc(tmem + (uint32_t)((t & 1) * TK), dq + (uint64_t)(((kk >> 2) * QBLK + (kk & 3) * 32) >> 4), k + (uint64_t)(((kk >> 2) * KBLK + (kk & 3) * 32) >> 4), id_s,
@@ -186,7 +180,7 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
       const uint32_t p = tmem + (uint32_t)((t & 1) * TK);
       const uint64_t v = dv + (uint64_t)((t & 1) * (SM::TILE >> 4));
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (elect()) {
+      if (elect_tc()) {
         for (int lo = 0; lo < (two ? 2 : 1); ++lo)  // 32 columns of hi, 32 of lo
 #pragma unroll
           for (int kk = 0; kk < TK / 16; ++kk) umma_ts_tc(t_o, p + (uint32_t)(lo * 32 + kk * 8), v + (uint64_t)(kk * 128), id_o, t > 0 || kk > 0 || lo > 0);
@@ -366,8 +360,8 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == NSOFT / 32) {
-    if (*dead)  // copies in flight land
-      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    drain_tc(dead);
+    if (lane == 0) report_tc(dead, a.status);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
@@ -425,7 +419,21 @@ cudaError_t launch_hd(const FastAttnArgs& a, int two_term, int parts, const Tens
   return cudaLaunchKernelEx(&cfg, attn_prompt_tc_kernel<HD>, a, two_term, parts, *reinterpret_cast<const CUtensorMap*>(&kvm));
 }
 
+__global__ void wait_selftest_kernel(int* status) {
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ int dead_s;
+  dead_s = 0;
+  mbar_init_tc(smem_u32(&bar), 1);
+  mbar_wait_tc(smem_u32(&bar), 0, &dead_s);
+  report_tc(&dead_s, status);
+}
+
 }  // namespace
+
+cudaError_t launch_wait_selftest(int* status, cudaStream_t st) {
+  wait_selftest_kernel<<<1, 1, 0, st>>>(status);
+  return cudaGetLastError();
+}
 
 bool attention_prompt_tc_takes(const FastAttnArgs& a) {
   return (a.kv.hd == 64 || a.kv.hd == 128) && a.kv.page_size == 16 && a.n_q % a.kv.n_kv == 0 &&

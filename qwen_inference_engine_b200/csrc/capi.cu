@@ -2,10 +2,12 @@
 #include <math.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
+#include <mutex>
 #include <string>
 
 #include "engine.h"
@@ -43,6 +45,48 @@ static bool aligned(size_t n, std::initializer_list<const void*> ps) {
   return true;
 }
 
+// ---------------------------------------------------------------- waits that ran out
+// Kernels whose waits have a limit (tc_ptx.cuh) report one that ran out through a word of mapped host memory: one of every engine, read where
+// the engine's stream has been waited for, and one for all operator calls, read when the next such operator is called (like CUDA's own
+// errors of earlier launches) or by qie_kernel_status.  Reading a report takes it back.
+static cudaError_t alloc_status_word(int** w) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the first operator call may be a captured one
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return e;
+  e = cudaHostAlloc(w, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e == cudaSuccess) **w = 0;
+  (void)cudaThreadExchangeStreamCaptureMode(&mode);
+  return e;
+}
+static std::atomic<int*> g_op_status{nullptr};
+static cudaError_t op_status(int** w) {
+  static std::mutex mu;
+  if ((*w = g_op_status.load(std::memory_order_acquire)) != nullptr) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(mu);
+  if ((*w = g_op_status.load(std::memory_order_acquire)) != nullptr) return cudaSuccess;
+  cudaError_t e = alloc_status_word(w);
+  if (e == cudaSuccess) g_op_status.store(*w, std::memory_order_release);
+  return e;
+}
+static bool take_status(int* w) { return w && *(volatile int*)w && __atomic_exchange_n(w, 0, __ATOMIC_RELAXED); }
+static int wait_failed(const char* whose) {
+  return fail(QIE_ECUDA, "a wait inside a kernel of %s ran out: its results are not numbers", whose);
+}
+static int engine_sync(qie_engine* e) {
+  CU(cudaStreamSynchronize(e->stream));
+  return take_status(e->wait_status) ? wait_failed("this engine") : QIE_OK;
+}
+#define ENGINE_SYNC(e)         \
+  do {                         \
+    int _r = engine_sync(e);   \
+    if (_r) return _r;         \
+  } while (0)
+// at the start of an operator that reports: the word, and an earlier call's report
+#define OP_STATUS(w)                                      \
+  int* w = nullptr;                                       \
+  CU(op_status(&w));                                      \
+  if (take_status(w)) return wait_failed("an earlier operator call")
+
 // ---------------------------------------------------------------- operator level
 int qie_embedding(qie_bf16* out, const qie_bf16* table, const int* ids, size_t hidden, size_t n_tok, qie_stream st) {
   CU(launch_embedding((bf16*)out, (const bf16*)table, ids, hidden, n_tok, (cudaStream_t)st));
@@ -57,6 +101,7 @@ int qie_matmul(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, 
   // reference argument meaning (helpers.cuh:81): N = inner dim, K = output columns
   if (M < 0 || N <= 0 || K <= 0 || (N & 7)) return fail(QIE_EINVAL, "matmul: need N %% 8 == 0 (got M=%d N=%d K=%d)", M, N, K);
   if (M > 0 && !aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul: A and B must start on a 16-byte boundary");
+  OP_STATUS(status);
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -68,7 +113,7 @@ int qie_matmul(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, 
   g.nseg = 1;
   g.epi = EPI_STORE;
   g.seg[0] = GemmSeg{(const bf16*)B, nullptr, (bf16*)C, K, K};
-  CU(launch_gemm_ref_rows(g, sms, (cudaStream_t)st, 0, nullptr));  // B may have been written by the caller's previous kernel
+  CU(launch_gemm_ref_rows(g, sms, (cudaStream_t)st, 0, nullptr, status));  // B may have been written by the caller's previous kernel
   return QIE_OK;
 }
 int qie_qknorm(qie_bf16* x, const qie_bf16* w, int head_dim, int n_tok, int row_dim, int n_heads, qie_stream st) {
@@ -214,6 +259,7 @@ static int scratch(void** p, size_t* cap, size_t need) {
 int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st) {
   if (M < 1 || N < 64 || (N % 8) || K < 1) return fail(QIE_EINVAL, "matmul_fast: need M>=1, N>=64, N%%8==0");
   if (!aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul_fast: A and B must start on a 16-byte boundary");
+  OP_STATUS(status);
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -230,6 +276,7 @@ int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, in
   t.out = (bf16*)C;
   t.ld_out = K;
   t.w_static = 0;  // B may have been written by the caller's previous kernel
+  t.status = status;
   CU(launch_gemm_tcgen05(t, sms, (cudaStream_t)st, nullptr));
   return QIE_OK;
 }
@@ -283,6 +330,7 @@ int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16*
     return fail(QIE_EINVAL, "attention_prefill_fast: need n_q %% n_kv == 0 and head_dim 64 or 128");
   if (n_tok > 0 && (!aligned(16, {kv->pool, Q}) || !aligned(4, {out})))
     return fail(QIE_EINVAL, "attention_prefill_fast: the pool and Q must start on a 16-byte, out on a 4-byte boundary");
+  OP_STATUS(status);
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -294,6 +342,7 @@ int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16*
   a.n_q = n_q_heads;
   a.layer = layer;
   a.n_splits = 1;
+  a.status = status;
   a.max_kv_len = max_pages * kv->page_size;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)kv->head_dim);
   a.kv = geom_of(kv);
@@ -307,6 +356,7 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_prefill_tc: bad layer");
   if (n_q_heads % kv->n_kv_heads || kv->head_dim != 128) return fail(QIE_EINVAL, "attention_prefill_tc: head_dim must be 128");
   if (n_tok > 0 && !aligned(16, {kv->pool, Q, out})) return fail(QIE_EINVAL, "attention_prefill_tc: the pool, Q and out must start on a 16-byte boundary");
+  OP_STATUS(status);
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -318,10 +368,23 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
   a.n_q = n_q_heads;
   a.layer = layer;
   a.n_splits = 1;
+  a.status = status;
   a.max_kv_len = max_pages * kv->page_size;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)kv->head_dim);
   a.kv = geom_of(kv);
   CU(launch_attention_prefill_tc(a, variant, (cudaStream_t)st));
+  return QIE_OK;
+}
+
+int qie_kernel_status(void) { return take_status(g_op_status.load(std::memory_order_acquire)) ? wait_failed("an earlier operator call") : QIE_OK; }
+int qie_wait_selftest(qie_engine* e, qie_stream st) {
+  if (e) {
+    CU(cudaSetDevice(e->opts.device));
+    CU(launch_wait_selftest(e->wait_status, e->stream));
+    return engine_sync(e);
+  }
+  OP_STATUS(status);
+  CU(launch_wait_selftest(status, (cudaStream_t)st));
   return QIE_OK;
 }
 
@@ -421,6 +484,7 @@ static void engine_free(qie_engine* e) {
   if (e->block_table_h) cudaFreeHost(e->block_table_h);
   if (e->stage_h) cudaFreeHost(e->stage_h);
   if (e->sampled_h) cudaFreeHost(e->sampled_h);
+  if (e->wait_status) cudaFreeHost(e->wait_status);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
 }
@@ -669,7 +733,9 @@ static int engine_begin(const qie_engine_opts* opts, qie_engine** out_e) {
   e->opts = o;
   cudaError_t r = cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, o.device);
   if (r == cudaSuccess) r = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
+  if (r == cudaSuccess) r = alloc_status_word(&e->wait_status);
   if (r != cudaSuccess) {
+    if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
     return cuda_fail(r, "engine init");
   }
@@ -1040,7 +1106,7 @@ int qie_prefill(qie_engine* e, int seq, const int32_t* h_ids, int n, int32_t* h_
     int m = std::min(R, n - c0);
     bool last = c0 + m == n;
     int* st = e->stage_h;
-    CU(cudaStreamSynchronize(e->stream));  // staging buffer reuse
+    ENGINE_SYNC(e);  // staging buffer reuse
     for (int i = 0; i < m; ++i) {
       st[i] = h_ids[c0 + i];
       st[R + i] = s.len + c0 + i;
@@ -1055,7 +1121,7 @@ int qie_prefill(qie_engine* e, int seq, const int32_t* h_ids, int n, int32_t* h_
     CU(forward_rows(e, m, s.len + c0 + m, m - 1, last ? 1 : 0, e->temp_prefill, false));
   }
   CU(cudaMemcpyAsync(e->sampled_h, e->sampled_d, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   *h_token = e->sampled_h[0];
   s.len += n;
   s.step += 1;  // iengine.cu:419
@@ -1128,7 +1194,7 @@ static int decode_prepare(qie_engine* e, const int* h_seqs, int n, int* max_kv_l
 static int decode_stage_inputs(qie_engine* e, const int* h_seqs, const int32_t* h_tokens_in, int n) {
   const int R = e->opts.max_batch_tokens;
   int* st = e->stage_h;
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   for (int i = 0; i < n; ++i) {
     if (h_tokens_in[i] < 0 || h_tokens_in[i] >= e->cfg.vocab) return fail(QIE_EINVAL, "decode: token id %d out of range", h_tokens_in[i]);
     const Sequence& s = e->seqs[h_seqs[i]];
@@ -1155,7 +1221,7 @@ int qie_decode_step(qie_engine* e, const int* h_seqs, const int32_t* h_tokens_in
   rc = decode_launch(e, n, mk);
   if (rc) return rc;
   CU(cudaMemcpyAsync(e->sampled_h, e->sampled_d, n * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   for (int i = 0; i < n; ++i) {
     h_tokens_out[i] = e->sampled_h[i];
     e->seqs[h_seqs[i]].len += 1;
@@ -1169,7 +1235,7 @@ int qie_decode_run(qie_engine* e, const int* h_seqs, const int32_t* h_tokens_in,
   if (!h_tokens_in || !h_tokens_out || steps <= 0) return fail(QIE_EINVAL, "decode_run: bad arguments");
   if (!e) return fail(QIE_EINVAL, "null engine");
   if ((size_t)n * steps > e->sampled_h_cap) {
-    CU(cudaStreamSynchronize(e->stream));
+    ENGINE_SYNC(e);
     if (e->sampled_h) cudaFreeHost(e->sampled_h);
     e->sampled_h = nullptr;
     e->sampled_h_cap = (size_t)n * steps;
@@ -1192,7 +1258,7 @@ int qie_decode_run(qie_engine* e, const int* h_seqs, const int32_t* h_tokens_in,
       e->seqs[h_seqs[i]].step += 1;
     }
   }
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   memcpy(h_tokens_out, e->sampled_h, (size_t)n * steps * sizeof(int));
   return QIE_OK;
 }
@@ -1213,7 +1279,7 @@ int qie_decode_step_device(qie_engine* e, const int* h_seqs, int n) {
 
 int qie_sync(qie_engine* e) {
   if (!e) return fail(QIE_EINVAL, "null engine");
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   return QIE_OK;
 }
 
@@ -1230,7 +1296,7 @@ long qie_capture_read(qie_engine* e, const char* tag, int layer, qie_bf16* h_out
   auto it = e->cap.find(key);
   if (it == e->cap.end() || !it->second.d) return fail(QIE_EINVAL, "no capture for %s", key.c_str());
   size_t n = std::min(max_elems, it->second.elems);
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   CU(cudaMemcpy(h_out, it->second.d, n * sizeof(bf16), cudaMemcpyDeviceToHost));
   return (long)it->second.elems;
 }
@@ -1352,7 +1418,7 @@ int qie_seq_fill_synthetic(qie_engine* e, int seq, int n_pos, uint64_t seed) {
   if (rc) CU(push_block_row(e, seq));
   CU(launch_kv_fill(e->kv, e->block_table_d + (size_t)seq * e->max_pages_per_seq, s.len, n_pos,
                     seed + 0x51ull * (uint64_t)seq, e->stream));
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   s.len += n_pos;
   if (s.step == 0) s.step = 1;
   return QIE_OK;
@@ -1374,7 +1440,7 @@ int qie_engine_set_int(qie_engine* e, const char* key, long value) {
   else if (k == "inject_x") e->inject_x = value != 0;
   else return fail(QIE_EINVAL, "unknown option %s", key);
   // captured graphs bake these choices in
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   for (auto& kvp : e->graphs)
     if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
   e->graphs.clear();
@@ -1391,7 +1457,7 @@ long qie_mega_prof_read(qie_engine* e, uint64_t* h_out, size_t max_values) {
   if (!e->mega_prof_d) return fail(QIE_ESTATE, "persistent decode kernel not available for this checkpoint");
   // layout: [16L+8] globaltimer ns, then [16L+8] SM clock counter values of the same points
   size_t n = std::min<size_t>(max_values, (size_t)2 * (16 * e->cfg.layers + 8) + 16);
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   CU(cudaMemcpy(h_out, e->mega_prof_d, n * sizeof(uint64_t), cudaMemcpyDeviceToHost));
   return (long)n;
 }
@@ -1411,7 +1477,7 @@ long qie_engine_read_activation(qie_engine* e, const char* name, void* h_out, si
     else if (k == "sampled") p = e->sampled_d, nb = R * sizeof(int);
     if (!p) return fail(QIE_EINVAL, "unknown activation %s", name);
     nb = std::min(nb, max_bytes);
-    CU(cudaStreamSynchronize(e->stream));
+    ENGINE_SYNC(e);
     CU(cudaMemcpy(h_out, p, nb, cudaMemcpyDeviceToHost));
     return (long)nb;
   }
@@ -1426,7 +1492,7 @@ long qie_engine_read_activation(qie_engine* e, const char* name, void* h_out, si
   else if (k == "kv") src = e->kv.pool, bytes = (size_t)e->kv.n_pages * e->kv.page_stride() * 2;
   else return fail(QIE_EINVAL, "unknown activation %s", name);
   bytes = std::min(bytes, max_bytes);
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   CU(cudaMemcpy(h_out, src, bytes, cudaMemcpyDeviceToHost));
   return (long)bytes;
 }
@@ -1437,7 +1503,7 @@ long qie_engine_write_activation(qie_engine* e, const char* name, const void* h_
   const size_t cap = (size_t)e->opts.max_batch_tokens * e->cfg.hidden * 2;
   if (bytes > cap) return fail(QIE_EINVAL, "write_activation: %zu bytes > %zu", bytes, cap);
   CU(cudaSetDevice(e->opts.device));
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   CU(cudaMemcpy(e->x, h_in, bytes, cudaMemcpyHostToDevice));
   return (long)bytes;
 }
@@ -1466,6 +1532,7 @@ int qie_decode_step_profile(qie_engine* e, const int* h_seqs, const int32_t* h_t
   cudaError_t fe = forward_rows(e, n, ((mk + 127) / 128) * 128, 0, n, e->temp_decode, true);
   e->prof_on = false;
   cudaError_t se = cudaStreamSynchronize(e->stream);
+  const bool gave_up = take_status(e->wait_status);
   for (int i = 0; i < n_kinds; ++i) {
     ms_by_kind[i] = 0.f;
     launches_by_kind[i] = 0;
@@ -1482,6 +1549,7 @@ int qie_decode_step_profile(qie_engine* e, const int* h_seqs, const int32_t* h_t
   e->prof.clear();
   if (fe != cudaSuccess) return cuda_fail(fe, "forward (profile)");
   if (se != cudaSuccess) return cuda_fail(se, "sync (profile)");
+  if (gave_up) return wait_failed("this engine");
   for (int i = 0; i < n; ++i) {
     e->seqs[h_seqs[i]].len += 1;
     e->seqs[h_seqs[i]].step += 1;
@@ -1600,7 +1668,7 @@ int qie_forward_batch(qie_engine* e, int n_entries, const int* h_seqs, const int
   long row0 = 0;  // index of the forward's first row in the batch's token list
   while (row0 < total) {
     const int n = (int)std::min<long>(R, total - row0);
-    CU(cudaStreamSynchronize(e->stream));  // staging buffers are reused
+    ENGINE_SYNC(e);  // staging buffers are reused
     int* stg = e->stage_h;
     seg_start.clear(), seg_slot.clear(), out_rows.clear();
     int r = 0, max_kv = 0;
@@ -1637,7 +1705,7 @@ int qie_forward_batch(qie_engine* e, int n_entries, const int* h_seqs, const int
     if (n_out && h_logits)
       CU(cudaMemcpyAsync(h_logits + (size_t)want0 * e->cfg.vocab, m->logits, (size_t)n_out * e->cfg.vocab * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
     if (n_out && h_sampled) CU(cudaMemcpyAsync(h_sampled + want0, e->sampled_d, n_out * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    CU(cudaStreamSynchronize(e->stream));  // seg_start / out_rows live on this stack frame's vectors
+    ENGINE_SYNC(e);  // seg_start / out_rows live on this stack frame's vectors
     row0 += n;
   }
   return QIE_OK;
@@ -1648,7 +1716,7 @@ int qie_forward_batch(qie_engine* e, int n_entries, const int* h_seqs, const int
 // (they run eagerly, an event pair around every launch), end sums the classes (names: qie_kernel_kind_name).
 int qie_profile_begin(qie_engine* e) {
   if (!e) return fail(QIE_EINVAL, "null engine");
-  CU(cudaStreamSynchronize(e->stream));
+  ENGINE_SYNC(e);
   for (auto& r : e->prof) {
     cudaEventDestroy(r.a);
     cudaEventDestroy(r.b);
@@ -1662,6 +1730,7 @@ int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int
   if (!e || !ms_by_kind || !launches_by_kind || n_kinds < KK_COUNT) return fail(QIE_EINVAL, "profile_end: need %d kinds", (int)KK_COUNT);
   e->prof_on = false;
   cudaError_t se = cudaStreamSynchronize(e->stream);
+  const bool gave_up = take_status(e->wait_status);
   for (int i = 0; i < n_kinds; ++i) ms_by_kind[i] = 0.f, launches_by_kind[i] = 0;
   for (auto& r : e->prof) {
     float ms = 0.f;
@@ -1671,6 +1740,7 @@ int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int
   }
   e->prof.clear();
   if (se != cudaSuccess) return cuda_fail(se, "sync (profile)");
+  if (gave_up) return wait_failed("this engine");
   return QIE_OK;
 }
 

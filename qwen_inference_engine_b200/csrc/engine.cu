@@ -82,7 +82,7 @@ static void capture_copy(qie_engine* e, const char* tag, int layer, const bf16* 
 static cudaError_t gemm_rows(qie_engine* e, int kind, GemmArgs g, int n_rows) {
   g.M = n_rows;
   int nl = 0;
-  QIE_TRY(kind, launch_gemm_ref_rows(g, e->num_sms, e->stream, 1, &nl));
+  QIE_TRY(kind, launch_gemm_ref_rows(g, e->num_sms, e->stream, 1, &nl, e->wait_status));
   e->launches += nl - 1;  // QIE_TRY counts one
   return cudaSuccess;
 }
@@ -103,6 +103,7 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
   t.out = out;
   t.ld_out = ld_out;
   t.w_static = 1;
+  t.status = e->wait_status;
   int nl = 0;
   qie_engine::ProfRec pr{kind, nullptr, nullptr};
   if (e->prof_on) {
@@ -234,6 +235,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.layer = l;
       a.n_splits = 1;
       a.max_kv_len = max_kv_len;
+      a.status = e->wait_status;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.kv = e->kv;
       // head_dim 128 and at least one full 128-row query tile: tcgen05 / TMEM kernel (QIE_ATTN_TC=0 keeps mma.sync)

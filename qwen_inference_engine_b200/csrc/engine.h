@@ -60,6 +60,7 @@ struct qie_engine {
   qie_engine_opts opts{};
   int num_sms = 0;
   cudaStream_t stream = nullptr;
+  int* wait_status = nullptr;  // mapped host word: a kernel of this engine gave up a wait (capi.cu: engine_sync)
 
   // weights: ONE device blob, tensors addressed as blob + begin (helpers.cuh:18-29)
   qie::Checkpoint ck;

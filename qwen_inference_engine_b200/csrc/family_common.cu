@@ -230,6 +230,7 @@ cudaError_t TcProjector::gemm_bf16(qie_engine* e, const bf16* A, const bf16* W, 
   t.out = C;
   t.ld_out = N;
   t.w_static = 0;  // the operand comes from the kernel in front
+  t.status = e->wait_status;
   int nl = 0;
   cudaError_t r = launch_gemm_tcgen05(t, e->num_sms, st, &nl);
   if (r != cudaSuccess) return r;

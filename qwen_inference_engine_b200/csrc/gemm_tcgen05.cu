@@ -32,6 +32,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"
+#include "tc_ptx.cuh"
 
 namespace qie {
 
@@ -42,44 +43,9 @@ struct TcCfg {
   static constexpr int STAGES = BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : BN <= 128 ? 7 : 4;  // what 227 KiB hold (4 x 48 KiB at BN=256)
 };
 
-// ------------------------------------------------------------------ PTX wrappers
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
+// ------------------------------------------------------------------ PTX wrappers (tc_ptx.cuh has the rest)
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Waits for the phase of this parity.  After the limit (about a second) it sets *dead, and from then on no wait of the CTA waits: the
-// producers stop, the epilogue stores values that are not numbers, the CTA lets copies in flight land and returns.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
-  for (int i = 0; i < 4000000; ++i) {
-    uint32_t done = 0;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if ((i & 63) == 63 && *dead) return false;
-  }
-  *dead = 1;
-  return false;
-}
-__device__ __forceinline__ void dead_drain(const volatile int* dead) {
-  if (*dead)
-    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-}
-// one lane of the converged warp; under a branch on it the compiler emits tcgen05 and TMA instructions once (under a branch on the
-// lane number each of them goes through code for any set of active lanes)
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
@@ -96,46 +62,13 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+  tmem_ld16_tc(taddr, r);
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void mark_bad(uint32_t (&r)[16]) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) r[j] = 0x7fc00000u;
-}
-
-// K-major, SWIZZLE_128B shared-memory matrix descriptor (cute::UMMA::SmemDescriptor):
-// start>>4 [0,14) | LBO>>4 [16,30) (=1, unused for swizzled K-major) | SBO>>4 [32,46) =
-// 1024 B (8 rows x 128 B) | version=1 [46,48) | layout SWIZZLE_128B=2 [61,64)
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// kind::f16 instruction descriptor: D=F32 (bits 4-5 = 1), A=B=BF16 (bits 7-9, 10-12 = 1),
-// A,B K-major (bits 15,16 = 0), N>>3 at [17,23), M>>4 at [24,29)
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ float silu_ref_f(float x) {
@@ -163,6 +96,7 @@ struct TcArgs {
   int epi, dual, w_static;
   int exact;       // reference-order numerics: SiLU as the reference computes it (expf, IEEE division)
   int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
+  int* status;     // host word that a wait which ran out sets, or null
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
   TcSeg seg[3];
 };
@@ -211,10 +145,10 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     if (g.dual) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+      mbar_init_tc(full_bar(s), 1);
+      mbar_init_tc(empty_bar(s), 1);
     }
-    mbar_init(tmem_full_bar, 1);
+    mbar_init_tc(tmem_full_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(slot, TMEM_COLS);
@@ -239,7 +173,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   // whatever the tile's width (76 steps at K = 4864: 22.8 us on an idle chip); now 0.18 us (15.4 us).  The products of a step
   // themselves take 0.025 us at 16 tokens, 0.27 us at 256.
   if (warp == 0) {
-    if (elect_one()) {
+    if (elect_tc()) {
       // Weights never depend on the previous kernel: start streaming them BEFORE waiting for
       // it (programmatic dependent launch), so HBM stays busy across the kernel boundary.
       const int pre = g.w_static ? min(nkb, TC_STAGES) : 0;
@@ -253,7 +187,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       int s = pre == TC_STAGES ? 0 : pre;
       uint32_t ph = pre == TC_STAGES ? 0 : 1;  // the first pass over the ring waits for nothing
       for (int i = pre; i < nkb; ++i) {
-        if (!mbar_wait(empty_bar(s), ph, dead)) break;
+        if (!mbar_wait_tc(empty_bar(s), ph, dead)) break;
         mbar_expect_tx(full_bar(s), STAGE_BYTES);
         load_w(i, s);
         tma_load_2d(smem0 + s * STAGE_BYTES + A_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, tok_base);
@@ -262,24 +196,24 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
     __syncwarp();
   } else if (warp == 1) {
-    constexpr uint32_t idesc = make_idesc(BM, BN);
-    const uint64_t ad0 = make_desc(smem0), bd0 = make_desc(smem0 + A_BYTES);
+    const uint32_t idesc = idesc_tc(BM, BN, false);
+    const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0;
     uint32_t ph = 0;
     for (int i = 0; i < nkb; ++i) {
-      mbar_wait(full_bar(s), ph, dead);
+      mbar_wait_tc(full_bar(s), ph, dead);
       tc_fence_after();
       const uint64_t step = (uint64_t)(s * (STAGE_BYTES >> 4));
-      if (elect_one()) {
+      if (elect_tc()) {
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
-          umma_bf16(tmem_base, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (i | k) != 0);
-        umma_commit(empty_bar(s));  // frees the smem stage once the MMAs have read it
+          umma_tc(tmem_base, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (i | k) != 0);
+        umma_commit_tc(empty_bar(s));  // frees the smem stage once the MMAs have read it
       }
       __syncwarp();
       if (++s == TC_STAGES) s = 0, ph ^= 1;
     }
-    if (elect_one()) umma_commit(tmem_full_bar);  // accumulator complete
+    if (elect_tc()) umma_commit_tc(tmem_full_bar);  // accumulator complete
     __syncwarp();
   }
 
@@ -297,7 +231,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       const int qd = warp & 3;
       pdl_wait();  // `out` may still be read (residual) by the previous kernel
       if (nkb > 0) {
-        mbar_wait(tmem_full_bar, 0, dead);
+        mbar_wait_tc(tmem_full_bar, 0, dead);
         tc_fence_after();
       }
       const bool bad = *dead;
@@ -383,7 +317,8 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
     __syncthreads();
     if (warp == 1) {
-      dead_drain(dead);
+      drain_tc(dead);
+    if (lane == 0) report_tc(dead, g.status);
       tc_fence_after();
       tmem_dealloc(tmem_base, TMEM_COLS);
     }
@@ -403,7 +338,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   if (epi_warp) {
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
     if (nkb > 0) {
-      mbar_wait(tmem_full_bar, 0, dead);
+      mbar_wait_tc(tmem_full_bar, 0, dead);
       tc_fence_after();
     }
     const bool bad = *dead;
@@ -525,7 +460,8 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   }
   __syncthreads();
   if (warp == 1) {
-    dead_drain(dead);
+    drain_tc(dead);
+    if (lane == 0) report_tc(dead, g.status);
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
@@ -579,12 +515,12 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w2) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     for (int s = 0; s < stages; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+      mbar_init_tc(full_bar(s), 1);
+      mbar_init_tc(empty_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(tfull_bar(b), 1);
-      mbar_init(tempty_bar(b), 1);
+      mbar_init_tc(tfull_bar(b), 1);
+      mbar_init_tc(tempty_bar(b), 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -605,7 +541,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   };
 
   if (warp == 0) {
-    if (elect_one()) {
+    if (elect_tc()) {
       int s = 0;
       uint32_t ph = 1;
       bool go = true;
@@ -636,7 +572,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
           if (pre > 0) {  // (the first stages: nothing to wait for)
             --pre;
           } else {
-            if (!(go = mbar_wait(empty_bar(s), ph, dead))) break;
+            if (!(go = mbar_wait_tc(empty_bar(s), ph, dead))) break;
             mbar_expect_tx(full_bar(s), stage_bytes);
             load_w(kb, si, row0);
           }
@@ -647,28 +583,28 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     }
     __syncwarp();
   } else if (warp == 1) {
-    const uint32_t idesc = make_idesc(BM, bn);
-    const uint64_t ad0 = make_desc(smem0), bd0 = make_desc(smem0 + A_BYTES);
+    const uint32_t idesc = idesc_tc(BM, bn, false);
+    const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0, j = 0;
     uint32_t ph = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
       const int buf = j & 1;
-      mbar_wait(tempty_bar(buf), (((uint32_t)j >> 1) & 1) ^ 1, dead);  // epilogue has drained this accumulator
+      mbar_wait_tc(tempty_bar(buf), (((uint32_t)j >> 1) & 1) ^ 1, dead);  // epilogue has drained this accumulator
       tc_fence_after();
       const uint32_t acc = tmem_base + (uint32_t)buf * PBN;
       for (int kb = 0; kb < nkb; ++kb) {
-        mbar_wait(full_bar(s), ph, dead);
+        mbar_wait_tc(full_bar(s), ph, dead);
         tc_fence_after();
         const uint64_t step = (uint64_t)(s * (stage_bytes >> 4));
-        if (elect_one()) {
+        if (elect_tc()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_bf16(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
-          umma_commit(empty_bar(s));
+          for (int k = 0; k < BK / 16; ++k) umma_tc(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
+          umma_commit_tc(empty_bar(s));
         }
         __syncwarp();
         if (++s == stages) s = 0, ph ^= 1;
       }
-      if (elect_one()) umma_commit(tfull_bar(buf));
+      if (elect_tc()) umma_commit_tc(tfull_bar(buf));
       __syncwarp();
     }
   } else {
@@ -716,7 +652,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
             x[u] = *reinterpret_cast<const uint4*>(out + (size_t)(tok_base + h0 + (c >> 4)) * ld + w_row);
         }
         if (h0 == 0) {
-          mbar_wait(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
+          mbar_wait_tc(tfull_bar(buf), ((uint32_t)j >> 1) & 1, dead);
           tc_fence_after();
           bad = *dead;
         }
@@ -738,7 +674,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         asm volatile("bar.sync 2, 256;" ::: "memory");
-        if (h0 + P_STEP >= bn && tq == 0) mbar_arrive_local(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
+        if (h0 + P_STEP >= bn && tq == 0) mbar_arrive_tc(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
         if (bulk) {
           if (copier < n_tok) {
             bf16* dst = out + (size_t)(tok_base + h0 + copier) * ld + row0;
@@ -787,7 +723,8 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   }
   __syncthreads();
   if (warp == 1) {
-    dead_drain(dead);
+    drain_tc(dead);
+    if (lane == 0) report_tc(dead, g.status);
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
@@ -965,6 +902,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.dual = t.epi == EPI_SILU_MUL;
   g.w_static = t.w_static;
   g.exact = t.exact;
+  g.status = t.status;
   int tiles = 0, cols = 0;
   if (g.dual) {
     // segments = (gate, up) with equal row counts; the weight maps must have 64-row boxes
@@ -1034,7 +972,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
 // 12.6 (the mma.sync kernel runs 64 rows a launch and reads the weights again for each), at 16 rows 10.5 -> 4.7; 4864 x 896 at 400 rows
 // 737 -> 16.5; 896 x 151936 at 1 row 79 -> 47.  The mma.sync kernel keeps what TMA or the tile cannot express: K below one k-block, fp32 outputs (the partial sums
 // of tensor parallelism), column slices of a wider matrix.  Operands off a 16-byte boundary are refused: both kernels read 16 bytes at a time.
-cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches) {
+cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches, int* status) {
   if (launches) *launches = 0;
   bool tc = a.M >= 1 && a.K >= BK && a.K % 8 == 0 && a.lda == a.K && a.epi != EPI_STORE_F32 && a.nseg <= 3 &&
             (reinterpret_cast<uintptr_t>(a.A) & 15) == 0;
@@ -1048,6 +986,7 @@ cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st
     t.K = a.K;
     t.epi = a.epi;
     t.exact = 1;
+    t.status = status;
     t.w_static = w_static;
     t.out = a.seg[0].out;
     t.ld_out = a.seg[0].ld_out;

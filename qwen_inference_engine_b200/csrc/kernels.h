@@ -131,7 +131,10 @@ struct FastAttnArgs {
   float* ws_o;       // [n_splits][n_tok][n_q][hd]
   float* ws_ml;      // [n_splits][n_tok][n_q][2]
   KvGeom kv;
+  int* status;       // mapped host memory: set to 1 by a kernel of which a wait ran out (its results are not numbers); null: not reported
 };
+// a wait that nothing ends, through the same limit and report
+cudaError_t launch_wait_selftest(int* status, cudaStream_t st);
 cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st);
 constexpr int FD_CLUSTER = 8;  // splits that need no workspace
 int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms);
@@ -167,10 +170,11 @@ struct TcGemm {
   int lds[3];
   int exact;     // reference-order numerics: k ascending in one accumulator (no split over K), SiLU as the reference computes it
   int w_static;  // weights are not produced by a preceding kernel: prefetch them before the PDL wait
+  int* status;   // see FastAttnArgs
 };
 cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, int* launches);
 // reference-order GEMM of any number of rows (tcgen05, or launch_gemm_ref_order 64 rows at a time); *launches: kernels launched
-cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches);
+cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches, int* status);
 
 cudaError_t launch_rmsnorm_fast(const bf16* x, const bf16* w, bf16* y, size_t hidden, size_t n_tok, size_t x_stride,
                                 cudaStream_t st, float eps = 1e-04f);

@@ -1,5 +1,5 @@
 // tc_ptx.cuh -- tcgen05, TMEM and mbarrier instructions with waits that have a limit, for kernels whose CTA finishes without waiting
-// once a wait ran out (attn_gqa_tc.cu, gemm_grouped_tc.cu).
+// once a wait ran out.
 #pragma once
 #include "common.cuh"
 
@@ -7,9 +7,12 @@ namespace qie {
 
 __device__ __forceinline__ void mbar_init_tc(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
 __device__ __forceinline__ void mbar_arrive_tc(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// waits for the phase of this parity; after the limit it sets *dead, and from then on no wait of the CTA waits
-__device__ __forceinline__ void mbar_wait_tc(uint32_t bar, uint32_t parity, volatile int* dead) {
-  for (int i = 0; i < 2000000; ++i) {
+// Waits for the phase of this parity.  After about a second it sets *dead, and from then on no wait of the CTA waits: its kernel stores values
+// that are not numbers, lets copies in flight land (drain_tc), reports (report_tc) and returns.  The clock is read only where a wait is long.
+constexpr long long WAIT_CYCLES_TC = 2000000000ll;
+__device__ __forceinline__ bool mbar_wait_tc(uint32_t bar, uint32_t parity, volatile int* dead) {
+  long long t0 = 0;
+  for (int i = 0;; ++i) {
     uint32_t done = 0;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -18,10 +21,33 @@ __device__ __forceinline__ void mbar_wait_tc(uint32_t bar, uint32_t parity, vola
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
-    if (done) return;
-    if ((i & 63) == 63 && *dead) return;
+    if (done) return true;
+    if ((i & 31) == 31) {
+      if (*dead) return false;
+      if (i == 31) t0 = clock64();
+      else if (clock64() - t0 > WAIT_CYCLES_TC) break;
+    }
   }
   *dead = 1;
+  return false;
+}
+__device__ __forceinline__ void drain_tc(const volatile int* dead) {
+  if (*dead)
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+}
+// one thread, behind the CTA's last wait: status is a word that the host reads (mapped memory), or null
+__device__ __forceinline__ void report_tc(const volatile int* dead, int* status) {
+  if (*dead && status) {
+    *reinterpret_cast<volatile int*>(status) = 1;
+    __threadfence_system();
+  }
+}
+// one lane of the converged warp; under a branch on it the compiler emits tcgen05 and TMA instructions once (under a branch on the
+// lane number each of them goes through code for any set of active lanes)
+__device__ __forceinline__ bool elect_tc() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void umma_tc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile(
