@@ -346,8 +346,10 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
 #pragma unroll
       for (int p = 0; p < 8; ++p)
         if (p < n_parts) {
-          const float f = m[p] > -INFINITY ? ex2_tc(m[p] - top) : 0.f;  // (a row sees nothing of a part behind its position)
-          if (f > 0.f) {
+          // A row sees nothing of a part behind its position.  A sum that is no number (a wait ran out, or no score of the part is one) counts
+          // whatever the maximum beside it.
+          const float f = l[p] != l[p] ? l[p] : m[p] > -INFINITY ? ex2_tc(m[p] - top) : 0.f;
+          if (f != 0.f) {
             sum.x += o[p].x * f, sum.y += o[p].y * f, sum.z += o[p].z * f, sum.w += o[p].w * f;
             total += l[p] * f;
           }

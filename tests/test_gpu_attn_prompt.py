@@ -86,3 +86,23 @@ def test_same_bits_every_time(layers, entry, nq, nkv, hd, first, n):
             torch.cuda.synchronize()
     torch.cuda.synchronize()
     assert all(torch.equal(o.view(torch.int16), outs[0].view(torch.int16)) for o in outs[1:])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("lo,hi", [(1000, 1500), (0, 200), (700, 704)])
+def test_keys_that_are_not_numbers(layers, hd, lo, hi):
+    """parts of the cluster that see nothing else: the row is not a number, as in the reference's order, and does not go on without them"""
+    g = torch.Generator("cuda").manual_seed(hd)
+    nq, nkv, total, n = 4, 2, 1516, 16
+    pool = layers.KvPool((total + 15) // 16, 16, 1, nkv, hd, max_seqs=1)
+    k, v = (torch.randn(total, nkv * hd, generator=g, device="cuda").bfloat16() for _ in "kv")
+    k[lo:hi, :hd] = float("nan")  # the first kv head
+    at = torch.arange(total, dtype=torch.int32, device="cuda")
+    pool.store(0, k, v, at, torch.zeros_like(at))
+    q = torch.randn(n, nq * hd, generator=g, device="cuda").bfloat16()
+    pos, slot = at[total - n:].contiguous(), torch.zeros(n, dtype=torch.int32, device="cuda")
+    want, got = torch.zeros_like(q), torch.zeros_like(q)
+    layers.launch_attn(q, want, pool, 0, pos, slot, nq)
+    layers.launch_attn_prefill_fast(q, got, pool, 0, pos, slot, nq)
+    torch.cuda.synchronize()
+    assert torch.equal(got.isnan(), want.isnan()) and got.isnan().sum() == n * 2 * hd
