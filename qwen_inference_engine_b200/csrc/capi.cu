@@ -1484,6 +1484,7 @@ long qie_engine_read_activation(qie_engine* e, const char* name, void* h_out, si
   const void* src = nullptr;
   size_t bytes = 0;
   if (k == "x") src = e->x, bytes = R * c.hidden * 2;
+  else if (k == "xn") src = e->xn, bytes = R * c.hidden * 2;
   else if (k == "qkv") src = e->qkv, bytes = R * (Dq + 2 * Dkv) * 2;
   else if (k == "att") src = e->att, bytes = R * Dq * 2;
   else if (k == "h") src = e->h, bytes = R * c.inter * 2;

@@ -76,7 +76,7 @@ __device__ __forceinline__ float silu_ref_f(float x) {
   return __fmul_rn(x, sg);
 }
 
-// tolerance-mode SiLU for the prefill epilogue: ex2.approx + rcp.approx (relative error ~1e-6, far inside the bf16 rounding
+// tolerance-mode SiLU for the epilogue of prompts (more than 128 rows): ex2.approx + rcp.approx (relative error ~1e-6, far inside the bf16 rounding
 // that follows) instead of expf + an IEEE division (~35 instructions per element on the epilogue warps that pace the
 // K = 1536 gate/up tiles)
 __device__ __forceinline__ float silu_fast_f(float x) {
@@ -94,7 +94,7 @@ struct TcArgs {
   int M, K;
   int nseg, n_tiles, splits, kb_per_split, kb_total;
   int epi, dual, w_static;
-  int exact;       // reference-order numerics: SiLU as the reference computes it (expf, IEEE division)
+  int ref_silu;    // persistent kernel: SiLU as the reference computes it (expf, IEEE division); the others always do
   int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
   int* status;     // host word that a wait which ran out sets, or null
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
@@ -708,8 +708,8 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
             uint32_t o4[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float s0 = g.exact ? silu_ref_f(lo2f(gs[e])) : silu_fast_f(lo2f(gs[e]));
-              const float s1 = g.exact ? silu_ref_f(hi2f(gs[e])) : silu_fast_f(hi2f(gs[e]));
+              const float s0 = g.ref_silu ? silu_ref_f(lo2f(gs[e])) : silu_fast_f(lo2f(gs[e]));
+              const float s1 = g.ref_silu ? silu_ref_f(hi2f(gs[e])) : silu_fast_f(hi2f(gs[e]));
               const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(s0)));
               const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(s1)));
               o4[e] = pack2(f2bf(a0), f2bf(a1));
@@ -901,7 +901,9 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.epi = t.epi;
   g.dual = t.epi == EPI_SILU_MUL;
   g.w_static = t.w_static;
-  g.exact = t.exact;
+  // The short SiLU is for prompts, whose epilogue paces the tile at K = 1536.  Up to 128 rows no tile waits
+  // for it, and fast numerics keep the reference's.
+  g.ref_silu = t.exact || t.M <= 128;
   g.status = t.status;
   int tiles = 0, cols = 0;
   if (g.dual) {

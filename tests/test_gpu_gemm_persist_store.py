@@ -46,3 +46,29 @@ def test_residual_and_gate_up():
         e.close()
     assert got[0][0] == got[1][0]
     assert np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("rows", [9, 64, 128])
+def test_few_rows_keep_the_reference_silu(rows):
+    """gate/up of 7B widths (more tiles than SMs at any row count) in fast numerics: the sums are the reference order's, since nothing splits them, and
+    so are silu and the product, bit for bit"""
+    import ctypes as C
+    import qwen_inference_engine_b200 as q
+    from qwen_inference_engine_b200 import _lib
+    from qwen_inference_engine_b200 import layers as L
+    hidden, inter = 3584, 18944
+    cfg = q.make_config(dict(hidden=hidden, inter=inter, layers=1, n_q=28, n_kv=4, head_dim=128, vocab=4096), context=256)
+    e = q.Engine(synthetic=cfg, seed=5, context=256, max_seqs=1, max_batch_tokens=rows, max_pages=16, numerics="fast")
+    e.set_int("layer_count", 1)  # the layer alone: its operand stays in place
+    e.prefill(e.new_sequence(), prompt_ids(rows, 4096, seed=rows))
+    xn, h = (torch.from_numpy(e.read_activation(n, rows * w).view(np.int16)).cuda().view(torch.bfloat16) for n, w in (("xn", hidden), ("h", inter)))
+    gate, up = (torch.empty(rows, inter, dtype=torch.bfloat16, device="cuda") for _ in "gu")
+    torch.cuda.synchronize()
+    for name, out in (("gate", gate), ("up", up)):
+        _lib.check(_lib.lib().qie_matmul(C.c_void_p(xn.data_ptr()), C.c_void_p(e.weight_ptr("mlp.%s_proj.weight" % name, 0)[0]), C.c_void_p(out.data_ptr()), rows, hidden, inter,
+                                         torch.cuda.current_stream().cuda_stream))
+    L.launch_act(gate, gate.numel())
+    L.launch_elem(gate, up, gate, gate.numel())
+    torch.cuda.synchronize()
+    assert torch.equal(gate.view(torch.int16).view(rows, inter), h.view(torch.int16).view(rows, inter))
+    e.close()
