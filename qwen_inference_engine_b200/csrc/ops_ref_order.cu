@@ -765,8 +765,12 @@ __device__ __forceinline__ bool topk_valid(uint16_t b) {  // -inf and NaN are ne
   const uint16_t a = b & 0x7fffu;
   return !(a > 0x7f80u) && b != 0xff80u;
 }
-__device__ __noinline__ void topk_select_row(const bf16* __restrict__ logits, int* __restrict__ out, int rowi, size_t vocab, float temperature, int k,
-                                             uint64_t seed, uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
+__global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab,
+                                                                    float temperature, int k, uint64_t seed, uint64_t seed_stride,
+                                                                    const int* __restrict__ step_ptr, unsigned long long subsequence) {
+  pdl_wait();
+  pdl_trigger();
+  const int rowi = blockIdx.x;
   __shared__ unsigned hist[256];
   __shared__ unsigned long long sel[256];  // the selected keys, then sorted best first
   __shared__ float topk_vals[256];
@@ -888,19 +892,13 @@ __device__ __noinline__ void topk_select_row(const bf16* __restrict__ logits, in
   }
 }
 
-__global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab,
-                                                                    float temperature, int k, uint64_t seed, uint64_t seed_stride,
-                                                                    const int* __restrict__ step_ptr, unsigned long long subsequence) {
-  pdl_wait();
-  pdl_trigger();
-  topk_select_row(logits, out, blockIdx.x, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence);
-}
-
 // 1 < k <= TC_MOST: a cluster of 8 CTAs per row, each over an eighth of the row, 16 bytes a load.  The k-th largest of the threads' maxima is a
 // bound that at least k values of the slice reach; the values that reach it (about 1.1 k of them) are the slice's candidates.  The first
 // CTA gathers the candidates of all slices through distributed shared memory, finds the k-th value by bisection over its 16 bits,
 // ranks what is left by counting (all keys differ) and runs the reference's tail: quotients and exponentials by a thread each, the
-// two sums in the reference's order.  A slice with more candidates than fit (a row of equal logits) falls back to the radix select.
+// two sums in the reference's order.  Where ties (a row of equal logits) or fewer threads than k with a value (vocabularies of 4 to 8
+// thousand) leave more candidates than the lists hold, the k-th key itself is found by bisection over its 48 bits: in the slice by
+// counting passes over it, in the first CTA over what it gathered.
 // One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384; here 18.5 and 39.  The bound
 // is the latency of the steps, not memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 15.6 us, 29 here.
 constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;
@@ -908,7 +906,7 @@ template <int TC_THREADS>
 __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
                                uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
-  static_assert(TC_THREADS >= 256, "topk_select_row clears and sorts 256 entries, a thread each");
+  static_assert(TC_THREADS > TC_MOST && TC_CAP >= TC_MOST, "a thread for every exponential and one for the random number; k candidates fit");
   pdl_wait();
   pdl_trigger();
   __shared__ unsigned long long cand[TC_CAP];             // this slice's candidates
@@ -965,54 +963,69 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
       const int at = atomicAdd(&s_n, 1);
       if (at < TC_CAP) cand[at] = topk_key((uint16_t)b, i);
     });
+  __syncthreads();
+  // how many of the block's values: every thread's c summed up
+  auto block_sum = [&](int c) {
+    __syncthreads();
+    if (tid == 0) s_cnt = 0;
+    __syncthreads();
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((tid & 31) == 0 && c) atomicAdd(&s_cnt, c);
+    __syncthreads();
+    return s_cnt;
+  };
+  if (s_n > TC_CAP) {
+    unsigned long long thr = 0;
+#pragma unroll 1
+    for (int bit = 47; bit >= 0; --bit) {
+      const unsigned long long t = thr | (1ull << bit);
+      int c = 0;
+      if (mx >= bound) each([&](uint32_t o, uint32_t b, int i) { c += o >= bound && topk_key((uint16_t)b, i) >= t; });
+      if (block_sum(c) >= k) thr = t;
+    }
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    if (mx >= bound)
+      each([&](uint32_t o, uint32_t b, int i) {  // exactly k
+        const unsigned long long key = topk_key((uint16_t)b, i);
+        if (o >= bound && key >= thr) cand[atomicAdd(&s_n, 1)] = key;
+      });
+  }
   cluster_sync_all();
   if (slice == 0) {
     // ---- gather
     int n = 0;
-    bool over = false;
     for (int c = 0; c < TC_CTAS; ++c) {
       uint32_t an, ac;
       int cn;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(an) : "r"(smem_u32(&s_n)), "r"(c));
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ac) : "r"(smem_u32(cand)), "r"(c));
       asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(cn) : "r"(an) : "memory");
-      over = over || cn > TC_CAP;
-      for (int i = tid; i < min(cn, TC_CAP); i += TC_THREADS)
+      for (int i = tid; i < cn; i += TC_THREADS)
         asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(all[n + i]) : "r"(ac + 8u * (uint32_t)i) : "memory");
-      n += min(cn, TC_CAP);
+      n += cn;
     }
     __syncthreads();
     const int actual_k = min(k, n);
-    // ---- the actual_k-th value, by bisection over its 16 bits
-    uint32_t kth = 0;
-    if (!over && actual_k > 0) {
+    // ---- those that reach the actual_k-th value, by bisection over its 16 bits; the actual_k-th key where they are too many
+    unsigned long long kth = 0;
+    int m = n;  // keys that reach it
+    if (actual_k > 0) {
 #pragma unroll 1
-      for (int bit = 15; bit >= 0; --bit) {
-        const uint32_t t = kth | (1u << bit);
-        if (tid == 0) s_cnt = 0;
-        __syncthreads();
+      for (int bit = 47; bit >= 0 && (bit >= 32 || m > TC_CAP); --bit) {
+        const unsigned long long t = kth | (1ull << bit);
         int c = 0;
-        for (int i = tid; i < n; i += TC_THREADS) c += (uint32_t)(all[i] >> 32) >= t;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if ((tid & 31) == 0 && c) atomicAdd(&s_cnt, c);
-        __syncthreads();
-        if (s_cnt >= actual_k) kth = t;
-        __syncthreads();
+        for (int i = tid; i < n; i += TC_THREADS) c += all[i] >= t;
+        c = block_sum(c);
+        if (c >= actual_k) kth = t, m = c;
       }
-    }
-    if (tid == 0) s_tot = 0;
-    __syncthreads();
-    if (!over && actual_k > 0)
+      if (tid == 0) s_tot = 0;
+      __syncthreads();
       for (int i = tid; i < n; i += TC_THREADS)
-        if ((uint32_t)(all[i] >> 32) >= kth) {
-          const int at = atomicAdd(&s_tot, 1);
-          if (at < TC_CAP) best[at] = all[i];
-        }
+        if (all[i] >= kth) best[atomicAdd(&s_tot, 1)] = all[i];
+    }
     __syncthreads();
-    const int m = s_tot;
-    if (over || m > TC_CAP) {
-      topk_select_row(logits, out, rowi, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence);
-    } else if (actual_k == 0) {
+    if (actual_k == 0) {
       if (tid == 0) out[rowi] = -1;
     } else {
       // ---- rank by counting

@@ -34,7 +34,7 @@ def row(kind, vocab, rng):
 
 
 @pytest.mark.parametrize("kind", ["normal", "ties", "equal", "few", "one slice", "zeros"])
-@pytest.mark.parametrize("vocab,rows", [(151936, 3), (32001, 5), (1000, 2), (519, 9)])
+@pytest.mark.parametrize("vocab,rows", [(151936, 3), (32001, 5), (8200, 2), (6001, 20), (1000, 2), (519, 9)])
 @pytest.mark.parametrize("k", [1, 2, 50, 128])
 def test_rows_against_the_restatement(layers, oracle, vocab, rows, kind, k):
     rng = np.random.default_rng(vocab + k)
