@@ -861,6 +861,8 @@ struct TcTile {
 //    (1536 outputs at 4096 rows: 107 -> 86 with 176; a few per cent less on paper were none: 8960 outputs 82.7 with 256, 85.5 with
 //    224).  Below 160 tokens the loop, not the tensor core, sets a tile's time, so of those the narrowest wins, whose ring holds most
 //    k-blocks: 151936 x 896 for one row 79 -> 47.
+//    Outputs that 16-byte stores cannot reach (an odd number of columns) take one tile per CTA at any number of tiles, no wider than the rows
+//    (1 x 896 x 20001: 45 us with 256, 7.5 with 16).
 //  * Few tiles and a long K: a cluster of 2, 4 or 8 CTAs splits K (never in the reference's order).  Its reduction costs about
 //    1.1 us + (0.1, 0.055, 0.045) us x tokens, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
 //    clusters have to run at once (`most` clusters of a size fit; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
@@ -883,7 +885,10 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool m
       }
     return best;
   }
-  if (!vec) return best;  // outputs that 16-byte stores cannot reach: one tile per CTA
+  if (!vec) {  // outputs that 16-byte stores cannot reach: one tile per CTA, no wider than the rows
+    for (best.bn = 16; best.bn < 256 && best.bn < M;) best.bn *= 2;
+    return best;
+  }
   best.persist = true;
   auto waves = [&](int bn) { return (ctas(bn) + num_sms - 1) / num_sms * std::max(bn, 160); };
   long cost = waves(256) * 9 / 10;
