@@ -11,7 +11,8 @@
 //                is then no power of two and gets rounded.)
 //   warp 4     : the products.  warp 5: copies, TMA boxes of a page x 64 columns with the 128-byte swizzle into two stages of K and of V.
 //                (One warp for both was the bottleneck: a request costs it 50 cycles, 400 - 600 a tile.)
-// Tiles whose rows see at most `two_term` positions keep the weights as bf16 hi + lo pairs (two products), as attn_prefill_fast.cu does.
+// Query tiles whose first 64 rows see at most `two_term` positions keep the weights as bf16 hi + lo pairs (two products): every row has them for
+// which attn_prefill_fast.cu, with its tiles of 64 rows, does, and up to 64 rows more.
 // Short launches split a query tile's keys over a cluster (pick_parts), summed through distributed shared memory.
 // What bounds it: the chain of a tile, 1500 - 1600 cycles alone on an SM: exponentials 620 (512 are the unit's floor), maximum 190, scaling O
 // 140 - 220 and waiting for its product 140, waiting for S 250, TMEM reads and writes 140.  14 heads of 64, 3000 rows: 105 us with mma.sync,
@@ -90,7 +91,7 @@ __device__ __forceinline__ unsigned long long twice(float x) {
   return v;
 }
 template <int HD>
-__global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a, int two_term, int parts, const __grid_constant__ CUtensorMap kvm) {
+__global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a, int two_term, int parts_max, int alone, const __grid_constant__ CUtensorMap kvm) {
   using SM = PromptSmem<HD>;
   constexpr int NB = HD / 64;  // column blocks
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -106,10 +107,15 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
   int* s_pages = reinterpret_cast<int*>(sg + SM::PAGES);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // parts of a query tile are the CTAs of a cluster; then heads, longest query tiles first
-  const int part = blockIdx.x % parts, h = blockIdx.x / parts, qt = gridDim.y - 1 - blockIdx.y, G = a.n_q / a.kv.n_kv, kvh = h / G;
+  const int part = blockIdx.x % parts_max, h = blockIdx.x / parts_max, qt = gridDim.y - 1 - blockIdx.y, G = a.n_q / a.kv.n_kv, kvh = h / G;
   const int t0 = qt * TQ, n_rows = min(TQ, a.n_tok - t0), Dq = a.n_q * HD;
   const int* bt = a.block_table + (size_t)a.slot[t0] * a.max_pages;
   const int pos_first = a.pos[t0], kv_len = pos_first + n_rows, all_tiles = (kv_len + TK - 1) / TK, n_pages = (kv_len + 15) / 16;
+  // The host knows the block table's width and not the sequence's length: where sharing out the tiles that there are saves fewer than the sum over
+  // the cluster costs, its first CTA does them all and the others are done.
+  const bool split = parts_max > 1 && all_tiles - (all_tiles + parts_max - 1) / parts_max > alone;
+  if (!split && part > 0) return;
+  const int parts = split ? parts_max : 1;
   const int per = (all_tiles + parts - 1) / parts, first = min(all_tiles, part * per), n_tiles = min(all_tiles, first + per) - first;
   const bool two = pos_first + min(n_rows, 64) <= two_term;
   if (tid == 0) {
@@ -374,24 +380,27 @@ __global__ void __launch_bounds__(NTHR, 2) attn_prompt_tc_kernel(FastAttnArgs a,
 // at once and most have an SM to themselves.  Measured (us; 1, 2, 4, 8 parts): 128 rows behind 1500, 12 heads of 128: 29 24 19 14; 16 rows behind 800, 14 heads of 64: 15 12
 // 10 10; 1000 rows behind 1000, 12 heads of 128: 35 30 40 49; 2000 rows, 12 heads of 128: 36 41 53 85; 64 rows of 64: 5.3 8.5 7.8 7.1.
 template <int HD>
-int pick_parts(const FastAttnArgs& a) {
+int pick_parts(const FastAttnArgs& a, int* alone) {
   const float tile = HD == 64 ? 0.78f : 0.85f, shared = HD == 64 ? 1.25f : 1.45f;
   const float sum[4] = {0.f, HD == 64 ? 3.9f : 6.3f, HD == 64 ? 2.5f : 4.2f, HD == 64 ? 1.8f : 3.2f};
   const int tiles = (a.max_kv_len + TK - 1) / TK;
   const long ctas = (long)a.n_q * ((a.n_tok + TQ - 1) / TQ);
-  int best = 1;
+  int best = 0;
   float cost = 0.f;
   for (int i = 0; i < 4; ++i) {
     const int p = 1 << i;
     if (p > 1 && ctas * p > (HD == 64 ? 240 : 200)) break;  // (700 rows, 12 heads of 128: 15, with 288 CTAs 22)
     const float c = (float)((tiles + p - 1) / p) * tile * (ctas * p > 148 ? shared : 1.f) + sum[i];
-    if (i == 0 || c < cost) cost = c, best = p;
+    if (i == 0 || c < cost) cost = c, best = i;
   }
-  return best;
+  *alone = (int)(sum[best] / tile);
+  return 1 << best;
 }
 
 template <int HD>
-cudaError_t launch_hd(const FastAttnArgs& a, int two_term, int parts, const TensorMap2D& kvm, cudaStream_t st) {
+cudaError_t launch_hd(const FastAttnArgs& a, int two_term, const TensorMap2D& kvm, cudaStream_t st) {
+  int alone = 0;
+  const int parts = pick_parts<HD>(a, &alone);
   static PerDeviceOnce set;
   if (set.need()) {
     cudaError_t e = cudaFuncSetAttribute(attn_prompt_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, PromptSmem<HD>::TOTAL);
@@ -418,7 +427,7 @@ cudaError_t launch_hd(const FastAttnArgs& a, int two_term, int parts, const Tens
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, attn_prompt_tc_kernel<HD>, a, two_term, parts, *reinterpret_cast<const CUtensorMap*>(&kvm));
+  return cudaLaunchKernelEx(&cfg, attn_prompt_tc_kernel<HD>, a, two_term, parts, alone, *reinterpret_cast<const CUtensorMap*>(&kvm));
 }
 
 __global__ void wait_selftest_kernel(int* status) {
@@ -449,7 +458,7 @@ cudaError_t launch_attention_prompt_tc(const FastAttnArgs& a, int two_term, cuda
   TensorMap2D kvm;
   cudaError_t e = make_tensor_map_kv(&kvm, a.kv.pool, (unsigned long long)a.kv.n_pages * a.kv.n_layers * 2ull * a.kv.n_kv * 16, a.kv.hd, 16);
   if (e != cudaSuccess) return e;
-  return a.kv.hd == 64 ? launch_hd<64>(a, two_term, pick_parts<64>(a), kvm, st) : launch_hd<128>(a, two_term, pick_parts<128>(a), kvm, st);
+  return a.kv.hd == 64 ? launch_hd<64>(a, two_term, kvm, st) : launch_hd<128>(a, two_term, kvm, st);
 }
 
 }  // namespace qie

@@ -52,9 +52,11 @@ def test_against_reference_order(layers, entry, nq, nkv, hd, first, n):
 
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("spare", [0, 4, 30, 200])
-def test_more_parts_than_keys(layers, hd, spare):
-    """a block table for more positions than the sequence has: parts of the cluster without a key, parts that a row does not see"""
-    check(layers, "launch_attn_prefill_fast", 4, 2, hd, 70, 90, spare)
+@pytest.mark.parametrize("first,n", [(70, 90), (200, 100), (0, 300)])
+def test_more_parts_than_keys(layers, hd, spare, first, n):
+    """a block table for more positions than the sequence has: parts of the cluster without a key, parts that a row does not see, query tiles
+    that the cluster's first CTA does alone beside others"""
+    check(layers, "launch_attn_prefill_fast", 4, 2, hd, first, n, spare)
 
 
 def test_growing_maxima(layers):
