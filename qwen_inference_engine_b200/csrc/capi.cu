@@ -172,9 +172,12 @@ int qie_kv_store(const qie_kv_view* kv, int layer, const qie_bf16* K, const qie_
                      (cudaStream_t)st));
   return QIE_OK;
 }
+// whole groups of query heads per kv head (hosts divide by them)
+static bool heads_ok(int n_q, int n_kv) { return n_kv > 0 && n_q >= n_kv && n_q % n_kv == 0; }
 int qie_attention(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16* out, const int* pos, const int* slot,
                   const int* block_table, int max_pages, int n_tok, int n_q_heads, qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention: bad layer");
+  if (!heads_ok(n_q_heads, kv->n_kv_heads)) return fail(QIE_EINVAL, "attention: %d query heads on %d kv heads", n_q_heads, kv->n_kv_heads);
   AttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -193,8 +196,7 @@ int qie_attention(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16*
 int qie_attention_pagelist(const qie_bf16* const* d_k_pages, const qie_bf16* const* d_v_pages, int n_pages, int page_size,
                            int n_layers, int layer, int n_kv_heads, int head_dim, const qie_bf16* Q, qie_bf16* out, const int* pos,
                            int n_tok, int n_q_heads, qie_stream st) {
-  if (!d_k_pages || !d_v_pages || n_pages <= 0 || page_size <= 0 || layer < 0 || layer >= n_layers || n_kv_heads <= 0 ||
-      n_q_heads % n_kv_heads)
+  if (!d_k_pages || !d_v_pages || n_pages <= 0 || page_size <= 0 || layer < 0 || layer >= n_layers || !heads_ok(n_q_heads, n_kv_heads))
     return fail(QIE_EINVAL, "attention_pagelist: bad geometry");
   AttnArgs a{};
   a.q = (const bf16*)Q;
@@ -285,7 +287,7 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
                               const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads,
                               int n_splits, qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_decode_fast: bad layer");
-  if (n_q_heads % kv->n_kv_heads || n_q_heads / kv->n_kv_heads > 16 || (kv->head_dim != 64 && kv->head_dim != 128))
+  if (!heads_ok(n_q_heads, kv->n_kv_heads) || n_q_heads / kv->n_kv_heads > 16 || (kv->head_dim != 64 && kv->head_dim != 128))
     return fail(QIE_EINVAL, "attention_decode_fast: need n_q/n_kv <= 16 and head_dim 64 or 128");
   if (n_tok > 0 && (!aligned(16, {kv->pool}) || !aligned(4, {Q}))) return fail(QIE_EINVAL, "attention_decode_fast: the pool must start on a 16-byte, Q on a 4-byte boundary");
   static thread_local void *wo = nullptr, *wml = nullptr;
@@ -326,7 +328,7 @@ int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16*
                                const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads,
                                qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_prefill_fast: bad layer");
-  if (n_q_heads % kv->n_kv_heads || (kv->head_dim != 64 && kv->head_dim != 128))
+  if (!heads_ok(n_q_heads, kv->n_kv_heads) || (kv->head_dim != 64 && kv->head_dim != 128))
     return fail(QIE_EINVAL, "attention_prefill_fast: need n_q %% n_kv == 0 and head_dim 64 or 128");
   if (n_tok > 0 && (!aligned(16, {kv->pool, Q}) || !aligned(4, {out})))
     return fail(QIE_EINVAL, "attention_prefill_fast: the pool and Q must start on a 16-byte, out on a 4-byte boundary");
@@ -354,7 +356,7 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
                              const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads, int variant,
                              qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention_prefill_tc: bad layer");
-  if (n_q_heads % kv->n_kv_heads || kv->head_dim != 128) return fail(QIE_EINVAL, "attention_prefill_tc: head_dim must be 128");
+  if (!heads_ok(n_q_heads, kv->n_kv_heads) || kv->head_dim != 128) return fail(QIE_EINVAL, "attention_prefill_tc: head_dim must be 128");
   if (n_tok > 0 && !aligned(16, {kv->pool, Q, out})) return fail(QIE_EINVAL, "attention_prefill_tc: the pool, Q and out must start on a 16-byte boundary");
   OP_STATUS(status);
   FastAttnArgs a{};

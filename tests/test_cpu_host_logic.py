@@ -199,3 +199,15 @@ def test_operands_off_their_boundary_are_refused(name, args, at):
         p[3] = C.byref(view)
         assert getattr(lib, name)(*args(p)) == -1
         assert b"boundary" in lib.qie_last_error()
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(1, 2), (0, 2), (5, 2), (4, 0), (4, -1)])
+def test_heads_that_make_no_groups_are_refused(n_q, n_kv):
+    """the choice of the reference-order kernel divides by the group's size on the host: no such call gets there"""
+    from qwen_inference_engine_b200._lib import KvView
+    lib, kv = q.lib(), KvView(4096, 8, 16, 1, n_kv, 64)
+    ptr = [4096 * i for i in range(1, 6)]
+    assert lib.qie_attention(C.byref(kv), 0, *ptr, 8, 4, n_q, None) == -1
+    assert lib.qie_attention_prefill_fast(C.byref(kv), 0, *ptr, 8, 4, n_q, None) == -1
+    assert lib.qie_attention_decode_fast(C.byref(kv), 0, *ptr, 8, 4, n_q, 0, None) == -1
+    assert lib.qie_attention_pagelist(*ptr[:2], 8, 16, 1, 0, n_kv, 64, *ptr[2:], 4, n_q, None) == -1
