@@ -147,14 +147,14 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
 
 /* FAST-numerics causal attention for PREFILL rows (same contract as qie_attention with the
  * restriction that the n_tok rows are consecutive positions pos[0]+t of ONE sequence
- * slot[0], which is what llm()'s prefill branch produces, qwen_main.cu:160-176):
- * FlashAttention-2 style tiling on mma.sync, K/V streamed from the paged pool. */
+ * slot[0], which is what llm()'s prefill branch produces, qwen_main.cu:160-176): tiles of 128 rows x 64 keys on tcgen05 / TMEM for
+ * pages of 16 positions, on mma.sync for other pages and the shortest contexts.  Softmax weights are bf16 hi + lo pairs where a tile sees at most
+ * 1024 positions. */
 int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16* out, const int* pos,
                                const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads,
                                qie_stream st);
 
-/* The same prefill attention on tcgen05 / TMEM (head_dim 128): S = QK^T and O_t = PV as tcgen05.mma with the
- * accumulators in tensor memory, softmax by one thread per query row over tcgen05.ld.  variant = 0. */
+/* The same with one bf16 term per softmax weight, head_dim 128, on tcgen05 / TMEM for every page size.  `variant` is ignored. */
 int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16* out, const int* pos,
                              const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads, int variant,
                              qie_stream st);

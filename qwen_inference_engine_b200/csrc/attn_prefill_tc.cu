@@ -12,12 +12,13 @@
 // One elected thread of the last warp issues the MMAs; all threads copy K/V tiles with 16-byte cp.async into the
 // swizzled layout the descriptors expect, the next tile's
 // copies are in flight while the current tile is multiplied.  Replaces the mma.sync kernel (141 TFLOP/s, bound by
-// ldmatrix + softmax issue between the MMAs) for head_dim 128 and >= 256 rows.
+// ldmatrix + softmax issue between the MMAs) for head_dim 128 and >= 256 rows.  A wait that runs out makes the results NaN and is reported.
 #include <cuda.h>
 
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"
+#include "tc_ptx.cuh"
 
 namespace qie {
 namespace {
@@ -37,36 +38,6 @@ constexpr int SM_TOTAL = SM_PAGES + MAXP * 4 + 1024;
 constexpr int NSOFT = 256;                  // 8 softmax warps: two threads per query row (keys / head-dim halves)
 constexpr int NTHR = NSOFT + 32;            // + the copy/MMA warp
 
-__device__ __forceinline__ void mbar_init_(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-// (pure polling with test_wait instead of try_wait was measured: no difference)
-__device__ __forceinline__ void mbar_wait_(uint32_t bar, uint32_t parity) {
-  uint32_t done = 0;
-  const long long t0 = clock64();
-  while (true) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return;
-    if (clock64() - t0 > 4000000000ll) __trap();
-  }
-}
-__device__ __forceinline__ void umma_(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,"
@@ -78,36 +49,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// K-major operand, SWIZZLE_128B, 8-row atoms 1024 bytes apart (same encoding as gemm_tcgen05.cu)
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// MN-major operand (V as stored: [key][hd], hd contiguous), SWIZZLE_128B: column blocks of 64 hd values are `lbo`
-// bytes apart, groups of 8 keys `sbo` bytes apart
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// D = F32, A = B = BF16, N >> 3 at [17,23), M >> 4 at [24,29), bit 16: B is MN-major
-__host__ __device__ constexpr uint32_t idesc_(int m, int n, bool b_mn) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-__device__ __forceinline__ float ex2(float x) {  // one MUFU instruction; 2^(-inf) = 0
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // byte offset of 16-byte chunk `ch` (0..15) of row r in a [128][128] bf16 operand made of two 64-column blocks
 __device__ __forceinline__ uint32_t tile_off(int r, int ch) {
   return (uint32_t)((ch >> 3) * BLK + r * 128 + (((ch & 7) ^ (r & 7)) << 4));
@@ -115,15 +56,15 @@ __device__ __forceinline__ uint32_t tile_off(int r, int ch) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a, int lbo_sbo_swap) {
+__global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int dead_s;
+  volatile int* dead = &dead_s;
   const uint32_t s0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* sg = smem_raw + (s0 - smem_u32(smem_raw));
-  // mbarriers: S product done (two: TMEM buffer t & 1; the copy path uses the first), P V done, K tile landed (two
-  // buffers), V tile landed (two)
-  const uint32_t bar_s = s0 + SM_BAR, bar_o = bar_s + 16, slot = bar_s + 24;
+  const uint32_t bar_s = s0 + SM_BAR, bar_o = bar_s + 8, slot = bar_s + 16;  // S product done, P V done
   int* s_pages = reinterpret_cast<int*>(sg + SM_PAGES);
   float* xmax = reinterpret_cast<float*>(sg + SM_X);  // [2][128]
   float* xsum = xmax + 256;                            // [2][128]
@@ -143,13 +84,13 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
   const int Dq = a.n_q * HDX;
 
   if (threadIdx.x == 0) {
-    mbar_init_(bar_s, 1);
-    mbar_init_(bar_s + 8, 1);
-    mbar_init_(bar_o, 1);
+    dead_s = 0;
+    mbar_init_tc(bar_s, 1);
+    mbar_init_tc(bar_o, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == MMA_WARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(512u) : "memory");  // S[2] (2 x 128 columns) + O (128): the next power of two
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(256u) : "memory");  // S, O: 128 columns each
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   const int n_pg = min(MAXP, (kv_len - 1) / psz + 1);
@@ -197,8 +138,7 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
   // the exp + bf16-pack pass 53 us (16 384 ex2 + 8 192 cvt per tile on the 16-lane XU pipe), everything else --
   // tile copies, TMEM loads, row max, O fold, P stores, barriers, CTA prologue/epilogue -- 94 us.  An MN-major V
   // descriptor costs the same as a K-major one.
-  const uint32_t lbo = (lbo_sbo_swap & 1) ? 1024u : (uint32_t)BLK, sbo = (lbo_sbo_swap & 1) ? (uint32_t)BLK : 1024u;
-  constexpr uint32_t ID_S = idesc_(128, 128, false), ID_O = idesc_(128, 128, true);
+  const uint32_t ID_S = idesc_tc(128, 128, false), ID_O = idesc_tc(128, 128, true);
   const float sl2 = a.scale_log2;
   // softmax thread: query row `row` (= TMEM lane), half `hf`: keys [64 hf, 64 hf + 64) of every tile for the softmax,
   // head-dim columns [64 hf, 64 hf + 64) of O.  Warps w and w + 4 share a TMEM lane quarter (warp % 4).
@@ -212,8 +152,8 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
   for (int i = 0; i < 64; ++i) o[i] = 0.f;
   auto fold_o = [&]() {  // o = o * corr + (P V of the last tile), this thread's 64 head-dim columns
     uint32_t r[32], r2[32];
-    tmem_ld32(lane_addr + 256 + 64 * hf, r);
-    tmem_ld32(lane_addr + 256 + 64 * hf + 32, r2);
+    tmem_ld32(lane_addr + 128 + 64 * hf, r);
+    tmem_ld32(lane_addr + 128 + 64 * hf + 32, r2);
     tmem_wait_ld();
 #pragma unroll
     for (int j = 0; j < 32; ++j) o[j] = fmaf(o[j], corr, __uint_as_float(r[j]));
@@ -221,13 +161,13 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     for (int j = 0; j < 32; ++j) o[32 + j] = fmaf(o[32 + j], corr, __uint_as_float(r2[j]));
   };
 
-  // softmax of tile `it` for this thread's query row / key half: S from TMEM buffer sbuf, P (bf16) -> shared memory
-  auto softmax_tile = [&](int it, int sbuf) {
+  // softmax of tile `it` for this thread's query row / key half: S from TMEM, P (bf16) -> shared memory
+  auto softmax_tile = [&](int it) {
     const int p0 = it * TK + 64 * hf;  // first key of this thread's half
     // ---- this thread's 64 scores stay in registers between the max and the exp pass
     uint32_t r[32], r2[32];
-    tmem_ld32(lane_addr + (uint32_t)sbuf * 128u + 64 * hf, r);
-    tmem_ld32(lane_addr + (uint32_t)sbuf * 128u + 64 * hf + 32, r2);
+    tmem_ld32(lane_addr + 64 * hf, r);
+    tmem_ld32(lane_addr + 64 * hf + 32, r2);
     tmem_wait_ld();
     const bool need_mask = p0 + 63 > my_pos;
     float mx = -INFINITY;
@@ -243,15 +183,15 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     xmax[hf * 128 + row] = mx;
     asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");  // the two warps that share these 32 rows meet
     const float m_new = fmaxf(m_run, fmaxf(mx, xmax[(hf ^ 1) * 128 + row]));
-    corr = ex2((m_run - m_new) * sl2);
+    corr = ex2_tc((m_run - m_new) * sl2);
     m_run = m_new;
     const float nms = -m_new * sl2;
     float rs = 0.f;
     uint32_t pk[32];
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
-      const float e0 = ex2(fmaf(__uint_as_float(r[j]), sl2, nms)), e1 = ex2(fmaf(__uint_as_float(r[j + 1]), sl2, nms));
-      const float e2 = ex2(fmaf(__uint_as_float(r2[j]), sl2, nms)), e3 = ex2(fmaf(__uint_as_float(r2[j + 1]), sl2, nms));
+      const float e0 = ex2_tc(fmaf(__uint_as_float(r[j]), sl2, nms)), e1 = ex2_tc(fmaf(__uint_as_float(r[j + 1]), sl2, nms));
+      const float e2 = ex2_tc(fmaf(__uint_as_float(r2[j]), sl2, nms)), e3 = ex2_tc(fmaf(__uint_as_float(r2[j + 1]), sl2, nms));
       rs += (e0 + e1) + (e2 + e3);
       pk[j >> 1] = pack2(f2bf(e0), f2bf(e1));
       pk[16 + (j >> 1)] = pack2(f2bf(e2), f2bf(e3));
@@ -265,15 +205,15 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // P (generic stores) -> tensor core
   };
-  auto issue_s = [&](int t, int sbuf) {  // MMA thread: S(t) = Q K(t)^T into TMEM buffer sbuf
+  auto issue_s = [&](int t) {  // MMA thread: S(t) = Q K(t)^T
     const uint32_t kb = s0 + SM_K0 + (t & 1) * TILE_B;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
     for (int kk = 0; kk < HDX / 16; ++kk) {
       const uint32_t ko = (uint32_t)((kk >> 2) * BLK + (kk & 3) * 32);
-      umma_(tmem + (uint32_t)sbuf * 128u, desc_kmajor(s0 + SM_Q + ko), desc_kmajor(kb + ko), ID_S, kk != 0);
+      umma_tc(tmem, desc_k_tc(s0 + SM_Q + ko), desc_k_tc(kb + ko), ID_S, kk != 0);
     }
-    umma_commit_(bar_s + 8u * (uint32_t)sbuf);
+    umma_commit_tc(bar_s);
   };
   auto issue_pv = [&](int t) {  // MMA thread: O_t = P V(t)
     const uint32_t vb = s0 + SM_V0 + (t & 1) * TILE_B;
@@ -282,9 +222,9 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     for (int kk = 0; kk < TK / 16; ++kk) {
       const uint32_t po = (uint32_t)((kk >> 2) * BLK + (kk & 3) * 32);   // P: K-major, K = keys
       const uint32_t vo = (uint32_t)(kk * 16 * 128);                     // V: 16 keys further down = 2 atoms of 8 rows
-      umma_(tmem + 256, desc_kmajor(s0 + SM_P + po), desc_mnmajor(vb + vo, lbo, sbo), ID_O, kk != 0);
+      umma_tc(tmem + 128, desc_k_tc(s0 + SM_P + po), desc_mn_tc(vb + vo, BLK), ID_O, kk != 0);
     }
-    umma_commit_(bar_o);
+    umma_commit_tc(bar_o);
   };
 
   for (int it = 0; it < n_tiles; ++it) {
@@ -293,32 +233,32 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // cp.async (generic proxy) data -> tensor core (async proxy)
     __syncthreads();
     // ---- S = Q K^T
-    if (warp == MMA_WARP && lane == 0) issue_s(it, 0);
+    if (warp == MMA_WARP && lane == 0) issue_s(it);
     // Behind the S product (queued right after the previous tile's P V in the tensor pipe): the buffer tile it+1 goes
     // into was read by the P V product of tile it-1, so wait for that MMA, then request the copies.
-    if (it > 0) mbar_wait_(bar_o, (uint32_t)((it - 1) & 1));
+    if (it > 0) mbar_wait_tc(bar_o, (uint32_t)((it - 1) & 1), dead);
     if (it + 1 < n_tiles) load_tile(it + 1, buf ^ 1);
     if (soft) {
       if (it > 0) {  // fold the previous tile's P V product while the tensor core works on this tile's S
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         fold_o();
       }
-      mbar_wait_(bar_s, (uint32_t)(it & 1));
+      mbar_wait_tc(bar_s, (uint32_t)(it & 1), dead);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      softmax_tile(it, 0);
+      softmax_tile(it);
     }
     __syncthreads();
     // ---- O_t = P V
     if (warp == MMA_WARP && lane == 0) issue_pv(it);
   }
   if (soft) {
-    mbar_wait_(bar_o, (uint32_t)((n_tiles - 1) & 1));
+    mbar_wait_tc(bar_o, (uint32_t)((n_tiles - 1) & 1), dead);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     fold_o();
     xsum[hf * 128 + row] = l_run;
     asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
     if (row < n_rows) {
-      const float inv = 1.f / (l_run + xsum[(hf ^ 1) * 128 + row]);
+      const float inv = *dead ? __int_as_float(0x7fc00000) : 1.f / (l_run + xsum[(hf ^ 1) * 128 + row]);
       bf16* dst = a.out + (size_t)(t0 + row) * Dq + (size_t)h * HDX + 64 * hf;
 #pragma unroll
       for (int c = 0; c < 64; c += 8) {
@@ -334,13 +274,14 @@ __global__ void __launch_bounds__(NTHR, 1) attn_prefill_tc_kernel(FastAttnArgs a
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == MMA_WARP) {
+    if (lane == 0) report_tc(dead, a.status);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
   }
 }
 
 // rows = consecutive positions of one sequence; head_dim 128 only
-cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap, cudaStream_t st) {
+cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, cudaStream_t st) {
   if (a.n_tok == 0) return cudaSuccess;
   if (a.kv.hd != HDX || a.n_q % a.kv.n_kv) return cudaErrorInvalidValue;
   if (attention_prompt_tc_takes(a)) return launch_attention_prompt_tc(a, 0, st);
@@ -351,7 +292,7 @@ cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap,
     set.done();
   }
   dim3 grid(a.n_q, (a.n_tok + TQ - 1) / TQ);
-  (void)launch_k(attn_prefill_tc_kernel, grid, dim3(NTHR), (size_t)SM_TOTAL, st, a, lbo_sbo_swap);
+  (void)launch_k(attn_prefill_tc_kernel, grid, dim3(NTHR), (size_t)SM_TOTAL, st, a);
   return cudaGetLastError();
 }
 

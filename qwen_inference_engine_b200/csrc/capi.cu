@@ -374,7 +374,7 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
   a.max_kv_len = max_pages * kv->page_size;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)kv->head_dim);
   a.kv = geom_of(kv);
-  CU(launch_attention_prefill_tc(a, variant, (cudaStream_t)st));
+  CU(launch_attention_prefill_tc(a, (cudaStream_t)st));
   return QIE_OK;
 }
 

@@ -238,10 +238,10 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.status = e->wait_status;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.kv = e->kv;
-      // head_dim 128 and at least one full 128-row query tile: tcgen05 / TMEM kernel (QIE_ATTN_TC=0 keeps mma.sync)
-      static const bool tc_on = [] { const char* v = getenv("QIE_ATTN_TC"); return !(v && v[0] == '0'); }();
-      if (tc_on && hd == 128 && n >= 128)
-        QIE_TRY(KK_ATTN, launch_attention_prefill_tc(a, 0, st));
+      // head_dim 128 and a full 128-row query tile: one bf16 term per softmax weight, else hi + lo pairs up to 1024 positions (pages of 16 take the
+      // same tcgen05 kernel either way, others tcgen05 and mma.sync)
+      if (hd == 128 && n >= 128)
+        QIE_TRY(KK_ATTN, launch_attention_prefill_tc(a, st));
       else
         QIE_TRY(KK_ATTN, launch_attention_prefill_fast(a, st));
     } else {

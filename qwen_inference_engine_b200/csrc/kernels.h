@@ -141,12 +141,12 @@ int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num
 // causal tiled attention for prefill rows (attn_prefill_fast.cu): rows are consecutive positions
 // pos[0]+t of one sequence (slot[0]); n_splits / ws_* unused
 cudaError_t launch_attention_prefill_fast(const FastAttnArgs& a, cudaStream_t st);
-// the same on tcgen05 / TMEM (attn_prompt_tc.cu), head_dim 64 or 128, pages of 16; tiles that see at most two_term positions keep their
-// softmax weights as bf16 hi + lo pairs
+// the same on tcgen05 / TMEM (attn_prompt_tc.cu), head_dim 64 or 128, pages of 16; query tiles whose first 64 rows see at most two_term positions
+// keep their softmax weights as bf16 hi + lo pairs
 bool attention_prompt_tc_takes(const FastAttnArgs& a);
 cudaError_t launch_attention_prompt_tc(const FastAttnArgs& a, int two_term, cudaStream_t st);
-// the same on tcgen05 / TMEM (attn_prefill_tc.cu), head_dim 128; lbo_sbo_swap: descriptor probe, 0 in production
-cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, int lbo_sbo_swap, cudaStream_t st);
+// the same with one bf16 term per weight, head_dim 128: attn_prompt_tc.cu, or for pages of other than 16 positions attn_prefill_tc.cu
+cudaError_t launch_attention_prefill_tc(const FastAttnArgs& a, cudaStream_t st);
 
 // tcgen05 GEMM (fast numerics; without a split over K also the reference's order)
 struct TensorMap2D {

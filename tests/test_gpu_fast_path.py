@@ -85,15 +85,17 @@ def test_flash_decoding_vs_reference_order_attention(layers, hd, n_q, n_kv, B, t
     assert rel_err(got, want) < TOL_BF16
 
 
-@pytest.mark.parametrize("hd,n_q,n_kv,prefix,T", [(64, 14, 2, 0, 64), (64, 14, 2, 0, 1), (64, 14, 2, 0, 200), (64, 14, 2, 37, 91),
-                                                   (128, 12, 2, 0, 257), (128, 28, 4, 130, 70), (64, 4, 4, 15, 17),
-                                                   (128, 2, 1, 64, 128)])
-def test_prefill_attention_vs_reference_order_attention(layers, hd, n_q, n_kv, prefix, T):
+# pages of other than 16 positions: the mma.sync kernel at every length
+@pytest.mark.parametrize("hd,n_q,n_kv,prefix,T,ps", [(64, 14, 2, 0, 64, 16), (64, 14, 2, 0, 1, 16), (64, 14, 2, 0, 200, 16), (64, 14, 2, 37, 91, 16),
+                                                      (128, 12, 2, 0, 257, 16), (128, 28, 4, 130, 70, 16), (64, 4, 4, 15, 17, 16),
+                                                      (128, 2, 1, 64, 128, 16), (64, 14, 2, 37, 700, 8), (128, 12, 2, 0, 257, 32), (128, 4, 2, 77, 1100, 4),
+                                                      (64, 4, 2, 900, 300, 3)])
+def test_prefill_attention_vs_reference_order_attention(layers, hd, n_q, n_kv, prefix, T, ps):
     """prefill chunk of T rows at positions prefix..prefix+T-1 of sequence 1 (sequence 0 holds other
     data); the cache already contains the prefix (chunked prefill) and the chunk's own K/V."""
     rng = np.random.default_rng(hd * 3 + n_q + prefix + T)
     Dq, Dkv = n_q * hd, n_kv * hd
-    n_layers, layer, ps = 2, 1, 16
+    n_layers, layer = 2, 1
     total = prefix + T
     pool = layers.KvPool(n_pages=2 * ((total + ps - 1) // ps + 1), page_size=ps, n_layers=n_layers, n_kv_heads=n_kv,
                          head_dim=hd, max_seqs=2)
@@ -114,15 +116,17 @@ def test_prefill_attention_vs_reference_order_attention(layers, hd, n_q, n_kv, p
     assert rel_err(got, want) < TOL_BF16
 
 
+@pytest.mark.parametrize("ps", [16, 8, 32, 3])
 @pytest.mark.parametrize("n_q,n_kv,prefix,T", [(12, 2, 0, 257), (28, 4, 130, 70), (2, 1, 64, 128), (4, 2, 77, 1000),
                                                 (2, 2, 0, 1), (6, 1, 300, 129)])
-def test_prefill_attention_tcgen05_vs_reference_order_attention(layers, n_q, n_kv, prefix, T):
+def test_prefill_attention_tcgen05_vs_reference_order_attention(layers, n_q, n_kv, prefix, T, ps):
     """the tcgen05 / TMEM prefill attention (head_dim 128: S and P V on the 5th-gen tensor cores, softmax over
-    tcgen05.ld) against the reference-order kernel: ragged last tile, cache prefix, GQA groups, one-row chunk."""
+    tcgen05.ld) against the reference-order kernel: ragged last tile, cache prefix, GQA groups, one-row chunk.  Pages of 16
+    positions are attn_prompt_tc.cu, others attn_prefill_tc.cu."""
     hd = 128
     rng = np.random.default_rng(n_q * 31 + prefix + T)
     Dq, Dkv = n_q * hd, n_kv * hd
-    n_layers, layer, ps = 2, 1, 16
+    n_layers, layer = 2, 1
     total = prefix + T
     pool = layers.KvPool(n_pages=2 * ((total + ps - 1) // ps + 1), page_size=ps, n_layers=n_layers, n_kv_heads=n_kv,
                          head_dim=hd, max_seqs=2)
