@@ -366,20 +366,28 @@ static cudaError_t launch_hd(const FastAttnArgs& a, cudaStream_t st) {
   return e;
 }
 
-// The most splits, up to a cluster of 8, whose CTAs are all on the chip (hd 64: 4 of 48 KiB an SM, hd 128: 2), no more than 64-position tiles, none for
-// one or two tiles.  Measured (us; 1, 2, 4, 8, 16 splits): 64 x 2048, 64 wide, 128 CTAs a split: 30 21 18 23 29; 33 x 700: 12 9.5 7.8 9.3 18; 1 x
-// 2500: 35 20 12 8.1 9.0; 64 x 2048, 128 wide: 47 33 39 51 61; 8 x 300: 10 9.5 8.0 7.2 11; 64 x 100, 64 wide: 4.7 6.2 7.6 13 23.
-int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms) {
-  const int tiles = (max_kv_len + TILE - 1) / TILE;
-  const long fit = (hd == 64 ? 7L : 4L) * num_sms / 2;
+// CTAs on the chip at once: hd 64 four of 48 KiB an SM (3.5 counted: a cluster does not find every gap), hd 128 two.  Splits beyond that wait for the
+// first ones to end, and a cluster for all its CTAs: 64 x 100, 28 heads of 128 on 4, 8 splits 56 us, one 11.
+int attention_decode_most_splits(int n_tok, int n_kv, int hd, int num_sms) {
+  return (int)std::max(1L, (hd == 64 ? 7L : 4L) * num_sms / 2 / ((long)n_tok * n_kv));
+}
+
+// The most splits, up to a cluster of 8, whose CTAs are all on the chip, no more than 64-position tiles, none for one or two tiles; 16 and the
+// combining kernel from 4096 positions on, if the caller has the workspace.  Measured (us; 1, 2, 4, 8, 16 splits): 64 x 2048, 64 wide, 128 CTAs a split: 30 21 18 23 29;
+// 33 x 700: 12 9.5 7.8 9.3 18; 1 x 2500: 35 20 12 8.1 9.0; 64 x 2048, 128 wide: 47 33 39 51 61; 8 x 300: 10 9.5 8.0 7.2 11; 64 x 100, 64 wide: 4.7 6.2 7.6 13
+// 23; 8 and 16 splits: 1 x 4096 10.5 10.0, 8 x 8192 20.1 16.1, 128 wide 1 x 8192 25.8 17.7, 8 x 8192 30.9 21.9.  (Clusters of 16 find room for a few at a time: the
+// last one 35.)
+int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms, int most) {
+  const int tiles = (max_kv_len + TILE - 1) / TILE, fit = attention_decode_most_splits(n_tok, n_kv, hd, num_sms);
   int s = 1;
-  while (tiles > 2 && 2 * s <= std::min(tiles, FD_CLUSTER) && 2L * s * n_tok * n_kv <= fit) s *= 2;
+  while (tiles > 2 && 2 * s <= std::min({tiles, fit, tiles >= 64 ? most : FD_CLUSTER})) s *= 2;
   return s;
 }
 
-cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st) {
+cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st, int* launches) {
   if (a.n_tok == 0) return cudaSuccess;
-  if (a.n_q % a.kv.n_kv || a.n_q / a.kv.n_kv > 16) return cudaErrorInvalidValue;
+  if (a.n_q % a.kv.n_kv || a.n_q / a.kv.n_kv > 16 || (a.n_splits > FD_CLUSTER && !a.ws_o)) return cudaErrorInvalidValue;
+  if (launches) *launches = a.n_splits > FD_CLUSTER ? 2 : 1;
   switch (a.kv.hd) {
     case 64: return launch_hd<64>(a, st);
     case 128: return launch_hd<128>(a, st);

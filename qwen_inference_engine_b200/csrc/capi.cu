@@ -292,13 +292,12 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   if (n_tok > 0 && (!aligned(16, {kv->pool}) || !aligned(4, {Q}))) return fail(QIE_EINVAL, "attention_decode_fast: the pool must start on a 16-byte, Q on a 4-byte boundary");
   static thread_local void *wo = nullptr, *wml = nullptr;
   static thread_local size_t wo_cap = 0, wml_cap = 0;
-  if (n_splits <= 0) {
-    int dev = 0, sms = 0;
-    CU(cudaGetDevice(&dev));
-    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    n_splits = attention_decode_splits(n_tok, kv->n_kv_heads, kv->head_dim, max_pages * kv->page_size, sms);
-  }
-  n_splits = std::min(n_splits, 64);
+  if (n_tok == 0) return QIE_OK;
+  int dev = 0, sms = 0;
+  CU(cudaGetDevice(&dev));
+  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (n_splits <= 0) n_splits = attention_decode_splits(n_tok, kv->n_kv_heads, kv->head_dim, max_pages * kv->page_size, sms, FD_CLUSTER);
+  else n_splits = std::min({n_splits, 64, attention_decode_most_splits(n_tok, kv->n_kv_heads, kv->head_dim, sms)});
   if (n_splits > FD_CLUSTER) {
     int rc = scratch(&wo, &wo_cap, (size_t)n_splits * n_tok * n_q_heads * kv->head_dim * 4);
     if (rc) return rc;

@@ -212,16 +212,15 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.n_tok = n;
       a.n_q = c.n_q;
       a.layer = l;
-      static const int ns_env = [] { const char* v = getenv("QIE_ATTN_SPLITS"); return v ? atoi(v) : 0; }();  // tuning knob
-      const int ns = ns_env > 0 ? std::max(1, std::min(ns_env, std::min(e->attn_max_splits, (max_kv_len + 63) / 64)))
-                                : attention_decode_splits(n, c.n_kv, hd, max_kv_len, e->num_sms);
+      const int ns = attention_decode_splits(n, c.n_kv, hd, max_kv_len, e->num_sms, FD_MOST);
       a.n_splits = ns;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.ws_o = e->attn_ws_o;
       a.ws_ml = e->attn_ws_ml;
       a.kv = e->kv;
-      QIE_TRY(KK_ATTN, launch_attention_decode_fast(a, st));
-      if (ns > FD_CLUSTER) ++e->launches;  // + combine kernel
+      int nl = 0;
+      QIE_TRY(KK_ATTN, launch_attention_decode_fast(a, st, &nl));
+      e->launches += nl - 1;
     } else if (fast_prefill) {
       FastAttnArgs a{};
       a.q = e->q;

@@ -135,9 +135,10 @@ struct FastAttnArgs {
 };
 // a wait that nothing ends, through the same limit and report
 cudaError_t launch_wait_selftest(int* status, cudaStream_t st);
-cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st);
-constexpr int FD_CLUSTER = 8;  // splits that need no workspace
-int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms);
+cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st, int* launches = nullptr);
+constexpr int FD_CLUSTER = 8, FD_MOST = 16;  // splits that need no workspace; the most that attention_decode_splits picks
+int attention_decode_most_splits(int n_tok, int n_kv, int hd, int num_sms);  // as many as have all their CTAs on the chip
+int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms, int most);
 // causal tiled attention for prefill rows (attn_prefill_fast.cu): rows are consecutive positions
 // pos[0]+t of one sequence (slot[0]); n_splits / ws_* unused
 cudaError_t launch_attention_prefill_fast(const FastAttnArgs& a, cudaStream_t st);

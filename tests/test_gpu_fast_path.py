@@ -56,7 +56,11 @@ def test_tcgen05_gemm_vs_reference_kernel(layers, ref, M, N, K):
 
 @pytest.mark.parametrize("hd,n_q,n_kv,B,t,splits", [(64, 14, 2, 4, 300, 1), (64, 14, 2, 3, 1000, 4), (64, 14, 2, 2, 64, 0),
                                                      (64, 14, 2, 5, 1, 2), (128, 12, 2, 3, 515, 3), (128, 28, 4, 2, 130, 0),
-                                                     (64, 4, 4, 2, 77, 5), (64, 16, 1, 2, 200, 2)])
+                                                     (64, 4, 4, 2, 77, 5), (64, 16, 1, 2, 200, 2),
+                                                     # clusters of every size, more splits than tiles, the combining kernel, what `0` picks at length
+                                                     (64, 14, 2, 2, 100, 6), (128, 12, 2, 2, 700, 7), (64, 14, 2, 3, 700, 8), (64, 4, 2, 2, 1000, 12),
+                                                     (128, 12, 2, 1, 1500, 16), (64, 14, 2, 2, 300, 16), (64, 14, 2, 2, 2300, 24), (128, 4, 2, 2, 900, 40),
+                                                     (64, 14, 2, 2, 4200, 0), (128, 28, 4, 1, 4100, 0), (64, 14, 2, 40, 600, 16)])
 def test_flash_decoding_vs_reference_order_attention(layers, hd, n_q, n_kv, B, t, splits):
     """ragged batch: sequence b has t - 13*b (>=1) cached positions."""
     rng = np.random.default_rng(hd + n_q + t)
