@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
+#include <map>
 #include <mutex>
 #include <string>
 
@@ -248,15 +249,43 @@ int qie_repetition_penalty(qie_bf16* logits, const int* context_tokens, size_t c
   return QIE_OK;
 }
 
-static int scratch(void** p, size_t* cap, size_t need) {
-  if (*cap >= need) return QIE_OK;
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  *cap = 0;
-  CU(cudaMalloc(p, need));
-  *cap = need;
-  return QIE_OK;
-}
+// Memory of one call, in the order of its stream (under capture: of the graph): from a pool of this library per device that keeps up to 16 MiB.
+struct CallMemory {
+  void* p = nullptr;
+  cudaStream_t st = nullptr;
+  cudaError_t alloc(size_t bytes, cudaStream_t stream) {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool;
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      auto it = pools.find(dev);
+      if (it == pools.end()) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = 16ull << 20;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
+        e = cudaMemPoolCreate(&pool, &props);
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        (void)cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return e;
+        it = pools.emplace(dev, pool).first;
+      }
+      pool = it->second;
+    }
+    st = stream;
+    return cudaMallocFromPoolAsync(&p, bytes, pool, stream);
+  }
+  ~CallMemory() {
+    if (p) cudaFreeAsync(p, st);
+  }
+};
 
 int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st) {
   if (M < 1 || N < 64 || (N % 8) || K < 1) return fail(QIE_EINVAL, "matmul_fast: need M>=1, N>=64, N%%8==0");
@@ -290,20 +319,15 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   if (!heads_ok(n_q_heads, kv->n_kv_heads) || n_q_heads / kv->n_kv_heads > 16 || (kv->head_dim != 64 && kv->head_dim != 128))
     return fail(QIE_EINVAL, "attention_decode_fast: need n_q/n_kv <= 16 and head_dim 64 or 128");
   if (n_tok > 0 && (!aligned(16, {kv->pool}) || !aligned(4, {Q}))) return fail(QIE_EINVAL, "attention_decode_fast: the pool must start on a 16-byte, Q on a 4-byte boundary");
-  static thread_local void *wo = nullptr, *wml = nullptr;
-  static thread_local size_t wo_cap = 0, wml_cap = 0;
   if (n_tok == 0) return QIE_OK;
   int dev = 0, sms = 0;
   CU(cudaGetDevice(&dev));
   CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (n_splits <= 0) n_splits = attention_decode_splits(n_tok, kv->n_kv_heads, kv->head_dim, max_pages * kv->page_size, sms, FD_CLUSTER);
   else n_splits = std::min({n_splits, 64, attention_decode_most_splits(n_tok, kv->n_kv_heads, kv->head_dim, sms)});
-  if (n_splits > FD_CLUSTER) {
-    int rc = scratch(&wo, &wo_cap, (size_t)n_splits * n_tok * n_q_heads * kv->head_dim * 4);
-    if (rc) return rc;
-    rc = scratch(&wml, &wml_cap, (size_t)n_splits * n_tok * n_q_heads * 2 * 4);
-    if (rc) return rc;
-  }
+  CallMemory ws;
+  const size_t parts = (size_t)n_splits * n_tok * n_q_heads;
+  if (n_splits > FD_CLUSTER) CU(ws.alloc(parts * (kv->head_dim + 2) * sizeof(float), (cudaStream_t)st));
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -316,8 +340,8 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   a.layer = layer;
   a.n_splits = n_splits;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)kv->head_dim);
-  a.ws_o = (float*)wo;
-  a.ws_ml = (float*)wml;
+  a.ws_o = (float*)ws.p;
+  a.ws_ml = a.ws_o ? a.ws_o + parts * kv->head_dim : nullptr;
   a.kv = geom_of(kv);
   CU(launch_attention_decode_fast(a, (cudaStream_t)st));
   return QIE_OK;
@@ -474,7 +498,7 @@ static void engine_free(qie_engine* e) {
   if (!e->blob_owned) e->blob = nullptr;
   void* dev[] = {e->blob, e->cos_d, e->sin_d, e->kv.pool, e->block_table_d, e->ids_d, e->pos_d, e->slot_d,
                  e->sampled_d, e->rowstep_d, e->x, e->xn, e->q, e->k, e->v, e->att, e->h, e->logits, e->qkv,
-                 e->attn_ws_o, e->attn_ws_ml, e->mega_layers_d, e->mega_cand_d,
+                 e->attn_ws, e->mega_layers_d, e->mega_cand_d,
                  e->mega_bar_d, e->mega_prof_d, e->mega_wmaps_d[0], e->mega_wmaps_d[1], e->tp_buf, e->tp_cand, e->tp_xbuf, e->x2,
                  e->mega_wmaps_tp_d[0], e->mega_wmaps_tp_d[1], e->mega_kvmap_d, e->mega_hmap_d, e->gemv_part_d};
   for (int r = 0; r < MEGA_MAX_TP; ++r)
@@ -707,8 +731,10 @@ static int engine_finish_setup(qie_engine* e) {
       CU(make_tensor_map_2d(&m.down, w.down, (int)H, (int)I, 128));
     }
     CU(make_tensor_map_2d(&e->lm_head_map, e->lm_head, c.vocab, (int)H, 128));
-    CU(cudaMalloc(&e->attn_ws_o, (size_t)e->attn_max_splits * R * Dq * sizeof(float)));
-    CU(cudaMalloc(&e->attn_ws_ml, (size_t)e->attn_max_splits * R * c.n_q * 2 * sizeof(float)));
+    // what FD_MOST splits of as many rows as have them (attention_decode_most_splits) write: 2 to 20 MB
+    const int decode_rows = attention_decode_most_splits(1, c.n_kv, c.head_dim, e->num_sms) / FD_MOST;
+    e->attn_ws_rows = (size_t)FD_MOST * std::max(1, decode_rows) * c.n_q;
+    CU(cudaMalloc(&e->attn_ws, e->attn_ws_rows * (c.head_dim + 2) * sizeof(float)));
   }
   CU(cudaStreamSynchronize(e->stream));
   return QIE_OK;

@@ -96,8 +96,8 @@ struct qie_engine {
   std::vector<LayerMaps> wmaps;  // TMA descriptors of the weight matrices (box 128 x 64)
   qie::TensorMap2D lm_head_map;
   qie::bf16* qkv = nullptr;      // fused [rows, Dq + 2*Dkv] projection output
-  float *attn_ws_o = nullptr, *attn_ws_ml = nullptr;
-  int attn_max_splits = 16;
+  float* attn_ws = nullptr;      // partial results of a decode step whose keys are split more than FD_CLUSTER ways
+  size_t attn_ws_rows = 0;       // (split, row, head) of them
 
   // persistent decode kernel (decode_mega.cu): reference-order decode steps of <= 8 rows
   bool use_mega = true;              // QIE_MEGA=0 disables

@@ -89,6 +89,38 @@ def test_flash_decoding_vs_reference_order_attention(layers, hd, n_q, n_kv, B, t
     assert rel_err(got, want) < TOL_BF16
 
 
+def test_flash_decoding_workspace_of_several_streams(layers):
+    """more splits than a cluster has write partial results: calls on two streams of one thread, and a captured one, each have memory of their own"""
+    rng = np.random.default_rng(1)
+    n_q, n_kv, hd, t, n = 14, 2, 64, 3000, 2
+    pool = layers.KvPool(n_pages=n * ((t + 15) // 16), page_size=16, n_layers=1, n_kv_heads=n_kv, head_dim=hd, max_seqs=n)
+    pool.pool.normal_(generator=torch.Generator("cuda").manual_seed(2))
+    pos, slot = torch.full((n,), t - 1, dtype=torch.int32, device="cuda"), torch.arange(n, dtype=torch.int32, device="cuda")
+    qs = [to_dev(rand_bf16(rng, (n, n_q * hd), 1.0)) for _ in range(2)]
+    outs = [[torch.empty_like(x) for _ in range(20)] for x in qs]
+    want = [torch.empty_like(x) for x in qs]
+    for x, o in zip(qs, want):
+        layers.launch_attn_decode_fast(x, o, pool, 0, pos, slot, n_q, 40)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in qs]
+    for i in range(20):
+        for x, o, st in zip(qs, outs, streams):
+            with torch.cuda.stream(st):
+                layers.launch_attn_decode_fast(x, o[i], pool, 0, pos, slot, n_q, 40)
+    torch.cuda.synchronize()
+    for o, w in zip(outs, want):
+        assert all(torch.equal(x.view(torch.int16), w.view(torch.int16)) for x in o)
+    g, x, o = torch.cuda.CUDAGraph(), qs[0].clone(), torch.empty_like(qs[0])
+    with torch.cuda.graph(g, stream=streams[0]):
+        layers.launch_attn_decode_fast(x, o, pool, 0, pos, slot, n_q, 40)
+    for src, w in ((1, want[1]), (0, want[0])):
+        x.copy_(qs[src])
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(o.view(torch.int16), w.view(torch.int16))
+    del g
+
+
 # pages of other than 16 positions: the mma.sync kernel at every length
 @pytest.mark.parametrize("hd,n_q,n_kv,prefix,T,ps", [(64, 14, 2, 0, 64, 16), (64, 14, 2, 0, 1, 16), (64, 14, 2, 0, 200, 16), (64, 14, 2, 37, 91, 16),
                                                       (128, 12, 2, 0, 257, 16), (128, 28, 4, 130, 70, 16), (64, 4, 4, 15, 17, 16),
