@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
     }
   };
   // ---- scores
+  fetch(0, 0);  // on its way beside the queries
   {
     const int c = lane % SP, r = lane / SP % R, ks = lane / (SP * R);
     float q[64];
@@ -140,7 +141,6 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
       for (int j = 0; j < 64; ++j) q[j] = 0.f;
     }
     const float den = __fsqrt_rn((float)HD);
-    fetch(0, 0);
     put(0, 0);
     __syncthreads();
     const int len = s_len[r];
@@ -148,8 +148,10 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
     for (int tl = 0; tl < n_tiles; ++tl) {
       if (tl + 1 < n_tiles) fetch(tl + 1, 0);
       const float* kt = tile + (tl & 1) * TILE_F;
+      const int end = min(TK, max_len - tl * TK);  // (a warp's lanes go round together: its first key decides)
 #pragma unroll 1
-      for (int kk = warp * KS + ks; kk < TK; kk += NWARP * KS) {
+      for (int k0 = warp * KS; k0 < end; k0 += NWARP * KS) {
+        const int kk = k0 + ks;
         const float4* kr = reinterpret_cast<const float4*>(kt + (kk * SP + c) * 68);
         // the tree with strides 32 ... 1 over the lane's 64 elements, depth first: part[b] is the sum over the elements b modulo 8
         // folded down to stride 8, with the tree's own pairs
@@ -282,7 +284,9 @@ cudaError_t launch_rows(const AttnArgs& a, int rows, size_t smem, cudaStream_t s
 // the second CTA.  Measured (us, 32 / 16 / 8 virtual rows; one block per row and head): 500 rows behind 300 positions, 14 heads on 2, 64
 // wide 128 / 112 / 137; 820.  64 rows behind 800: 98 / 61 / 42; 291.  One row at 801: 89 / 56 / 39; 120.  12 heads on 2, 128 wide, 500
 // rows behind 300: - / 185 / 223; 981.
+// Up to 16 positions one block per row and head is quicker (16 rows, 12 heads of 128: 6.0, 6.7 here).
 int attention_ref_tile_rows(const AttnArgs& a, int num_sms, int* virtual_rows) {
+  if (a.max_kv_len <= 16) return 0;
   const int G = a.n_q / a.kv.n_kv, np = a.kv.hd / 64;
   int best = 0;
   for (int R = 32 / np; R >= 8 && R >= G; R /= 2) {
