@@ -977,11 +977,12 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
 // sums, subnormals, overflow, infinities, NaN) showed no difference, and tests/test_gpu_gemm_exact.py repeats a part of them.  So
 // the reference order takes the tcgen05 kernels without the split over K, at every row count: 896 x 4864 at 1000 rows 290 us ->
 // 12.6 (the mma.sync kernel runs 64 rows a launch and reads the weights again for each), at 16 rows 10.5 -> 4.7; 4864 x 896 at 400 rows
-// 737 -> 16.5; 896 x 151936 at 1 row 79 -> 47.  The mma.sync kernel keeps what TMA or the tile cannot express: K below one k-block, fp32 outputs (the partial sums
+// 737 -> 16.5; 896 x 151936 at 1 row 79 -> 47.  The mma.sync kernel keeps what TMA or the tile cannot express: K below one k-block (two for up to 8 rows), fp32 outputs (the partial sums
 // of tensor parallelism), column slices of a wider matrix.  Operands off a 16-byte boundary are refused: both kernels read 16 bytes at a time.
 cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st, int w_static, int* launches, int* status) {
   if (launches) *launches = 0;
-  bool tc = a.M >= 1 && a.K >= BK && a.K % 8 == 0 && a.lda == a.K && a.epi != EPI_STORE_F32 && a.nseg <= 3 &&
+  // (up to 8 rows of less than two k-blocks: the mma.sync kernel starts up quicker, 8 x 64 x 512 in 1.95 us, 2.05 here; from 128 on no longer)
+  bool tc = a.M >= 1 && a.K >= (a.M <= 8 ? 2 * BK : BK) && a.K % 8 == 0 && a.lda == a.K && a.epi != EPI_STORE_F32 && a.nseg <= 3 &&
             (reinterpret_cast<uintptr_t>(a.A) & 15) == 0;
   for (int i = 0; i < a.nseg; ++i) tc = tc && (a.seg[i].ldw == 0 || a.seg[i].ldw == a.K);
   if (tc) {

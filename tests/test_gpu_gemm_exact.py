@@ -41,11 +41,21 @@ def matmul(layers, a, b):
 @pytest.mark.parametrize("kind", ["normal", "wide", "small", "special"])
 @pytest.mark.parametrize("rows", [1, 8, 17, 64, 200])
 def test_same_bits_as_the_mma_sync_kernel(layers, rows, kind):
-    """An inner dimension below one k-block takes the mma.sync kernel; with zeros appended up to a k-block the same sums take tcgen05
+    """An inner dimension below one k-block takes the mma.sync kernel; with zeros appended up to a k-block (two for up to 8 rows) the same sums take tcgen05
     (a product with zeros leaves an accumulator as it is; infinities stay out of the zero columns)."""
     a, b = draw((rows, 56), kind, 3 + rows), draw((520, 56), "normal" if kind == "special" else kind, 4)
+    pad, more = torch.nn.functional.pad, 8 if rows > 8 else 72
+    assert torch.equal(matmul(layers, a, b), matmul(layers, pad(a, (0, more)), pad(b, (0, more))))
+
+
+@pytest.mark.parametrize("kind", ["normal", "wide", "small"])
+@pytest.mark.parametrize("rows", [1, 5, 8])
+def test_same_bits_over_more_than_one_block(layers, rows, kind):
+    """up to 8 rows of less than two k-blocks take the mma.sync kernel too: chains of 5 to 7 products against two blocks of a tcgen05 tile"""
     pad = torch.nn.functional.pad
-    assert torch.equal(matmul(layers, a, b), matmul(layers, pad(a, (0, 8)), pad(b, (0, 8))))
+    for inner in (72, 104, 120):
+        a, b = draw((rows, inner), kind, inner + rows), draw((1000, inner), kind, inner)
+        assert torch.equal(matmul(layers, a, b), matmul(layers, pad(a, (0, 136 - inner)), pad(b, (0, 136 - inner))))
 
 
 @pytest.mark.parametrize("inner,outer", [(896, 4864), (4864, 896), (72, 20000), (1536, 264)])
