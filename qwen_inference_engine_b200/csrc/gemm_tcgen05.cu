@@ -864,7 +864,7 @@ struct TcTile {
 //    Outputs that 16-byte stores cannot reach (an odd number of columns) take one tile per CTA at any number of tiles, no wider than the rows
 //    (1 x 896 x 20001: 45 us with 256, 7.5 with 16).
 //  * Few tiles and a long K: a cluster of 2, 4 or 8 CTAs splits K (never in the reference's order).  Its reduction costs about
-//    1.1 us + (0.1, 0.055, 0.045) us x tokens, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
+//    1.1 us + (0.1, 0.055, 0.045) us x tokens that are there, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
 //    clusters have to run at once (`most` clusters of a size fit; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
 //    against 27 with 4).
 static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool may_split) {
@@ -880,7 +880,7 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool m
       for (int bn = 16; bn <= 128; bn *= 2) {
         const int s = 2 << i;
         if (nkb < 2 * s || ctas(bn) > most[i] || (bn > 16 && bn / 2 >= M)) continue;
-        const float c = 0.19f * ((nkb + s - 1) / s) + 1.1f + per_token[i] * bn;
+        const float c = 0.19f * ((nkb + s - 1) / s) + 1.1f + per_token[i] * std::min(bn, M);
         if (c < cost) cost = c, best.bn = bn, best.splits = s;
       }
     return best;
