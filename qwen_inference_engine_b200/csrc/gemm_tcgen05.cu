@@ -5,7 +5,7 @@
 // may split K (a fixed-order sum of the splits) and match it within the bf16 tolerance.
 //
 // Swap-AB: the weight tile is the UMMA "A" operand (M = 128 weight rows = 128 TMEM lanes),
-// the activations are the "B" operand (N = BN tokens, 16..256), both K-major, 128-byte
+// the activations are the "B" operand (N = BN tokens, 16..128; up to 256 in the persistent kernel), both K-major, 128-byte
 // swizzle, BLOCK_K = 64 bf16.  D[w_row, token] lives in TMEM: lane = weight row, column =
 // token.  Decode is HBM-bound on the weights: each CTA streams its [128 x Kslice] weight
 // slab exactly once through a TMA/mbarrier ring.
@@ -38,9 +38,9 @@ namespace qie {
 
 static constexpr int BM = 128;  // weight rows per CTA (UMMA M)
 static constexpr int BK = 64;   // k elements per stage (128 B rows, SWIZZLE_128B)
-template <int BN>
-struct TcCfg {
-  static constexpr int STAGES = BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : BN <= 128 ? 7 : 4;  // what 227 KiB hold (4 x 48 KiB at BN=256)
+template <int BN, bool HALF>
+struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens)
+  static constexpr int STAGES = HALF ? 6 : BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : 7;  // what 227 KiB hold
 };
 
 // ------------------------------------------------------------------ PTX wrappers (tc_ptx.cuh has the rest)
@@ -97,11 +97,12 @@ struct TcArgs {
   int ref_silu;    // persistent kernel: SiLU as the reference computes it (expf, IEEE division); the others always do
   int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
   int* status;     // host word that a wait which ran out sets, or null
+  int vec;         // persistent kernel: rows of the output take 16-byte stores
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
   TcSeg seg[3];
 };
 
-template <int BN>
+template <int BN, bool HALF>
 __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
-  constexpr int TC_STAGES = TcCfg<BN>::STAGES;
+  constexpr int TC_STAGES = TcCfg<BN, HALF>::STAGES;
   static_assert(TC_STAGES * STAGE_BYTES >= BN * (BM + 32) * 4, "reduction tile must fit in the pipeline ring");
   // 1024-byte alignment for SWIZZLE_128B (same offset in every CTA of a cluster: the dynamic
   // shared window starts at the same address in all CTAs of a kernel)
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
       return v;
     };
-    const bool bulk = !g.dual && g.epi == EPI_STORE;
+    const bool bulk = g.vec && !g.dual && g.epi == EPI_STORE;
     const int copier = lane < P_STEP / 8 ? (warp - 2) * (P_STEP / 8) + lane : P_STEP;  // the token whose copy this thread issues
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
     int j = 0, it = 0;
@@ -682,6 +683,13 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
                          "r"(2 * min(BM, seg_rows - row0))
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        } else if (!g.vec) {  // an odd number of columns (plain results only): 2 bytes a thread, neighbours side by side
+          for (int c = tq; c < n_tok * BM; c += P_EPI) {
+            const int tok = c / BM, r = c % BM;
+            unsigned short y;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(y) : "r"(st0 + (uint32_t)tok * PITCH + (uint32_t)r * 2u) : "memory");
+            if (row0 + r < seg_rows) out[(size_t)(tok_base + h0 + tok) * ld + row0 + r] = __ushort_as_bfloat16(y);
           }
         } else if (!g.dual) {
 #pragma unroll
@@ -811,15 +819,15 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN>
+template <int BN, bool HALF = false>
 static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int STAGE_BYTES = BM * BK * 2 + BN * BK * 2;
-  constexpr size_t smem = (size_t)TcCfg<BN>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  constexpr size_t smem = (size_t)TcCfg<BN, HALF>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     set.done();
   }
@@ -847,12 +855,12 @@ static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, const TensorMap2D
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN>, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF>, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g);
 }
 
 struct TcTile {
   int bn, splits;
-  bool persist;
+  bool persist, half;
 };
 // Tokens of a tile and splits over K.  Measured on B200 in graphs of the same launch, weights in L2 (us):
 //  * One wave of CTAs: the smallest of 16 ... 128 tokens whose tiles all fit on the SMs.  A k-block takes the same time at any width up
@@ -867,9 +875,9 @@ struct TcTile {
 //    1.1 us + (0.1, 0.055, 0.045) us x tokens that are there, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
 //    clusters have to run at once (`most` clusters of a size fit; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
 //    against 27 with 4).
-static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool may_split) {
+static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool may_split) {
   auto ctas = [&](int bn) { return (long)tiles * ((M + bn - 1) / bn); };
-  TcTile best{16, 1, false};
+  TcTile best{16, 1, false, false};
   while (best.bn < 256 && ctas(best.bn) > num_sms) best.bn *= 2;
   if (best.bn < 256) {
     if (!may_split) return best;
@@ -885,8 +893,8 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool vec, bool m
       }
     return best;
   }
-  if (!vec) {  // outputs that 16-byte stores cannot reach: one tile per CTA, no wider than the rows
-    for (best.bn = 16; best.bn < 256 && best.bn < M;) best.bn *= 2;
+  if (M <= 16 && tiles <= 2 * num_sms) {
+    best.bn = 16, best.half = true;
     return best;
   }
   best.persist = true;
@@ -926,19 +934,22 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   }
   g.n_tiles = tiles;
   g.kb_total = (t.K + BK - 1) / BK;
-  bool vec = true;  // the epilogue through a staging tile stores 16 bytes
+  bool vec = true;  // 16-byte stores reach every row of the outputs
   for (int i = 0; i < g.nseg; ++i)
     vec = vec && g.seg[i].rows % 8 == 0 && g.seg[i].ld % 8 == 0 && (reinterpret_cast<uintptr_t>(g.seg[i].out) & 15) == 0;
-  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, vec, !t.exact);
+  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, !t.exact);
   const int token_tiles = (t.M + tl.bn - 1) / tl.bn;
   g.kb_per_split = (g.kb_total + tl.splits - 1) / tl.splits;
   g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
   g.staged = g.splits == 1 && vec;
+  g.vec = vec;
   TensorMap2D x;
   cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
   if (e != cudaSuccess) return e;
   if (launches) *launches = 1;
   if (tl.persist) {
+    // (widths of the residual stream and of the feed-forward are inner dimensions too, so multiples of 8)
+    if (!vec && t.epi != EPI_STORE) return cudaErrorInvalidValue;
     constexpr size_t smem = (size_t)P_RING + P_STAGING + 1024 /*align*/ + 256 /*barriers*/;
     static PerDeviceOnce set;
     if (set.need()) {
@@ -964,11 +975,10 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
   }
   switch (tl.bn) {
-    case 16: return launch_bn<16>(t, g, x, token_tiles, st);
+    case 16: return tl.half ? launch_bn<16, true>(t, g, x, token_tiles, st) : launch_bn<16>(t, g, x, token_tiles, st);
     case 32: return launch_bn<32>(t, g, x, token_tiles, st);
     case 64: return launch_bn<64>(t, g, x, token_tiles, st);
-    case 128: return launch_bn<128>(t, g, x, token_tiles, st);
-    default: return launch_bn<256>(t, g, x, token_tiles, st);
+    default: return launch_bn<128>(t, g, x, token_tiles, st);
   }
 }
 
