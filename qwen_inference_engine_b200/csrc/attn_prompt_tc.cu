@@ -389,8 +389,9 @@ int pick_parts(const FastAttnArgs& a, int* alone) {
   float cost = 0.f;
   for (int i = 0; i < 4; ++i) {
     const int p = 1 << i;
-    if (p > 1 && ctas * p > (HD == 64 ? 240 : 200)) break;  // (700 rows, 12 heads of 128: 15, with 288 CTAs 22)
-    const float c = (float)((tiles + p - 1) / p) * tile * (ctas * p > 148 ? shared : 1.f) + sum[i];
+    // (240 and 200 CTAs of 148 SMs' 296 places: clusters do not find every gap.  700 rows, 12 heads of 128: 15, with 288 CTAs 22)
+    if (p > 1 && ctas * p * 148 > (HD == 64 ? 240L : 200L) * a.num_sms) break;
+    const float c = (float)((tiles + p - 1) / p) * tile * (ctas * p > a.num_sms ? shared : 1.f) + sum[i];
     if (i == 0 || c < cost) cost = c, best = i;
   }
   *alone = (int)(sum[best] / tile);

@@ -88,6 +88,12 @@ static int engine_sync(qie_engine* e) {
   CU(op_status(&w));                                      \
   if (take_status(w)) return wait_failed("an earlier operator call")
 
+static cudaError_t sm_count(int* n) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  return e == cudaSuccess ? cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev) : e;
+}
+
 // ---------------------------------------------------------------- operator level
 int qie_embedding(qie_bf16* out, const qie_bf16* table, const int* ids, size_t hidden, size_t n_tok, qie_stream st) {
   CU(launch_embedding((bf16*)out, (const bf16*)table, ids, hidden, n_tok, (cudaStream_t)st));
@@ -103,9 +109,8 @@ int qie_matmul(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, 
   if (M < 0 || N <= 0 || K <= 0 || (N & 7)) return fail(QIE_EINVAL, "matmul: need N %% 8 == 0 (got M=%d N=%d K=%d)", M, N, K);
   if (M > 0 && !aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul: A and B must start on a 16-byte boundary");
   OP_STATUS(status);
-  int dev = 0, sms = 0;
-  CU(cudaGetDevice(&dev));
-  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int sms = 0;
+  CU(sm_count(&sms));
   GemmArgs g{};
   g.A = (const bf16*)A;
   g.lda = N;
@@ -291,9 +296,8 @@ int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, in
   if (M < 1 || N < 64 || (N % 8) || K < 1) return fail(QIE_EINVAL, "matmul_fast: need M>=1, N>=64, N%%8==0");
   if (!aligned(16, {A, B})) return fail(QIE_EINVAL, "matmul_fast: A and B must start on a 16-byte boundary");
   OP_STATUS(status);
-  int dev = 0, sms = 0;
-  CU(cudaGetDevice(&dev));
-  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int sms = 0;
+  CU(sm_count(&sms));
   TensorMap2D wmap;
   CU(make_tensor_map_2d(&wmap, (const bf16*)B, K, N, 128));
   TcGemm t{};
@@ -320,9 +324,8 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
     return fail(QIE_EINVAL, "attention_decode_fast: need n_q/n_kv <= 16 and head_dim 64 or 128");
   if (n_tok > 0 && (!aligned(16, {kv->pool}) || !aligned(4, {Q}))) return fail(QIE_EINVAL, "attention_decode_fast: the pool must start on a 16-byte, Q on a 4-byte boundary");
   if (n_tok == 0) return QIE_OK;
-  int dev = 0, sms = 0;
-  CU(cudaGetDevice(&dev));
-  CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int sms = 0;
+  CU(sm_count(&sms));
   if (n_splits <= 0) n_splits = attention_decode_splits(n_tok, kv->n_kv_heads, kv->head_dim, max_pages * kv->page_size, sms, FD_CLUSTER);
   else n_splits = std::min({n_splits, 64, attention_decode_most_splits(n_tok, kv->n_kv_heads, kv->head_dim, sms)});
   CallMemory ws;
@@ -357,6 +360,7 @@ int qie_attention_prefill_fast(const qie_kv_view* kv, int layer, const qie_bf16*
     return fail(QIE_EINVAL, "attention_prefill_fast: the pool and Q must start on a 16-byte, out on a 4-byte boundary");
   OP_STATUS(status);
   FastAttnArgs a{};
+  CU(sm_count(&a.num_sms));
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
   a.pos = pos;
@@ -383,6 +387,7 @@ int qie_attention_prefill_tc(const qie_kv_view* kv, int layer, const qie_bf16* Q
   if (n_tok > 0 && !aligned(16, {kv->pool, Q, out})) return fail(QIE_EINVAL, "attention_prefill_tc: the pool, Q and out must start on a 16-byte boundary");
   OP_STATUS(status);
   FastAttnArgs a{};
+  CU(sm_count(&a.num_sms));
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
   a.pos = pos;

@@ -234,6 +234,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.layer = l;
       a.n_splits = 1;
       a.max_kv_len = max_kv_len;
+      a.num_sms = e->num_sms;
       a.status = e->wait_status;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.kv = e->kv;

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   if (warp == 0) {
     if (elect_tc()) {
       // Weights never depend on the previous kernel: start streaming them BEFORE waiting for
-      // it (programmatic dependent launch), so HBM stays busy across the kernel boundary.
+      // it (programmatic dependent launch), as soon as its CTAs leave room for the ring.
       const int pre = g.w_static ? min(nkb, TC_STAGES) : 0;
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), STAGE_BYTES);
@@ -868,12 +868,11 @@ struct TcTile {
 //  * More tiles than that: the persistent kernel.  256 tokens, unless a width with fuller waves takes less than 0.9 of waves x width
 //    (1536 outputs at 4096 rows: 107 -> 86 with 176; a few per cent less on paper were none: 8960 outputs 82.7 with 256, 85.5 with
 //    224).  Below 160 tokens the loop, not the tensor core, sets a tile's time, so of those the narrowest wins, whose ring holds most
-//    k-blocks: 151936 x 896 for one row 79 -> 47.
-//    Outputs that 16-byte stores cannot reach (an odd number of columns) take one tile per CTA at any number of tiles, no wider than the rows
-//    (1 x 896 x 20001: 45 us with 256, 7.5 with 16).
+//    k-blocks: 151936 x 896 for one row 79 -> 47.  (Odd output widths too, with 2-byte stores: one 256-token tile per CTA took 45 us for 1 x 896 x
+//    20001.)  Up to 16 rows and two tiles an SM: one tile per CTA, two CTAs an SM beside each other (1 x 896 x 20001, weights from memory: persistent 11.3, 9.0).
 //  * Few tiles and a long K: a cluster of 2, 4 or 8 CTAs splits K (never in the reference's order).  Its reduction costs about
 //    1.1 us + (0.1, 0.055, 0.045) us x tokens that are there, a k-block 0.19 us: 4864 x 896 at 64 tokens 16.0 without, 6.9 with 8 x 32 tokens.  All
-//    clusters have to run at once (`most` clusters of a size fit; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
+//    clusters have to run at once (`most` clusters of a size fit on 148 SMs; they do not pack every SM: 28 clusters of 5 took two rounds, 49 us
 //    against 27 with 4).
 static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool may_split) {
   auto ctas = [&](int bn) { return (long)tiles * ((M + bn - 1) / bn); };
@@ -887,7 +886,7 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool may_split) 
     for (int i = 0; i < 3; ++i)
       for (int bn = 16; bn <= 128; bn *= 2) {
         const int s = 2 << i;
-        if (nkb < 2 * s || ctas(bn) > most[i] || (bn > 16 && bn / 2 >= M)) continue;
+        if (nkb < 2 * s || ctas(bn) * 148 > (long)most[i] * num_sms || (bn > 16 && bn / 2 >= M)) continue;
         const float c = 0.19f * ((nkb + s - 1) / s) + 1.1f + per_token[i] * std::min(bn, M);
         if (c < cost) cost = c, best.bn = bn, best.splits = s;
       }

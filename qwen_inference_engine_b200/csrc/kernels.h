@@ -128,6 +128,7 @@ struct FastAttnArgs {
   int max_pages, n_tok, n_q, layer, n_splits;
   float scale_log2;  // log2(e) / sqrt(hd)
   int max_kv_len;    // prompts: upper bound on the positions a row sees (how the work is split)
+  int num_sms;       // the same
   float* ws_o;       // [n_splits][n_tok][n_q][hd]
   float* ws_ml;      // [n_splits][n_tok][n_q][2]
   KvGeom kv;
