@@ -1,6 +1,6 @@
 // ops_ref_order.cu -- the non-GEMM operators of the forward, written so that every
 // floating-point result is produced by the same sequence of IEEE operations as the
-// reference kernel it replaces (citations relative to /root/reference/layers/), while
+// reference kernel it replaces (citations relative to the reference's layers/), while
 // the work is spread over warps/blocks instead of one thread per token:
 //   rmsNorm        src/normalization.cu:5-26   sequential FFMA chain (kept: it IS the spec)
 //   qkNorm         src/qk_norm.cu:43-80        shared-memory tree  -> same tree in shuffles
@@ -239,7 +239,7 @@ cudaError_t launch_rope_ref(const float* cos_t, const float* sin_t, bf16* x, int
 // ---- fused q/k-norm + RoPE + KV store: replaces 2x qkNorm + 2x RoPE + the
 // cudaMemcpy2D scatter of kv_copy_layer_to_cache_* (include_cuda.cu:165-279) ------------
 // One warp = up to QP_HEADS consecutive heads (q heads, then k heads, then v heads) of one token: the token's position,
-// page and RoPE row are looked up once, the heads' rows are requested together and processed one after the other (r02:
+// page and RoPE row are looked up once, the heads' rows are requested together and processed one after the other (
 // one warp per (token, head) ran a chain of three dependent global loads per 256 bytes of payload -- 23.9 us for 33 MB
 // on a 4096-token prefill).  The arithmetic per head is unchanged (head_norm / head_rope).
 constexpr int QP_HEADS = 4;
@@ -555,7 +555,7 @@ cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
 
 // ------------------------------------------------------------------ sampling
 // The reference runs ONE block of 256 threads and, for each of k rounds, a strided scan
-// + shared-memory arg-max whose tie-break is a function of (idx & 255) (SURVEY 8a S1):
+// + shared-memory arg-max whose tie-break is a function of (idx & 255):
 // value, then the larger bit-reversed low byte of idx, then the lower idx.  That is a
 // total order, so the scan can use any number of threads and still pick the same token.
 __global__ void __launch_bounds__(1024) sample_topk_kernel(const bf16* __restrict__ logits, int* __restrict__ out,
@@ -896,12 +896,123 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
 // bound that at least k values of the slice reach; the values that reach it (about 1.1 k of them) are the slice's candidates.  The first
 // CTA gathers the candidates of all slices through distributed shared memory, finds the k-th value by bisection over its 16 bits,
 // ranks what is left by counting (all keys differ) and runs the reference's tail: quotients and exponentials by a thread each, the
-// two sums in the reference's order.  Where ties (a row of equal logits) or fewer threads than k with a value (vocabularies of 4 to 8
-// thousand) leave more candidates than the lists hold, the k-th key itself is found by bisection over its 48 bits: in the slice by
-// counting passes over it, in the first CTA over what it gathered.
+// two sums in the reference's order.  Where ties (a row of equal logits) leave more candidates than the lists hold, the slice takes four more
+// passes to pick its k best, and the first CTA bisects the lower half of the keys.
 // One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384; here 18.5 and 39.  The bound
 // is the latency of the steps, not memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 15.6 us, 29 here.
 constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;
+// order-preserving 16 bits; 0: never selected
+__device__ __forceinline__ uint32_t topk_order16(uint32_t b) {
+  if (!topk_valid((uint16_t)b)) return 0u;
+  if (b == 0x8000u) b = 0;  // -0.0 == +0.0
+  return (b & 0x8000u) ? (uint32_t)(uint16_t)~b : (b | 0x8000u);
+}
+template <int TC_THREADS>
+struct TopkSlice {  // elements in front of the first 16-byte boundary and behind the last whole piece belong to the first slice
+  const uint16_t* row;
+  size_t v0, v1;
+  int head, tail0, loose;
+  template <class F>
+  __device__ __forceinline__ void each(F&& f) const {  // f(order16, bits, index) for this thread's share of the slice
+    const int tid = threadIdx.x;
+    constexpr int U = 4;  // loads on their way together, whatever the compiler makes of the loop
+    for (size_t v = v0 + tid; v < v1; v += U * TC_THREADS) {
+      uint32_t w[U][4];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint16_t* p = row + head + min(v + u * TC_THREADS, v1 - 1) * 8;
+        asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[u][0]), "=r"(w[u][1]), "=r"(w[u][2]), "=r"(w[u][3]) : "l"(p));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i0 = head + (int)(v + u * TC_THREADS) * 8;
+        if (v + u * TC_THREADS < v1) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            f(topk_order16(w[u][e] & 0xffffu), w[u][e] & 0xffffu, i0 + 2 * e);
+            f(topk_order16(w[u][e] >> 16), w[u][e] >> 16, i0 + 2 * e + 1);
+          }
+        }
+      }
+    }
+    if (tid < loose) {
+      const int i = tid < head ? tid : tail0 + tid - head;
+      f(topk_order16(row[i]), (uint32_t)row[i], i);
+    }
+  }
+};
+// Every thread's c summed up, one barrier a sum: three counters in turn, the next one cleared in front of the barrier behind which it is added to and
+// after all have read what it held.  They start at zero.
+struct TopkSums {
+  int* cnt;
+  int at;
+  __device__ __forceinline__ int operator()(int c) {
+    const int next = at == 2 ? 0 : at + 1;
+    if (threadIdx.x == 0) cnt[next] = 0;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&cnt[at], c);
+    __syncthreads();
+    c = cnt[at];
+    at = next;
+    return c;
+  }
+};
+// Exactly k of a slice of which more than TC_CAP values reach `bound`.  v: the value that the slice's k-th has (the bound itself, unless many large
+// values share few threads); of those that equal it the best by the key's lower half: bit-reversed low byte of the index, largest first, then index.
+// cls: 256 ints (ties by low byte); tie: indices of one low byte, a 2048-th of the row and one more.  Not inlined: beside the kernel's own passes its
+// copies of the loop cost those 15 %.
+template <int TC_THREADS>
+__device__ __noinline__ void topk_slice_ties(const TopkSlice<TC_THREADS> sl, TopkSums sum, uint32_t mx, uint32_t bound, int k, unsigned long long* cand, int* cls,
+                                              int* tie, int* s_n, int* s_tot) {
+  const int tid = threadIdx.x;
+  auto count = [&](uint32_t t) {  // values that reach t
+    int c = 0;
+    if (mx >= t) sl.each([&](uint32_t o, uint32_t, int) { c += o >= t; });
+    return sum(c);
+  };
+  uint32_t v = bound;
+  int above = count(v + 1);
+  if (above >= k) {
+    v = 0;
+#pragma unroll 1
+    for (int bit = 15; bit >= 0; --bit)
+      if (count(v | (1u << bit)) >= k) v |= 1u << bit;
+    above = count(v + 1);
+  }
+  int need = k - above;
+  if (tid < 256) cls[tid] = 0;
+  __syncthreads();
+  if (mx >= v) sl.each([&](uint32_t o, uint32_t, int i) { if (o == v) atomicAdd(&cls[i & 255], 1); });
+  __syncthreads();
+  const int mine = tid < 256 ? cls[__brev((uint32_t)tid << 24)] : 0;  // thread = reversed byte
+  uint32_t rv = 0;  // the reversed byte in which the last needed tie lies
+#pragma unroll 1
+  for (int bit = 7; bit >= 0; --bit)
+    if (sum(tid >= (int)(rv | (1u << bit)) ? mine : 0) >= need) rv |= 1u << bit;
+  need -= sum(tid > (int)rv ? mine : 0);
+  const int byte = (int)__brev(rv << 24);
+  if (tid == 0) *s_n = 0;
+  __syncthreads();
+  if (mx >= v) sl.each([&](uint32_t o, uint32_t, int i) { if (o == v && (i & 255) == byte) tie[atomicAdd(s_n, 1)] = i; });
+  __syncthreads();
+  const int n_tie = *s_n;
+  for (int i = tid; i < n_tie; i += TC_THREADS) {
+    int before = 0;
+    for (int j = 0; j < n_tie; ++j) before += tie[j] < tie[i];
+    if (before == need - 1) *s_tot = tie[i];
+  }
+  __syncthreads();
+  const int last = *s_tot;
+  if (tid == 0) *s_n = 0;
+  __syncthreads();
+  if (mx >= v)
+    sl.each([&](uint32_t o, uint32_t b, int i) {
+      const uint32_t r = __brev((uint32_t)i << 24);
+      if (o > v || (o == v && (r > rv || (r == rv && i <= last)))) cand[atomicAdd(s_n, 1)] = topk_key((uint16_t)b, i);
+    });
+  __syncthreads();
+  if (tid < 3) sum.cnt[tid] = 0;
+}
 template <int TC_THREADS>
 __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
@@ -914,39 +1025,20 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   __shared__ unsigned long long best[TC_CAP];         // first CTA: those that reach the k-th value
   __shared__ float vals[TC_MOST];
   __shared__ int idxs[TC_MOST];
-  __shared__ int s_n, s_cnt, s_tot;
+  __shared__ int s_n, s_cnt[3], s_tot;
   __shared__ float s_u;
   const int tid = threadIdx.x, slice = blockIdx.x, rowi = blockIdx.y;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(logits) + (size_t)rowi * vocab;
   if (!(temperature > 0.0f)) temperature = 1.0f;
   k = min(k, (int)min(vocab, (size_t)TC_MOST));
-  // elements in front of the first 16-byte boundary and behind the last whole piece belong to the first slice
-  const int head = (int)min((size_t)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / 2, vocab);
-  const size_t nvec = (vocab - head) / 8, per = (nvec + TC_CTAS - 1) / TC_CTAS, v0 = min(nvec, slice * per), v1 = min(nvec, v0 + per);
-  const int tail0 = head + (int)nvec * 8, loose = slice == 0 ? head + (int)vocab - tail0 : 0;
-  // order-preserving 16 bits; 0: never selected
-  auto order16 = [](uint32_t b) -> uint32_t {
-    if (!topk_valid((uint16_t)b)) return 0u;
-    if (b == 0x8000u) b = 0;  // -0.0 == +0.0
-    return (b & 0x8000u) ? (uint32_t)(uint16_t)~b : (b | 0x8000u);
-  };
-  auto each = [&](auto&& f) {  // f(order16, bits, index) for this thread's share of the slice
-    for (size_t v = v0 + tid; v < v1; v += TC_THREADS) {
-      const uint4 q = *reinterpret_cast<const uint4*>(row + head + v * 8);
-      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        f(order16(w[e] & 0xffffu), w[e] & 0xffffu, head + (int)v * 8 + 2 * e);
-        f(order16(w[e] >> 16), w[e] >> 16, head + (int)v * 8 + 2 * e + 1);
-      }
-    }
-    if (tid < loose) {
-      const int i = tid < head ? tid : tail0 + tid - head;
-      f(order16(row[i]), (uint32_t)row[i], i);
-    }
-  };
+  TopkSlice<TC_THREADS> sl;
+  sl.row = row;
+  sl.head = (int)min((size_t)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / 2, vocab);
+  const size_t nvec = (vocab - sl.head) / 8, per = (nvec + TC_CTAS - 1) / TC_CTAS;
+  sl.v0 = min(nvec, slice * per), sl.v1 = min(nvec, sl.v0 + per);
+  sl.tail0 = sl.head + (int)nvec * 8, sl.loose = slice == 0 ? sl.head + (int)vocab - sl.tail0 : 0;
   uint32_t mx = 0;
-  each([&](uint32_t o, uint32_t, int) { mx = max(mx, o); });
+  sl.each([&](uint32_t o, uint32_t, int) { mx = max(mx, o); });
   // the largest bound that k maxima reach (1 if fewer threads have a value: then every value is a candidate)
   uint32_t bound = 0;
 #pragma unroll 1
@@ -956,41 +1048,16 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   }
   bound = max(bound, 1u);
   if (tid == 0) s_n = 0;
+  if (tid < 3) s_cnt[tid] = 0;
   __syncthreads();
   if (mx >= bound)
-    each([&](uint32_t o, uint32_t b, int i) {
+    sl.each([&](uint32_t o, uint32_t b, int i) {
       if (o < bound) return;
       const int at = atomicAdd(&s_n, 1);
       if (at < TC_CAP) cand[at] = topk_key((uint16_t)b, i);
     });
   __syncthreads();
-  // how many of the block's values: every thread's c summed up
-  auto block_sum = [&](int c) {
-    __syncthreads();
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    c = __reduce_add_sync(0xffffffffu, c);
-    if ((tid & 31) == 0 && c) atomicAdd(&s_cnt, c);
-    __syncthreads();
-    return s_cnt;
-  };
-  if (s_n > TC_CAP) {
-    unsigned long long thr = 0;
-#pragma unroll 1
-    for (int bit = 47; bit >= 0; --bit) {
-      const unsigned long long t = thr | (1ull << bit);
-      int c = 0;
-      if (mx >= bound) each([&](uint32_t o, uint32_t b, int i) { c += o >= bound && topk_key((uint16_t)b, i) >= t; });
-      if (block_sum(c) >= k) thr = t;
-    }
-    if (tid == 0) s_n = 0;
-    __syncthreads();
-    if (mx >= bound)
-      each([&](uint32_t o, uint32_t b, int i) {  // exactly k
-        const unsigned long long key = topk_key((uint16_t)b, i);
-        if (o >= bound && key >= thr) cand[atomicAdd(&s_n, 1)] = key;
-      });
-  }
+  if (s_n > TC_CAP) topk_slice_ties<TC_THREADS>(sl, TopkSums{s_cnt, 0}, mx, bound, k, cand, reinterpret_cast<int*>(best), reinterpret_cast<int*>(all), &s_n, &s_tot);
   cluster_sync_all();
   if (slice == 0) {
     // ---- gather
@@ -1010,13 +1077,24 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     // ---- those that reach the actual_k-th value, by bisection over its 16 bits; the actual_k-th key where they are too many
     unsigned long long kth = 0;
     int m = n;  // keys that reach it
+    TopkSums sum{s_cnt, 0};
     if (actual_k > 0) {
+      uint32_t top = 0;
 #pragma unroll 1
-      for (int bit = 47; bit >= 0 && (bit >= 32 || m > TC_CAP); --bit) {
+      for (int bit = 15; bit >= 0; --bit) {
+        const uint32_t t = top | (1u << bit);
+        int c = 0;
+        for (int i = tid; i < n; i += TC_THREADS) c += (uint32_t)(all[i] >> 32) >= t;
+        c = sum(c);
+        if (c >= actual_k) top = t, m = c;
+      }
+      kth = (unsigned long long)top << 32;
+#pragma unroll 1
+      for (int bit = 31; bit >= 0 && m > TC_CAP; --bit) {
         const unsigned long long t = kth | (1ull << bit);
         int c = 0;
         for (int i = tid; i < n; i += TC_THREADS) c += all[i] >= t;
-        c = block_sum(c);
+        c = sum(c);
         if (c >= actual_k) kth = t, m = c;
       }
       if (tid == 0) s_tot = 0;
@@ -1111,18 +1189,21 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
     (void)launch_k(greedy_merge_kernel, dim3((n_rows + 63) / 64), dim3(64), 0, st, (const Cand*)cands, out_tokens, n_rows);
     return cudaGetLastError();
   }
-  if (k > 1 && k <= TC_MOST && vocab < (1u << 24) && n_rows <= 65535) {
-    // many rows: 256 threads, so that more clusters are on the chip at once (64 rows of 151936, k = 50: 39 us, 42 with 512); few rows:
-    // 512, for shorter passes (1 row 18.5, 22 with 256)
+  // (slices longer than a candidate list of which fewer than k threads hold a value, vocabularies of 4 to 8 thousand with large k, have no bound to
+  // start from: 64 rows of 8000, k = 128, 44 us by the radix select, 86 here)
+  if (k > 1 && k <= TC_MOST && vocab <= (1u << 23) && n_rows <= 65535 && (vocab <= (size_t)TC_CTAS * TC_CAP || vocab / (TC_CTAS * 8) > (size_t)k)) {
+    // many rows: 256 threads, so that more clusters are on the chip at once (64 rows of 151936, k = 50: 39 us, 42 with 512), and 5 KB of shared
+    // memory more than they need, so that no SM takes five CTAs while others have two (44); few rows: 512, for shorter passes (1 row 18.5, 22
+    // with 256)
     if (n_rows > 16)
-      (void)launch_k(sample_topk_cluster_kernel<256>, dim3(TC_CTAS, n_rows), dim3(256), 0, st, logits, out_tokens, vocab, temperature, k, seed,
+      (void)launch_k(sample_topk_cluster_kernel<256>, dim3(TC_CTAS, n_rows), dim3(256), 5120, st, logits, out_tokens, vocab, temperature, k, seed,
                      seed_stride, step_ptr, (unsigned long long)subsequence);
     else
       (void)launch_k(sample_topk_cluster_kernel<512>, dim3(TC_CTAS, n_rows), dim3(512), 0, st, logits, out_tokens, vocab, temperature, k, seed,
                      seed_stride, step_ptr, (unsigned long long)subsequence);
     return cudaGetLastError();
   }
-  // more than TC_MOST candidates: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the
+  // more than TC_MOST candidates, and the above: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the
   // 24-bit index field of the key cannot hold, and for k < 1
   if (k > 1 && vocab < (1u << 24))
     (void)launch_k(sample_topk_select_kernel, dim3(n_rows), dim3(1024), 0, st, logits, out_tokens, vocab, temperature, k, seed, seed_stride,

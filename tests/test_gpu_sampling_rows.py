@@ -30,10 +30,16 @@ def row(kind, vocab, rng):
         x[vocab // 2:vocab // 2 + 300] += 40
     if kind == "zeros":
         x = np.where(x > 3, 0.0, -0.0) - (x < 0)
+    if kind == "two values":  # ties at the top over all slices, fewer than k above them
+        x = np.where(rng.random(vocab) < 0.5, 2.0, np.minimum(x, 1.0)).astype(np.float32)
+        x[rng.integers(0, vocab, size=3)] = 5.0
+    if kind == "few threads":  # more large values than a list holds, in the 16-byte pieces of 30 threads of a slice
+        piece = np.arange(vocab) // 8
+        x[piece % max(1, (vocab // 8 + 7) // 8) % 512 < 30] += 25
     return f32_to_bf16(x)
 
 
-@pytest.mark.parametrize("kind", ["normal", "ties", "equal", "few", "one slice", "zeros"])
+@pytest.mark.parametrize("kind", ["normal", "ties", "equal", "few", "one slice", "zeros", "two values", "few threads"])
 @pytest.mark.parametrize("vocab,rows", [(151936, 3), (32001, 5), (8200, 2), (6001, 20), (1000, 2), (519, 9)])
 @pytest.mark.parametrize("k", [1, 2, 50, 128])
 def test_rows_against_the_restatement(layers, oracle, vocab, rows, kind, k):
