@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """bench.py -- the reference's headline metric on B200.
 
-Metric: decode tokens/s.  Workload at N=1 = BASELINE.json configs[1]:
+Metric: decode tokens/s.  Workload at N=1:
 Qwen2.5-0.5B-arch bf16, batch 64 decode, 2048-token context, KV cache resident on one
 B200.  A "step" is one decode step of the whole batch (64 tokens).  N>1 (torchrun, one
 process per GPU) is data-parallel over independent sequences, no data-path collective:
@@ -18,7 +18,7 @@ max-over-ranks device time.
   cpu_baseline : the plain-C oracle (oracle/qie_oracle.c, "port") timed on the host cores
               on a bounded sample.  bench.py is one of the places allowed to run oracle/.
   --impl reference : the reference's own kernels (oracle/_ref, built from
-              /root/reference/layers/src) replaying llm()'s launch order on the GPU --
+              layers/src) replaying llm()'s launch order on the GPU --
               the reference has no CPU implementation; its only implementation is CUDA.
 """
 import argparse
@@ -193,7 +193,7 @@ def _ref_model_on_device(arch_dims):
 
 
 ARCH_DIMS = dict(hidden=896, inter=4864, layers=24, n_q=14, n_kv=2, head_dim=64, vocab=151936, context=32786)
-PROMPT32 = [151643, 785, 50802, 1525, 3818] + list(range(100, 127))  # configs[0]: 32-token prompt
+PROMPT32 = [151643, 785, 50802, 1525, 3818] + list(range(100, 127))  # a 32-token prompt
 
 
 def run_reference(args):
@@ -220,7 +220,7 @@ def run_reference(args):
     dt = time.perf_counter() - t0
     rs.close()
     val = args.steps / dt
-    # configs[0] on the reference's CUDA path: 32-token prompt through its prefill branch, then greedy decode
+    # batch 1 on the reference's CUDA path: 32-token prompt through its prefill branch, then greedy decode
     # (qwen_main.cu:74-247 / :250-404 with k = 1), llm()'s per-op device syncs kept
     extra = {}
     try:
@@ -238,12 +238,12 @@ def run_reference(args):
         tp2 = time.perf_counter()
         r1.close()
         extra["config1_reference_cuda"] = {
-            "workload": "configs[0]: 0.5B-arch, batch 1, 32-token prompt, greedy decode (64 of the 128 tokens timed), the "
+            "workload": "0.5B-arch, batch 1, 32-token prompt, greedy decode (64 of the 128 tokens timed), the "
                         "reference's kernels in llm()'s launch order with its per-op cudaDeviceSynchronize",
             "prefill_ms": 1e3 * (tp1 - tp0), "decode_tokens_per_s": n_dec / (tp2 - tp1), "us_per_token": 1e6 * (tp2 - tp1) / n_dec}
     except Exception as ex:
         extra["config1_reference_cuda_error"] = str(ex)
-    sample = (f"reference CUDA kernels (sm_100a build of /root/reference/layers/src, launch order + syncs of llm() "
+    sample = (f"reference CUDA kernels (sm_100a build of layers/src, launch order + syncs of llm() "
               f"decode) on ONE sequence at context {CTX}.. (KV pages pre-allocated, zero-filled), {args.steps} tokens; "
               "the reference has no batching: a batch of 64 is 64 such calls, so tokens/s is the per-call rate")
     line = {"impl": "reference", "metric": METRIC, "value": val, "unit": "tokens/s", "n_gpus": args.gpus,
@@ -260,7 +260,7 @@ def run_reference(args):
 
 
 def config4_leg(q, torch, np, rank, world, local, use_dist):
-    """the configs[0] workload x 256 sequences (distinct seeded 32-token prompts, greedy decode),
+    """The batch-1 workload x 256 sequences (distinct seeded 32-token prompts, greedy decode),
     256 / N sequences per GPU, full weight replica per GPU, no collective.  Total work is fixed -> strong scaling.
     More than 64 rows run as consecutive persistent launches of <= 64 rows."""
     n_seq = 256 // world
@@ -301,7 +301,7 @@ def config4_leg(q, torch, np, rank, world, local, use_dist):
 
 
 def tp_leg(q, torch, np, rank, world, local):
-    """BASELINE configs[4] inside the driver-visible run: Qwen2.5-7B-arch sharded over the N ranks of this torchrun
+    """Qwen2.5-7B-arch sharded over the N ranks of this torchrun
     (heads / intermediate / vocabulary; o_proj and down_proj partial sums exchanged inside the persistent kernel over
     NVLink peer memory, NCCL all-reduce on the per-operator path), batch 1 and 16; on rank 0 the same model on one GPU
     for the speed-up; a parity run of a 3-layer model against tp_size 1; exchange latency from in-kernel timestamps."""
@@ -736,7 +736,7 @@ def main():
                          "step; fast: the 1e-2-tolerance per-operator path (tcgen05 GEMM, flash-decoding)")
     ap.add_argument("--no-fast-extra", action="store_true", help="skip the fast-numerics side measurement")
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-extra", action="store_true", help="skip the batch-1 (configs[0]) side measurement")
+    ap.add_argument("--no-extra", action="store_true", help="skip the batch-1 side measurement")
     ap.add_argument("--family-compare", action="store_true",
                     help="side measurement (not the contract line): prefill / decode throughput of the Nogatar family beside the "
                          "Qwen family at equal size, with per-kernel-class device times")
@@ -897,7 +897,7 @@ def main():
     peak, peak_src = measured_peaks()
     H, I, hd = cfg.hidden, cfg.inter, cfg.head_dim
     Dq, Dkv = cfg.n_q * hd, cfg.n_kv * hd
-    alg_bytes = {  # algorithmic bytes of ONE launch of each class (DESIGN.md "roofline arithmetic")
+    alg_bytes = {  # algorithmic bytes of ONE launch of each class
         "attention": B * ctx_now * 2 * Dkv * 2 + 2 * B * Dq * 2,
         "gemm_qkv": 2 * H * (Dq + 2 * Dkv) + B * 2 * (H + Dq + 2 * Dkv),
         "gemm_o": 2 * Dq * H + B * 2 * (Dq + 2 * H),
@@ -905,7 +905,7 @@ def main():
         "gemm_down": 2 * H * I + B * 2 * (I + 2 * H),
         "lm_head": 2 * cfg.vocab * H + B * 2 * (H + cfg.vocab),
     }
-    step_bytes = int(q.weight_bytes(cfg) + B * ctx_leg_mean * kvpp + B * kvpp + B * 2 * H)  # SURVEY 8d, context of the TIMED leg
+    step_bytes = int(q.weight_bytes(cfg) + B * ctx_leg_mean * kvpp + B * kvpp + B * 2 * H)  # context of the TIMED leg
     traffic = None
     tp = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if mega:
@@ -1000,7 +1000,7 @@ def main():
         except Exception as ex:
             line.setdefault("extra", {})["fast_numerics_error"] = str(ex)
     if rank == 0 and world == 1 and not args.no_extra:
-        # configs[0] side measurement: batch 1, 32-token prompt, 128 greedy tokens (the parity case)
+        # side measurement: batch 1, 32-token prompt, 128 greedy tokens (the parity case)
         try:
             ids = np.array([151643, 785, 50802, 1525, 3818] + list(range(100, 127)), np.int32)
             s1 = eng.new_sequence()
@@ -1012,7 +1012,7 @@ def main():
             dt = time.perf_counter() - t0
             b1_bytes = q.weight_bytes(cfg) + kvpp * (eng.seq_len(s1) - 60)
             line.setdefault("extra", {})["batch1"] = {
-                "workload": "configs[0]: batch 1, 32-token prompt, greedy decode (qie_decode_run, 120 tokens)",
+                "workload": "batch 1, 32-token prompt, greedy decode (qie_decode_run, 120 tokens)",
                 "persistent_kernel": bool(eng.uses_mega(1, 200)),
                 "tokens_per_s": 120 / dt, "us_per_token": 1e6 * dt / 120,
                 "frac_of_hbm_peak": (b1_bytes * 120 / dt / 1e9) / peak}
@@ -1030,7 +1030,7 @@ def main():
                 eng.decode_run([s1], [int(t_first)], 120)
                 dtf = time.perf_counter() - t0
                 line["extra"]["batch1_fast_numerics"] = {
-                    "workload": "configs[0] batch 1, fast numerics: the GEMV decode kernel (decode_gemv.cu: one persistent launch "
+                    "workload": "batch 1, fast numerics: the GEMV decode kernel (decode_gemv.cu: one persistent launch "
                                 "per token, weight rows streamed by bulk copies, warp-per-row-group FHFMA dot products, "
                                 "split-KV flash decoding, no grid barrier between the phases -- consumers poll per-layer "
                                 "activation buffers; 1e-2 tolerance per layer, tokens not bit-exact)",
@@ -1041,7 +1041,7 @@ def main():
             line.setdefault("extra", {})["batch1_error"] = str(ex)
     eng.close()
     if rank == 0 and world == 1 and not args.no_extra:
-        # configs[2] side measurement: Qwen2.5-1.5B-arch prefill of 4096 tokens (tcgen05 GEMMs + tiled causal
+        # side measurement: Qwen2.5-1.5B-arch prefill of 4096 tokens (tcgen05 GEMMs + tiled causal
         # attention, fast numerics), through qie_prefill with HOST ids in / HOST token out
         try:
             cfg15 = q.make_config("qwen2.5-1.5b", context=8192)
@@ -1073,7 +1073,7 @@ def main():
             except Exception:
                 tpeak = 1377.7
             line.setdefault("extra", {})["prefill_1p5b_4096"] = {
-                "workload": "configs[2]: qwen2.5-1.5b prefill of 4096 tokens in one forward (fast numerics: tcgen05/TMEM/TMA "
+                "workload": "qwen2.5-1.5b prefill of 4096 tokens in one forward (fast numerics: tcgen05/TMEM/TMA "
                             "GEMMs, FlashAttention-2 style causal attention on mma.sync), qie_prefill end to end",
                 "ms": msp, "tokens_per_s": T / (msp / 1e3), "alg_tflop": flop / 1e12,
                 "achieved_tflops": flop / 1e12 / (msp / 1e3), "frac_of_tensor_peak": flop / 1e12 / (msp / 1e3) / tpeak}
@@ -1081,13 +1081,13 @@ def main():
         except Exception as ex:
             line.setdefault("extra", {})["prefill_error"] = str(ex)
 
-    # ---------------- configs[3]: 256 sequences, 32-token prompts, sharded 256 / N per GPU (STRONG scaling) ----------
+    # ---------------- 256 sequences, 32-token prompts, sharded 256 / N per GPU (STRONG scaling) ----------
     if not args.no_extra:
         try:
             line.setdefault("extra", {})["config4_256seq"] = config4_leg(q, torch, np, rank, world, local, use_dist)
         except Exception as ex:
             line.setdefault("extra", {})["config4_error"] = str(ex)
-    # ---------------- configs[4]: Qwen2.5-7B-arch tensor parallel over the N GPUs of this run ---------------------
+    # ---------------- Qwen2.5-7B-arch tensor parallel over the N GPUs of this run ---------------------
     if use_dist and not args.no_extra:
         try:
             line.setdefault("extra", {})["tp"] = tp_leg(q, torch, np, rank, world, local)
@@ -1100,7 +1100,7 @@ def main():
         except Exception as ex:
             line["cpu_baseline"] = {"value": None, "unit": "tokens/s", "cores": os.cpu_count(), "kind": "port",
                                     "sample": f"failed: {ex}"}
-        try:  # the north star's "scalar C++ CPU forward": the same port on ONE thread
+        try:  # a scalar C++ CPU forward: the same port on ONE thread
             line.setdefault("extra", {})["cpu_scalar_1thread"] = cpu_baseline_port(ARCH, sample_tokens=2, prompt_len=4, cores=1)
         except Exception as ex:
             line.setdefault("extra", {})["cpu_scalar_1thread_error"] = str(ex)

@@ -1,5 +1,5 @@
 // include/layers/iengine_compat.hh -- the reference's host-side types and entry points
-// (/root/reference/layers/include/{iengine.cuh,utils.hh,tensor_parser.hh,helpers.cuh,
+// (layers/include/{iengine.cuh,utils.hh,tensor_parser.hh,helpers.cuh,
 // layers_include.cuh}) re-declared on top of libqie_b200, so that iengine's main()
 // (src/iengine.cu:226-482) and llm()'s call sites (src/qwen_main.cu) compile against the
 // B200 library.  Same names, argument order and meaning; what changes is behind them:

@@ -4,7 +4,7 @@
  *
  * Everything here is `extern "C"`, plain pointers / integers / sizes; no C++ or torch
  * types cross the boundary.  Two levels, mirroring the two levels of the reference's
- * header API; citations are relative to /root/reference/layers/:
+ * header API; citations are relative to the reference's layers/:
  *
  *   (1) operator level  -- one entry point per reference __global__ / launch_* wrapper
  *                          (include/layers_include.cuh:15-35, include/helpers.cuh:45-166).
@@ -81,7 +81,7 @@ int qie_elem_mul(const qie_bf16* a, const qie_bf16* b, qie_bf16* c, size_t n, qi
 int qie_residual_add(qie_bf16* a, const qie_bf16* b, size_t n, qie_stream st);
 
 /* KV pool geometry used by the operator-level attention / store entry points.
- * B200 layout (DESIGN.md "KV pool"): one allocation,
+ * B200 layout: one allocation,
  *   pool[page][layer][k|v][kv_head][slot][head_dim]   (bf16)
  * replacing the reference's linked list of per-page cudaMallocs laid out
  * [slot][layer][kv_dim] (include/iengine.cuh:42-48, src/include_cuda.cu:165-279). */
@@ -202,7 +202,7 @@ typedef struct {
  * are bit-identical to the reference's kernels (greedy tokens, logits, activations).
  * FAST: rows > 8 use the tcgen05/TMEM GEMM (+ split-K), decode attention is split-KV
  * flash-decoding, RMSNorm reduces in parallel; results agree with the reference within
- * the 1e-2 bf16 tolerance of BASELINE.json, not bit for bit. */
+ * the 1e-2 bf16 tolerance, not bit for bit. */
 #define QIE_NUMERICS_REFERENCE_ORDER 0
 #define QIE_NUMERICS_FAST 1
 
@@ -258,7 +258,7 @@ int qie_engine_create_synthetic_json(const char* config_json, uint64_t seed, con
 const char* qie_model_families(void);
 const char* qie_engine_family(const qie_engine* e);
 
-/* Tensor parallelism (BASELINE configs[4]; the reference is single-GPU, SURVEY 8e): one
+/* Tensor parallelism (the reference is single-GPU): one
  * process per GPU, every rank creates the engine with the same checkpoint and
  * opts.tp_rank / opts.tp_size, then all ranks call qie_engine_tp_connect with the 128-byte
  * id that rank 0 obtained from qie_tp_unique_id (carried between the processes by the
@@ -415,7 +415,7 @@ long qie_engine_read_activation(qie_engine* e, const char* name, void* h_out, si
 /* Layer-isolation parity hook of the per-operator forward: qie_engine_set_int keys "layer_first" / "layer_count"
  * (run only these layers, no final norm / lm_head; 0 = the whole model) and "inject_x" (1: the residual stream is
  * what qie_engine_write_activation(e, "x", rows, bytes) stored, the embedding gather is skipped).  Lets a test feed
- * layer l of one numerics mode the layer input of another and compare ONE layer's output (north-star 1e-2 bar). */
+ * layer l of one numerics mode the layer input of another and compare ONE layer's output (1e-2 bar). */
 long qie_engine_write_activation(qie_engine* e, const char* name, const void* h_in, size_t bytes);
 
 #ifdef __cplusplus

@@ -1,10 +1,10 @@
 """Generate the golden fixtures in tests/golden/ by running the REFERENCE'S OWN KERNELS
-(oracle/_ref/libqie_ref.so, built from /root/reference/layers/src) on a B200.
+(oracle/_ref/libqie_ref.so, built from layers/src) on a B200.
 
-The reference ships no golden vectors (SURVEY.md section 4), so these fixtures are what
+The reference ships no golden vectors, so these fixtures are what
 pins the oracle: inputs are stored next to the reference outputs, everything is seeded.
-Run on the GPU box:   python oracle/gen_golden.py gpurun_out/golden
-then copy gpurun_out/golden/*.npz to tests/golden/.  TEST INFRASTRUCTURE ONLY.
+Run where there is a GPU:   python oracle/gen_golden.py OUT
+then copy OUT/*.npz to tests/golden/.  TEST INFRASTRUCTURE ONLY.
 """
 import os
 import sys
@@ -140,7 +140,7 @@ def main(out_dir):
             e2e[f"{arch}_L0_{tag}"] = taps[(tag, 0)]
             e2e[f"{arch}_L{last}_{tag}"] = taps[(tag, last)]
         eng.close()
-    # BASELINE.json configs[0]: 0.5B-arch, 32-token prompt, 128 greedy tokens
+    # 0.5B-arch, 32-token prompt, 128 greedy tokens
     eng = q.Engine(synthetic="qwen2.5-0.5b", seed=1234, max_batch_tokens=64, kv_bytes=256 << 20)
     ids = prompt_ids(32, eng.config.vocab)
     rs = RefSeq(ref, ref.model_desc(eng), page_size=4)
@@ -163,4 +163,4 @@ def main(out_dir):
 
 
 if __name__ == "__main__":
-    main(sys.argv[1] if len(sys.argv) > 1 else "gpurun_out/golden")
+    main(sys.argv[1] if len(sys.argv) > 1 else "golden_out")

@@ -2,7 +2,7 @@
 
   * `Oracle`  -> oracle/libqie_oracle.so, the plain-C CPU restatement (qie_oracle.c)
   * `Ref`     -> oracle/_ref/libqie_ref.so, the reference's OWN CUDA kernels compiled from
-                 /root/reference/layers/src (oracle/Makefile) + ref_driver.cu. Needs a GPU.
+                 layers/src (oracle/Makefile) + ref_driver.cu. Needs a GPU.
 
 Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs
 import this module.  The product package never does.

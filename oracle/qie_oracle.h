@@ -6,14 +6,14 @@
  * legs may load this library.  The product (qwen_inference_engine_b200/) never links,
  * imports or executes anything under oracle/.
  *
- * Parity pin: the reference ships no golden vectors or tests (SURVEY.md section 4), so
+ * Parity pin: the reference ships no golden vectors or tests, so
  * this restatement is pinned against outputs of the reference's OWN kernels compiled
- * from /root/reference/layers/src into oracle/_ref/libqie_ref.so and run on a B200
+ * from layers/src into oracle/_ref/libqie_ref.so and run on a B200
  * (oracle/gen_golden.py -> tests/golden/).  Until those fixtures exist the oracle is
  * "parity unpinned".
  *
  * Every function cites the reference file:line it follows (paths relative to
- * /root/reference/layers/).
+ * layers/).
  */
 #ifndef QIE_ORACLE_H
 #define QIE_ORACLE_H
@@ -62,7 +62,7 @@ void orc_matmul(const orc_bf16* A, const orc_bf16* B, orc_bf16* C, int M, int N,
 /* src/qk_norm.cu:43-80 qkNorm (in place; one block per head, tree reduction) */
 void orc_qknorm(orc_bf16* qk, const orc_bf16* w, int head_dim, int n_tok, int row_dim, int n_heads);
 void orc_qknorm_eps(orc_bf16* qk, const orc_bf16* w, int head_dim, int n_tok, int row_dim, int n_heads, float eps);
-/* Qwen2.5 / HF semantics that the reference does not have (SURVEY 8f rank 1) */
+/* Qwen2.5 / HF semantics that the reference does not have */
 void orc_rope_half(const float* cos_values, const float* sin_values, orc_bf16* x, int n_tok, int head_dim, int row_dim, int n_heads);
 void orc_add_bias(orc_bf16* y, const orc_bf16* b, int n_tok, int dim);
 
@@ -101,7 +101,7 @@ void orc_attention(const orc_bf16* Q, orc_bf16* out, size_t seq_len_q, size_t se
  * (block of 256 threads, k rounds of blockArgMax :19-33, XORWOW draw :255-268). */
 int orc_sample_topk(const orc_bf16* logits, float temperature, int k, size_t vocab, uint64_t seed,
                     uint64_t subseq);
-/* the k=1 special case, spelled out as the closed-form tie-break rule (SURVEY 8a S1) */
+/* the k=1 special case, spelled out as the closed-form tie-break rule */
 int orc_argmax_ref_tiebreak(const orc_bf16* logits, size_t vocab);
 void orc_repetition_penalty(orc_bf16* logits, const int* context_tokens, size_t context_len, int vocab, float penalty);
 

@@ -1,12 +1,12 @@
 // ref_driver.cu -- TEST INFRASTRUCTURE ONLY (oracle/).  Thin extern "C" driver around
 // the reference's OWN kernels and launch wrappers, compiled from the sources where they
-// lie under /root/reference/layers (see oracle/Makefile; nothing of the reference is
+// lie under layers (see oracle/Makefile; nothing of the reference is
 // copied into this repository).  It exists so that tests can compare libqie_b200's
 // results with the reference's on a B200 bit for bit, and so that bench.py --impl
 // reference can time the reference's CUDA path.
 //
 // Why a replay and not llm() itself: llm() (src/qwen_main.cu:64-417) hard-wires the
-// Qwen3-14B dimensions (literal 5120s, SURVEY.md fact 2) and prints/dumps per layer.
+// Qwen3-14B dimensions (literal 5120s) and prints/dumps per layer.
 // ref_forward_* below issues exactly llm()'s kernel sequence through the reference's
 // helpers.cuh wrappers with the dimensions taken from a struct instead, including the
 // cudaDeviceSynchronize() calls llm() makes in its decode branch.
@@ -29,7 +29,7 @@
 // The SAME driver compiles two ways (oracle/Makefile):
 //   default            against the reference's own helpers.cuh + kernels            -> _ref/libqie_ref.so
 //   -DQIE_COMPAT_REPLAY against include/layers/iengine_compat.hh + libqie_b200.so   -> _compat/libqie_compat_replay.so
-// The second build is the drop-in proof for the operator-level boundary (SURVEY 8b): llm()'s call sequence, written
+// The second build is the drop-in proof for the operator-level boundary: llm()'s call sequence, written
 // once against the reference's names (launch_rms, proj/launch_matmul, launch_qknorm, launch_rope[_single],
 // kv_copy_layer_to_cache_*, launch_attn over a page_table list, launch_act/elem/resadd, copy_*_vec, sample_topk_bf16,
 // create_page_list / allocate_page_buffers, ModelBuffers), links and runs against the B200 library unchanged; the two

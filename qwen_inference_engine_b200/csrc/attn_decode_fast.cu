@@ -1,10 +1,10 @@
 // attn_decode_fast.cu -- split-KV flash-decoding over the paged KV pool (fast numerics).
 //
-// Replaces selfattention (/root/reference/layers/src/self_attension.cu:10-149) for decode
+// Replaces selfattention (layers/src/self_attension.cu:10-149) for decode
 // rows when the context is long or the batch is large.  The reference walks a linked list
 // of pages for every kv position and runs the softmax in one thread; its arithmetic order
 // (sequential sum over positions) cannot be parallelised, so this kernel trades bit
-// equality for bandwidth: results agree with the reference within the north-star 1e-2
+// equality for bandwidth: results agree with the reference within 1e-2
 // bf16 tolerance (tests/test_gpu_fast_path.py), the reference-order kernel in
 // ops_ref_order.cu stays the bit-exact path.
 //

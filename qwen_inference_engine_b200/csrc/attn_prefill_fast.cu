@@ -1,11 +1,11 @@
 // attn_prefill_fast.cu -- causal tiled attention for prefill rows over the paged KV pool
 // (fast numerics).
 //
-// Replaces selfattention (/root/reference/layers/src/self_attension.cu:10-149) for the
+// Replaces selfattention (layers/src/self_attension.cu:10-149) for the
 // prefill branch of llm() (qwen_main.cu:160-176): there one block per head loops over the
 // query tokens, walks the page list for every (token, kv position) pair and runs the softmax
 // in one thread -- O(T^2) serial work per head.  Here the T x t score matrix is tiled the
-// FlashAttention-2 way; results agree with the reference within the north-star 1e-2 bf16
+// FlashAttention-2 way; results agree with the reference within 1e-2 bf16
 // tolerance (tests/test_gpu_fast_path.py); ops_ref_order.cu stays the bit-exact path.  attn_prompt_tc.cu takes pages of 16 positions,
 // but for contexts up to 128 of head_dim 64.
 //

@@ -1,5 +1,5 @@
 // attn_ref_rows.cu -- reference-order attention of many rows of one sequence (prompts), bit for bit what attention_ref_kernel
-// (ops_ref_order.cu) and the reference's selfattention (/root/reference/layers/src/self_attension.cu:10-149) compute per row and head.
+// (ops_ref_order.cu) and the reference's selfattention (layers/src/self_attension.cu:10-149) compute per row and head.
 //
 // The order is serial per row and head -- a product tree over the head, a sum of exponentials over the positions, an fma chain per output
 // -- but rows and heads are independent of each other.  A CTA takes `rows` consecutive rows times the G query heads of one kv head, up

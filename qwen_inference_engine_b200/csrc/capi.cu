@@ -551,7 +551,7 @@ static int engine_finish_setup(qie_engine* e) {
     if (!w.in_ln || !w.q || !w.k || !w.v || !w.o || !w.post_ln || !w.up || !w.gate || !w.down)
       return fail(QIE_EIO, "layer %d: missing tensor in checkpoint", l);
   }
-  // biases the forward does not apply would give wrong logits without an error (ADVICE r01): refuse them
+  // biases the forward does not apply would give wrong logits without an error: refuse them
   for (const TensorInfo& t : e->ck.tensors) {
     const std::string& sn = t.short_name;
     const bool is_bias = sn.size() > 5 && sn.compare(sn.size() - 5, 5, ".bias") == 0;

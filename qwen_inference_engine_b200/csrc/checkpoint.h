@@ -1,6 +1,6 @@
 // checkpoint.h -- the reference's on-disk model format: weights.bin (raw bf16 tensors
 // back to back) + model_files/meta_data.txt (the text operator<< of
-// /root/reference/layers/src/tensor_parser.cpp:19-28 emits, 6 lines per tensor).
+// layers/src/tensor_parser.cpp:19-28 emits, 6 lines per tensor).
 // The reference only WRITES that text (it re-parses safetensors at start-up,
 // tensor_parser.cpp:31-129); this loader READS it, addressing tensors by their
 // [begin,end) byte offsets and never by file order.

@@ -216,7 +216,7 @@ qie_engine* qie_compat_engine(__nv_bfloat16* blob) {
     return nullptr;
   }
   // the reference hard-codes top-k 50, T = 1.0 (prefill) / 0.7 (decode), seed 1234 + step (qwen_main.cu:241,381-388);
-  // QIE_COMPAT_TOPK overrides k (1 = the greedy mode BASELINE configs[0] asks for)
+  // QIE_COMPAT_TOPK overrides k (1 = greedy)
   int topk = 50;
   if (const char* v = getenv("QIE_COMPAT_TOPK")) topk = std::max(1, atoi(v));
   qie_engine_set_sampling(e, topk, 1.0f, 0.7f, 1234, 1);

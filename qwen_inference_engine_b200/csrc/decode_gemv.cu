@@ -1,10 +1,10 @@
 // decode_gemv.cu -- the fast-numerics decode step of <= 4 sequences as ONE persistent cooperative kernel built from
-// memory-bound GEMVs (sm_100a).  BASELINE.json's named target is batch-1 decode against the HBM roofline; the
+// memory-bound GEMVs (sm_100a).  The target is batch-1 decode against the HBM roofline; the
 // reference-order kernel (decode_mega.cu) cannot get there because the reference's arithmetic order is a chain of
-// dependent HMMAs / FFMAs per output (DESIGN 3a).  This kernel keeps the reference's ROUNDING POINTS (every operator
+// dependent HMMAs / FFMAs per output.  This kernel keeps the reference's ROUNDING POINTS (every operator
 // output is rounded to bf16 where the reference rounds: matrix_mul.cu, normalization.cu, qk_norm.cu, RoPE.cu, SiLU.cu,
 // element_add.cu, residual_add.cu, self_attension.cu) but sums in whatever order is fastest, so results are within the
-// north star's 1e-2 tolerance per layer, not bit-exact (tests/test_gpu_mega.py, tests/test_gpu_layer_isolation.py).
+// 1e-2 tolerance per layer, not bit-exact (tests/test_gpu_mega.py, tests/test_gpu_layer_isolation.py).
 //
 //   * one CTA per SM, resident for the whole step; weight rows are dealt to the CTAs as CONTIGUOUS row ranges, so a
 //     CTA's share of a projection is one contiguous piece of HBM.  A producer warp streams it with 1-D bulk copies
@@ -359,7 +359,7 @@ struct GvRing {
 // A warp owns an ITEM = R weight rows that share the activation loads (gate/up: two gate rows and their two up rows;
 // lm_head: four neighbouring rows; else two): 32 lanes x 16 bytes per step, the loads of G steps issued in one batch
 // in front of their FMAs.  The step is bound by the length of a warp's dependent instruction stream, not by issue
-// slots or shared-memory bandwidth (DESIGN 3b), so the per-row overhead is what counts: lanes beyond the row read the
+// slots or shared-memory bandwidth, so the per-row overhead is what counts: lanes beyond the row read the
 // weights of step 0 against a block of zeros instead of being predicated (no register clearing), and the R sums of a
 // lane are reduced together -- every exchange halves the values a lane carries; in the end lanes 8 g + i hold row g.
 template <int NB, int KIND>
@@ -1083,7 +1083,7 @@ __device__ __forceinline__ void gv_load_rows(unsigned char* dst, const bf16* src
 }
 
 // phase stamp of a profiled launch (CTA 0, thread 0).  One out-of-line copy: the kernel's straight-line code is several
-// times the 32 KB instruction cache, so everything that is not on the hot path is kept out of it (DESIGN 3b).
+// times the 32 KB instruction cache, so everything that is not on the hot path is kept out of it.
 __device__ __noinline__ void gv_stamp(const MegaArgs& a, int prof_i) {
   if (a.prof && blockIdx.x == 0 && threadIdx.x == 0) {
     a.prof[prof_i] = globaltimer();

@@ -1,7 +1,7 @@
 // decode_mega.cu -- the whole decode step as ONE persistent cooperative kernel (sm_100a).
 //
 // The reference runs a decode token as 18 kernels + 2-4 memcpys per layer, most of them
-// followed by a device sync (llm(), /root/reference/layers/src/qwen_main.cu:250-404).
+// followed by a device sync (llm(), layers/src/qwen_main.cu:250-404).
 // Even with 8 fused launches per layer the step stays launch/latency bound
 // (profiles/r01a_*).  Here one CTA per SM stays resident for the whole step:
 //
@@ -116,7 +116,7 @@ __device__ __forceinline__ unsigned long long globaltimer() {
 // bar.sync orders the CTA's writes before thread 0's release; the release/acquire pair on
 // the counter publishes them device-wide.  Readers fetch activations with ld.cg /
 // cp.async.cg (L2), never through L1.
-// The poll is an acquire load (r02: ld.relaxed + a trailing fence.acq_rel.gpu cost ~0.3 us more per barrier --
+// The poll is an acquire load (ld.relaxed + a trailing fence.acq_rel.gpu cost ~0.3 us more per barrier --
 // batch 64 2954 -> 2918 us per step, batch 1 1042 -> 1007 us per token); it reads the head of the release sequence the
 // CTAs' red.release additions form, so it synchronises with all of them.
 // Measured alternatives (B200, batch 1 and 64): arrivals sharded over 8 counters on separate
@@ -503,7 +503,7 @@ __device__ __forceinline__ void mma_chunk(float (&acc)[MT == 0 ? 1 : MT][4], flo
   // nk16 is a multiple of 4 (chunks are whole 64-wide k blocks), GS divides 4.  The HMMAs of a chain are dependent
   // (20.7 cycles apart) and a warp issues in order, so the fragment loads of the NEXT group are placed BETWEEN the
   // HMMAs of the current one -- step s of the other set right behind step s -- where they issue in the latency
-  // shadow of the HMMA just issued.  (r01 issued a whole group of loads, then the group's HMMAs: both are asm
+  // shadow of the HMMA just issued.  (The first form issued a whole group of loads, then the group's HMMAs: both are asm
   // volatile and keep their order, so ~36 load / address instructions sat on the chain: 59 cycles per k-step at one
   // chain per warp.)
 #pragma unroll
@@ -557,7 +557,7 @@ __device__ __forceinline__ void lm_store(const MegaArgs& a, int tok, int n, floa
 }
 
 // One output pair (token tok, columns n, n+1) of a GEMM phase: the reference's rounding points
-// (R3, R8, R9 of SURVEY 8a).
+// (the reference's rounding points).
 template <int MT>
 __device__ __forceinline__ void epilogue_store(const MegaArgs& a, const Phase& p, int seg, int tok, int n, float v0, float v1,
                                                float w0, float w1, uint32_t res_old) {
@@ -746,7 +746,7 @@ __device__ __forceinline__ void gemm_inner(const MegaArgs& a, const Phase& p, ui
 // Tile-split GEMM phase (more than 16 rows, phases with at most one unit per CTA in the default mapping: QKV, O, DOWN of
 // the 0.5B shape).  The default mapping gives such a phase ONE unit per CTA and spreads its token tiles over warps, so
 // every CTA needs the activations of ALL rows: for down_proj that is the whole [64, I] operand (622 KB at I = 4864)
-// copied from L2 by each of the 148 CTAs, 92 MB of L2 traffic per layer and 29 us (r01).  Here CTA c owns token tile
+// copied from L2 by each of the 148 CTAs, 92 MB of L2 traffic per layer and 29 us at first.  Here CTA c owns token tile
 // c % T and the units c / T, c / T + G, ... (G = grid / T): warp w runs the HMMA chain of its unit for that ONE tile, the
 // A operand is 16 rows -- resident for K = H (29 KB instead of 115 KB), streamed in KC-wide chunks through a 4-stage
 // cp.async ring for down_proj (155 KB per CTA instead of 622 KB, one barrier per chunk) -- and the weights of a unit
@@ -1605,7 +1605,7 @@ __device__ __forceinline__ void attention_phase(const MegaArgs& a, int layer, un
 //  * softmax: one warp per head; the sum chain runs in lane 0 with its operands requested 16 positions ahead;
 //  * PV: warps 0..3 own heads w, w+4, w+8, w+12 with lane l on output dims 2l, 2l+1: one LDS.32 of a V row feeds
 //    the fma chains of all heads of the warp (packed fma (fma.rn.f32x2): two IEEE fp32 fmas per instruction), the four
-//    probabilities of a head arrive with one broadcast LDS.128.  (r01: one warp per head re-read every V row
+//    probabilities of a head arrive with one broadcast LDS.128.  (At first one warp per head re-read every V row
 //    7 times and the phase was bound by shared-memory wavefronts: 27 cycles per position, now ~8.)
 constexpr int AT = NTC;            // positions per K/V tile
 constexpr int AT_BYTES = AT * 128;  // head_dim 64, bf16
@@ -1682,7 +1682,7 @@ __device__ __noinline__ void attention_group_phase(const MegaArgs& a, int layer,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // a task is (row, kv head, part): the query group of a kv head (hsk heads) is cut into parts of hp heads while all
   // tasks still fit one wave of CTAs (batch 64: one part of 7 heads, 128 tasks; batch 32: 4 + 3 heads, 128 tasks; batch
-  // 16: 2 + 2 + 2 + 1, 128 tasks) -- r02 first version: one task per (row, kv head) left most SMs idle below 64 rows
+  // 16: 2 + 2 + 2 + 1, 128 tasks) -- the first form, one task per (row, kv head), left most SMs idle below 64 rows
   const int hsk = a.n_q / a.n_kv, hp = a.attn_hp, nparts = (hsk + hp - 1) / hp;
   const int Dq = a.n_q * HD, Dkv = a.n_kv * HD, QKV = Dq + 2 * Dkv;
   const int ntask = a.B * a.n_kv * nparts;

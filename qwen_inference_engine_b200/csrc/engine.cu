@@ -356,7 +356,7 @@ static int mega_tile_set(const qie_engine* e, int n, int max_kv_len) {
   return 0;
 }
 
-// Tensor-parallel forward (7B-arch over 2/4 GPUs).  Every rank holds the full
+// Tensor-parallel forward (7B-arch over 2 or 4 GPUs, for instance).  Every rank holds the full
 // weight blob and works on its shard by pointer arithmetic: q/k/v/gate/up/lm_head by output rows,
 // o_proj/down_proj by input columns (row stride = the full width).  The two row-parallel GEMMs
 // produce fp32 partial sums (the HMMA accumulators, not yet rounded) that are summed over ranks with
@@ -510,7 +510,7 @@ bool decode_uses_mega(const qie_engine* e, int n, int max_kv_len) {
                                 e->mega_kc[mega_tile_set(e, n, max_kv_len)], 0, e->kv.page_size);
   }
   const int fast = e->opts.numerics == QIE_NUMERICS_FAST;  // fast numerics: persistent kernel for <= 8 rows
-  // more rows than one launch takes (BASELINE configs[3]: 256 sequences on one GPU) run as consecutive launches of
+  // more rows than one launch takes (256 sequences on one GPU) run as consecutive launches of
   // <= MEGA_ROWS_PER_LAUNCH rows: both block sizes must fit
   const int nb = std::min(n, MEGA_ROWS_PER_LAUNCH), tail = n % MEGA_ROWS_PER_LAUNCH;
   if (n > MEGA_ROWS_PER_LAUNCH && (fast || e->mega_layers_run > 0)) return false;

@@ -1,6 +1,6 @@
 // gemm_ref_order.cu -- skinny GEMM  C[M,Nout] = A[M,K] * W[Nout,K]^T  for what the tcgen05 kernels of the reference
 // order (launch_gemm_ref_rows, gemm_tcgen05.cu) do not take, reproducing the accumulation order of the reference's wmma kernel
-// (/root/reference/layers/src/matrix_mul.cu:165-288):
+// (layers/src/matrix_mul.cu:165-288):
 //   * activations are the A operand (row-major 16 x 16 tiles, rows >= M are zero),
 //     weight rows are the B operand ("col" = k-contiguous), exactly as the reference
 //     feeds nvcuda::wmma m16n16k16 (:199-201) which lowers to two HMMA.16816.F32.BF16;
@@ -14,7 +14,7 @@
 //   EPI_STORE     C = bf16(acc)
 //   EPI_RESIDUAL  x = bf16(float(x) + float(bf16(acc)))          (residual_add.cu:7-18)
 //   EPI_SILU_MUL  h = bf16(bf16(up) * bf16(silu(bf16(gate))))    (SiLU.cu:10-23, element_add.cu:4-13)
-// The rounding points are the reference's (SURVEY.md 8a list R3, R8, R9).
+// The rounding points are the reference's.
 #include "common.cuh"
 #include "kernels.h"
 #include "launch.h"

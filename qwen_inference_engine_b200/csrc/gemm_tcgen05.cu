@@ -1,7 +1,7 @@
 // gemm_tcgen05.cu -- C[M,Nout] = A[M,K] * W[Nout,K]^T on the 5th-gen tensor cores
 // (tcgen05.mma, accumulator in TMEM, operands staged by TMA): batched decode
 // (M = sequences) and prefill (M = prompt tokens).  Without a split over K the results are the bits of the
-// reference's wmma kernel (/root/reference/layers/src/matrix_mul.cu:165-288; launch_gemm_ref_rows); fast numerics
+// reference's wmma kernel (layers/src/matrix_mul.cu:165-288; launch_gemm_ref_rows); fast numerics
 // may split K (a fixed-order sum of the splits) and match it within the bf16 tolerance.
 //
 // Swap-AB: the weight tile is the UMMA "A" operand (M = 128 weight rows = 128 TMEM lanes),
@@ -18,7 +18,7 @@
 // own shared memory, the cluster synchronises, and CTA r sums rows [r*128/S, (r+1)*128/S)
 // of all S partials through distributed shared memory (ld.shared::cluster) in rank order
 // -- deterministic -- and applies the epilogue.  No partials in HBM/L2, no second launch.
-// Epilogues keep the reference's rounding points (R3, R8, R9 of SURVEY.md 8a):
+// Epilogues keep the reference's rounding points:
 //   EPI_STORE     C = bf16(acc)
 //   EPI_RESIDUAL  x = bf16(float(x) + float(bf16(acc)))
 //   EPI_SILU_MUL  h = bf16(bf16(up) * bf16(silu(bf16(gate))));  the CTA's 128-lane tile is
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       __syncwarp();
     }
   } else {
-    // ---- epilogue warps 2-9: two warps per TMEM lane quarter, each draining half of the columns (r02: with four warps the
+    // ---- epilogue warps 2-9: two warps per TMEM lane quarter, each draining half of the columns (with four warps the
     // epilogue of a K = 1536 tile -- drain, SiLU * up, 64 KiB of stores -- took longer than the tile's mainloop).  64 tokens at a time
     // go through one of two staging tiles, so one barrier a step is enough: who drains into a tile has passed the barrier behind its
     // last readers.  Plain results leave by bulk copies, a token's 256 bytes each; residuals are requested before the drain.

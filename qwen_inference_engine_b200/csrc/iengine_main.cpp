@@ -1,5 +1,5 @@
 // iengine -- host driver, the B200 counterpart of the reference's main()
-// (/root/reference/layers/src/iengine.cu:226-482): load weights.bin + meta_data.txt, create
+// (layers/src/iengine.cu:226-482): load weights.bin + meta_data.txt, create
 // sequences, prefill, then decode token by token.  Differences that are the point:
 // prompts come from the command line instead of a literal (iengine.cu:325), generation stops
 // at EOS 151645 (the reference checks it at qwen_main.cu:257 but main() loops forever on

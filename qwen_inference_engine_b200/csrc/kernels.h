@@ -78,7 +78,7 @@ struct QkvPostArgs {
   const int* block_table;  // [*, max_pages]
   int max_pages, n_tok, n_q, layer;
   KvGeom kv;
-  // model semantics beyond the reference's (data / option driven, SURVEY 8f rank 1): projection biases (Qwen2.5),
+  // model semantics beyond the reference's (data / option driven): projection biases (Qwen2.5),
   // RMS epsilon (1e-4 in the reference, normalization.cu:9 / qk_norm.cu:46; 1e-6 in HF), half-rotation RoPE
   const bf16 *q_bias = nullptr, *k_bias = nullptr, *v_bias = nullptr;
   float eps = 1e-04f;

@@ -3,7 +3,8 @@
 // prerequisite grids complete, their writes visible) before it touches global memory, and
 // calls pdl_trigger() (griddepcontrol.launch_dependents) right away so the NEXT kernel's
 // CTAs can be scheduled, set up their barriers/TMEM/tensor-map prefetch and -- for the
-// GEMMs -- start streaming weights while this kernel is still running.  Launched without
+// GEMMs -- start streaming weights while this kernel is still running, where shared memory holds CTAs of both (a GEMM's ring of 192 to 224 KB
+// lets it in beside a kernel of a few KB, or when CTAs of this one have left).  Launched without
 // the attribute both instructions are no-ops, so the same kernels work eagerly.
 #pragma once
 #include <cuda_runtime.h>

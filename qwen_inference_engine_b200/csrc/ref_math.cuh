@@ -1,5 +1,5 @@
 // ref_math.cuh -- device functions that reproduce the reference's arithmetic op for op
-// (citations relative to /root/reference/layers/).  Shared by the per-operator kernels
+// (citations relative to the reference's layers/).  Shared by the per-operator kernels
 // (ops_ref_order.cu, gemm_ref_order.cu) and the persistent decode kernel (decode_mega.cu).
 // Translation units including this header are compiled with -fmad=false: every fused
 // multiply-add that nvcc's default contraction makes of the reference's source expressions is
@@ -70,7 +70,7 @@ __device__ __forceinline__ void head_rope(float (&x)[NP][2], const float* __rest
   }
 }
 
-// "HF-correct" RoPE (transformers' rotate_half; Qwen2.5 / Qwen3 checkpoints, SURVEY 8f rank 1): element j of a head
+// "HF-correct" RoPE (transformers' rotate_half; Qwen2.5 / Qwen3 checkpoints): element j of a head
 // pairs with j + hd/2 and both use table column j.  Lane l holds elements 64p + 2l, 64p + 2l + 1: for hd = 128 the
 // partner (+64) is the same lane's p = 1 value; for hd = 64 the partner (+32) lives in lane l ^ 16, same slot.
 template <int NP>
@@ -134,8 +134,8 @@ __device__ __forceinline__ float silu_ref(float x) {
 }
 
 
-// arg-max candidate order of the reference sampler (logit_decode.cu:15-33,182-223; SURVEY 8a
-// S1): value, then the larger bit-reversed low byte of the index, then the lower index.
+// arg-max candidate order of the reference sampler (logit_decode.cu:15-33,182-223):
+// value, then the larger bit-reversed low byte of the index, then the lower index.
 struct Cand {
   float val;
   int idx;

@@ -1,6 +1,6 @@
 // safetensors_convert.cpp -- HF safetensors shards -> the reference's weights.bin + meta_data.txt.
 //
-// What parsed_tensors() does in the reference (/root/reference/layers/src/tensor_parser.cpp:31-129): for every
+// What parsed_tensors() does in the reference (layers/src/tensor_parser.cpp:31-129): for every
 // shard, in the order given, read the 8-byte little-endian header length and the JSON header, walk its keys in
 // byte-lexicographic order (nlohmann::json objects are std::map, :71), keep keys that start with "model." or
 // "lm_" (:74,102), give each kept tensor the running byte range [global_offset, +size) (:94-99), derive

@@ -1,7 +1,7 @@
 // scheduler.cpp -- continuous batching on top of the driver-level C ABI.
 //
 // The reference only sketches this: `enum State {prefill, decode}` and one `batch_metadata` per sequence
-// (/root/reference/layers/include/iengine.cuh:23-37), a second sequence commented out in main()
+// (layers/include/iengine.cuh:23-37), a second sequence commented out in main()
 // (src/iengine.cu:369-373,448-452), the EOS test `generated_token == 151645` at the top of the decode branch
 // (src/qwen_main.cu:257) and a decode loop that never ends (iengine.cu:422).  Here requests queue up, are
 // admitted FIFO while sequence slots and KV pages allow (prefill = llm() in state prefill), all running requests

@@ -23,7 +23,7 @@ bool tp_plan(const qie_config& c, int rank, int size, TpPlan* out) {
     p.kv_row0 = rank * p.n_kv * c.head_dim;
     p.q_row0 = rank * p.n_q * c.head_dim;
   } else if (size % c.n_kv == 0) {
-    // more ranks than kv heads (Qwen2.5-7B: 28 q / 4 kv heads over 8 GPUs, SURVEY 7 "hard parts"): `rep` ranks share one
+    // more ranks than kv heads (Qwen2.5-7B: 28 q / 4 kv heads over 8 GPUs): `rep` ranks share one
     // kv head -- each keeps its own copy of that head's K/V cache -- and split its query group between them as evenly
     // as it goes (7 heads over 2 ranks: 4 + 3).  No padded heads: o_proj takes the columns of the heads a rank owns.
     const int rep = size / c.n_kv, kvh = rank / rep, sub = rank % rep;

@@ -1,7 +1,6 @@
 // tp_nccl.h -- tensor-parallel plumbing: NCCL (loaded at run time, only when tp_size > 1) for the
 // all-reduce after o_proj / down_proj and the all-gather of arg-max candidates, plus the shard plan.
-// The reference has no multi-GPU path at all; BASELINE configs[4] asks for
-// Qwen2.5-7B-arch tensor parallel over NVLink with an NCCL all-reduce after o_proj and down_proj.
+// The reference has no multi-GPU path at all.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>

@@ -1,5 +1,5 @@
 """Data-parallel plumbing: one process per GPU, independent sequences, NO data-path
-collective (SURVEY.md 8e: the reference keeps all state per sequence -- batch_metadata +
+collective (the reference keeps all state per sequence -- batch_metadata +
 ModelBuffers + page list -- so sequences shard naturally).  torch.distributed is used only
 to gather token ids on the host side and to take max-over-ranks timings."""
 import torch

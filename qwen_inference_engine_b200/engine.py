@@ -1,6 +1,6 @@
 """Python mirror of the driver-level C ABI (include/qie_b200.h, section 2).
 
-Names follow the reference's host driver (/root/reference/layers/src/iengine.cu): an
+Names follow the reference's host driver (layers/src/iengine.cu): an
 Engine owns the weight blob + KV pages (main(), iengine.cu:226-482), a sequence is what
 create_new_sequence() returns (iengine.cu:25-47), prefill()/decode_step() are llm() in
 its two states (src/qwen_main.cu:74-247 / 250-404).  All compute happens in
@@ -13,7 +13,7 @@ import numpy as np
 from . import _lib
 from ._lib import Config, EngineOpts, KvView, QieError, check  # noqa: F401
 
-# Qwen2.5 shape table (SURVEY.md 8d). Operator semantics are the reference's (q/k-norm,
+# Qwen2.5 shape table. Operator semantics are the reference's (q/k-norm,
 # no bias, explicit lm_head, interleaved RoPE, eps 1e-4).
 ARCHS = {
     "qwen2.5-0.5b": dict(hidden=896, inter=4864, layers=24, n_q=14, n_kv=2, head_dim=64, vocab=151936),
@@ -24,7 +24,7 @@ ARCHS = {
     "small": dict(hidden=256, inter=640, layers=3, n_q=4, n_kv=2, head_dim=64, vocab=4096),
     "small128": dict(hidden=256, inter=512, layers=2, n_q=2, n_kv=1, head_dim=128, vocab=2048),
 }
-REF_CONTEXT = 32786  # sic: /root/reference/layers/src/utills.cu:14
+REF_CONTEXT = 32786  # sic: layers/src/utills.cu:14
 
 
 def make_config(arch, context=REF_CONTEXT, **over):
@@ -35,7 +35,7 @@ def make_config(arch, context=REF_CONTEXT, **over):
 
 
 def weight_bytes(cfg):
-    """bf16 bytes read per decode step (all layers + norms + lm_head), SURVEY 8d."""
+    """bf16 bytes read per decode step (all layers + norms + lm_head)."""
     H, I, L, hd = cfg.hidden, cfg.inter, cfg.layers, cfg.head_dim
     Dq, Dkv = cfg.n_q * hd, cfg.n_kv * hd
     return 2 * (L * (H * Dq + 2 * H * Dkv + Dq * H + 3 * H * I + 2 * H + 2 * hd) + H + cfg.vocab * H)
@@ -136,7 +136,7 @@ class Engine:
         except Exception:
             pass
 
-    # -- tensor parallel (one process per GPU; SURVEY 8e) ---------------------------
+    # -- tensor parallel (one process per GPU) ---------------------------
     @staticmethod
     def tp_unique_id():
         """128-byte NCCL id; rank 0 creates it and ships it to the other ranks."""

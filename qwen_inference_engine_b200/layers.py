@@ -1,6 +1,6 @@
 """Operator-level mirror of the reference's `layers/` API.
 
-Same names and argument meaning as /root/reference/layers/include/helpers.cuh:45-166
+Same names and argument meaning as layers/include/helpers.cuh:45-166
 (launch_rms, launch_rope, launch_rope_single, launch_matmul, launch_elem, launch_act,
 launch_resadd, launch_attn, launch_qknorm, sample_topk_bf16), so a parity test reads like
 the reference's call site in llm() (src/qwen_main.cu).  Tensors are torch CUDA tensors

@@ -1,5 +1,5 @@
 // tests/compat/main_callseq.cpp -- TEST PROGRAM.  The call sequence of the reference's host driver, main()
-// (/root/reference/layers/src/iengine.cu:226-482), written against include/layers/iengine_compat.hh and linked with
+// (layers/src/iengine.cu:226-482), written against include/layers/iengine_compat.hh and linked with
 // libqie_b200.so: same names, same argument order, same order of calls --
 //   build_indexed_tensors (:245) -> weights.bin into ONE device blob (:117-223) -> create_new_sequence +
 //   initialize_model_buffers (:25-47) -> create_page_list + allocate_page_buffers per page (:334-351) ->

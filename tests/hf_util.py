@@ -2,7 +2,7 @@
 no bias -- the family the reference targets) models, built offline from their configs (no download), saved as bf16
 safetensors and converted with the product's own converter: the fixture for the "HF-correct" semantics tests.  The HF
 model evaluated in fp32 on the bf16 weights is the ground truth the oracle and the engine are held to (1e-2, the
-north-star tolerance)."""
+1e-2 tolerance)."""
 import os
 
 import numpy as np
@@ -62,7 +62,7 @@ def hf_bf16_error(model, ids):
 
 
 def hf_tolerance(model, ids):
-    """1e-2 (north star) where transformers' own bf16 run meets it, else 1.25 x its error + 2e-3"""
+    """1e-2 where transformers' own bf16 run meets it, else 1.25 x its error + 2e-3"""
     return max(1e-2, 1.25 * hf_bf16_error(model, ids) + 2e-3)
 
 

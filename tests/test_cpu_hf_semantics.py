@@ -1,6 +1,6 @@
 """not-gpu: the C oracle's "HF-correct" semantics (half-rotation RoPE, eps 1e-6, q/k/v bias, optional q/k-norm, tied
 lm_head) pinned against Hugging Face transformers itself: tiny random-init Qwen2 and Qwen3 models, converted with the
-product's safetensors converter, forward of the oracle vs the HF model in fp32 (SURVEY 8f rank 1).  The reference's own
+product's safetensors converter, forward of the oracle vs the HF model in fp32.  The reference's own
 semantics on the same checkpoints must NOT match (the switch does something)."""
 import numpy as np
 import pytest

@@ -131,7 +131,7 @@ def test_reference_meta_data_parses_when_present():
         pytest.skip("reference tree not present (GPU box)")
     cfg, total, n = q.inspect_checkpoint(ref_meta)
     assert (cfg.hidden, cfg.inter, cfg.layers, cfg.n_q, cfg.n_kv, cfg.head_dim, cfg.vocab) == (5120, 17408, 40, 40, 8, 128, 151936)
-    assert total == 29536614400  # SURVEY 8d: weights.bin bytes of Qwen3-14B
+    assert total == 29536614400  # weights.bin bytes of Qwen3-14B
 
 
 def test_rope_tables_host_function(oracle):
@@ -156,7 +156,7 @@ def test_tiebreak_closed_form_equals_block_reduction(oracle):
 
 def test_shape_table_and_roofline_bytes():
     c = q.make_config("qwen2.5-0.5b")
-    assert q.weight_bytes(c) == 988016384 and q.kv_bytes_per_pos(c) == 12288  # SURVEY 8d
+    assert q.weight_bytes(c) == 988016384 and q.kv_bytes_per_pos(c) == 12288
     assert q.weight_bytes(q.make_config("qwen2.5-1.5b")) == 3087328256
     assert q.weight_bytes(q.make_config("qwen2.5-7b")) == 14140994560
 

@@ -1,7 +1,7 @@
 """not-gpu: the plain-C oracle (oracle/qie_oracle.c) against the golden fixtures produced
 by the REFERENCE'S OWN KERNELS on a B200 (oracle/gen_golden.py -> tests/golden/*.npz).
 This is what pins the oracle.  Bit-exact wherever a CPU can restate the arithmetic; the
-written tolerance (1e-2 relative, bf16 -- BASELINE.json) where it cannot: GEMM accumulation
+written tolerance (1e-2 relative, bf16) where it cannot: GEMM accumulation
 runs through HMMA on the GPU, and device expf differs from glibc expf in the last ulp."""
 import os
 
@@ -112,7 +112,7 @@ def test_forward_against_reference_kernels(oracle, e2e, arch, tmp_path):
 
 
 def test_config1_fixture_is_sane(e2e):
-    """BASELINE.json configs[0] golden: 128 greedy tokens of the 0.5B-arch model from the
+    """golden: 128 greedy tokens of the 0.5B-arch model from the
     reference kernels; exact top-2 ties occur, so the tie-break rule is load-bearing."""
     toks, margins = e2e["config1_greedy"], e2e["config1_top2_margin"]
     assert toks.shape == (128,) and e2e["config1_prompt"].shape == (32,)

@@ -1,6 +1,6 @@
-"""not-gpu: safetensors -> weights.bin + meta_data.txt converter (SURVEY 8f rank 1).
+"""not-gpu: safetensors -> weights.bin + meta_data.txt converter.
 The expected layout is derived here, independently, from the reference's parsed_tensors()
-(/root/reference/layers/src/tensor_parser.cpp:31-129): shards in the given order, keys in byte-lexicographic
+(layers/src/tensor_parser.cpp:31-129): shards in the given order, keys in byte-lexicographic
 order (nlohmann::json = std::map), only "model." / "lm_" keys, running offsets, lm_* -> short_name "logits"."""
 import json
 import os

@@ -1,7 +1,7 @@
-"""not-gpu: tensor-parallel host logic (SURVEY 8e, BASELINE configs[4]).
+"""not-gpu: tensor-parallel host logic.
 * qie_tp_plan: the shards of all ranks tile heads / intermediate / vocabulary exactly, vocabulary
   shards start at multiples of 256 (the sampler's tie-break key is idx mod 256,
-  /root/reference/layers/src/logit_decode.cu:15-33), indivisible shapes are refused.
+  layers/src/logit_decode.cu:15-33), indivisible shapes are refused.
 * world_size 2 over gloo: column-sharded gate/up + row-sharded down_proj with the plan's
   offsets, partial sums all-reduced, equals the unsharded product (fp64, exact up to sum order)."""
 import os
@@ -50,7 +50,7 @@ def test_plan_refuses_indivisible_shapes():
 
 @pytest.mark.parametrize("arch,tp", [("qwen2.5-7b", 8), ("qwen2.5-0.5b", 4), ("small128", 2), ("qwen2.5-1.5b", 4)])
 def test_plan_with_more_ranks_than_kv_heads(arch, tp):
-    """BASELINE configs[4] names 2/4/8 GPUs; Qwen2.5-7B has 28 q / 4 kv heads.  With more ranks than kv heads, `rep`
+    """2, 4 and 8 GPUs; Qwen2.5-7B has 28 q / 4 kv heads.  With more ranks than kv heads, `rep`
     ranks share one kv head (each caches it) and split its query group: every q head is owned exactly once, a rank's
     q heads all belong to its kv head, o_proj columns = the owned q rows, MLP and vocabulary tile as always."""
     cfg = q.make_config(arch)

@@ -5,7 +5,7 @@
     launch_act / launch_elem / launch_resadd, copy_*_vec, sample_topk_bf16, create_page_list / allocate_page_buffers,
     ModelBuffers; qwen_main.cu:74-247,250-404) -- is compiled TWICE: against the reference's helpers.cuh + kernels
     (oracle/_ref) and against include/layers/iengine_compat.hh + libqie_b200.so (oracle/_compat).  Same source, same
-    exported ref_* functions; this file runs BASELINE configs[0] through both and requires identical tokens, logits and
+    exported ref_* functions; this file runs the batch-1 workload (0.5B-arch, 32-token prompt, greedy) through both and requires identical tokens, logits and
     cache pages.
 (2) tests/compat/main_callseq.cpp -- main()'s call sequence (iengine.cu:226-482: build_indexed_tensors, the weight
     blob, create_new_sequence / initialize_model_buffers, create_page_list / allocate_page_buffers, the llm() loop)

@@ -2,7 +2,7 @@
 reference's own kernels replaying llm()'s launch order (oracle/_ref) on the SAME device
 weight blob, and against the plain-C CPU oracle.
 
-North-star bar (BASELINE.json): greedy token ids bit-exact for the first 128 tokens;
+The bar: greedy token ids bit-exact for the first 128 tokens;
 per-layer activations and logits within 1e-2 relative error in bf16.  Because the
 reference-order kernels reproduce the reference's arithmetic, this file asserts the
 stronger property -- activations and logits BIT-EXACT -- and states the 1e-2 tolerance
@@ -18,7 +18,7 @@ from util import bf16_to_f32, prompt_ids, rel_err, ulp_diff
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-TOL_BF16 = 1e-2  # north_star: per-layer activations and logits, relative, bf16
+TOL_BF16 = 1e-2  # per-layer activations and logits, relative, bf16
 
 
 @pytest.fixture(scope="module")
@@ -66,7 +66,7 @@ def test_greedy_tokens_and_logits_bit_exact_small(qie, ref, arch, n_prompt, n_ne
 
 
 def test_config1_qwen05b_128_greedy_tokens_bit_exact(qie, ref):
-    """BASELINE.json configs[0]: Qwen2.5-0.5B-arch random-init bf16, batch 1, 32-token
+    """Qwen2.5-0.5B-arch random-init bf16, batch 1, 32-token
     prompt, 128-token greedy decode -- token ids identical to the reference's kernels."""
     eng = qie.Engine(synthetic="qwen2.5-0.5b", seed=1234, max_batch_tokens=64, kv_bytes=256 << 20)
     ids = prompt_ids(32, eng.config.vocab)
@@ -156,7 +156,7 @@ def test_checkpoint_file_load_equals_synthetic_and_cpu_oracle(qie, oracle):
 
 
 def test_batched_decode_equals_single_sequence(qie):
-    """batch > 1 has no reference counterpart (SURVEY fact 3): parity = every sequence of a
+    """batch > 1 has no reference counterpart: parity = every sequence of a
     batch produces exactly the tokens it produces alone."""
     eng = qie.Engine(synthetic="small", seed=3, context=256, max_batch_tokens=64, max_seqs=16)
     prompts = [prompt_ids(n, eng.config.vocab, seed=n) for n in (3, 17, 8, 30, 1, 12, 5, 9, 21)]

@@ -1,7 +1,7 @@
 """-m gpu: the FAST-numerics kernels (tcgen05/TMEM/TMA GEMM with split-K, split-KV
 flash-decoding, parallel RMSNorm) against the reference's own kernels and the
-reference-order path.  These kernels change the fp32 summation order, so the bar is the
-north-star tolerance -- 1e-2 relative error in bf16 -- and it is written here."""
+reference-order path.  These kernels change the fp32 summation order, so the bar is a
+tolerance -- 1e-2 relative error in bf16 -- and it is written here."""
 import numpy as np
 import pytest
 
@@ -10,7 +10,7 @@ from util import bf16_to_f32, prompt_ids, rand_bf16, rel_err, rel_l2, to_dev, to
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-TOL_BF16 = 1e-2      # north star: relative error in bf16 (||a-b||/||b|| for a tensor; max-norm for one op)
+TOL_BF16 = 1e-2      # relative error in bf16 (||a-b||/||b|| for a tensor; max-norm for one op)
 TOL_MAXNORM = 3.2e-2  # whole-forward sanity bound: max|a-b|/max|b| <= 4 bf16 ulps of the largest value
                       # (two pipelines that round to bf16 ~20 times per layer differ by an ulp or two per element)
 

@@ -1,7 +1,7 @@
 """-m gpu: the GEMV decode kernel (csrc/decode_gemv.cu: fast numerics, <= 4 rows, one persistent launch per step)
 against the reference-order persistent kernel, which tests/test_gpu_mega.py pins bit for bit to the reference's own
 kernels.  Both engines are fed the SAME input tokens every step (the reference-order engine's samples), so a
-rounding flip in one sampled token cannot turn into a different continuation.  Tolerance: the north star's 1e-2
+rounding flip in one sampled token cannot turn into a different continuation.  Tolerance: 1e-2
 relative error in bf16 on the logits (||a-b|| / ||b||) for models of <= 3 layers, and the KV rows the kernel stores."""
 import numpy as np
 import pytest

@@ -1,4 +1,4 @@
-"""-m gpu: "HF-correct" model semantics through the engine (SURVEY 8f rank 1): real-checkpoint-shaped tiny Qwen2
+"""-m gpu: "HF-correct" model semantics through the engine: real-checkpoint-shaped tiny Qwen2
 (Qwen2.5 family: q/k/v bias, no q/k-norm, tied lm_head) and Qwen3 (q/k-norm, the reference's family) models from
 Hugging Face transformers, converted by qie_convert_safetensors, run with semantics="hf" (half-rotation RoPE, eps 1e-6)
 in both numerics modes -- against transformers in fp32 and against the C oracle's restatement (which
@@ -60,7 +60,7 @@ def test_engine_hf_semantics(oracle, tmp_path, kind, numerics):
 
 
 def test_checkpoint_with_an_unapplied_bias_is_refused(tmp_path):
-    """ADVICE r01: a bias tensor the forward would silently ignore must fail the load, not produce wrong logits"""
+    """a bias tensor the forward would silently ignore must fail the load, not produce wrong logits"""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     import qwen_inference_engine_b200 as q

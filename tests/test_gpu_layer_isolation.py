@@ -1,9 +1,9 @@
-"""-m gpu: the north-star tolerance "per-layer activations within 1e-2 relative error in bf16" checked PER LAYER
-at the full depth and width of the BASELINE architectures (0.5B: 24 layers, 1.5B: 28, 7B: 28) for the FAST
+"""-m gpu: the tolerance "per-layer activations within 1e-2 relative error in bf16" checked PER LAYER
+at the full depth and width of the architectures (0.5B: 24 layers, 1.5B: 28, 7B: 28) for the FAST
 numerics path (tcgen05/TMEM GEMMs with split-K, tiled prefill attention incl. the tcgen05 kernel, split-KV
 flash-decoding, parallel RMSNorm).
 
-Method (VERDICT r01 item 1c): the reference-order engine -- bit-identical to the reference's kernels,
+Method: the reference-order engine -- bit-identical to the reference's kernels,
 tests/test_gpu_e2e_vs_reference.py -- runs the whole model once and keeps every layer's output; then layer l of
 the FAST engine is fed the reference-order INPUT of layer l (qie_engine_write_activation + "layer_first" /
 "layer_count") and its output is compared with the reference-order output of the same layer.  Errors therefore
@@ -17,7 +17,7 @@ from util import prompt_ids, rel_l2
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-TOL = 1e-2  # BASELINE.json north_star: per-layer activations and logits, relative, bf16
+TOL = 1e-2  # per-layer activations and logits, relative, bf16
 
 
 @pytest.fixture(scope="module")
@@ -113,7 +113,7 @@ def test_fast_decode_layers_in_isolation(qie, arch, B, ctx):
 
 
 def test_fast_prefill_1p5b_T4096_one_layer(qie):
-    """BASELINE configs[2] at its stated size: ONE layer of the 1.5B architecture over 4096 prompt tokens -- the
+    """ONE layer of the 1.5B architecture over 4096 prompt tokens -- the
     persistent tcgen05 GEMM (K = 1536 and K = 8960, N = 1536 / 8960 / 2048) and the tcgen05/TMEM attention kernel at
     T = 4096 -- against the reference-order kernels on the same layer input."""
     arch, T = "qwen2.5-1.5b", 4096

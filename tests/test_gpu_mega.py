@@ -50,7 +50,7 @@ def _run(qie, arch, n_seq, n_prompt, n_steps, use_mega):
 @pytest.mark.parametrize("arch,n_seq,n_prompt,n_steps", [
     ("tiny", 1, 3, 20), ("small", 1, 9, 40), ("small", 3, 5, 24), ("small128", 2, 7, 20), ("small", 8, 4, 12),
     ("small", 16, 4, 10), ("small", 40, 3, 8), ("small128", 33, 3, 6), ("tiny", 64, 2, 6),
-    ("small", 150, 2, 5),  # more rows than one launch takes: 64 + 64 + 22 (256 sequences per GPU at N = 1)
+    ("small", 150, 2, 5),  # more rows than one launch takes: 64 + 64 + 22 (256 sequences on one GPU)
 ])
 def test_mega_equals_per_operator_path(qie, arch, n_seq, n_prompt, n_steps):
     want_t, want_l, want_kv = _run(qie, arch, n_seq, n_prompt, n_steps, use_mega=False)
@@ -92,7 +92,7 @@ def test_mega_layer_activations(qie, n_layers):
 
 @pytest.mark.parametrize("arch,n_seq", [("qwen2.5-1.5b", 3), ("qwen2.5-7b", 1)])
 def test_mega_larger_architectures(qie, arch, n_seq):
-    """BASELINE configs[2] / [4] shapes (head_dim 128, 28 layers): the persistent kernel equals the
+    """1.5B and 7B shapes (head_dim 128, 28 layers): the persistent kernel equals the
     per-operator path on the 1.5B and 7B architectures too."""
     want_t, want_l, _ = _run(qie, arch, n_seq, 5, 4, use_mega=False)
     got_t, got_l, _ = _run(qie, arch, n_seq, 5, 4, use_mega=True)
@@ -102,7 +102,7 @@ def test_mega_larger_architectures(qie, arch, n_seq):
 
 
 def test_mega_qwen05b_batch64_long_context(qie):
-    """BASELINE configs[1] shape: 0.5B-arch, 64 sequences, synthetic KV of 300..363 positions
+    """0.5B-arch, 64 sequences, synthetic KV of 300..363 positions
     (several V tiles, ragged lengths) -- tokens and logits equal the per-operator path."""
     cfg = qie.make_config("qwen2.5-0.5b")
     res = {}
@@ -128,7 +128,7 @@ def test_mega_qwen05b_batch64_long_context(qie):
 
 
 def test_mega_config2_batch64_ctx2048_vs_reference_kernels(qie, ref):
-    """BASELINE configs[1] at its stated size: 0.5B-arch, 64 sequences with 2048 cached positions each, ONE persistent
+    """0.5B-arch, 64 sequences with 2048 cached positions each, ONE persistent
     kernel step -- and for three of the 64 rows the reference's own kernels (oracle/_ref, llm()'s decode branch) run
     on the SAME cache contents and input token: logits and the greedy token must be bit-identical."""
     from oracle.oracle import RefSeq
@@ -185,7 +185,7 @@ def test_mega_graph_replay_and_topk(qie):
 
 
 def test_mega_config1_vs_reference_kernels(qie, ref):
-    """BASELINE configs[0] through the persistent kernel: 128 greedy tokens identical to the
+    """the batch-1 workload through the persistent kernel: 128 greedy tokens identical to the
     reference's own kernels."""
     from test_gpu_e2e_vs_reference import _ref_generate
     eng = qie.Engine(synthetic="qwen2.5-0.5b", seed=1234, max_batch_tokens=64, kv_bytes=256 << 20)
@@ -199,7 +199,7 @@ def test_mega_config1_vs_reference_kernels(qie, ref):
 @pytest.mark.parametrize("arch,n_seq", [("small", 1), ("small", 5), ("small128", 3), ("qwen2.5-0.5b", 1)])
 def test_mega_fast_numerics_tolerance(qie, arch, n_seq):
     """FAST numerics in the persistent kernel (<= 8 rows: K split over the warps of a CTA,
-    parallel RMSNorm) against the reference-order kernel: logits within the north-star 1e-2
+    parallel RMSNorm) against the reference-order kernel: logits within 1e-2
     relative error in bf16 (||a-b||/||b||); the sum order differs, so no bit-exactness."""
     from util import rel_l2
     outs = {}
@@ -218,7 +218,7 @@ def test_mega_fast_numerics_tolerance(qie, arch, n_seq):
         outs[numerics] = (cur.copy(), eng.read_activation("logits", n_seq * eng.config.vocab))
         eng.close()
     a, b = outs["fast"][1], outs["reference_order"][1]
-    # <= 3 layers: the north-star 1e-2.  The 24-layer model accumulates the per-layer rounding flips
+    # <= 3 layers: 1e-2.  The 24-layer model accumulates the per-layer rounding flips
     # (every op rounds to bf16; a different fp32 sum order moves values that sit on a rounding
     # boundary), so its final logits are held to 5e-2 and the per-layer bar is carried by the small models.
     assert rel_l2(a, b) < (1e-2 if eng.config.layers <= 3 else 5e-2)
@@ -256,7 +256,7 @@ def test_mega_group_attention_tma_page_sizes_and_ragged_contexts(qie, page_size)
 
 @pytest.mark.parametrize("n_seq,ctx", [(1, 12600), (40, 13000)])
 def test_reference_order_decode_above_12k_context(qie, n_seq, ctx):
-    """SURVEY 8f rank 4: reference-order decode with more than 12 k cached positions (the reference's practical limit):
+    """reference-order decode with more than 12 k cached positions (the reference's practical limit):
     the persistent kernel where the score rows fit its shared memory, the per-operator kernels otherwise -- both give
     the same tokens, logits and cache."""
     res = {}

@@ -1,5 +1,5 @@
 """-m gpu: every operator of libqie_b200 (through the C ABI) against the reference's OWN
-kernel (oracle/_ref, compiled from /root/reference/layers/src) on the same seeded inputs.
+kernel (oracle/_ref, compiled from layers/src) on the same seeded inputs.
 The bar is BIT-EXACT: the reference-order kernels reproduce the reference's arithmetic
 order, so there is no tolerance in this file.  The same calls are also checked against
 the plain-C oracle (bit-exact where the CPU can restate the arithmetic; tolerance where it
@@ -142,7 +142,7 @@ def test_embedding_bit_exact(layers, ref, oracle):
     (128, 12, 2, 2, 19, 1, 0),     # 1.5B head geometry
     (128, 4, 4, 1, 9, 9, 1),       # MHA
     (64, 4, 1, 2, 160, 1, 0),      # config-1 final context length
-    (64, 14, 2, 1, 2048, 1, 0),    # BASELINE configs[1] context: 0.5B head geometry at t = 2048
+    (64, 14, 2, 1, 2048, 1, 0),    # 0.5B head geometry at t = 2048
     (128, 12, 2, 1, 2049, 1, 0),   # 1.5B head geometry, odd length across the 2048 boundary
     (64, 2, 1, 1, 700, 700, 1),    # causal prefill rows over many pages
 ])

@@ -1,4 +1,4 @@
-"""-m gpu: the sampling surface beyond greedy (SURVEY 8f rank 3).
+"""-m gpu: the sampling surface beyond greedy.
 * radix-select top-k kernel vs the reference's k-round scan (oracle/_ref) on adversarial rows: long runs of ties across
   the k-th boundary, +-0, +inf, -inf / NaN entries, fewer finite logits than k, every k from 2 to 256;
 * repetition penalty (declared, never defined in the reference, layers_include.cuh:33): the CUDA operator vs the C oracle

@@ -107,7 +107,7 @@ def test_kv_swap_out_and_in_keeps_generation_bit_exact():
 
 
 def test_bad_requests_are_refused_and_never_wedge_the_queue():
-    """ADVICE r01: a request that can never run (prompt + budget beyond the context, token id outside the vocabulary)
+    """a request that can never run (prompt + budget beyond the context, token id outside the vocabulary)
     is refused at submit; max_running is clamped to what a decode step takes; the good requests around it finish."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")

@@ -28,7 +28,7 @@ def to_host(t):
 
 
 def rel_err(a_u16, b_u16):
-    """max |a-b| / max|b| over bf16 arrays (the north-star 'relative error in bf16')."""
+    """max |a-b| / max|b| over bf16 arrays ('relative error in bf16')."""
     a, b = bf16_to_f32(a_u16).astype(np.float64), bf16_to_f32(b_u16).astype(np.float64)
     return float(np.max(np.abs(a - b)) / (np.max(np.abs(b)) + 1e-30))
 

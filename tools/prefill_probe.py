@@ -1,9 +1,9 @@
-"""Prefill probe (BASELINE configs[2]: Qwen2.5-1.5B-arch bf16, prefill 4096 tokens + decode).
+"""Prefill probe (Qwen2.5-1.5B-arch bf16, prefill 4096 tokens + decode).
 
   python tools/prefill_probe.py --arch qwen2.5-1.5b --tokens 4096 --numerics fast
 
 Times qie_prefill (HOST ids in, HOST token out) with CUDA events on the engine stream; reports
-tokens/s and algorithmic TFLOP/s (SURVEY 8d: 2*T*L*params/layer + 2*V*H + L*n_q*4*hd*T^2/2)
+tokens/s and algorithmic TFLOP/s (2*T*L*params/layer + 2*V*H + L*n_q*4*hd*T^2/2)
 against the measured dense bf16 peak, then a short greedy decode.  One JSON line."""
 import argparse
 import json

@@ -1,4 +1,4 @@
-"""Tensor-parallel probe (BASELINE configs[4]): run under torchrun, one rank per GPU.
+"""Tensor-parallel probe: run under torchrun, one rank per GPU.
 
   python -m torch.distributed.run --nnodes=1 --nproc-per-node 2 --master-addr 127.0.0.1 \
       --master-port 29511 tools/tp_probe.py --arch qwen2.5-7b --steps 64 [--check]
@@ -7,7 +7,7 @@ Every rank builds the same synthetic checkpoint on its GPU, takes its shard by p
 arithmetic (qie_tp_plan) and decodes greedily; o_proj / down_proj partial sums are
 all-reduced with NCCL over NVLink inside the engine.  --check also builds a tp_size 1 engine
 on rank 0 and compares tokens and final logits (tolerance: the bf16 all-reduce rounds the
-partial sums, SURVEY 8e).  Prints ONE JSON line on rank 0; times are CUDA-event device times,
+partial sums).  Prints ONE JSON line on rank 0; times are CUDA-event device times,
 max over ranks."""
 import argparse
 import json
