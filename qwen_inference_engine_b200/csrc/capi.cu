@@ -7,7 +7,6 @@
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
-#include <map>
 #include <mutex>
 #include <string>
 
@@ -260,15 +259,15 @@ struct CallMemory {
   cudaStream_t st = nullptr;
   cudaError_t alloc(size_t bytes, cudaStream_t stream) {
     static std::mutex mu;
-    static std::map<int, cudaMemPool_t> pools;
+    static cudaMemPool_t pools[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     cudaMemPool_t pool;
     {
       std::lock_guard<std::mutex> lock(mu);
-      auto it = pools.find(dev);
-      if (it == pools.end()) {
+      if (!pools[dev]) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -280,9 +279,9 @@ struct CallMemory {
         if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
         (void)cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) return e;
-        it = pools.emplace(dev, pool).first;
+        pools[dev] = pool;
       }
-      pool = it->second;
+      pool = pools[dev];
     }
     st = stream;
     return cudaMallocFromPoolAsync(&p, bytes, pool, stream);

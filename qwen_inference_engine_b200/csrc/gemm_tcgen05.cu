@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
     __syncwarp();
   } else if (warp == 1) {
+    pdl_wait();  // (a wait's limit counts this kernel's time, not its predecessor's)
     const uint32_t idesc = idesc_tc(BM, BN, false);
     const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0;
@@ -584,6 +585,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     }
     __syncwarp();
   } else if (warp == 1) {
+    pdl_wait();  // as above
     const uint32_t idesc = idesc_tc(BM, bn, false);
     const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0, j = 0;

@@ -7,9 +7,9 @@ namespace qie {
 
 __device__ __forceinline__ void mbar_init_tc(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
 __device__ __forceinline__ void mbar_arrive_tc(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// Waits for the phase of this parity.  After about a second it sets *dead, and from then on no wait of the CTA waits: its kernel stores values
+// Waits for the phase of this parity.  After about two seconds it sets *dead, and from then on no wait of the CTA waits: its kernel stores values
 // that are not numbers, lets copies in flight land (drain_tc), reports (report_tc) and returns.  The clock is read only where a wait is long.
-constexpr long long WAIT_CYCLES_TC = 2000000000ll;
+constexpr long long WAIT_CYCLES_TC = 4000000000ll;
 __device__ __forceinline__ bool mbar_wait_tc(uint32_t bar, uint32_t parity, volatile int* dead) {
   long long t0 = 0;
   for (int i = 0;; ++i) {
