@@ -139,7 +139,8 @@ int qie_repetition_penalty(qie_bf16* logits, const int* context_tokens, size_t c
 /* FAST-numerics operators (same contracts as qie_matmul / qie_attention, results within
  * the 1e-2 bf16 tolerance instead of bit-exact): tcgen05/TMEM/TMA GEMM with split-K, and
  * split-KV flash-decoding (one query token per row).  n_splits = 0 picks by what fits on the chip; a number is an upper bound (64 at most, and no
- * more than fit).  Above 8 splits the call takes memory in the order of its stream. */
+ * more than fit).  Above 8 splits, and where a number's clusters would not all find room, the call takes memory in the
+ * order of its stream. */
 int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, int N, int K, qie_stream st);
 int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16* out, const int* pos,
                               const int* slot, const int* block_table, int max_pages, int n_tok, int n_q_heads,

@@ -18,9 +18,9 @@
 //           ldmatrix.trans (V) conflict-free
 //   softmax: online (running max / sum in fp32, exp2f with the scale folded in), P split into
 //           bf16 hi + lo parts for the PV MMA (two MMAs, 16 mantissa bits)
-//   splits: up to FD_CLUSTER of them are a cluster and meet in distributed shared memory; more write partial results (max, sum,
-//           unnormalised O) for attn_combine_kernel.  64 sequences of 2048 positions, 14 heads of 64, 4 splits: 20.7 us
-//           with the second kernel, 18.0 as a cluster
+//   splits: up to FD_CLUSTER of them are a cluster and meet in distributed shared memory; more, and those whose clusters would not all
+//           find room (attention_decode_by_cluster), write partial results (max, sum, unnormalised O) for attn_combine_kernel.  64
+//           sequences of 2048 positions, 14 heads of 64, 4 splits: 20.7 us with the second kernel, 18.0 as a cluster
 #include <algorithm>
 
 #include "cluster.cuh"
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(128) attn_decode_fast_kernel(FastAttnArgs a) {
   }
   __syncthreads();
   // splits of one cluster meet in distributed shared memory: a head's rows, then maxima and sums
-  const bool cluster = a.n_splits > 1 && a.n_splits <= FD_CLUSTER;
+  const bool cluster = a.n_splits > 1 && !a.ws_o;
   float* part = red_ml + 4 * 16 * 2;  // [G][HD], [G][2]
   for (int i = threadIdx.x; i < G * HD; i += 128) {
     const int r = i / HD, d = i % HD;
@@ -326,21 +326,39 @@ __global__ void attn_combine_kernel(FastAttnArgs a, int hd) {
   a.out[(size_t)b * a.n_q * hd + (size_t)h * hd + d] = f2bf(O / L);
 }
 
+// Clusters are placed whole and as many CTAs on an SM as fit, so how many there are decides how they lie.  `cluster_room`: the CTAs in clusters of n_splits that
+// run at once.  Two CTAs an SM of head size 128 and a few GPCs that are no multiple of the cluster leave 240 to 296 of 296 (us, 1400 positions, 12 heads: 17
+// sequences 7 splits 12.4, 18 7 14.0 and 6 12.4, 16 8 11.1 and 17 18.5, 34 4 16.0 and 36 27.4, 44 3 18.8 and 48 33.3, 70 2 24.7).  Head size 64 has room for four an SM, but up to
+// 416 CTAs that would leave SMs idle beside full ones: `three_an_sm` asks for a third of the shared memory (14 heads, 4 splits: 40 sequences 14.6 - 12.7,
+// 52 14.6 - 13.3, 60 14.8 - 21; 8 splits: 18 10.1 - 9.2, 24 10.6 - 9.3, 28 10.7 - 15).  Below 304 CTAs of up to 4 splits it gives nothing (36: 13.7, 12.5, 5 splits 11.4).
+static constexpr int THREE = 228 * 1024 / 3 - 1024 - 256;
+static long cluster_room(int n_splits, int hd, int num_sms) {
+  if (hd == 64) return (n_splits > 4 ? 384L : 512L) * num_sms / 148;
+  return (n_splits > FD_CLUSTER - 1 ? 256L : n_splits > 4 ? 240L : n_splits > 3 ? 272L : n_splits > 2 ? 264L : 296L) * num_sms / 148;
+}
+static bool three_an_sm(long ctas, int n_splits, int hd, int num_sms) {
+  return hd == 64 && ctas > (n_splits > 4 ? 256L : 264L) * num_sms / 148 && ctas <= (n_splits > 4 ? 384L : 416L) * num_sms / 148;
+}
+// splits that meet in a cluster; else they need the workspace
+bool attention_decode_by_cluster(int n_tok, int n_kv, int hd, int n_splits, int num_sms) {
+  return n_splits <= FD_CLUSTER && (hd == 64 || (long)n_splits * n_tok * n_kv <= cluster_room(n_splits, hd, num_sms));
+}
+
 template <int HD>
 static cudaError_t launch_hd(const FastAttnArgs& a, cudaStream_t st) {
   static PerDeviceOnce set;
   constexpr int smem = FastAttnSmem<HD>::TOTAL;
   static_assert(FastAttnSmem<HD>::RING >= 4 * 16 * HD * 4 + 4 * 16 * 2 * 4 + 16 * (HD + 2) * 4, "merge scratch must fit in the KV ring");
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_fast_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_fast_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(smem, THREE));
     if (e != cudaSuccess) return e;
     set.done();
   }
-  const bool cluster = a.n_splits > 1 && a.n_splits <= FD_CLUSTER;
+  const bool cluster = a.n_splits > 1 && !a.ws_o;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(a.n_splits, a.kv.n_kv, a.n_tok);
   cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = cluster && three_an_sm((long)a.n_splits * a.kv.n_kv * a.n_tok, a.n_splits, HD, a.num_sms) ? std::max(smem, THREE) : smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   int na = 0;
@@ -359,7 +377,7 @@ static cudaError_t launch_hd(const FastAttnArgs& a, cudaStream_t st) {
   cfg.numAttrs = na;
   cudaError_t e = cudaLaunchKernelEx(&cfg, attn_decode_fast_kernel<HD>, a);
   if (e != cudaSuccess) return e;
-  if (a.n_splits > FD_CLUSTER) {
+  if (a.n_splits > 1 && !cluster) {
     (void)launch_k(attn_combine_kernel, dim3(dim3(a.n_q, a.n_tok)), dim3(HD), 0, st, a, HD);
     e = cudaGetLastError();
   }
@@ -372,22 +390,31 @@ int attention_decode_most_splits(int n_tok, int n_kv, int hd, int num_sms) {
   return (int)std::max(1L, (hd == 64 ? 7L : 4L) * num_sms / 2 / ((long)n_tok * n_kv));
 }
 
-// The most splits, up to a cluster of 8, whose CTAs are all on the chip, no more than 64-position tiles, none for one or two tiles; 16 and the
-// combining kernel from 4096 positions on, if the caller has the workspace.  Measured (us; 1, 2, 4, 8, 16 splits): 64 x 2048, 64 wide, 128 CTAs a split: 30 21 18 23 29;
+// The most splits, up to a cluster of 8, that find room at once, no more than 64-position tiles, none for one or two tiles; 16 and the combining kernel from
+// 4096 positions on, if the caller allows it.  Measured (us; 1, 2, 4, 8, 16 splits): 64 x 2048, 64 wide, 128 CTAs a split: 30 21 18 23 29;
 // 33 x 700: 12 9.5 7.8 9.3 18; 1 x 2500: 35 20 12 8.1 9.0; 64 x 2048, 128 wide: 47 33 39 51 61; 8 x 300: 10 9.5 8.0 7.2 11; 64 x 100, 64 wide: 4.7 6.2 7.6 13
 // 23; 8 and 16 splits: 1 x 4096 10.5 10.0, 8 x 8192 20.1 16.1, 128 wide 1 x 8192 25.8 17.7, 8 x 8192 30.9 21.9.  (Clusters of 16 find room for a few at a time: the
-// last one 35.)
+// last one 35.)  Not powers of two only (2, 3, 4, 5, 6, 7, 8 splits, 1400 positions; 14 heads of 64, 20 sequences: 13.4 11.1 10.6 9.8 8.9 10.2 9.2, 36: 13.5 12.9 12.5 11.4 12.1 12.1 12.1;
+// 12 heads of 128, 17: 20.1 15.9 15.2 14.4 12.4 12.4 18.5, 24: 20.1 18.5 15.8 14.4 23 23 23).  35 to 37 sequences of 12 heads of 128: 4 with the combining kernel 16.6, 3 in a
+// cluster 18.8, but at 300 positions 10.1 and 9.4.
 int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms, int most) {
   const int tiles = (max_kv_len + TILE - 1) / TILE, fit = attention_decode_most_splits(n_tok, n_kv, hd, num_sms);
-  int s = 1;
-  while (tiles > 2 && 2 * s <= std::min({tiles, fit, tiles >= 64 ? most : FD_CLUSTER})) s *= 2;
+  const long each = (long)n_tok * n_kv;
+  if (tiles <= 2) return 1;
+  if (tiles >= 64 && most > FD_CLUSTER && fit >= most) return most;
+  if (tiles >= 16 && most > FD_CLUSTER && hd == 128 && fit == 4 && 4 * each > cluster_room(4, hd, num_sms)) return 4;
+  int s = std::min({tiles, fit, FD_CLUSTER});
+  while (s > 1 && s * each > cluster_room(s, hd, num_sms)) --s;
   return s;
 }
 
-cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st, int* launches) {
-  if (a.n_tok == 0) return cudaSuccess;
-  if (a.n_q % a.kv.n_kv || a.n_q / a.kv.n_kv > 16 || (a.n_splits > FD_CLUSTER && !a.ws_o)) return cudaErrorInvalidValue;
-  if (launches) *launches = a.n_splits > FD_CLUSTER ? 2 : 1;
+cudaError_t launch_attention_decode_fast(const FastAttnArgs& args, cudaStream_t st, int* launches) {
+  if (args.n_tok == 0) return cudaSuccess;
+  FastAttnArgs a = args;
+  const bool combine = a.n_splits > 1 && !attention_decode_by_cluster(a.n_tok, a.kv.n_kv, a.kv.hd, a.n_splits, a.num_sms);
+  if (a.n_q % a.kv.n_kv || a.n_q / a.kv.n_kv > 16 || (combine && !a.ws_o)) return cudaErrorInvalidValue;
+  if (!combine) a.ws_o = nullptr;  // tells the kernel (a field of its own in FastAttnArgs took the loop of head size 64 from 128 registers to 100, 34.6 us to 40.1 for 2500 positions in one split)
+  if (launches) *launches = combine ? 2 : 1;
   switch (a.kv.hd) {
     case 64: return launch_hd<64>(a, st);
     case 128: return launch_hd<128>(a, st);

@@ -329,7 +329,8 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   else n_splits = std::min({n_splits, 64, attention_decode_most_splits(n_tok, kv->n_kv_heads, kv->head_dim, sms)});
   CallMemory ws;
   const size_t parts = (size_t)n_splits * n_tok * n_q_heads;
-  if (n_splits > FD_CLUSTER) CU(ws.alloc(parts * (kv->head_dim + 2) * sizeof(float), (cudaStream_t)st));
+  if (n_splits > 1 && !attention_decode_by_cluster(n_tok, kv->n_kv_heads, kv->head_dim, n_splits, sms))
+    CU(ws.alloc(parts * (kv->head_dim + 2) * sizeof(float), (cudaStream_t)st));
   FastAttnArgs a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -341,6 +342,7 @@ int qie_attention_decode_fast(const qie_kv_view* kv, int layer, const qie_bf16* 
   a.n_q = n_q_heads;
   a.layer = layer;
   a.n_splits = n_splits;
+  a.num_sms = sms;
   a.scale_log2 = 1.4426950408889634f / sqrtf((float)kv->head_dim);
   a.ws_o = (float*)ws.p;
   a.ws_ml = a.ws_o ? a.ws_o + parts * kv->head_dim : nullptr;
@@ -735,9 +737,8 @@ static int engine_finish_setup(qie_engine* e) {
       CU(make_tensor_map_2d(&m.down, w.down, (int)H, (int)I, 128));
     }
     CU(make_tensor_map_2d(&e->lm_head_map, e->lm_head, c.vocab, (int)H, 128));
-    // what FD_MOST splits of as many rows as have them (attention_decode_most_splits) write: 2 to 20 MB
-    const int decode_rows = attention_decode_most_splits(1, c.n_kv, c.head_dim, e->num_sms) / FD_MOST;
-    e->attn_ws_rows = (size_t)FD_MOST * std::max(1, decode_rows) * c.n_q;
+    // what the splits of a step write, as many as have all their CTAs on the chip (attention_decode_most_splits): about 1 MB
+    e->attn_ws_rows = (size_t)std::max(FD_MOST, attention_decode_most_splits(1, c.n_kv, c.head_dim, e->num_sms)) * c.n_q;
     CU(cudaMalloc(&e->attn_ws, e->attn_ws_rows * (c.head_dim + 2) * sizeof(float)));
   }
   CU(cudaStreamSynchronize(e->stream));

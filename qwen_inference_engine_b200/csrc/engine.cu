@@ -214,6 +214,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.layer = l;
       const int ns = attention_decode_splits(n, c.n_kv, hd, max_kv_len, e->num_sms, FD_MOST);
       a.n_splits = ns;
+      a.num_sms = e->num_sms;
       a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
       a.ws_o = e->attn_ws;
       a.ws_ml = e->attn_ws + e->attn_ws_rows * hd;

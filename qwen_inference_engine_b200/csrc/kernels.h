@@ -128,7 +128,7 @@ struct FastAttnArgs {
   int max_pages, n_tok, n_q, layer, n_splits;
   float scale_log2;  // log2(e) / sqrt(hd)
   int max_kv_len;    // prompts: upper bound on the positions a row sees (how the work is split)
-  int num_sms;       // the same
+  int num_sms;       // the same, and for decode rows
   float* ws_o;       // [n_splits][n_tok][n_q][hd]
   float* ws_ml;      // [n_splits][n_tok][n_q][2]
   KvGeom kv;
@@ -137,7 +137,8 @@ struct FastAttnArgs {
 // a wait that nothing ends, through the same limit and report
 cudaError_t launch_wait_selftest(int* status, cudaStream_t st);
 cudaError_t launch_attention_decode_fast(const FastAttnArgs& a, cudaStream_t st, int* launches = nullptr);
-constexpr int FD_CLUSTER = 8, FD_MOST = 16;  // splits that need no workspace; the most that attention_decode_splits picks
+constexpr int FD_CLUSTER = 8, FD_MOST = 16;  // the largest cluster of splits; the most that attention_decode_splits picks
+bool attention_decode_by_cluster(int n_tok, int n_kv, int hd, int n_splits, int num_sms);  // else ws_o / ws_ml are needed
 int attention_decode_most_splits(int n_tok, int n_kv, int hd, int num_sms);  // as many as have all their CTAs on the chip
 int attention_decode_splits(int n_tok, int n_kv, int hd, int max_kv_len, int num_sms, int most);
 // causal tiled attention for prefill rows (attn_prefill_fast.cu): rows are consecutive positions

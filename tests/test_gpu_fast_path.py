@@ -60,7 +60,12 @@ def test_tcgen05_gemm_vs_reference_kernel(layers, ref, M, N, K):
                                                      # clusters of every size, more splits than tiles, the combining kernel, what `0` picks at length
                                                      (64, 14, 2, 2, 100, 6), (128, 12, 2, 2, 700, 7), (64, 14, 2, 3, 700, 8), (64, 4, 2, 2, 1000, 12),
                                                      (128, 12, 2, 1, 1500, 16), (64, 14, 2, 2, 300, 16), (64, 14, 2, 2, 2300, 24), (128, 4, 2, 2, 900, 40),
-                                                     (64, 14, 2, 2, 4200, 0), (128, 28, 4, 1, 4100, 0), (64, 14, 2, 40, 600, 16)])
+                                                     (64, 14, 2, 2, 4200, 0), (128, 28, 4, 1, 4100, 0), (64, 14, 2, 40, 600, 16),
+                                                     # as many splits as find room at once: 8, 7, 6, 5, 4, 3, 2 of them, three CTAs an SM, and 4 that
+                                                     # find none as clusters
+                                                     (64, 14, 2, 20, 260, 0), (64, 14, 2, 36, 500, 0), (64, 14, 2, 40, 600, 0), (64, 14, 2, 60, 700, 0),
+                                                     (64, 14, 2, 70, 600, 0), (128, 12, 2, 16, 220, 0), (128, 12, 2, 17, 300, 0), (128, 12, 2, 20, 300, 0),
+                                                     (128, 12, 2, 24, 330, 0), (128, 12, 2, 36, 480, 0), (128, 12, 2, 48, 640, 0), (128, 12, 2, 36, 480, 4)])
 def test_flash_decoding_vs_reference_order_attention(layers, hd, n_q, n_kv, B, t, splits):
     """ragged batch: sequence b has t - 13*b (>=1) cached positions."""
     rng = np.random.default_rng(hd + n_q + t)
