@@ -52,48 +52,105 @@ cudaError_t launch_embedding(bf16* out, const bf16* table, const int* ids, size_
 }
 
 // ------------------------------------------------------------------ rmsNorm
-// One block per token.  The reference's sum is a strictly sequential fp32 FFMA chain
-// over the hidden dimension (one thread per token); fp32 addition is not associative, so
-// the chain order is part of the result.  Thread 0 walks the chain out of shared memory
-// (4-cycle dependent FFMA issue, loads hoisted), the block does the rest in parallel.
-__global__ void __launch_bounds__(128) rmsnorm_ref_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                           bf16* __restrict__ y, int hidden, size_t x_stride, float eps) {
+// The reference's sum is a strictly sequential fp32 FFMA chain over the hidden dimension (one thread per token); fp32 addition is not
+// associative, so the chain's order is part of the result.  A block takes R rows into shared memory as they are (bf16), R lanes of one warp
+// walk a chain each side by side, and the block does the rest in parallel.
+// What bounds it: the chain, 4 cycles an element (896 wide 1.9 us).  Its loads are 16 bytes and a group of 32 elements ahead: single floats read
+// inside the loop cost the chain as much again.  us at 1 / 1000 / 4000 rows, before (one row a block, fp32 in shared memory) and now: 896 wide 5.9
+// 6.4 15.7 and 3.9 5.2 8.6; 1536 wide 9.3 9.9 25.9 and 5.6 7.3 12.4; 3584 wide 20.3 21.4 74 and 11.0 13.8 28.0.
+// VEC: rows, weights and results in pieces of 16 bytes; other widths and addresses are taken element by element.
+// Four rows a block from RMS_MANY rows on: from there more than one chain falls to each of an SM's schedulers, and the lanes of one warp share
+// their issue slots (1 and 4 rows a block: 512 rows of 1536 6.1 6.6, 1000 rows 7.4 7.3, 2000 13.8 8.6).
+constexpr size_t RMS_MANY = 6 * 148;
+template <int R, bool VEC>
+__global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, int hidden,
+                                                                        size_t x_stride, int n_tok, float eps) {
+  constexpr int RMS_NT = R > 1 ? 256 : 128;
   pdl_wait();
   pdl_trigger();
-  extern __shared__ float xs[];
-  __shared__ float s_rms;
-  const bf16* xr = x + (size_t)blockIdx.x * x_stride;
-  bf16* yr = y + (size_t)blockIdx.x * hidden;
-  for (int i = threadIdx.x; i < hidden; i += blockDim.x) xs[i] = bf2f(xr[i]);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float sum = 0.f;
-    int i = 0;
-    for (; i + 8 <= hidden; i += 8) {
-      float v0 = xs[i], v1 = xs[i + 1], v2 = xs[i + 2], v3 = xs[i + 3];
-      float v4 = xs[i + 4], v5 = xs[i + 5], v6 = xs[i + 6], v7 = xs[i + 7];
-      sum = __fmaf_rn(v0, v0, sum);
-      sum = __fmaf_rn(v1, v1, sum);
-      sum = __fmaf_rn(v2, v2, sum);
-      sum = __fmaf_rn(v3, v3, sum);
-      sum = __fmaf_rn(v4, v4, sum);
-      sum = __fmaf_rn(v5, v5, sum);
-      sum = __fmaf_rn(v6, v6, sum);
-      sum = __fmaf_rn(v7, v7, sum);
-    }
-    for (; i < hidden; ++i) sum = __fmaf_rn(xs[i], xs[i], sum);
-    s_rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps));  // eps 1e-4 in the reference (normalization.cu:9)
+  extern __shared__ __align__(16) unsigned char rms_rows[];
+  __shared__ float s_rms[R];
+  const int pitch = ((hidden + 7) / 8 + 1) * 16;  // bytes of a row: whole pieces and one more, so that R lanes read different banks
+  const int row0 = blockIdx.x * R, n = min(R, n_tok - row0), tid = threadIdx.x;
+  if constexpr (VEC) {  // all pieces on their way at once
+    const int nv = hidden / 8;
+    const uint32_t dst = smem_u32(rms_rows);
+    for (int r = 0; r < n; ++r)
+      for (int i = tid; i < nv; i += RMS_NT) cp_async16(dst + (uint32_t)(r * pitch + i * 16), x + (size_t)(row0 + r) * x_stride + i * 8);
+    cp_async_commit();
+    cp_async_wait<0>();
+  } else {
+    for (int r = 0; r < n; ++r)
+      for (int i = tid; i < hidden; i += RMS_NT) reinterpret_cast<bf16*>(rms_rows + (size_t)r * pitch)[i] = x[(size_t)(row0 + r) * x_stride + i];
   }
   __syncthreads();
-  const float rms = s_rms;
-  for (int i = threadIdx.x; i < hidden; i += blockDim.x)
-    yr[i] = f2bf(__fmul_rn(__fdiv_rn(xs[i], rms), bf2f(w[i])));
+  if (tid < n) {
+    const uint4* p = reinterpret_cast<const uint4*>(rms_rows + (size_t)tid * pitch);
+    float sum = 0.f;
+    const int groups = hidden / 32;
+    uint4 cur[4], nxt[4];
+    auto add = [&](uint32_t u) {
+      const float a = lo2f(u), b = hi2f(u);
+      sum = __fmaf_rn(a, a, sum);
+      sum = __fmaf_rn(b, b, sum);
+    };
+    if (groups > 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cur[j] = p[j];
+    }
+#pragma unroll 2
+    for (int g = 0; g < groups; ++g) {
+      const uint4* q = p + 4 * min(g + 1, groups - 1);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) nxt[j] = q[j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) add(cur[j].x), add(cur[j].y), add(cur[j].z), add(cur[j].w);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
+    }
+    for (int i = groups * 32; i < hidden; ++i) {
+      const float a = bf2f(reinterpret_cast<const bf16*>(p)[i]);
+      sum = __fmaf_rn(a, a, sum);
+    }
+    s_rms[tid] = __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps));  // eps 1e-4 in the reference (normalization.cu:9)
+  }
+  __syncthreads();
+  if constexpr (VEC) {
+    const int nv = hidden / 8;
+    for (int i = tid; i < nv; i += RMS_NT) {
+      const uint4 wv = reinterpret_cast<const uint4*>(w)[i];
+      const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (r >= n) break;
+        const uint4 v = *reinterpret_cast<const uint4*>(rms_rows + (size_t)r * pitch + i * 16);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+        const float rms = s_rms[r];
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          o[j] = pack2(f2bf(__fmul_rn(__fdiv_rn(lo2f(u[j]), rms), lo2f(ww[j]))), f2bf(__fmul_rn(__fdiv_rn(hi2f(u[j]), rms), hi2f(ww[j]))));
+        reinterpret_cast<uint4*>(y + (size_t)(row0 + r) * hidden)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  } else {
+    for (int r = 0; r < n; ++r)
+      for (int i = tid; i < hidden; i += RMS_NT)
+        y[(size_t)(row0 + r) * hidden + i] = f2bf(__fmul_rn(__fdiv_rn(bf2f(reinterpret_cast<const bf16*>(rms_rows + (size_t)r * pitch)[i]), s_rms[r]), bf2f(w[i])));
+  }
 }
 
 cudaError_t launch_rmsnorm_ref(const bf16* x, const bf16* w, bf16* y, size_t hidden, size_t n_tok, size_t x_stride,
                                cudaStream_t st, float eps) {
   if (n_tok == 0) return cudaSuccess;
-  (void)launch_k(rmsnorm_ref_kernel, dim3((unsigned)n_tok), dim3(128), hidden * sizeof(float), st, x, w, y, (int)hidden, x_stride, eps);
+  const size_t pitch = ((hidden + 7) / 8 + 1) * 16;
+  const bool vec = hidden % 8 == 0 && x_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  if (vec && n_tok >= RMS_MANY && 4 * pitch <= 40 * 1024)
+    (void)launch_k(rmsnorm_ref_kernel<4, true>, dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+  else if (vec)
+    (void)launch_k(rmsnorm_ref_kernel<1, true>, dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+  else
+    (void)launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
   return cudaGetLastError();
 }
 
