@@ -47,7 +47,7 @@ __global__ void embedding_kernel(bf16* __restrict__ out, const bf16* __restrict_
 cudaError_t launch_embedding(bf16* out, const bf16* table, const int* ids, size_t hidden, size_t n_tok,
                              cudaStream_t st) {
   if (n_tok == 0) return cudaSuccess;
-  (void)launch_k(embedding_kernel, dim3((unsigned)n_tok), dim3(128), 0, st, out, table, ids, hidden);
+  (void)launch_spread<embedding_kernel>(dim3((unsigned)n_tok), dim3(128), 0, st, out, table, ids, hidden);
   return cudaGetLastError();
 }
 
@@ -146,9 +146,9 @@ cudaError_t launch_rmsnorm_ref(const bf16* x, const bf16* w, bf16* y, size_t hid
   const size_t pitch = ((hidden + 7) / 8 + 1) * 16;
   const bool vec = hidden % 8 == 0 && x_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   if (vec && n_tok >= RMS_MANY && 4 * pitch <= 40 * 1024)
-    (void)launch_k(rmsnorm_ref_kernel<4, true>, dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+    (void)launch_spread<rmsnorm_ref_kernel<4, true>>(dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
   else if (vec)
-    (void)launch_k(rmsnorm_ref_kernel<1, true>, dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+    (void)launch_spread<rmsnorm_ref_kernel<1, true>>(dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
   else
     (void)launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
   return cudaGetLastError();
@@ -226,7 +226,7 @@ cudaError_t launch_rmsnorm_fast(const bf16* x, const bf16* w, bf16* y, size_t hi
   // (every row count takes this kernel when the layout allows: a row's result must not depend on how a prompt is chunked)
   if (hidden % 8 == 0 && x_stride % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
-    (void)launch_k(rmsnorm_fast_rows_kernel, dim3((unsigned)((n_tok + 7) / 8)), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps,
+    (void)launch_spread<rmsnorm_fast_rows_kernel>(dim3((unsigned)((n_tok + 7) / 8)), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps,
                    (int)n_tok);
     return cudaGetLastError();
   }
@@ -362,7 +362,7 @@ cudaError_t launch_qkv_post(const QkvPostArgs& a, cudaStream_t st) {
   int warps = a.n_tok * ((heads + QP_HEADS - 1) / QP_HEADS);
   if (warps == 0) return cudaSuccess;
   int blocks = (warps + 3) / 4;
-  QIE_DISPATCH_HD(a.kv.hd, ((void)launch_k(qkv_post_kernel<NP>, dim3(blocks), dim3(128), 0, st, a)));
+  QIE_DISPATCH_HD(a.kv.hd, ((void)launch_spread<qkv_post_kernel<NP>>(dim3(blocks), dim3(128), 0, st, a)));
   return cudaGetLastError();
 }
 
