@@ -1,0 +1,244 @@
+// head_ops.cu -- what stands between the q/k/v projections and attention: head norms (layers/src/qk_norm.cu:43-80), rotary positions
+// (layers/src/RoPE.cu:6-22) and the store into the KV pool (layers/src/include_cuda.cu:165-279), as one kernel for the engine
+// and as single operators.  Compiled with -fmad=false, every result by the reference's sequence of IEEE operations (ref_math.cuh).
+//
+// A head of 64 NP values belongs to LH = 4 NP lanes, a warp has 32 / LH heads; they may be of different tokens and kinds.  Lane l holds the 16-byte
+// pieces l and l + LH: the tree's first stride (half a head) is in the lane, the strides down to 8 are exchanges between the LH lanes, 4, 2, 1
+// are in the lane again; interleaved and half-rotation partners are in the lane as well.  Square root, reciprocal and page lookup are done once
+// for all heads of a warp.  One head after the other on 32 lanes with 4-byte accesses took about 250 instructions a head of 128, here 75.
+// What bounds it now: latency of the loads and DRAM; behind a projection 4096 tokens of 16 heads of 128 took 23.5 us
+// and take 11.2, 512 tokens of 18 heads of 64 6.5 and 3.1; head norms and positions alone, 1000 x 12 heads of 128, 3.4 and 3.0, now 2.3 and 2.0.
+#include <initializer_list>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "launch.h"
+#include "ref_math.cuh"
+
+namespace qie {
+namespace {
+
+// 16 bytes; V: the address is a multiple of 16, else of 4
+template <bool V>
+__device__ __forceinline__ uint4 load16(const void* p) {
+  if constexpr (V) return *reinterpret_cast<const uint4*>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+template <bool V>
+__device__ __forceinline__ void store16(void* p, const uint4& v) {
+  if constexpr (V) {
+    *reinterpret_cast<uint4*>(p) = v;
+  } else {
+    uint32_t* w = reinterpret_cast<uint32_t*>(p);
+    w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+  }
+}
+template <bool V>
+__device__ __forceinline__ void load8f(float* f, const bf16* p) {
+  const uint4 u = load16<V>(p);
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[2 * i] = lo2f(w[i]), f[2 * i + 1] = hi2f(w[i]);
+}
+// a lane's share of a head: elements 8 l .. and HD / 2 + 8 l ..
+template <int NP>
+struct Head {
+  static constexpr int LH = 4 * NP, HALF = 32 * NP;
+  float x[16];
+  template <bool V>
+  __device__ __forceinline__ void load(const bf16* p, int l) {
+    load8f<V>(x, p + 8 * l);
+    load8f<V>(x + 8, p + HALF + 8 * l);
+  }
+  template <bool V>
+  __device__ __forceinline__ void store(bf16* p, int l) const {
+#pragma unroll
+    for (int c = 0; c < 16; c += 8)
+      store16<V>(p + c / 8 * HALF + 8 * l, make_uint4(pack2f(x[c], x[c + 1]), pack2f(x[c + 2], x[c + 3]), pack2f(x[c + 4], x[c + 5]), pack2f(x[c + 6], x[c + 7])));
+  }
+  __device__ __forceinline__ void round() {
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+      const uint32_t p = pack2f(x[i], x[i + 1]);
+      x[i] = lo2f(p), x[i + 1] = hi2f(p);
+    }
+  }
+  template <bool V>
+  __device__ __forceinline__ void add_bias(const bf16* b, int l) {  // y = bf16(y + b) on the rounded projection output
+    Head h;
+    h.load<V>(b, l);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = __fadd_rn(x[i], h.x[i]);
+    round();
+  }
+  // sum of the head's squares: for (stride = hd / 2; stride > 0; stride /= 2) buf[t] += buf[t + stride] for t < stride; every lane of the warp takes part
+  __device__ __forceinline__ float squares() const {
+    float s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(__fmul_rn(x[i], x[i]), __fmul_rn(x[i + 8], x[i + 8]));
+#pragma unroll
+    for (int m = LH / 2; m >= 1; m >>= 1)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i] = __fadd_rn(s[i], __shfl_xor_sync(0xffffffffu, s[i], m));
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1)
+#pragma unroll
+      for (int i = 0; i < m; ++i) s[i] = __fadd_rn(s[i], s[i + m]);
+    return s[0];
+  }
+  template <bool V>
+  __device__ __forceinline__ void norm(float sum, const bf16* w, int l, float eps) {  // qk_norm.cu:46-78 (the division by hd, a power of two, is a product)
+    Head h;
+    h.load<V>(w, l);
+    quot16(x, quot_of(__fsqrt_rn(__fadd_rn(__fmul_rn(sum, 1.f / (64 * NP)), eps))));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = __fmul_rn(x[i], h.x[i]);
+    round();
+  }
+  template <bool V>
+  __device__ __forceinline__ static void load4(float* f, const float* p) {
+    const uint4 u = load16<V>(p);
+    f[0] = __uint_as_float(u.x), f[1] = __uint_as_float(u.y), f[2] = __uint_as_float(u.z), f[3] = __uint_as_float(u.w);
+  }
+  template <bool V>
+  __device__ __forceinline__ void rope(const float* cos_row, const float* sin_row, int l) {  // RoPE.cu:15-18: pair j is elements 2 j, 2 j + 1
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float co[4], si[4];
+      load4<V>(co, cos_row + c * (HALF / 2) + 4 * l);
+      load4<V>(si, sin_row + c * (HALF / 2) + 4 * l);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float &x0 = x[8 * c + 2 * i], &x1 = x[8 * c + 2 * i + 1];
+        const float v = __fmaf_rn(x0, co[i], -__fmul_rn(x1, si[i]));
+        x1 = __fmaf_rn(co[i], x1, __fmul_rn(x0, si[i]));
+        x0 = v;
+      }
+    }
+  }
+  template <bool V>
+  __device__ __forceinline__ void rope_half(const float* cos_row, const float* sin_row, int l) {  // rotate_half: element j pairs with j + hd / 2, table column j
+#pragma unroll
+    for (int c = 0; c < 8; c += 4) {
+      float co[4], si[4];
+      load4<V>(co, cos_row + 8 * l + c);
+      load4<V>(si, sin_row + 8 * l + c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float &x0 = x[c + i], &x1 = x[8 + c + i];
+        const float v = __fmaf_rn(x0, co[i], -__fmul_rn(x1, si[i]));
+        x1 = __fmaf_rn(co[i], x1, __fmul_rn(x0, si[i]));
+        x0 = v;
+      }
+    }
+  }
+};
+
+template <int NP, bool V>
+__global__ void __launch_bounds__(128) qkv_post_kernel(QkvPostArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  using H = Head<NP>;
+  constexpr int HD = 64 * NP;
+  const int heads = a.n_q + 2 * a.kv.n_kv, all = a.n_tok * heads;  // q heads, k heads, v heads
+  const int at = (blockIdx.x * 128 + threadIdx.x) / H::LH, l = threadIdx.x % H::LH;
+  const int g = min(at, all - 1), tok = g / heads, h = g - tok * heads;
+  const int kind = h < a.n_q ? 0 : h < a.n_q + a.kv.n_kv ? 1 : 2, kh = h - a.n_q - (kind == 2 ? a.kv.n_kv : 0);  // kh: head within k / v
+  const bf16* src = kind == 0 ? a.q_in + (size_t)tok * a.q_in_stride + (size_t)h * HD : (kind == 1 ? a.k : a.v) + (size_t)tok * a.kv_stride + (size_t)kh * HD;
+  H x;
+  x.template load<V>(src, l);
+  const int ps = a.pos[tok];
+  bf16* dst = a.q + (size_t)tok * a.n_q * HD + (size_t)h * HD;
+  if (kind != 0) {
+    const int page = a.block_table[(size_t)a.slot[tok] * a.max_pages + ps / a.kv.page_size];
+    dst = a.kv.chunk(page, a.layer, kind - 1, kh) + (size_t)(ps % a.kv.page_size) * HD;
+  }
+  const bf16* bias = kind == 0 ? a.q_bias : kind == 1 ? a.k_bias : a.v_bias;
+  if (bias) x.template add_bias<V>(bias + (size_t)(kind == 0 ? h : kh) * HD, l);
+  const float sum = x.squares();
+  const bf16* w = kind == 0 ? a.q_norm_w : a.k_norm_w;
+  if (kind != 2) {
+    if (w) x.template norm<V>(sum, w, l, a.eps);
+    const float *co = a.cos_t + (size_t)ps * H::HALF, *si = a.sin_t + (size_t)ps * H::HALF;
+    if (a.rope_half)
+      x.template rope_half<V>(co, si, l);
+    else
+      x.template rope<V>(co, si, l);
+  }
+  if (at < all) x.template store<V>(dst, l);  // (v: bf16 -> fp32 -> bf16 is the identity)
+}
+
+template <int NP, bool V>
+__global__ void __launch_bounds__(128) qknorm_ref_kernel(bf16* x, const bf16* __restrict__ w, int n_tok, int row_dim, int n_heads) {
+  pdl_wait();
+  pdl_trigger();
+  using H = Head<NP>;
+  const int all = n_tok * n_heads, at = (blockIdx.x * 128 + threadIdx.x) / H::LH, l = threadIdx.x % H::LH;
+  const int g = min(at, all - 1), tok = g / n_heads;
+  bf16* p = x + (size_t)tok * row_dim + (size_t)(g - tok * n_heads) * 64 * NP;
+  H v;
+  v.template load<V>(p, l);
+  v.template norm<V>(v.squares(), w, l, 1e-04f);
+  if (at < all) v.template store<V>(p, l);
+}
+
+template <int NP, bool V>
+__global__ void __launch_bounds__(128) rope_ref_kernel(const float* __restrict__ cos_t, const float* __restrict__ sin_t, bf16* x, int n_tok, const int* __restrict__ pos,
+                                                       int pos0, int row_dim, int n_heads) {
+  pdl_wait();
+  pdl_trigger();
+  using H = Head<NP>;
+  const int all = n_tok * n_heads, at = (blockIdx.x * 128 + threadIdx.x) / H::LH, l = threadIdx.x % H::LH;
+  if (at >= all) return;
+  const int tok = at / n_heads, ps = pos ? pos[tok] : pos0 + tok;
+  bf16* p = x + (size_t)tok * row_dim + (size_t)(at - tok * n_heads) * 64 * NP;
+  H v;
+  v.template load<V>(p, l);
+  v.template rope<V>(cos_t + (size_t)ps * H::HALF, sin_t + (size_t)ps * H::HALF, l);
+  v.template store<V>(p, l);
+}
+
+bool on16(std::initializer_list<const void*> ps) {
+  for (const void* p : ps)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+
+}  // namespace
+
+// (head sizes are multiples of 64, so heads of an aligned row are aligned; strides off 8 elements and other addresses take 4-byte accesses)
+#define QIE_HEADS(hd, vec, CALL)                                                                                  \
+  if (hd == 64) { constexpr int NP = 1; if (vec) { constexpr bool V = true; CALL; } else { constexpr bool V = false; CALL; } }         \
+  else if (hd == 128) { constexpr int NP = 2; if (vec) { constexpr bool V = true; CALL; } else { constexpr bool V = false; CALL; } }   \
+  else if (hd == 256) { constexpr int NP = 4; if (vec) { constexpr bool V = true; CALL; } else { constexpr bool V = false; CALL; } }   \
+  else return cudaErrorInvalidValue
+
+static unsigned blocks_of(long heads, int hd) { return (unsigned)((heads * (hd / 16) + 127) / 128); }
+
+cudaError_t launch_qkv_post(const QkvPostArgs& a, cudaStream_t st) {
+  const long heads = (long)a.n_tok * (a.n_q + 2 * a.kv.n_kv);
+  if (heads == 0) return cudaSuccess;
+  const bool vec = on16({a.q, a.q_in, a.k, a.v, a.q_norm_w, a.k_norm_w, a.cos_t, a.sin_t, a.q_bias, a.k_bias, a.v_bias, a.kv.pool}) && a.q_in_stride % 8 == 0 &&
+                   a.kv_stride % 8 == 0;
+  QIE_HEADS(a.kv.hd, vec, (void)(launch_spread<qkv_post_kernel<NP, V>>(dim3(blocks_of(heads, a.kv.hd)), dim3(128), 0, st, a)));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_qknorm_ref(bf16* x, const bf16* w, int hd, int n_tok, int row_dim, int n_heads, cudaStream_t st) {
+  const long heads = (long)n_tok * n_heads;
+  if (heads == 0) return cudaSuccess;
+  QIE_HEADS(hd, (on16({x, w}) && row_dim % 8 == 0),
+            (void)launch_k(qknorm_ref_kernel<NP, V>, dim3(blocks_of(heads, hd)), dim3(128), 0, st, x, w, n_tok, row_dim, n_heads));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_rope_ref(const float* cos_t, const float* sin_t, bf16* x, int n_tok, const int* pos, int pos0, int hd, int row_dim, int n_heads, cudaStream_t st) {
+  const long heads = (long)n_tok * n_heads;
+  if (heads == 0) return cudaSuccess;
+  QIE_HEADS(hd, (on16({x, cos_t, sin_t}) && row_dim % 8 == 0),
+            (void)launch_k(rope_ref_kernel<NP, V>, dim3(blocks_of(heads, hd)), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads));
+  return cudaGetLastError();
+}
+
+}  // namespace qie

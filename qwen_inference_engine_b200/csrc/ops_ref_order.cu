@@ -56,11 +56,20 @@ cudaError_t launch_embedding(bf16* out, const bf16* table, const int* ids, size_
 // associative, so the chain's order is part of the result.  A block takes R rows into shared memory as they are (bf16), R lanes of one warp
 // walk a chain each side by side, and the block does the rest in parallel.
 // What bounds it: the chain, 4 cycles an element (896 wide 1.9 us).  Its loads are 16 bytes and a group of 32 elements ahead: single floats read
-// inside the loop cost the chain as much again.  us at 1 / 1000 / 4000 rows, before (one row a block, fp32 in shared memory) and now: 896 wide 5.9
-// 6.4 15.7 and 3.9 5.2 8.6; 1536 wide 9.3 9.9 25.9 and 5.6 7.3 12.4; 3584 wide 20.3 21.4 74 and 11.0 13.8 28.0.
+// inside the loop cost the chain as much again.  us at 1 / 1000 / 4000 rows, before (one row a block, fp32 in shared memory, a division an element) and
+// now: 896 wide 5.9 6.4 15.7 and 3.5 4.6 9.2; 1536 wide 9.3 9.9 25.9 and 5.2 6.3 13.2; 3584 wide 20.3 21.4 74 and 10.0 11.8 29.8.
 // VEC: rows, weights and results in pieces of 16 bytes; other widths and addresses are taken element by element.
 // Four rows a block from RMS_MANY rows on: from there more than one chain falls to each of an SM's schedulers, and the lanes of one warp share
-// their issue slots (1 and 4 rows a block: 512 rows of 1536 6.1 6.6, 1000 rows 7.4 7.3, 2000 13.8 8.6).
+// their issue slots (1 and 4 rows a block, with divisions: 512 rows of 1536 6.1 6.6, 1000 rows 7.4 7.3, 2000 13.8 8.6).
+// eight elements: RN(x / rms) w, rounded to bf16
+__device__ __forceinline__ void norm8(const uint32_t (&x)[4], const uint32_t (&w)[4], const Quot& rms, uint32_t (&o)[4]) {
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[2 * j] = lo2f(x[j]), v[2 * j + 1] = hi2f(x[j]);
+  quot16(v, rms);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[j] = pack2f(__fmul_rn(v[2 * j], lo2f(w[j])), __fmul_rn(v[2 * j + 1], hi2f(w[j])));
+}
 constexpr size_t RMS_MANY = 6 * 148;
 template <int R, bool VEC>
 __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, int hidden,
@@ -125,11 +134,8 @@ __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf
         if (r >= n) break;
         const uint4 v = *reinterpret_cast<const uint4*>(rms_rows + (size_t)r * pitch + i * 16);
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-        const float rms = s_rms[r];
         uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          o[j] = pack2(f2bf(__fmul_rn(__fdiv_rn(lo2f(u[j]), rms), lo2f(ww[j]))), f2bf(__fmul_rn(__fdiv_rn(hi2f(u[j]), rms), hi2f(ww[j]))));
+        norm8(u, ww, quot_of(s_rms[r]), o);
         reinterpret_cast<uint4*>(y + (size_t)(row0 + r) * hidden)[i] = make_uint4(o[0], o[1], o[2], o[3]);
       }
     }
@@ -183,7 +189,8 @@ __global__ void __launch_bounds__(256) rmsnorm_fast_kernel(const bf16* __restric
   }
 }
 // one WARP per row, 16-byte accesses, no block barrier -- the block-per-row kernel above ran at a quarter of the HBM
-// rate on the 4096 rows of a prefill (15.9 us for 25 MB: latency of one tiny block per row)
+// rate on the 4096 rows of a prefill (15.9 us for 25 MB: latency of one tiny block per row); a division an element cost 3 of the 11 us that
+// this one then took behind a projection
 __global__ void __launch_bounds__(256) rmsnorm_fast_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
                                                                  bf16* __restrict__ y, int hidden, size_t x_stride, float eps,
                                                                  int n_tok) {
@@ -207,14 +214,12 @@ __global__ void __launch_bounds__(256) rmsnorm_fast_rows_kernel(const bf16* __re
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  const float rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps));
+  const Quot rms = quot_of(__fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps)));
   for (int i = lane; i < nv; i += 32) {
     const uint4 v = xr[i], wv = wr[i];  // (the row is still in L1)
     const uint32_t u[4] = {v.x, v.y, v.z, v.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
     uint32_t o4[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      o4[j] = pack2(f2bf(__fmul_rn(__fdiv_rn(lo2f(u[j]), rms), lo2f(ww[j]))), f2bf(__fmul_rn(__fdiv_rn(hi2f(u[j]), rms), hi2f(ww[j]))));
+    norm8(u, ww, rms, o4);
     yr[i] = make_uint4(o4[0], o4[1], o4[2], o4[3]);
   }
 }
@@ -231,138 +236,6 @@ cudaError_t launch_rmsnorm_fast(const bf16* x, const bf16* w, bf16* y, size_t hi
     return cudaGetLastError();
   }
   (void)launch_k(rmsnorm_fast_kernel, dim3((unsigned)n_tok), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps);
-  return cudaGetLastError();
-}
-
-// ---- operator-level qkNorm / RoPE (one warp per (token, head)) ----------------------
-template <int NP>
-__global__ void qknorm_ref_kernel(bf16* __restrict__ x, const bf16* __restrict__ w, int n_tok, int row_dim,
-                                  int n_heads) {
-  pdl_wait();
-  pdl_trigger();
-  int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gw >= n_tok * n_heads) return;
-  int tok = gw / n_heads, h = gw % n_heads;
-  bf16* p = x + (size_t)tok * row_dim + (size_t)h * 64 * NP;
-  float v[NP][2];
-  head_load<NP>(v, p, lane);
-  head_norm<NP>(v, w, lane);
-  head_store<NP>(v, p, lane);
-}
-
-template <int NP>
-__global__ void rope_ref_kernel(const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                bf16* __restrict__ x, int n_tok, const int* __restrict__ pos, int pos0, int row_dim,
-                                int n_heads) {
-  pdl_wait();
-  pdl_trigger();
-  int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gw >= n_tok * n_heads) return;
-  int tok = gw / n_heads, h = gw % n_heads;
-  int ps = pos ? pos[tok] : pos0 + tok;
-  bf16* p = x + (size_t)tok * row_dim + (size_t)h * 64 * NP;
-  float v[NP][2];
-  head_load<NP>(v, p, lane);
-  head_rope<NP>(v, cos_t + (size_t)ps * 32 * NP, sin_t + (size_t)ps * 32 * NP, lane);
-  head_store<NP>(v, p, lane);
-}
-
-#define QIE_DISPATCH_HD(hd, CALL)                  \
-  switch (hd) {                                    \
-    case 64: { constexpr int NP = 1; CALL; break; }  \
-    case 128: { constexpr int NP = 2; CALL; break; } \
-    case 256: { constexpr int NP = 4; CALL; break; } \
-    default: return cudaErrorInvalidValue;         \
-  }
-
-cudaError_t launch_qknorm_ref(bf16* x, const bf16* w, int hd, int n_tok, int row_dim, int n_heads, cudaStream_t st) {
-  int warps = n_tok * n_heads;
-  if (warps == 0) return cudaSuccess;
-  int blocks = (warps + 3) / 4;
-  QIE_DISPATCH_HD(hd, ((void)launch_k(qknorm_ref_kernel<NP>, dim3(blocks), dim3(128), 0, st, x, w, n_tok, row_dim, n_heads)));
-  return cudaGetLastError();
-}
-
-cudaError_t launch_rope_ref(const float* cos_t, const float* sin_t, bf16* x, int n_tok, const int* pos, int pos0,
-                            int hd, int row_dim, int n_heads, cudaStream_t st) {
-  int warps = n_tok * n_heads;
-  if (warps == 0) return cudaSuccess;
-  int blocks = (warps + 3) / 4;
-  QIE_DISPATCH_HD(hd,
-                  ((void)launch_k(rope_ref_kernel<NP>, dim3(blocks), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads)));
-  return cudaGetLastError();
-}
-
-// ---- fused q/k-norm + RoPE + KV store: replaces 2x qkNorm + 2x RoPE + the
-// cudaMemcpy2D scatter of kv_copy_layer_to_cache_* (include_cuda.cu:165-279) ------------
-// One warp = up to QP_HEADS consecutive heads (q heads, then k heads, then v heads) of one token: the token's position,
-// page and RoPE row are looked up once, the heads' rows are requested together and processed one after the other (
-// one warp per (token, head) ran a chain of three dependent global loads per 256 bytes of payload -- 23.9 us for 33 MB
-// on a 4096-token prefill).  The arithmetic per head is unchanged (head_norm / head_rope).
-constexpr int QP_HEADS = 4;
-template <int NP>
-__global__ void qkv_post_kernel(QkvPostArgs a) {
-  pdl_wait();
-  pdl_trigger();
-  const int hd = 64 * NP;
-  const int heads = a.n_q + 2 * a.kv.n_kv;  // q heads, k heads, v heads
-  const int groups = (heads + QP_HEADS - 1) / QP_HEADS;
-  int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gw >= a.n_tok * groups) return;
-  const int tok = gw / groups, h0 = (gw - tok * groups) * QP_HEADS;
-  const int nh = min(QP_HEADS, heads - h0);
-  const int ps = a.pos[tok];
-  const float* cos_row = a.cos_t + (size_t)ps * 32 * NP;
-  const float* sin_row = a.sin_t + (size_t)ps * 32 * NP;
-  int page = 0, off = 0;
-  if (h0 + nh > a.n_q) {  // the group holds k / v heads
-    page = a.block_table[(size_t)a.slot[tok] * a.max_pages + ps / a.kv.page_size];
-    off = ps % a.kv.page_size;
-  }
-  auto src_of = [&](int h) -> const bf16* {
-    if (h < a.n_q) return a.q_in + (size_t)tok * a.q_in_stride + (size_t)h * hd;
-    if (h < a.n_q + a.kv.n_kv) return a.k + (size_t)tok * a.kv_stride + (size_t)(h - a.n_q) * hd;
-    return a.v + (size_t)tok * a.kv_stride + (size_t)(h - a.n_q - a.kv.n_kv) * hd;
-  };
-  float v[QP_HEADS][NP][2];
-#pragma unroll
-  for (int j = 0; j < QP_HEADS; ++j)
-    if (j < nh) head_load<NP>(v[j], src_of(h0 + j), lane);
-#pragma unroll
-  for (int j = 0; j < QP_HEADS; ++j) {
-    if (j >= nh) break;
-    const int h = h0 + j;
-    if (h < a.n_q) {
-      if (a.q_bias) head_add_bias<NP>(v[j], a.q_bias + (size_t)h * hd, lane);
-      if (a.q_norm_w) head_norm<NP>(v[j], a.q_norm_w, lane, a.eps);
-      if (a.rope_half)
-        head_rope_half<NP>(v[j], cos_row, sin_row, lane);
-      else
-        head_rope<NP>(v[j], cos_row, sin_row, lane);
-      head_store<NP>(v[j], a.q + (size_t)tok * a.n_q * hd + (size_t)h * hd, lane);
-    } else if (h < a.n_q + a.kv.n_kv) {
-      const int kh = h - a.n_q;
-      if (a.k_bias) head_add_bias<NP>(v[j], a.k_bias + (size_t)kh * hd, lane);
-      if (a.k_norm_w) head_norm<NP>(v[j], a.k_norm_w, lane, a.eps);
-      if (a.rope_half)
-        head_rope_half<NP>(v[j], cos_row, sin_row, lane);
-      else
-        head_rope<NP>(v[j], cos_row, sin_row, lane);
-      head_store<NP>(v[j], a.kv.chunk(page, a.layer, 0, kh) + (size_t)off * hd, lane);
-    } else {
-      const int vh = h - a.n_q - a.kv.n_kv;
-      if (a.v_bias) head_add_bias<NP>(v[j], a.v_bias + (size_t)vh * hd, lane);
-      head_store<NP>(v[j], a.kv.chunk(page, a.layer, 1, vh) + (size_t)off * hd, lane);  // (bf16 -> fp32 -> bf16 is the identity)
-    }
-  }
-}
-
-cudaError_t launch_qkv_post(const QkvPostArgs& a, cudaStream_t st) {
-  const int heads = a.n_q + 2 * a.kv.n_kv;
-  int warps = a.n_tok * ((heads + QP_HEADS - 1) / QP_HEADS);
-  if (warps == 0) return cudaSuccess;
-  int blocks = (warps + 3) / 4;
-  QIE_DISPATCH_HD(a.kv.hd, ((void)launch_spread<qkv_post_kernel<NP>>(dim3(blocks), dim3(128), 0, st, a)));
   return cudaGetLastError();
 }
 
