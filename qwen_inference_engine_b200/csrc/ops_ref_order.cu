@@ -610,7 +610,16 @@ __global__ void __launch_bounds__(1024) sample_topk_kernel(const bf16* __restric
 // arg-max in the reference's total order whatever the random draw, so the row can be scanned by several CTAs with
 // 16-byte loads -- the one-block-per-row scan above is latency bound (85 us for 152 k logits, 64 SMs busy at batch
 // 64).  Stage 1: CTA (slice, row) reduces its slice to one candidate; stage 2: one warp per row merges the slices.
-constexpr int GREEDY_SLICES = 8;
+// Eight logits are one packed maximum, looked at further only where it reaches the thread's best, and few long rows are cut into more slices: one row
+// of 151936 behind lm_head 22 us with 8 slices and a comparison in the full order for each, 4.2 now (alone 10.5 and 4.1); 16 rows 12.4 and 5.3, 64 rows 16.7
+// and 9.4.  Below 65536 logits 8 slices hold few pieces a thread as they are (32000: 4.8 and 3.7).
+constexpr int GREEDY_SLICES = 8, GREEDY_MOST = 64;
+static int greedy_slices(int n_rows, size_t vocab) { return vocab < 65536 || n_rows > 16 ? GREEDY_SLICES : n_rows > 4 ? 32 : GREEDY_MOST; }
+__device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {  // two bf16 each; a number wins over a NaN
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
 __global__ void __launch_bounds__(256) greedy_slice_kernel(const bf16* __restrict__ logits, Cand* __restrict__ cands, size_t vocab) {
   pdl_wait();
   pdl_trigger();
@@ -618,63 +627,66 @@ __global__ void __launch_bounds__(256) greedy_slice_kernel(const bf16* __restric
   const int slice = blockIdx.x, rowi = blockIdx.y;
   const bf16* row = logits + (size_t)rowi * vocab;
   const size_t nvec = vocab >> 3;  // 8 logits per 16-byte load (rows are 16-byte aligned: vocab % 8 == 0, checked by the launcher)
-  const size_t per = (nvec + GREEDY_SLICES - 1) / GREEDY_SLICES;
+  const size_t per = (nvec + gridDim.x - 1) / gridDim.x;
   const size_t v0 = (size_t)slice * per, v1 = min(nvec, v0 + per);
   float bv = -CUDART_INF_F;
   int bi = -1;
-  for (size_t v = v0 + threadIdx.x; v < v1; v += 256) {
-    const uint4 q = ld_nc_v4(reinterpret_cast<const uint4*>(row) + v);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  constexpr int U = 4;  // loads on their way together
+  for (size_t v = v0 + threadIdx.x; v < v1; v += U * 256) {
+    uint4 q[U];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float f0 = lo2f(w[e]), f1 = hi2f(w[e]);
-      const int i0 = (int)(v * 8) + 2 * e;
-      if (f0 > -CUDART_INF_F && cand_better(f0, i0, bv, bi)) {
-        bv = f0;
-        bi = i0;
-      }
-      if (f1 > -CUDART_INF_F && cand_better(f1, i0 + 1, bv, bi)) {
-        bv = f1;
-        bi = i0 + 1;
-      }
+    for (int u = 0; u < U; ++u) q[u] = ld_nc_v4(reinterpret_cast<const uint4*>(row) + min(v + u * 256, v1 - 1));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t w[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+      const uint32_t m = max2(max2(w[0], w[1]), max2(w[2], w[3]));
+      const float f = fmaxf(lo2f(m), hi2f(m));
+      if (!(v + u * 256 < v1 && f >= bv && f > -CUDART_INF_F)) continue;  // (maxima that are NaN or -inf fail)
+      // of those that equal it the first in the reference's order, the largest reversed low bits: 7, 3, 5, 1, 6, 2, 4, 0
+      int e = 0;
+      if (lo2f(w[2]) == f) e = 4;
+      if (lo2f(w[1]) == f) e = 2;
+      if (lo2f(w[3]) == f) e = 6;
+      if (hi2f(w[0]) == f) e = 1;
+      if (hi2f(w[2]) == f) e = 5;
+      if (hi2f(w[1]) == f) e = 3;
+      if (hi2f(w[3]) == f) e = 7;
+      const int i = (int)(v + u * 256) * 8 + e;
+      if (cand_better(f, i, bv, bi)) bv = f, bi = i;
     }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (cand_better(ov, oi, bv, bi)) {
-      bv = ov;
-      bi = oi;
-    }
+    if (cand_better(ov, oi, bv, bi)) bv = ov, bi = oi;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) s_c[warp] = Cand{bv, bi};
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w2 = 1; w2 < 8; ++w2)
-      if (cand_better(s_c[w2].val, s_c[w2].idx, bv, bi)) {
-        bv = s_c[w2].val;
-        bi = s_c[w2].idx;
-      }
-    cands[(size_t)rowi * GREEDY_SLICES + slice] = Cand{bv, bi};
+      if (cand_better(s_c[w2].val, s_c[w2].idx, bv, bi)) bv = s_c[w2].val, bi = s_c[w2].idx;
+    cands[(size_t)rowi * gridDim.x + slice] = Cand{bv, bi};
   }
 }
-__global__ void greedy_merge_kernel(const Cand* __restrict__ cands, int* __restrict__ out, int n_rows) {
+__global__ void greedy_merge_kernel(const Cand* __restrict__ cands, int* __restrict__ out, int n_rows, int slices) {  // a warp per row
   pdl_wait();
   pdl_trigger();
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
   if (r >= n_rows) return;
   float bv = -CUDART_INF_F;
   int bi = -1;
-  for (int s2 = 0; s2 < GREEDY_SLICES; ++s2) {
-    const Cand c = cands[(size_t)r * GREEDY_SLICES + s2];
-    if (cand_better(c.val, c.idx, bv, bi)) {
-      bv = c.val;
-      bi = c.idx;
-    }
+  for (int s2 = lane; s2 < slices; s2 += 32) {
+    const Cand c = cands[(size_t)r * slices + s2];
+    if (cand_better(c.val, c.idx, bv, bi)) bv = c.val, bi = c.idx;
   }
-  out[r] = bi;  // -1 if the row holds no finite logit, like the scan above
+  for (int o = slices >= 32 ? 16 : 4; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (cand_better(ov, oi, bv, bi)) bv = ov, bi = oi;
+  }
+  if (lane == 0) out[r] = bi;  // -1 if the row holds no finite logit, like the scan above
 }
 
 // Top-k (k > 1) without k scans.  The reference selects by k rounds of "arg-max over everything not chosen yet"
@@ -828,8 +840,11 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
 // ranks what is left by counting (all keys differ) and runs the reference's tail: quotients and exponentials by a thread each, the
 // two sums in the reference's order.  Where ties (a row of equal logits) leave more candidates than the lists hold, the slice takes four more
 // passes to pick its k best, and the first CTA bisects the lower half of the keys.
-// One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384; here 18.5 and 39.  The bound
-// is the latency of the steps, not memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 15.6 us, 29 here.
+// One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384.  The cluster with both passes over memory,
+// every value brought into its order and the gathering CTA by CTA: 18.2 and 39.2.  Now a piece of eight values is one packed maximum and the second pass
+// looks into those that reach the bound (a few per cent), the slice is read from memory once, all counts and then all candidates are
+// gathered at once, and the draw is compared with the running sums of the one chain: 13.8 and 25.1.  The bound is the latency of the steps, not
+// memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 9.4 us.
 constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;
 // order-preserving 16 bits; 0: never selected
 __device__ __forceinline__ uint32_t topk_order16(uint32_t b) {
@@ -943,20 +958,25 @@ __device__ __noinline__ void topk_slice_ties(const TopkSlice<TC_THREADS> sl, Top
   __syncthreads();
   if (tid < 3) sum.cnt[tid] = 0;
 }
-template <int TC_THREADS>
+// STAGED: the slice is copied to shared memory once, its two passes read it there (up to TC_STAGE bytes, 48 KB with the 9.6 KB of the rest, so that four
+// CTAs share an SM; the first CTA's gathered candidates go over it).
+constexpr int TC_STAGE = 38 * 1024, TC_ALL = TC_CTAS * TC_CAP * 8;  // bytes
+template <int TC_THREADS, bool STAGED>
 __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
                                uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
   static_assert(TC_THREADS > TC_MOST && TC_CAP >= TC_MOST, "a thread for every exponential and one for the random number; k candidates fit");
   pdl_wait();
   pdl_trigger();
+  extern __shared__ __align__(16) unsigned char tc_buf[];
   __shared__ unsigned long long cand[TC_CAP];             // this slice's candidates
-  __shared__ unsigned long long all[TC_CTAS * TC_CAP];    // first CTA: everybody's
   __shared__ unsigned long long best[TC_CAP];         // first CTA: those that reach the k-th value
-  __shared__ float vals[TC_MOST];
+  __shared__ __align__(16) float vals[TC_MOST];
+  __shared__ float cums[TC_MOST];
   __shared__ int idxs[TC_MOST];
-  __shared__ int s_n, s_cnt[3], s_tot;
+  __shared__ int s_n, s_cnt[3], s_tot, s_ns[TC_CTAS];
   __shared__ float s_u;
+  unsigned long long* all = reinterpret_cast<unsigned long long*>(tc_buf);  // first CTA: everybody's
   const int tid = threadIdx.x, slice = blockIdx.x, rowi = blockIdx.y;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(logits) + (size_t)rowi * vocab;
   if (!(temperature > 0.0f)) temperature = 1.0f;
@@ -967,8 +987,37 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   const size_t nvec = (vocab - sl.head) / 8, per = (nvec + TC_CTAS - 1) / TC_CTAS;
   sl.v0 = min(nvec, slice * per), sl.v1 = min(nvec, sl.v0 + per);
   sl.tail0 = sl.head + (int)nvec * 8, sl.loose = slice == 0 ? sl.head + (int)vocab - sl.tail0 : 0;
-  uint32_t mx = 0;
-  sl.each([&](uint32_t o, uint32_t, int) { mx = max(mx, o); });
+  const bool loose = tid < sl.loose;  // this thread's element in front of the first 16-byte boundary or behind the last whole piece
+  const int loose_at = tid < sl.head ? tid : sl.tail0 + tid - sl.head;
+  const uint32_t loose_bits = loose ? (uint32_t)row[loose_at] : 0xff80u;
+  // f(eight values, the largest of them, index of the first) for this thread's pieces
+  auto pieces = [&](auto&& f) {
+    constexpr int U = STAGED ? 1 : 4;
+    for (size_t v = sl.v0 + tid; v < sl.v1; v += U * TC_THREADS) {
+      uint4 q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const size_t at = min(v + u * TC_THREADS, sl.v1 - 1);
+        if constexpr (STAGED) q[u] = *reinterpret_cast<const uint4*>(tc_buf + (at - sl.v0) * 16);
+        else asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[u].x), "=r"(q[u].y), "=r"(q[u].z), "=r"(q[u].w) : "l"(row + sl.head + at * 8));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (v + u * TC_THREADS < sl.v1) {
+          const uint32_t m = max2(max2(q[u].x, q[u].y), max2(q[u].z, q[u].w));
+          f(q[u], max2(m, __byte_perm(m, 0, 0x1032)), sl.head + (int)(v + u * TC_THREADS) * 8);
+        }
+    }
+  };
+  if constexpr (STAGED) {  // (a thread reads what it has copied)
+    const uint32_t dst = smem_u32(tc_buf);
+    for (size_t v = sl.v0 + tid; v < sl.v1; v += TC_THREADS) cp_async16(dst + (uint32_t)(v - sl.v0) * 16u, row + sl.head + v * 8);
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
+  uint32_t m2 = 0xff80ff80u;  // -inf twice: what stays where there is no number
+  pieces([&](const uint4&, uint32_t m, int) { m2 = max2(m2, m); });
+  const uint32_t mx = max(topk_order16(m2 & 0xffffu), topk_order16(loose_bits));
   // the largest bound that k maxima reach (1 if fewer threads have a value: then every value is a candidate)
   uint32_t bound = 0;
 #pragma unroll 1
@@ -980,26 +1029,42 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   if (tid == 0) s_n = 0;
   if (tid < 3) s_cnt[tid] = 0;
   __syncthreads();
-  if (mx >= bound)
-    sl.each([&](uint32_t o, uint32_t b, int i) {
-      if (o < bound) return;
+  if (mx >= bound) {
+    auto take = [&](uint32_t b, int i) {
+      if (topk_order16(b) < bound) return;
       const int at = atomicAdd(&s_n, 1);
       if (at < TC_CAP) cand[at] = topk_key((uint16_t)b, i);
+    };
+    pieces([&](const uint4& q, uint32_t m, int i0) {
+      if (topk_order16(m & 0xffffu) < bound) return;
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) take(w[e] & 0xffffu, i0 + 2 * e), take(w[e] >> 16, i0 + 2 * e + 1);
     });
+    if (loose) take(loose_bits, loose_at);
+  }
   __syncthreads();
-  if (s_n > TC_CAP) topk_slice_ties<TC_THREADS>(sl, TopkSums{s_cnt, 0}, mx, bound, k, cand, reinterpret_cast<int*>(best), reinterpret_cast<int*>(all), &s_n, &s_tot);
+  if (s_n > TC_CAP) topk_slice_ties<TC_THREADS>(sl, TopkSums{s_cnt, 0}, mx, bound, k, cand, reinterpret_cast<int*>(best), reinterpret_cast<int*>(tc_buf), &s_n, &s_tot);
   cluster_sync_all();
   if (slice == 0) {
-    // ---- gather
+    // ---- gather: all counts at once, then all candidates
+    if (tid < TC_CTAS) {
+      uint32_t an;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(an) : "r"(smem_u32(&s_n)), "r"(tid));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(s_ns[tid]) : "r"(an) : "memory");
+    }
+    __syncthreads();
     int n = 0;
+#pragma unroll
     for (int c = 0; c < TC_CTAS; ++c) {
-      uint32_t an, ac;
-      int cn;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(an) : "r"(smem_u32(&s_n)), "r"(c));
+      uint32_t ac;
+      const int cn = s_ns[c];
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ac) : "r"(smem_u32(cand)), "r"(c));
-      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(cn) : "r"(an) : "memory");
-      for (int i = tid; i < cn; i += TC_THREADS)
-        asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(all[n + i]) : "r"(ac + 8u * (uint32_t)i) : "memory");
+      for (int i = tid; i < cn; i += TC_THREADS) {
+        unsigned long long key;
+        asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(key) : "r"(ac + 8u * (uint32_t)i));
+        all[n + i] = key;
+      }
       n += cn;
     }
     __syncthreads();
@@ -1010,11 +1075,20 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     TopkSums sum{s_cnt, 0};
     if (actual_k > 0) {
       uint32_t top = 0;
+      uint32_t own[4];  // this thread's values, where they are few
+      const bool few = n <= 4 * TC_THREADS;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) own[u] = tid + u * TC_THREADS < n ? (uint32_t)(all[tid + u * TC_THREADS] >> 32) : 0u;
 #pragma unroll 1
       for (int bit = 15; bit >= 0; --bit) {
         const uint32_t t = top | (1u << bit);
         int c = 0;
-        for (int i = tid; i < n; i += TC_THREADS) c += (uint32_t)(all[i] >> 32) >= t;
+        if (few) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) c += own[u] >= t;
+        } else {
+          for (int i = tid; i < n; i += TC_THREADS) c += (uint32_t)(all[i] >> 32) >= t;
+        }
         c = sum(c);
         if (c >= actual_k) top = t, m = c;
       }
@@ -1036,16 +1110,22 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     if (actual_k == 0) {
       if (tid == 0) out[rowi] = -1;
     } else {
-      // ---- rank by counting
+      // ---- rank by counting.  A key holds its value, but for the sign of a zero, which no exponential below sees.
       for (int i = tid; i < m; i += TC_THREADS) {
         const unsigned long long key = best[i];
         int rank = 0;
         for (int j = 0; j < m; ++j) rank += best[j] > key;
         if (rank < actual_k) {
-          const int idx = (int)(0xFFFFFFu - (unsigned)(key & 0xFFFFFFull));
-          idxs[rank] = idx;
-          vals[rank] = __fdiv_rn(bf2f(logits[(size_t)rowi * vocab + idx]), temperature);
+          const uint32_t o = (uint32_t)(key >> 32);
+          idxs[rank] = (int)(0xFFFFFFu - (unsigned)(key & 0xFFFFFFull));
+          vals[rank] = __fdiv_rn(lo2f(o & 0x8000u ? o ^ 0x8000u : ~o & 0xffffu), temperature);
         }
+      }
+      if (tid == TC_THREADS - 1) {  // (a warp of its own, where it has no key to rank)
+        curandState rng;
+        const unsigned long long sd = seed + (unsigned long long)rowi * seed_stride + (step_ptr ? (unsigned)step_ptr[rowi] : 0u);
+        curand_init(sd, subsequence, 0, &rng);
+        s_u = curand_uniform(&rng);
       }
       __syncthreads();
       // ---- the reference's tail, logit_decode.cu:225-273: the best quotient is the largest (division by a positive number keeps the order)
@@ -1054,32 +1134,41 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
       } else {
         const float max_val = vals[0];
         __syncthreads();
-        if (tid < actual_k) vals[tid] = expf(__fsub_rn(vals[tid], max_val));
-        if (tid == TC_THREADS - 1) {  // (a warp of its own)
-          curandState rng;
-          const unsigned long long sd = seed + (unsigned long long)rowi * seed_stride + (step_ptr ? (unsigned)step_ptr[rowi] : 0u);
-          curand_init(sd, subsequence, 0, &rng);
-          s_u = curand_uniform(&rng);
-        }
+        if (tid < TC_MOST) vals[tid] = tid < actual_k ? expf(__fsub_rn(vals[tid], max_val)) : 0.f;
         __syncthreads();
-        if (tid == 0) {
-          float sum = 0.0f, cum = 0.0f;
-          for (int i = 0; i < actual_k; ++i) sum = __fadd_rn(sum, vals[i]);
-          const float u = __fmul_rn(s_u, sum);
-          int picked = idxs[actual_k - 1];
-          for (int i = 0; i < actual_k; ++i) {
-            cum = __fadd_rn(cum, vals[i]);
-            if (u <= cum) {
-              picked = idxs[i];
-              break;
+        if (tid < 32) {
+          // the sum and the running sums that the draw is compared with are the same chain
+          if (tid == 0) {
+            float sum = 0.0f;
+            for (int i = 0; i < actual_k; i += 4) {
+              const float4 v = *reinterpret_cast<const float4*>(vals + i);
+              cums[i] = sum = __fadd_rn(sum, v.x);
+              cums[i + 1] = sum = __fadd_rn(sum, v.y);
+              cums[i + 2] = sum = __fadd_rn(sum, v.z);
+              cums[i + 3] = sum = __fadd_rn(sum, v.w);
             }
           }
-          out[rowi] = picked;
+          __syncwarp();
+          const float u = __fmul_rn(s_u, cums[actual_k - 1]);
+          int at = actual_k - 1;
+#pragma unroll
+          for (int c = TC_MOST - 32; c >= 0; c -= 32) {
+            const uint32_t hit = __ballot_sync(0xffffffffu, c + tid < actual_k && u <= cums[c + tid]);
+            if (hit) at = c + __ffs(hit) - 1;
+          }
+          if (tid == 0) out[rowi] = idxs[at];
         }
       }
     }
   }
   cluster_sync_all();  // nobody leaves while the first CTA reads its candidates
+}
+template <int TC_THREADS, bool STAGED>
+static cudaError_t launch_topk_cluster(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature, int k, uint64_t seed, uint64_t seed_stride,
+                                       const int* step_ptr, unsigned long long subsequence, cudaStream_t st) {
+  const size_t slice = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16, smem = STAGED ? std::max<size_t>(slice, TC_ALL) : TC_ALL;
+  return launch_k(sample_topk_cluster_kernel<TC_THREADS, STAGED>, dim3(TC_CTAS, n_rows), dim3(TC_THREADS), smem, st, logits, out_tokens, vocab, temperature, k, seed,
+                  seed_stride, step_ptr, subsequence);
 }
 
 cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature,
@@ -1107,31 +1196,27 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
       if (!cands) {
         Scratch sc;
         sc.cap = std::max(n_rows, 256);
-        cudaError_t e = cudaMalloc(&sc.p, (size_t)sc.cap * GREEDY_SLICES * sizeof(Cand));
+        cudaError_t e = cudaMalloc(&sc.p, std::max<size_t>(256 * GREEDY_MOST, (size_t)sc.cap * GREEDY_SLICES) * sizeof(Cand));
         if (e != cudaSuccess) return e;
         v.push_back(sc);
         cands = sc.p;
       }
     }
-    (void)launch_k(greedy_slice_kernel, dim3(GREEDY_SLICES, n_rows), dim3(256), 0, st, logits, cands, vocab);
+    const int slices = greedy_slices(n_rows, vocab);
+    (void)launch_k(greedy_slice_kernel, dim3(slices, n_rows), dim3(256), 0, st, logits, cands, vocab);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    (void)launch_k(greedy_merge_kernel, dim3((n_rows + 63) / 64), dim3(64), 0, st, (const Cand*)cands, out_tokens, n_rows);
+    (void)launch_k(greedy_merge_kernel, dim3((n_rows + 3) / 4), dim3(128), 0, st, (const Cand*)cands, out_tokens, n_rows, slices);
     return cudaGetLastError();
   }
   // (slices longer than a candidate list of which fewer than k threads hold a value, vocabularies of 4 to 8 thousand with large k, have no bound to
   // start from: 64 rows of 8000, k = 128, 44 us by the radix select, 86 here)
   if (k > 1 && k <= TC_MOST && vocab <= (1u << 23) && n_rows <= 65535 && (vocab <= (size_t)TC_CTAS * TC_CAP || vocab / (TC_CTAS * 8) > (size_t)k)) {
-    // many rows: 256 threads, so that more clusters are on the chip at once (64 rows of 151936, k = 50: 39 us, 42 with 512), and 5 KB of shared
-    // memory more than they need, so that no SM takes five CTAs while others have two (44); few rows: 512, for shorter passes (1 row 18.5, 22
-    // with 256)
-    if (n_rows > 16)
-      (void)launch_k(sample_topk_cluster_kernel<256>, dim3(TC_CTAS, n_rows), dim3(256), 5120, st, logits, out_tokens, vocab, temperature, k, seed,
-                     seed_stride, step_ptr, (unsigned long long)subsequence);
-    else
-      (void)launch_k(sample_topk_cluster_kernel<512>, dim3(TC_CTAS, n_rows), dim3(512), 0, st, logits, out_tokens, vocab, temperature, k, seed,
-                     seed_stride, step_ptr, (unsigned long long)subsequence);
-    return cudaGetLastError();
+    // many rows: 256 threads, so that all clusters are on the chip at once; few rows: 512, for shorter passes
+    const bool staged = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16 <= (size_t)TC_STAGE;
+    auto launch = n_rows > 16 ? (staged ? launch_topk_cluster<256, true> : launch_topk_cluster<256, false>)
+                              : (staged ? launch_topk_cluster<512, true> : launch_topk_cluster<512, false>);
+    return launch(logits, out_tokens, n_rows, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence, st);
   }
   // more than TC_MOST candidates, and the above: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the
   // 24-bit index field of the key cannot hold, and for k < 1
