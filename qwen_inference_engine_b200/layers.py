@@ -22,7 +22,8 @@ def _p(t):
 
 
 def _st():
-    return torch.cuda.current_stream().cuda_stream
+    """cudaStream_t of torch's current stream.  (torch.cuda.current_stream() builds an object around it: 3.4 us of an operator call of 8, here 0.3.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def embedding(out, table, ids):
@@ -101,11 +102,13 @@ def launch_attn(Q, out, pool, layer, pos, slot, n_q_heads):
 def sample_topk_bf16(logits_d, vocab, temperature, topk, seed, step=0):
     """helpers.cuh:157-166 -- returns the sampled token ids (one per row of logits)."""
     rows = logits_d.numel() // vocab
-    out = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    # The kernel writes the tokens into page-locked memory itself: a device buffer, its clearing and a copy to pageable memory were 20 us of 72 (64 rows).
+    out = torch.empty(rows, dtype=torch.int32, pin_memory=True)
     # the reference hands `step` to the kernel as the cuRAND subsequence (helpers.cuh:157-166)
-    check(_lib.lib().qie_sample_topk_subseq(_p(logits_d), _p(out), rows, vocab, float(temperature), topk, seed, 0, step,
+    check(_lib.lib().qie_sample_topk_subseq(_p(logits_d), out.data_ptr(), rows, vocab, float(temperature), topk, seed, 0, step,
                                             _st()))
-    return out.cpu().numpy()
+    torch.cuda.current_stream().synchronize()
+    return out.numpy().copy()
 
 
 def apply_repetition_penalty(logits_d, context_tokens_d, vocab, penalty):
