@@ -39,6 +39,29 @@ __device__ __forceinline__ void quot16(float (&x)[N], const Quot& d) {
   }
 }
 
+// The same for fp32 numerators of no matter how many bits: the first correction leaves the quotient or a neighbour of it, the second rounds correctly
+// (Markstein).  Zeros are fine where they are positive.
+__device__ __forceinline__ bool quot32_ok(float x) { return __float_as_uint(x) == 0u || (fabsf(x) >= 0x1p-100f && fabsf(x) <= 0x1p100f); }
+__device__ __forceinline__ float quot32_fast(float x, const Quot& d) {
+  float q = __fmul_rn(x, d.y);
+  q = __fmaf_rn(__fmaf_rn(-d.b, q, x), d.y, q);
+  return __fmaf_rn(__fmaf_rn(-d.b, q, x), d.y, q);
+}
+__device__ __forceinline__ float quot1(float x, const Quot& d) { return d.ok && quot32_ok(x) ? quot32_fast(x, d) : __fdiv_rn(x, d.b); }
+template <int N>
+__device__ __forceinline__ void quot32(float (&x)[N], const Quot& d) {
+  bool ok = d.ok;
+#pragma unroll
+  for (int i = 0; i < N; ++i) ok = ok && quot32_ok(x[i]);
+  if (ok) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = quot32_fast(x[i], d);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) x[i] = __fdiv_rn(x[i], d.b);
+  }
+}
+
 // ------------------------------------------------------------------ per-head tree sum
 // Lane l holds, for p in [0,NP): elements t = 64p + 2l and 64p + 2l + 1 of a head of
 // hd = 64*NP values.  Reproduces  for (stride = hd/2; stride > 0; stride >>= 1)
