@@ -301,6 +301,7 @@ int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, in
   CU(make_tensor_map_2d(&wmap, (const bf16*)B, K, N, 128));
   TcGemm t{};
   t.w[0] = &wmap;
+  t.wp[0] = (const bf16*)B;
   t.x = (const bf16*)A;
   t.rows[0] = K;
   t.nseg = 1;

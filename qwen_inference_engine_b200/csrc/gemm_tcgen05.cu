@@ -38,9 +38,9 @@ namespace qie {
 
 static constexpr int BM = 128;  // weight rows per CTA (UMMA M)
 static constexpr int BK = 64;   // k elements per stage (128 B rows, SWIZZLE_128B)
-template <int BN, bool HALF>
-struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens)
-  static constexpr int STAGES = HALF ? 6 : BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : 7;  // what 227 KiB hold
+template <int BN, bool HALF, int KB>
+struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens); KB: k-blocks of a stage
+  static constexpr int STAGES = (HALF ? 6 : BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : 7) / KB;  // what 227 KiB hold
 };
 
 // ------------------------------------------------------------------ PTX wrappers (tc_ptx.cuh has the rest)
@@ -51,6 +51,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
@@ -102,7 +108,7 @@ struct TcArgs {
   TcSeg seg[3];
 };
 
-template <int BN, bool HALF>
+template <int BN, bool HALF, int KB>
 __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
@@ -112,11 +118,11 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   __shared__ int dead_s;
   volatile int* const dead = &dead_s;
   if (threadIdx.x == 0) dead_s = 0;  // (a barrier follows before any wait)
-  constexpr int A_BYTES = BM * BK * 2;  // 16 KiB
-  constexpr int B_BYTES = BN * BK * 2;
+  constexpr int A_BLK = BM * BK * 2, A_BYTES = KB * A_BLK;  // 16 KiB a k-block
+  constexpr int B_BLK = BN * BK * 2, B_BYTES = KB * B_BLK;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
-  constexpr int TC_STAGES = TcCfg<BN, HALF>::STAGES;
+  constexpr int TC_STAGES = TcCfg<BN, HALF, KB>::STAGES;
   static_assert(TC_STAGES * STAGE_BYTES >= BN * (BM + 32) * 4, "reduction tile must fit in the pipeline ring");
   // 1024-byte alignment for SWIZZLE_128B (same offset in every CTA of a cluster: the dynamic
   // shared window starts at the same address in all CTAs of a kernel)
@@ -138,7 +144,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   bf16* const out = g.seg[si].out;
   const int kb0 = split * g.kb_per_split;
   const int kb1 = min(g.kb_total, kb0 + g.kb_per_split);
-  const int nkb = max(0, kb1 - kb0);
+  const int nkb = max(0, kb1 - kb0), nst = (nkb + KB - 1) / KB;  // k-blocks, stages of them
   const int tok_base = ttile * BN;
 
   if (warp == 0 && lane == 0) {
@@ -161,6 +167,10 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 
   auto load_w = [&](int i, int s) {
     const uint32_t sa = smem0 + s * STAGE_BYTES;
+    if constexpr (KB > 1) {  // one request for the k-blocks of a stage (behind the matrix: zeros, which no product reads)
+      tma_load_3d(sa, map_w, full_bar(s), row0, kb0 + i * KB);
+      return;
+    }
     if (g.dual) {  // two 64-row boxes: gate rows -> lanes 0-63, up rows -> lanes 64-127
       tma_load_2d(sa, &map_w0, full_bar(s), (kb0 + i) * BK, row0);
       tma_load_2d(sa + A_BYTES / 2, &map_w1, full_bar(s), (kb0 + i) * BK, row0);
@@ -169,29 +179,35 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     }
   };
 
+  auto load_x = [&](int i, int s) {
+    const uint32_t sb = smem0 + s * STAGE_BYTES + A_BYTES;
+    if constexpr (KB > 1) tma_load_3d(sb, &map_x, full_bar(s), tok_base, kb0 + i * KB);
+    else tma_load_2d(sb, &map_x, full_bar(s), (kb0 + i) * BK, tok_base);
+  };
+
   // The loops of both roles carry stage, parity and descriptors from step to step, and the MMA loop runs on the whole warp with one
   // elected lane.  With a division by the stage count, a clock read per wait and descriptors built per product a step took 0.27 us
-  // whatever the tile's width (76 steps at K = 4864: 22.8 us on an idle chip); now 0.18 us (15.4 us).  The products of a step
-  // themselves take 0.025 us at 16 tokens, 0.27 us at 256.
+  // whatever the tile's width (76 steps at K = 4864: 22.8 us on an idle chip), then 0.18 us (15.7 us).  The products of a step
+  // themselves take 0.025 us at 16 tokens, 0.27 us at 256.  With two k-blocks a stage (KB) a k-block takes 0.13 us: us before and after, in graphs, in the
+  // reference's order: 64 rows of 896 x 896 4.6 4.1, 4864 x 896 15.7 12.3, 8960 x 1536 27.3 20.7, 18944 x 3584 56.2 42.8; 512 rows 4864 x 896 16.6 13.7.
   if (warp == 0) {
     if (elect_tc()) {
       // Weights never depend on the previous kernel: start streaming them BEFORE waiting for
       // it (programmatic dependent launch), as soon as its CTAs leave room for the ring.
-      const int pre = g.w_static ? min(nkb, TC_STAGES) : 0;
+      const int pre = g.w_static ? min(nst, TC_STAGES) : 0;
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), STAGE_BYTES);
         load_w(i, i);
       }
       pdl_wait();  // activations are produced by the previous kernel
-      for (int i = 0; i < pre; ++i)
-        tma_load_2d(smem0 + i * STAGE_BYTES + A_BYTES, &map_x, full_bar(i), (kb0 + i) * BK, tok_base);
+      for (int i = 0; i < pre; ++i) load_x(i, i);
       int s = pre == TC_STAGES ? 0 : pre;
       uint32_t ph = pre == TC_STAGES ? 0 : 1;  // the first pass over the ring waits for nothing
-      for (int i = pre; i < nkb; ++i) {
+      for (int i = pre; i < nst; ++i) {
         if (!mbar_wait_tc(empty_bar(s), ph, dead)) break;
         mbar_expect_tx(full_bar(s), STAGE_BYTES);
         load_w(i, s);
-        tma_load_2d(smem0 + s * STAGE_BYTES + A_BYTES, &map_x, full_bar(s), (kb0 + i) * BK, tok_base);
+        load_x(i, s);
         if (++s == TC_STAGES) s = 0, ph ^= 1;
       }
     }
@@ -202,14 +218,17 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0;
     uint32_t ph = 0;
-    for (int i = 0; i < nkb; ++i) {
+    for (int i = 0; i < nst; ++i) {
       mbar_wait_tc(full_bar(s), ph, dead);
       tc_fence_after();
       const uint64_t step = (uint64_t)(s * (STAGE_BYTES >> 4));
       if (elect_tc()) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
-          umma_tc(tmem_base, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (i | k) != 0);
+        for (int b = 0; b < KB; ++b)
+          if (b == 0 || i * KB + b < nkb)
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
+              umma_tc(tmem_base, ad0 + step + b * (A_BLK >> 4) + 2 * k, bd0 + step + b * (B_BLK >> 4) + 2 * k, idesc, (i | b | k) != 0);
         umma_commit_tc(empty_bar(s));  // frees the smem stage once the MMAs have read it
       }
       __syncwarp();
@@ -821,21 +840,18 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN, bool HALF = false>
-static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, const TensorMap2D& x, int token_tiles, cudaStream_t st) {
-  constexpr int STAGE_BYTES = BM * BK * 2 + BN * BK * 2;
-  constexpr size_t smem = (size_t)TcCfg<BN, HALF>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+template <int BN, bool HALF, int KB>
+static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
+  constexpr int STAGE_BYTES = KB * (BM * BK * 2 + BN * BK * 2);
+  constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     set.done();
   }
-  const CUtensorMap* w0 = reinterpret_cast<const CUtensorMap*>(t.w[0]);
-  const CUtensorMap* w1 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 1 ? 1 : 0]);
-  const CUtensorMap* w2 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 2 ? 2 : 0]);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(g.n_tiles, g.splits, token_tiles);
   cfg.blockDim = dim3(192);
@@ -857,7 +873,19 @@ static cudaError_t launch_bn(const TcGemm& t, const TcArgs& g, const TensorMap2D
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF>, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
+}
+
+template <int KB>
+static cudaError_t launch_tile(int bn, bool half, const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
+  switch (bn) {
+    case 16: return half ? launch_bn<16, true, KB>(g, w, x, token_tiles, st) : launch_bn<16, false, KB>(g, w, x, token_tiles, st);
+    case 32: return launch_bn<32, false, KB>(g, w, x, token_tiles, st);
+    case 64: return launch_bn<64, false, KB>(g, w, x, token_tiles, st);
+    default:
+      if constexpr (KB == 1) return launch_bn<128, false, 1>(g, w, x, token_tiles, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 struct TcTile {
@@ -944,10 +972,24 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
   g.staged = g.splits == 1 && vec;
   g.vec = vec;
+  const CUtensorMap* w[3];
+  for (int i = 0; i < 3; ++i) w[i] = reinterpret_cast<const CUtensorMap*>(t.w[i < t.nseg ? i : 0]);
   TensorMap2D x;
+  if (launches) *launches = 1;
+  // Two k-blocks a stage where tensor maps can express them (whole k-blocks, and the weights' place is known): half the requests, waits and commits.  Up
+  // to 64 tokens: of 128 the ring holds three such stages, too few on the way (8960 x 1536 at 1000 rows 34.8 with stages of one, 37.1).  Gate/up tiles
+  // are two boxes a k-block as they are.
+  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && t.wp[0]) {
+    TensorMap2D w3[3];
+    bool ok = make_tensor_map_w3d(&x, t.x, t.M, t.K, 2 * BK, 0, tl.bn) == cudaSuccess;
+    for (int i = 0; i < t.nseg; ++i) ok = ok && t.wp[i] && make_tensor_map_w3d(&w3[i], t.wp[i], t.rows[i], t.K, 2 * BK, 0, BM) == cudaSuccess;
+    if (ok) {
+      for (int i = 0; i < 3; ++i) w[i] = reinterpret_cast<const CUtensorMap*>(&w3[i < t.nseg ? i : 0]);
+      return launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
+    }
+  }
   cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
   if (e != cudaSuccess) return e;
-  if (launches) *launches = 1;
   if (tl.persist) {
     // (widths of the residual stream and of the feed-forward are inner dimensions too, so multiples of 8)
     if (!vec && t.epi != EPI_STORE) return cudaErrorInvalidValue;
@@ -960,9 +1002,6 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     }
     g.bn = tl.bn;
     g.stages = std::min(P_MAX_STAGES, P_RING / (BM * BK * 2 + tl.bn * BK * 2));
-    const CUtensorMap* w0 = reinterpret_cast<const CUtensorMap*>(t.w[0]);
-    const CUtensorMap* w1 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 1 ? 1 : 0]);
-    const CUtensorMap* w2 = reinterpret_cast<const CUtensorMap*>(t.w[t.nseg > 2 ? 2 : 0]);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)std::min<long>(num_sms, (long)tiles * token_tiles));
     cfg.blockDim = dim3(P_THREADS);
@@ -973,14 +1012,9 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = g_use_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w0, *w1, *w2, *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
+    return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
   }
-  switch (tl.bn) {
-    case 16: return tl.half ? launch_bn<16, true>(t, g, x, token_tiles, st) : launch_bn<16>(t, g, x, token_tiles, st);
-    case 32: return launch_bn<32>(t, g, x, token_tiles, st);
-    case 64: return launch_bn<64>(t, g, x, token_tiles, st);
-    default: return launch_bn<128>(t, g, x, token_tiles, st);
-  }
+  return launch_tile<1>(tl.bn, tl.half, g, w, x, token_tiles, st);
 }
 
 // Reference-order products of any number of rows.  The chain of tcgen05.mma over ascending k of 16 into one accumulator gives the bits of
@@ -1014,6 +1048,7 @@ cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st
       const GemmSeg& sg = a.seg[dual ? 0 : i];
       tc = make_tensor_map_2d(&w[i], dual && i ? sg.W2 : sg.W, sg.rows, a.K, dual ? BM / 2 : BM) == cudaSuccess;
       t.w[i] = &w[i];
+      t.wp[i] = dual && i ? sg.W2 : sg.W;
       t.rows[i] = sg.rows;
       t.outs[i] = sg.out;
       t.lds[i] = sg.ld_out;

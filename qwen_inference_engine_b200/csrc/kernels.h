@@ -164,6 +164,7 @@ cudaError_t make_tensor_map_kv(TensorMap2D* out, const bf16* pool, unsigned long
 cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_elems, int page_size, int n_pages, size_t page_elems, int box_rows);
 struct TcGemm {
   const TensorMap2D* w[3];  // weight maps, box rows = 128 (EPI_SILU_MUL: 64)
+  const bf16* wp[3];        // the weights themselves (null: stages of one k-block)
   const bf16* x;            // activations [M, K]
   int rows[3];
   int nseg, M, K, epi;
