@@ -1140,20 +1140,14 @@ int qie_prefill(qie_engine* e, int seq, const int32_t* h_ids, int n, int32_t* h_
     bool last = c0 + m == n;
     int* st = e->stage_h;
     ENGINE_SYNC(e);  // staging buffer reuse
-    for (int i = 0; i < m; ++i) {
-      st[i] = h_ids[c0 + i];
-      st[R + i] = s.len + c0 + i;
-      st[2 * R + i] = seq;
-      st[3 * R + i] = s.step;
-    }
-    CU(cudaMemcpyAsync(e->ids_d, st, m * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CU(cudaMemcpyAsync(e->pos_d, st + R, m * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    CU(cudaMemcpyAsync(e->slot_d, st + 2 * R, m * sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    // the sampled row is row 0 of the sampler -> its step lives in rowstep_d[0]
-    CU(cudaMemcpyAsync(e->rowstep_d, st + 3 * R, sizeof(int), cudaMemcpyHostToDevice, e->stream));
+    memcpy(st, h_ids + c0, m * sizeof(int));
+    // (the sampled row is row 0 of the sampler -> its step lives in rowstep_d[0])
+    CU(launch_stage_rows(st, m, s.len + c0, seq, s.step, e->ids_d, e->pos_d, e->slot_d, e->rowstep_d, e->stream));
+    ++e->launches;
     CU(forward_rows(e, m, s.len + c0 + m, m - 1, last ? 1 : 0, e->temp_prefill, false));
   }
-  CU(cudaMemcpyAsync(e->sampled_h, e->sampled_d, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+  CU(launch_publish_token(e->sampled_d, e->sampled_h, e->stream));
+  ++e->launches;
   ENGINE_SYNC(e);
   *h_token = e->sampled_h[0];
   s.len += n;

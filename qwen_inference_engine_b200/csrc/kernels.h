@@ -49,6 +49,9 @@ struct GemmArgs {
 cudaError_t launch_gemm_ref_order(const GemmArgs& args, int num_sms, cudaStream_t st);
 
 // ---------------------------------------------------------------- row-wise ops
+// a prompt's row descriptions out of page-locked memory, and its token back into it
+cudaError_t launch_stage_rows(const int* src, int n, int pos0, int seq, int step, int* ids, int* pos, int* slot, int* steps, cudaStream_t st);
+cudaError_t launch_publish_token(const int* token, int* dst, cudaStream_t st);
 cudaError_t launch_embedding(bf16* out, const bf16* table, const int* ids, size_t hidden, size_t n_tok,
                              cudaStream_t st);
 cudaError_t launch_rmsnorm_ref(const bf16* x, const bf16* w, bf16* y, size_t hidden, size_t n_tok,
