@@ -857,7 +857,7 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
   }
 }
 
-// 1 < k <= TC_MOST: a cluster of 8 CTAs per row, each over an eighth of the row, 16 bytes a load.  The k-th largest of the threads' maxima is a
+// 1 < k <= TC_MOST: a cluster of 8, 4 or 2 CTAs per row, each over its part of the row, 16 bytes a load.  The k-th largest of the threads' maxima is a
 // bound that at least k values of the slice reach; the values that reach it (about 1.1 k of them) are the slice's candidates.  The first
 // CTA gathers the candidates of all slices through distributed shared memory, finds the k-th value by bisection over its 16 bits,
 // ranks what is left by counting (all keys differ) and runs the reference's tail: quotients and exponentials by a thread each, the
@@ -866,9 +866,9 @@ __global__ void __launch_bounds__(1024) sample_topk_select_kernel(const bf16* __
 // One block per row read the row eight times, two bytes a load: k = 50 of 151936, 1 row 369 us, 64 rows 384.  The cluster with both passes over memory,
 // every value brought into its order and the gathering CTA by CTA: 18.2 and 39.2.  Now a piece of eight values is one packed maximum and the second pass
 // looks into those that reach the bound (a few per cent), the slice is read from memory once, all counts and then all candidates are
-// gathered at once, and the draw is compared with the running sums of the one chain: 13.8 and 25.1.  The bound is the latency of the steps, not
-// memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 9.4 us.
-constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;
+// gathered at once, and the draw is compared with the running sums of the one chain: 13.8 and 25.1, with clusters of two for
+// many rows 19.4.  The bound is the latency of the steps, not memory (19 MB).  Greedy (k = 1) stays with the two kernels above: 64 rows 9.4 us.
+constexpr int TC_CTAS = 8, TC_CAP = 512, TC_MOST = 128;  // TC_CTAS: the largest cluster
 // order-preserving 16 bits; 0: never selected
 __device__ __forceinline__ uint32_t topk_order16(uint32_t b) {
   if (!topk_valid((uint16_t)b)) return 0u;
@@ -983,9 +983,9 @@ __device__ __noinline__ void topk_slice_ties(const TopkSlice<TC_THREADS> sl, Top
 }
 // STAGED: the slice is copied to shared memory once, its two passes read it there (up to TC_STAGE bytes, 48 KB with the 9.6 KB of the rest, so that four
 // CTAs share an SM; the first CTA's gathered candidates go over it).
-constexpr int TC_STAGE = 38 * 1024, TC_ALL = TC_CTAS * TC_CAP * 8;  // bytes
-template <int TC_THREADS, bool STAGED>
-__global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
+constexpr int TC_STAGE = 38 * 1024;  // bytes in clusters of 8, twice and four times that in clusters of 4 and 2
+template <int TC_THREADS, bool STAGED, int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
                                uint64_t seed_stride, const int* __restrict__ step_ptr, unsigned long long subsequence) {
   static_assert(TC_THREADS > TC_MOST && TC_CAP >= TC_MOST, "a thread for every exponential and one for the random number; k candidates fit");
@@ -997,7 +997,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   __shared__ __align__(16) float vals[TC_MOST];
   __shared__ float cums[TC_MOST];
   __shared__ int idxs[TC_MOST];
-  __shared__ int s_n, s_cnt[3], s_tot, s_ns[TC_CTAS];
+  __shared__ int s_n, s_cnt[3], s_tot, s_ns[CTAS];
   __shared__ float s_u;
   unsigned long long* all = reinterpret_cast<unsigned long long*>(tc_buf);  // first CTA: everybody's
   const int tid = threadIdx.x, slice = blockIdx.x, rowi = blockIdx.y;
@@ -1007,7 +1007,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   TopkSlice<TC_THREADS> sl;
   sl.row = row;
   sl.head = (int)min((size_t)((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / 2, vocab);
-  const size_t nvec = (vocab - sl.head) / 8, per = (nvec + TC_CTAS - 1) / TC_CTAS;
+  const size_t nvec = (vocab - sl.head) / 8, per = (nvec + CTAS - 1) / CTAS;
   sl.v0 = min(nvec, slice * per), sl.v1 = min(nvec, sl.v0 + per);
   sl.tail0 = sl.head + (int)nvec * 8, sl.loose = slice == 0 ? sl.head + (int)vocab - sl.tail0 : 0;
   const bool loose = tid < sl.loose;  // this thread's element in front of the first 16-byte boundary or behind the last whole piece
@@ -1071,7 +1071,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   cluster_sync_all();
   if (slice == 0) {
     // ---- gather: all counts at once, then all candidates
-    if (tid < TC_CTAS) {
+    if (tid < CTAS) {
       uint32_t an;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(an) : "r"(smem_u32(&s_n)), "r"(tid));
       asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(s_ns[tid]) : "r"(an) : "memory");
@@ -1079,7 +1079,7 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     __syncthreads();
     int n = 0;
 #pragma unroll
-    for (int c = 0; c < TC_CTAS; ++c) {
+    for (int c = 0; c < CTAS; ++c) {
       uint32_t ac;
       const int cn = s_ns[c];
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ac) : "r"(smem_u32(cand)), "r"(c));
@@ -1186,12 +1186,21 @@ __global__ void __cluster_dims__(TC_CTAS, 1, 1) __launch_bounds__(TC_THREADS)
   }
   cluster_sync_all();  // nobody leaves while the first CTA reads its candidates
 }
-template <int TC_THREADS, bool STAGED>
+template <int TC_THREADS, bool STAGED, int CTAS>
 static cudaError_t launch_topk_cluster(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature, int k, uint64_t seed, uint64_t seed_stride,
                                        const int* step_ptr, unsigned long long subsequence, cudaStream_t st) {
-  const size_t slice = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16, smem = STAGED ? std::max<size_t>(slice, TC_ALL) : TC_ALL;
-  return launch_k(sample_topk_cluster_kernel<TC_THREADS, STAGED>, dim3(TC_CTAS, n_rows), dim3(TC_THREADS), smem, st, logits, out_tokens, vocab, temperature, k, seed,
-                  seed_stride, step_ptr, subsequence);
+  constexpr size_t all = (size_t)CTAS * TC_CAP * 8;
+  const size_t slice = (vocab / 8 + CTAS - 1) / CTAS * 16, smem = STAGED ? std::max(slice, all) : all;
+  if constexpr (STAGED && CTAS < TC_CTAS) {
+    static PerDeviceOnce set;
+    if (set.need()) {
+      cudaError_t e = cudaFuncSetAttribute(sample_topk_cluster_kernel<TC_THREADS, STAGED, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_STAGE * TC_CTAS / CTAS + 64);
+      if (e != cudaSuccess) return e;
+      set.done();
+    }
+  }
+  return launch_k(sample_topk_cluster_kernel<TC_THREADS, STAGED, CTAS>, dim3(CTAS, n_rows), dim3(TC_THREADS), smem, st, logits, out_tokens, vocab, temperature, k,
+                  seed, seed_stride, step_ptr, subsequence);
 }
 
 cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature,
@@ -1235,10 +1244,15 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
   // (slices longer than a candidate list of which fewer than k threads hold a value, vocabularies of 4 to 8 thousand with large k, have no bound to
   // start from: 64 rows of 8000, k = 128, 44 us by the radix select, 86 here)
   if (k > 1 && k <= TC_MOST && vocab <= (1u << 23) && n_rows <= 65535 && (vocab <= (size_t)TC_CTAS * TC_CAP || vocab / (TC_CTAS * 8) > (size_t)k)) {
-    // many rows: 256 threads, so that all clusters are on the chip at once; few rows: 512, for shorter passes
+    // Few rows take all the CTAs they can get; more rows fewer of them, whose first one has fewer candidates to rank and shares its SM with less (us of
+    // 151936, k = 50, 8 4 2 CTAs a row: 1 row 14.0 14.9 16.5, 8 14.2 15.4 17.1, 16 17.3 15.6 17.5, 32 17.9 17.3 17.9, 48 24.4 20.8 19.0, 64 25.2 21.9 19.4).  A
+    // slice has to hold more pieces than k, as above.
     const bool staged = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16 <= (size_t)TC_STAGE;
-    auto launch = n_rows > 16 ? (staged ? launch_topk_cluster<256, true> : launch_topk_cluster<256, false>)
-                              : (staged ? launch_topk_cluster<512, true> : launch_topk_cluster<512, false>);
+    auto holds = [&](int ctas) { return vocab <= (size_t)ctas * TC_CAP || vocab / (ctas * 8) > (size_t)k; };
+    auto launch = !staged ? (n_rows > 16 ? launch_topk_cluster<256, false, 8> : launch_topk_cluster<512, false, 8>)
+                  : n_rows > 32 && holds(2) ? launch_topk_cluster<512, true, 2>
+                  : n_rows > 8 && holds(4)  ? launch_topk_cluster<512, true, 4>
+                                            : launch_topk_cluster<512, true, 8>;
     return launch(logits, out_tokens, n_rows, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence, st);
   }
   // more than TC_MOST candidates, and the above: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the
