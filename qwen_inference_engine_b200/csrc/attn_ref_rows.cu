@@ -95,6 +95,19 @@ __device__ __forceinline__ void score_tree(float (&t)[4][2], int l, const Q& q, 
   }
 }
 
+// Softmax: the position that a thread reads as the u-th behind k0, where its positions are `step` apart; its first one again where that is behind
+// `end`, since the last one in front of the end is another thread's, which writes it in the same pass.
+__host__ __device__ constexpr int own_position(int k0, int u, int step, int end) { return k0 + u * step < end ? k0 + u * step : k0; }
+constexpr bool reads_own_positions(int step, int end) {
+  for (int first = 0; first < step; ++first)
+    for (int k0 = first; k0 < end; k0 += 8 * step)
+      for (int u = 0; u < 8; ++u)
+        if (own_position(k0, u, step, end) % step != first || own_position(k0, u, step, end) >= end) return false;
+  return true;
+}
+static_assert(reads_own_positions(NT / 8, 1) && reads_own_positions(NT / 8, 333) && reads_own_positions(NT / 16, 131) && reads_own_positions(NT / 32, 70),
+              "a position belongs to one thread");
+
 template <int NP, int R, bool ANY>
 __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, int rows) {
   pdl_wait();
@@ -284,7 +297,7 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
     for (int k0 = tid / R; k0 < max_len; k0 += U * KT) {
       float e[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = S[min(k0 + u * KT, max_len - 1) * R + r];
+      for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, max_len) * R + r];
 #pragma unroll
       for (int u = 0; u < U; ++u) e[u] = expf(__fsub_rn(e[u], m));
 #pragma unroll
@@ -315,7 +328,7 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
     for (int k0 = tid / R; k0 < len; k0 += U * KT) {
       float e[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = S[min(k0 + u * KT, len - 1) * R + r];
+      for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, len) * R + r];
       quot32(e, sum);
 #pragma unroll
       for (int u = 0; u < U; ++u)

@@ -105,3 +105,12 @@ def test_page_list(layers, hd, n, offset):
                                           C.c_void_p(torch.cuda.current_stream().cuda_stream)))
     torch.cuda.synchronize()
     assert np.array_equal(out.view(torch.int16).cpu().numpy(), got[1].cpu().numpy())
+
+
+@pytest.mark.parametrize("nq,nkv,hd,n", [(14, 2, 64, 400), (14, 2, 64, 3), (12, 2, 128, 5), (16, 2, 256, 7)])
+@pytest.mark.parametrize("end", [17, 63, 64, 65, 127, 128, 129, 255, 257, 300])
+def test_softmax_where_the_last_turn_is_short(layers, nq, nkv, hd, n, end):
+    """a thread's eight positions of a turn reach behind the end, by one to all but one"""
+    n = min(n, end)
+    got, _, _ = both(layers, nq, nkv, hd, 16, [end], [(0, end - n + i) for i in range(n)], end + hd)
+    assert torch.equal(got[0], got[1])
