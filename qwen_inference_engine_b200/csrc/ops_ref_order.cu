@@ -1246,13 +1246,15 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
   if (k > 1 && k <= TC_MOST && vocab <= (1u << 23) && n_rows <= 65535 && (vocab <= (size_t)TC_CTAS * TC_CAP || vocab / (TC_CTAS * 8) > (size_t)k)) {
     // Few rows take all the CTAs they can get; more rows fewer of them, whose first one has fewer candidates to rank and shares its SM with less (us of
     // 151936, k = 50, 8 4 2 CTAs a row: 1 row 14.0 14.9 16.5, 8 14.2 15.4 17.1, 16 17.3 15.6 17.5, 32 17.9 17.3 17.9, 48 24.4 20.8 19.0, 64 25.2 21.9 19.4).  A
-    // slice has to hold more pieces than k, as above.
+    // slice has to hold an eighth more pieces than k: with hardly more, the k-th of their maxima is a bound that most values reach, and the lists are
+    // long or overflow (33 rows of 2064, k = 128: 19.9 with eight CTAs, 25.3 with two; from 2304 on two are quicker).  More than 16 rows that stay
+    // with eight take 256 threads, so that all clusters are on the chip at once (256 rows of 2056, k = 128: 77 us, 132 with 512).
     const bool staged = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16 <= (size_t)TC_STAGE;
-    auto holds = [&](int ctas) { return vocab <= (size_t)ctas * TC_CAP || vocab / (ctas * 8) > (size_t)k; };
-    auto launch = !staged ? (n_rows > 16 ? launch_topk_cluster<256, false, 8> : launch_topk_cluster<512, false, 8>)
-                  : n_rows > 32 && holds(2) ? launch_topk_cluster<512, true, 2>
-                  : n_rows > 8 && holds(4)  ? launch_topk_cluster<512, true, 4>
-                                            : launch_topk_cluster<512, true, 8>;
+    auto holds = [&](int ctas) { return vocab <= (size_t)ctas * TC_CAP || vocab / (ctas * 8) >= (size_t)k + k / 8; };
+    auto launch = staged && n_rows > 32 && holds(2)  ? launch_topk_cluster<512, true, 2>
+                  : staged && n_rows > 8 && holds(4) ? launch_topk_cluster<512, true, 4>
+                  : n_rows > 16                      ? (staged ? launch_topk_cluster<256, true, 8> : launch_topk_cluster<256, false, 8>)
+                                                     : (staged ? launch_topk_cluster<512, true, 8> : launch_topk_cluster<512, false, 8>);
     return launch(logits, out_tokens, n_rows, vocab, temperature, k, seed, seed_stride, step_ptr, subsequence, st);
   }
   // more than TC_MOST candidates, and the above: the radix select; the k-round scan of the reference for vocabularies beyond 2^24 entries, which the

@@ -57,3 +57,21 @@ def test_nothing_to_choose(layers):
     x[1, 4098] = 3
     assert layers.sample_topk_bf16(to_dev(f32_to_bf16(x)), 4099, 1.0, 50, 1).tolist() == [-1, 4098]
     assert np.isinf(bf16_to_f32(f32_to_bf16(x))[0]).all()
+
+
+def some_rows(layers, oracle, lg, vocab, k, seed, check):
+    """rows against the restatement; the others are copies, and the same row gives the same token wherever it stands"""
+    got = layers.sample_topk_bf16(to_dev(lg), vocab, 0.7, k, seed)
+    for r in check:
+        want = oracle.argmax_tiebreak(lg[r]) if k == 1 else oracle.sample_topk(lg[r], 0.7, k, seed)
+        assert got[r] == want, (r, seed)
+    assert np.array_equal(got, np.tile(got[:len(check)], len(got) // len(check) + 1)[:len(got)])
+
+
+@pytest.mark.parametrize("kind", ["normal", "ties", "few"])
+@pytest.mark.parametrize("rows", [17, 33, 70])
+@pytest.mark.parametrize("vocab,k", [(1023, 128), (1040, 64), (2056, 128), (2064, 128), (2303, 128), (2304, 128), (4095, 120)])
+def test_slices_of_hardly_more_pieces_than_k(layers, oracle, vocab, k, rows, kind):
+    rng = np.random.default_rng(vocab + rows)
+    lg = np.stack([row(kind, vocab, rng) for _ in range(5)])
+    some_rows(layers, oracle, np.tile(lg, (rows // 5 + 1, 1))[:rows], vocab, k, 1234, range(5))
