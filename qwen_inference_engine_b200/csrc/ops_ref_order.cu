@@ -14,6 +14,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -75,15 +76,6 @@ cudaError_t launch_stage_rows(const int* src, int n, int pos0, int seq, int step
 cudaError_t launch_publish_token(const int* token, int* dst, cudaStream_t st) { return launch_k(publish_token_kernel, dim3(1), dim3(1), 0, st, token, (volatile int*)dst); }
 
 // ------------------------------------------------------------------ rmsNorm
-// The reference's sum is a strictly sequential fp32 FFMA chain over the hidden dimension (one thread per token); fp32 addition is not
-// associative, so the chain's order is part of the result.  A block takes R rows into shared memory as they are (bf16), R lanes of one warp
-// walk a chain each side by side, and the block does the rest in parallel.
-// What bounds it: the chain, 4 cycles an element (896 wide 1.9 us).  Its loads are 16 bytes and a group of 32 elements ahead: single floats read
-// inside the loop cost the chain as much again.  us at 1 / 1000 / 4000 rows, before (one row a block, fp32 in shared memory, a division an element) and
-// now: 896 wide 5.9 6.4 15.7 and 3.5 4.6 9.2; 1536 wide 9.3 9.9 25.9 and 5.2 6.3 13.2; 3584 wide 20.3 21.4 74 and 10.0 11.8 29.8.
-// VEC: rows, weights and results in pieces of 16 bytes; other widths and addresses are taken element by element.
-// Four rows a block from RMS_MANY rows on: from there more than one chain falls to each of an SM's schedulers, and the lanes of one warp share
-// their issue slots (1 and 4 rows a block, with divisions: 512 rows of 1536 6.1 6.6, 1000 rows 7.4 7.3, 2000 13.8 8.6).
 // eight elements: RN(x / rms) w, rounded to bf16
 __device__ __forceinline__ void norm8(const uint32_t (&x)[4], const uint32_t (&w)[4], const Quot& rms, uint32_t (&o)[4]) {
   float v[8];
@@ -93,38 +85,60 @@ __device__ __forceinline__ void norm8(const uint32_t (&x)[4], const uint32_t (&w
 #pragma unroll
   for (int j = 0; j < 4; ++j) o[j] = pack2f(__fmul_rn(v[2 * j], lo2f(w[j])), __fmul_rn(v[2 * j + 1], hi2f(w[j])));
 }
-constexpr size_t RMS_MANY = 6 * 148;
+
+// The reference's sum is a strictly sequential fp32 FFMA chain over the hidden dimension (one thread per token); fp32 addition is not
+// associative, so the chain's order is part of the result.  A block takes R rows into shared memory, R lanes of one warp walk a chain each
+// side by side, and the block does the rest in parallel.
+// What bounds it: the chain, 4 cycles an element (896 wide 1.9 us).  Its loads are 16 bytes and a group of four pieces ahead: single floats read
+// inside the loop cost the chain as much again.  us at 1 / 1000 / 4000 rows, before (one row a block, fp32 in shared memory, a division an element) and
+// now: 250 wide 2.7 3.3 6.6 and 2.7 3.3 6.7; 896 wide 6.2 6.6 15.7 and 3.8 4.8 9.4; 1536 wide 9.7 10.2 25.3 and 5.3 6.5 13.3; 3584 wide 20.9 21.5 58 and
+// 10.1 12.1 26.4.
+// VEC: rows (bf16 as they are), weights and results in pieces of 16 bytes.  Other widths and addresses: element by element, one row a block, and the row
+// in fp32, so that the chain unpacks nothing: its issue slots bound launches of many rows (1500 rows of 250: 3.9 us, 4.6 from bf16).
+// Four rows a block from RMS_MANY rows an SM on (twice as many where a row is narrow): from there more than one chain falls to each of an SM's schedulers,
+// and the lanes of one warp share their issue slots.  1 and 4 rows a block, us: 256 wide 1000 rows 2.6 3.2, 1500 3.0 3.3, 2000 4.3 3.4; 640 wide 888 rows 3.9
+// 4.2, 1500 5.0 4.5; 896 wide 700 rows 4.6 4.8, 1000 4.8 4.8, 2000 8.6 5.4; 1536 wide 700 rows 6.7 6.6, 1000 7.0 6.6, 2000 13.1 7.3.
+constexpr size_t RMS_MANY = 6, RMS_WIDE = 640;
+// bytes of a row in shared memory: whole pieces of 16 and one more, so that lanes that walk a row each read different banks
+__host__ __device__ inline size_t rms_pitch(size_t hidden, size_t elem) { return ((hidden * elem + 15) / 16 + 1) * 16; }
 template <int R, bool VEC>
 __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, int hidden,
                                                                         size_t x_stride, int n_tok, float eps) {
+  static_assert(VEC || R == 1, "one row element by element");
   constexpr int RMS_NT = R > 1 ? 256 : 128;
+  using T = std::conditional_t<VEC, bf16, float>;
+  constexpr int PIECE = 16 / sizeof(T), GROUP = 4 * PIECE;
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char rms_rows[];
   __shared__ float s_rms[R];
-  const int pitch = ((hidden + 7) / 8 + 1) * 16;  // bytes of a row: whole pieces and one more, so that R lanes read different banks
+  const int pitch = (int)rms_pitch(hidden, sizeof(T));
   const int row0 = blockIdx.x * R, n = min(R, n_tok - row0), tid = threadIdx.x;
+  uint4 w0 = make_uint4(0u, 0u, 0u, 0u);  // this thread's first weights: on their way beside the chain (with four rows the registers would cost a block on the SM)
   if constexpr (VEC) {  // all pieces on their way at once
     const int nv = hidden / 8;
     const uint32_t dst = smem_u32(rms_rows);
     for (int r = 0; r < n; ++r)
       for (int i = tid; i < nv; i += RMS_NT) cp_async16(dst + (uint32_t)(r * pitch + i * 16), x + (size_t)(row0 + r) * x_stride + i * 8);
     cp_async_commit();
+    if (R == 1 && tid < nv) w0 = reinterpret_cast<const uint4*>(w)[tid];
     cp_async_wait<0>();
   } else {
-    for (int r = 0; r < n; ++r)
-      for (int i = tid; i < hidden; i += RMS_NT) reinterpret_cast<bf16*>(rms_rows + (size_t)r * pitch)[i] = x[(size_t)(row0 + r) * x_stride + i];
+    for (int i = tid; i < hidden; i += RMS_NT) reinterpret_cast<float*>(rms_rows)[i] = bf2f(x[(size_t)row0 * x_stride + i]);
   }
   __syncthreads();
   if (tid < n) {
     const uint4* p = reinterpret_cast<const uint4*>(rms_rows + (size_t)tid * pitch);
     float sum = 0.f;
-    const int groups = hidden / 32;
+    const int groups = hidden / GROUP, rest = hidden - groups * GROUP;
     uint4 cur[4], nxt[4];
-    auto add = [&](uint32_t u) {
-      const float a = lo2f(u), b = hi2f(u);
-      sum = __fmaf_rn(a, a, sum);
-      sum = __fmaf_rn(b, b, sum);
+    auto add = [&](const uint4& v, int left) {  // a piece, or the `left` elements that there are of it
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < PIECE; ++j) {
+        const float a = !VEC ? __uint_as_float(u[j % 4]) : j & 1 ? hi2f(u[j / 2]) : lo2f(u[j / 2]);
+        if (j < left) sum = __fmaf_rn(a, a, sum);
+      }
     };
     if (groups > 0) {
 #pragma unroll
@@ -136,13 +150,17 @@ __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf
 #pragma unroll
       for (int j = 0; j < 4; ++j) nxt[j] = q[j];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) add(cur[j].x), add(cur[j].y), add(cur[j].z), add(cur[j].w);
+      for (int j = 0; j < 4; ++j) add(cur[j], PIECE);
 #pragma unroll
       for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
     }
-    for (int i = groups * 32; i < hidden; ++i) {
-      const float a = bf2f(reinterpret_cast<const bf16*>(p)[i]);
-      sum = __fmaf_rn(a, a, sum);
+    if (rest > 0) {  // up to four more pieces, the last one cut short (never with VEC)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j * PIECE < rest) cur[j] = p[4 * groups + j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j * PIECE < rest) add(cur[j], VEC ? PIECE : rest - j * PIECE);
     }
     s_rms[tid] = __fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps));  // eps 1e-4 in the reference (normalization.cu:9)
   }
@@ -150,7 +168,7 @@ __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf
   if constexpr (VEC) {
     const int nv = hidden / 8;
     for (int i = tid; i < nv; i += RMS_NT) {
-      const uint4 wv = reinterpret_cast<const uint4*>(w)[i];
+      const uint4 wv = R == 1 && i == tid ? w0 : reinterpret_cast<const uint4*>(w)[i];
       const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -163,24 +181,31 @@ __global__ void __launch_bounds__(R > 1 ? 256 : 128) rmsnorm_ref_kernel(const bf
       }
     }
   } else {
-    for (int r = 0; r < n; ++r)
-      for (int i = tid; i < hidden; i += RMS_NT)
-        y[(size_t)(row0 + r) * hidden + i] = f2bf(__fmul_rn(__fdiv_rn(bf2f(reinterpret_cast<const bf16*>(rms_rows + (size_t)r * pitch)[i]), s_rms[r]), bf2f(w[i])));
+    const float rms = s_rms[0];
+    for (int i = tid; i < hidden; i += RMS_NT)
+      y[(size_t)row0 * hidden + i] = f2bf(__fmul_rn(__fdiv_rn(reinterpret_cast<const float*>(rms_rows)[i], rms), bf2f(w[i])));
   }
 }
 
 cudaError_t launch_rmsnorm_ref(const bf16* x, const bf16* w, bf16* y, size_t hidden, size_t n_tok, size_t x_stride,
                                cudaStream_t st, float eps) {
   if (n_tok == 0) return cudaSuccess;
-  const size_t pitch = ((hidden + 7) / 8 + 1) * 16;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const size_t pitch = rms_pitch(hidden, sizeof(bf16)), sms = device_attribute<cudaDevAttrMultiProcessorCount>(dev);
   const bool vec = hidden % 8 == 0 && x_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  if (vec && n_tok >= RMS_MANY && 4 * pitch <= 40 * 1024)
-    (void)launch_spread<rmsnorm_ref_kernel<4, true>>(dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
-  else if (vec)
-    (void)launch_spread<rmsnorm_ref_kernel<1, true>>(dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
-  else
-    (void)launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
-  return cudaGetLastError();
+  if (vec && n_tok >= (hidden < RMS_WIDE ? 2 : 1) * RMS_MANY * sms && 4 * pitch <= 40 * 1024)
+    return launch_spread<rmsnorm_ref_kernel<4, true>>(dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+  if (vec)
+    return launch_spread<rmsnorm_ref_kernel<1, true>>(dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+  static PerDeviceOnce set;  // (12288 elements are a little more than the 48 KB that need no attribute)
+  if (set.need()) {
+    e = cudaFuncSetAttribute(rmsnorm_ref_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    if (e != cudaSuccess) return e;
+    set.done();
+  }
+  return launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), rms_pitch(hidden, sizeof(float)), st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
 }
 
 // fast-numerics variant: the sum of squares is reduced in parallel (warp shuffles), so it

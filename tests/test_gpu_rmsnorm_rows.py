@@ -39,3 +39,20 @@ def test_operands_off_a_16_byte_boundary(oracle, n_tok, off):
     xd, wd, y = placed(x, off[0]), placed(w, off[1]), placed(np.zeros_like(x), off[2])
     L.launch_rms(xd, wd, y, hidden, n_tok)
     assert np.array_equal(to_host(y), oracle.rmsnorm(x, w))
+
+
+@pytest.mark.parametrize("n_tok", [1, 889, 1775, 1776, 1777])
+@pytest.mark.parametrize("hidden", [8, 15, 16, 17, 31, 40, 250, 632, 640, 1001, 12287, 12288])
+def test_remainders_of_the_chain(oracle, hidden, n_tok):
+    """the last pieces of a row, whole and cut short; widths around the rule for four rows a block, at 6 and 12 rows an SM; the widest row in fp32"""
+    from qwen_inference_engine_b200 import layers as L
+    rng = np.random.default_rng(hidden * 3 + n_tok)
+    x, w = rand_bf16(rng, (n_tok, hidden), 1.5), rand_bf16(rng, (hidden,), 1.0)
+    want = oracle.rmsnorm(x, w)
+    for off in (0, 1):  # off 1: element by element at any width
+        buf = torch.zeros(x.size + 16, dtype=torch.bfloat16, device="cuda")
+        xd = buf[off:off + x.size].view(x.shape)
+        xd.copy_(to_dev(x))
+        y = torch.full_like(to_dev(x), 3.0)
+        L.launch_rms(xd, to_dev(w), y, hidden, n_tok)
+        assert np.array_equal(to_host(y), want), off
