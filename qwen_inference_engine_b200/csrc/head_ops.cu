@@ -7,7 +7,7 @@
 // are in the lane again; interleaved and half-rotation partners are in the lane as well.  Square root, reciprocal and page lookup are done once
 // for all heads of a warp.  One head after the other on 32 lanes with 4-byte accesses took about 250 instructions a head of 128, here 75.
 // What bounds it now: latency of the loads and DRAM; behind a projection 4096 tokens of 16 heads of 128 took 23.5 us
-// and take 11.2, 512 tokens of 18 heads of 64 6.5 and 3.1; head norms and positions alone, 1000 x 12 heads of 128, 3.4 and 3.0, now 2.3 and 2.0.
+// and take 11.2, 512 tokens of 18 heads of 64 6.5 and 3.1; head norms and positions alone, 1000 x 12 heads of 128, 3.4 and 3.0, now 2.3 and 2.0 (positions of few heads: 32 lanes a head, see the rule).
 #include <initializer_list>
 
 #include "common.cuh"
@@ -199,6 +199,27 @@ __global__ void __launch_bounds__(128) rope_ref_kernel(const float* __restrict__
   v.template store<V>(p, l);
 }
 
+// The same with a head on 32 lanes, 4 bytes an access: where there are so few heads that a lane's 16 elements are a chain and leave SMs idle.
+template <int NP>
+__global__ void __launch_bounds__(128) rope_ref_pairs_kernel(const float* __restrict__ cos_t, const float* __restrict__ sin_t, bf16* x, int n_tok, const int* __restrict__ pos,
+                                                             int pos0, int row_dim, int n_heads) {
+  pdl_wait();
+  pdl_trigger();
+  const int at = (blockIdx.x * 128 + threadIdx.x) / 32, l = threadIdx.x % 32;
+  if (at >= n_tok * n_heads) return;
+  const int tok = at / n_heads, ps = pos ? pos[tok] : pos0 + tok;
+  uint32_t* p = reinterpret_cast<uint32_t*>(x + (size_t)tok * row_dim + (size_t)(at - tok * n_heads) * 64 * NP) + l;
+  const float *co = cos_t + (size_t)ps * 32 * NP + l, *si = sin_t + (size_t)ps * 32 * NP + l;
+  uint32_t u[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) u[i] = p[32 * i];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const float c = co[32 * i], s = si[32 * i], x0 = lo2f(u[i]), x1 = hi2f(u[i]);
+    p[32 * i] = pack2f(__fmaf_rn(x0, c, -__fmul_rn(x1, s)), __fmaf_rn(c, x1, __fmul_rn(x0, s)));
+  }
+}
+
 bool on16(std::initializer_list<const void*> ps) {
   for (const void* p : ps)
     if (reinterpret_cast<uintptr_t>(p) & 15) return false;
@@ -236,8 +257,17 @@ cudaError_t launch_qknorm_ref(bf16* x, const bf16* w, int hd, int n_tok, int row
 cudaError_t launch_rope_ref(const float* cos_t, const float* sin_t, bf16* x, int n_tok, const int* pos, int pos0, int hd, int row_dim, int n_heads, cudaStream_t st) {
   const long heads = (long)n_tok * n_heads;
   if (heads == 0) return cudaSuccess;
-  QIE_HEADS(hd, (on16({x, cos_t, sin_t}) && row_dim % 8 == 0),
-            (void)launch_k(rope_ref_kernel<NP, V>, dim3(blocks_of(heads, hd)), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads));
+  // 16 elements a lane from 4096 heads of 64 on, as many elements of wider ones; off a 16-byte boundary from 6144 (256 wide from 40000 heads, since 32 lanes
+  // read whole sectors and 16 do not).  us with 32 lanes and with 16 elements: 17 heads of 64 1.2 1.3, 2800 1.6 1.8, 4000 1.7 1.8, 7168 2.5 1.8; off a
+  // boundary 1 head 1.2 1.4, 4000 1.8 2.0, 7168 2.6 2.2; 14000 of 256 there 4.5 5.5, 42000 11.7 10.9.
+  const bool vec = on16({x, cos_t, sin_t}) && row_dim % 8 == 0;
+  if (heads * hd > 64L * (vec ? 4096 : hd < 256 ? 6144 : 160000)) {
+    QIE_HEADS(hd, vec, (void)launch_k(rope_ref_kernel<NP, V>, dim3(blocks_of(heads, hd)), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads));
+    return cudaGetLastError();
+  }
+  const auto pairs = hd == 64 ? rope_ref_pairs_kernel<1> : hd == 128 ? rope_ref_pairs_kernel<2> : hd == 256 ? rope_ref_pairs_kernel<4> : nullptr;
+  if (!pairs) return cudaErrorInvalidValue;
+  (void)launch_k(pairs, dim3((unsigned)((heads + 3) / 4)), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads);
   return cudaGetLastError();
 }
 

@@ -74,3 +74,16 @@ def test_every_significand_of_the_numerator(oracle):
     y = torch.zeros(4000, 256, dtype=torch.bfloat16, device="cuda")
     L.launch_rms(to_dev(x), to_dev(w), y, 256, 4000)
     assert np.array_equal(to_host(y), oracle.rmsnorm(x, w))
+
+
+@pytest.mark.parametrize("hd,heads,rows,off", [(64, 14, 292, 0), (64, 14, 293, 0), (64, 14, 438, 2), (64, 14, 439, 2), (128, 12, 170, 0), (128, 12, 171, 0), (128, 12, 257, 2),
+                                               (256, 2, 512, 0), (256, 2, 513, 0), (256, 28, 1429, 2)])
+def test_positions_around_the_rule(oracle, hd, heads, rows, off):
+    """both layouts of a head, on and off a 16-byte boundary, on both sides of the number of heads that chooses between them"""
+    from qwen_inference_engine_b200 import layers as L
+    rng = np.random.default_rng(hd + rows)
+    x = rand_bf16(rng, (rows, heads * hd), 1.3)
+    cos, sin = L.precompute_cos_sin(rows, hd)
+    y = placed(x, off)
+    L.launch_rope(torch.from_numpy(cos).cuda(), torch.from_numpy(sin).cuda(), y, rows, hd, heads * hd, heads)
+    assert np.array_equal(to_host(y), oracle.rope(cos, sin, x, 0, hd, heads))
