@@ -98,15 +98,15 @@ __device__ __forceinline__ void score_tree(float (&t)[4][2], int l, const Q& q, 
 // Softmax: the position that a thread reads as the u-th behind k0, where its positions are `step` apart; its first one again where that is behind
 // `end`, since the last one in front of the end is another thread's, which writes it in the same pass.
 __host__ __device__ constexpr int own_position(int k0, int u, int step, int end) { return k0 + u * step < end ? k0 + u * step : k0; }
-constexpr bool reads_own_positions(int step, int end) {
+constexpr bool reads_own_positions(int turn, int step, int end) {
   for (int first = 0; first < step; ++first)
-    for (int k0 = first; k0 < end; k0 += 8 * step)
-      for (int u = 0; u < 8; ++u)
+    for (int k0 = first; k0 < end; k0 += turn * step)
+      for (int u = 0; u < turn; ++u)
         if (own_position(k0, u, step, end) % step != first || own_position(k0, u, step, end) >= end) return false;
   return true;
 }
-static_assert(reads_own_positions(NT / 8, 1) && reads_own_positions(NT / 8, 333) && reads_own_positions(NT / 16, 131) && reads_own_positions(NT / 32, 70),
-              "a position belongs to one thread");
+static_assert(reads_own_positions(8, NT / 8, 333) && reads_own_positions(8, NT / 16, 131) && reads_own_positions(8, NT / 32, 70) && reads_own_positions(2, NT / 8, 1) &&
+                  reads_own_positions(2, NT / 8, 45), "a position belongs to one thread");
 
 template <int NP, int R, bool ANY>
 __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, int rows) {
@@ -293,46 +293,68 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
 #pragma unroll
     for (int w = 1; w < NWARP; ++w) m = fmaxf(m, s_max[w][r]);
     constexpr int KT = NT / R;  // a thread's positions are KT apart; it takes eight at a time, whose chains run side by side
-    constexpr int U = 8;
-    for (int k0 = tid / R; k0 < max_len; k0 += U * KT) {
-      float e[U];
+    // Up to 4 KT positions: two at a time, the sums' loads in their own turn, plain divisions; the long forms are more instructions than there is work (cycles
+    // of the three steps at 17 positions 600 1250 730, so 330 770 330; 17 rows of 14 heads of 64 by the operator 6.5 us, so 6.0; one row at 200 with
+    // the short forms 11.4, with the long ones 9.9).
+    auto exponentials = [&](auto turn) {
+      constexpr int U = decltype(turn)::value;
+      for (int k0 = tid / R; k0 < max_len; k0 += U * KT) {
+        float e[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, max_len) * R + r];
+        for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, max_len) * R + r];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = expf(__fsub_rn(e[u], m));
+        for (int u = 0; u < U; ++u) e[u] = expf(__fsub_rn(e[u], m));
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k0 + u * KT < max_len) S[(k0 + u * KT) * R + r] = k0 + u * KT < len ? e[u] : 0.f;
-    }
+        for (int u = 0; u < U; ++u)
+          if (k0 + u * KT < max_len) S[(k0 + u * KT) * R + r] = k0 + u * KT < len ? e[u] : 0.f;
+      }
+    };
+    const bool few = max_len <= 4 * KT;
+    if (few) exponentials(std::integral_constant<int, 2>{});
+    else exponentials(std::integral_constant<int, 8>{});
     __syncthreads();
     if (tid < R) {  // one chain per virtual row; zeros behind a row's positions leave its sum as it is
       float sum = 0.f, e[16];
       int k = 0;
-      if (max_len >= 16) {
+      if (few) {
+        for (; k + 16 <= max_len; k += 16) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) e[i] = S[(size_t)i * R + tid];
+          for (int i = 0; i < 16; ++i) e[i] = S[(k + i) * R + tid];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) sum = __fadd_rn(sum, e[i]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) e[i] = S[i * R + tid];
+        for (; k + 16 <= max_len; k += 16) {
+          float next[16];
+          const float* p = S + min(k + 16, max_len - 16) * R + tid;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) next[i] = p[i * R], sum = __fadd_rn(sum, e[i]);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) e[i] = next[i];
+        }
       }
-      for (; k + 16 <= max_len; k += 16) {
-        float next[16];
-        const float* p = S + (size_t)min(k + 16, max_len - 16) * R + tid;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) next[i] = p[i * R], sum = __fadd_rn(sum, e[i]);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) e[i] = next[i];
-      }
-      for (; k < max_len; ++k) sum = __fadd_rn(sum, S[(size_t)k * R + tid]);
+      for (; k < max_len; ++k) sum = __fadd_rn(sum, S[k * R + tid]);
       s_sum[tid] = sum;
     }
     __syncthreads();
-    const Quot sum = quot_of(s_sum[r]);
-    for (int k0 = tid / R; k0 < len; k0 += U * KT) {
-      float e[U];
+    if (few) {
+      const float sum = s_sum[r];
+#pragma unroll 2
+      for (int k = tid / R; k < len; k += KT) S[k * R + r] = __fdiv_rn(S[k * R + r], sum);
+    } else {
+      constexpr int U = 8;
+      const Quot sum = quot_of(s_sum[r]);
+      for (int k0 = tid / R; k0 < len; k0 += U * KT) {
+        float e[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, len) * R + r];
-      quot32(e, sum);
+        for (int u = 0; u < U; ++u) e[u] = S[own_position(k0, u, KT, len) * R + r];
+        quot32(e, sum);
 #pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k0 + u * KT < len) S[(k0 + u * KT) * R + r] = e[u];
+        for (int u = 0; u < U; ++u)
+          if (k0 + u * KT < len) S[(k0 + u * KT) * R + r] = e[u];
+      }
     }
   }
   // ---- values: RP rows x 4 columns a lane; the threads that are left fetch the next tile
@@ -399,11 +421,19 @@ __global__ void __launch_bounds__(NT, 2) attention_ref_rows_kernel(AttnArgs a, i
         }
       }
       const int end = min(TK, max(len[0], len[RP - 1]) - tl * TK);  // (negative for lanes without a row)
-      for (; kk < end; ++kk) {
-        const float4 v = *reinterpret_cast<const float4*>(vt + kk * HD);
+      for (; kk < end; kk += U) {  // (loads U at a time here as well; one position after the other took as long as the rest of the values at 17)
 #pragma unroll
-        for (int i = 0; i < RP; ++i)
-          if (tl * TK + kk < len[i]) add(i, pt[kk * R + i], v);
+        for (int u = 0; u < U; ++u) {
+          const int at = min(kk + u, end - 1);
+          x[0][u] = *reinterpret_cast<const float4*>(vt + at * HD);
+#pragma unroll
+          for (int i = 0; i < RP; ++i) p[0][u][i] = pt[at * R + i];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int i = 0; i < RP; ++i)
+            if (tl * TK + kk + u < len[i]) add(i, p[0][u][i], x[0][u]);
       }
     }
     __syncthreads();
