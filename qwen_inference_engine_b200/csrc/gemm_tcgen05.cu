@@ -978,8 +978,10 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   if (launches) *launches = 1;
   // Two k-blocks a stage where tensor maps can express them (whole k-blocks, and the weights' place is known): half the requests, waits and commits.  Up
   // to 64 tokens: of 128 the ring holds three such stages, too few on the way (8960 x 1536 at 1000 rows 34.8 with stages of one, 37.1).  Gate/up tiles
-  // are two boxes a k-block as they are.
-  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && t.wp[0]) {
+  // are two boxes a k-block as they are.  Not for 3 or 5 k-blocks: the half of the last stage that is not there is a box of zeros to bring, a quarter of
+  // the operands (us with stages of one and of two, 1000 rows: 192 x 130 3.7 4.0, 320 x 130 4.3 4.6, 448 x 130 4.7 4.7, 576 x 130 4.5 4.2).
+  const bool whole = g.splits > 1 || g.kb_total % 2 == 0 || g.kb_total > 5;
+  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && t.wp[0]) {
     TensorMap2D w3[3];
     bool ok = make_tensor_map_w3d(&x, t.x, t.M, t.K, 2 * BK, 0, tl.bn) == cudaSuccess;
     for (int i = 0; i < t.nseg; ++i) ok = ok && t.wp[i] && make_tensor_map_w3d(&w3[i], t.wp[i], t.rows[i], t.K, 2 * BK, 0, BM) == cudaSuccess;

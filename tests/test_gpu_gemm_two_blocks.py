@@ -32,3 +32,10 @@ def test_split_over_the_inner_dimension(inner, rows, outer):
     a, b = (torch.randn(n, inner, generator=g, device="cuda").bfloat16() for n in (rows, outer))
     want = a.double() @ b.double().T
     assert ((product(L.launch_matmul_fast, a, b).double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5 * inner ** 0.5).all()
+
+
+@pytest.mark.parametrize("inner", [192, 320, 384, 448, 576])
+@pytest.mark.parametrize("rows,outer", [(7, 130), (64, 896), (1000, 130), (16, 20001)])
+def test_same_bits_around_the_rule_for_odd_numbers_of_k_blocks(inner, rows, outer):
+    """3 and 5 k-blocks stay with stages of one, 6, 7 and 9 do not"""
+    test_same_bits_in_the_references_order(inner, rows, outer)
