@@ -208,16 +208,11 @@ __global__ void __launch_bounds__(128) rope_ref_pairs_kernel(const float* __rest
   const int at = (blockIdx.x * 128 + threadIdx.x) / 32, l = threadIdx.x % 32;
   if (at >= n_tok * n_heads) return;
   const int tok = at / n_heads, ps = pos ? pos[tok] : pos0 + tok;
-  uint32_t* p = reinterpret_cast<uint32_t*>(x + (size_t)tok * row_dim + (size_t)(at - tok * n_heads) * 64 * NP) + l;
-  const float *co = cos_t + (size_t)ps * 32 * NP + l, *si = sin_t + (size_t)ps * 32 * NP + l;
-  uint32_t u[NP];
-#pragma unroll
-  for (int i = 0; i < NP; ++i) u[i] = p[32 * i];
-#pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    const float c = co[32 * i], s = si[32 * i], x0 = lo2f(u[i]), x1 = hi2f(u[i]);
-    p[32 * i] = pack2f(__fmaf_rn(x0, c, -__fmul_rn(x1, s)), __fmaf_rn(c, x1, __fmul_rn(x0, s)));
-  }
+  bf16* p = x + (size_t)tok * row_dim + (size_t)(at - tok * n_heads) * 64 * NP;
+  float v[NP][2];
+  head_load<NP>(v, p, l);
+  head_rope<NP>(v, cos_t + (size_t)ps * 32 * NP, sin_t + (size_t)ps * 32 * NP, l);
+  head_store<NP>(v, p, l);
 }
 
 bool on16(std::initializer_list<const void*> ps) {
