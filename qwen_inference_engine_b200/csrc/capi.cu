@@ -297,10 +297,7 @@ int qie_matmul_fast(const qie_bf16* A, const qie_bf16* B, qie_bf16* C, int M, in
   OP_STATUS(status);
   int sms = 0;
   CU(sm_count(&sms));
-  TensorMap2D wmap;
-  CU(make_tensor_map_2d(&wmap, (const bf16*)B, K, N, 128));
   TcGemm t{};
-  t.w[0] = &wmap;
   t.wp[0] = (const bf16*)B;
   t.x = (const bf16*)A;
   t.rows[0] = K;
@@ -729,15 +726,20 @@ static int engine_finish_setup(qie_engine* e) {
     for (int l = 0; l < c.layers; ++l) {
       const LayerWeights& w = e->L[l];
       qie_engine::LayerMaps& m = e->wmaps[l];
-      CU(make_tensor_map_2d(&m.q, w.q, (int)Dq, (int)H, 128));
-      CU(make_tensor_map_2d(&m.k, w.k, (int)Dkv, (int)H, 128));
-      CU(make_tensor_map_2d(&m.v, w.v, (int)Dkv, (int)H, 128));
-      CU(make_tensor_map_2d(&m.o, w.o, (int)H, (int)Dq, 128));
-      CU(make_tensor_map_2d(&m.gate, w.gate, (int)I, (int)H, 64));  // dual tile: 64 gate + 64 up rows
-      CU(make_tensor_map_2d(&m.up, w.up, (int)I, (int)H, 64));
-      CU(make_tensor_map_2d(&m.down, w.down, (int)H, (int)I, 128));
+      auto maps = [&](qie_engine::WeightMaps& wm, const bf16* p, size_t rows, size_t inner) {  // (inner dimensions are multiples of 64)
+        cudaError_t r = make_tensor_map_2d(&wm.one, p, (int)rows, (int)inner, 128);
+        return r != cudaSuccess ? r : make_tensor_map_w3d(&wm.two, p, (int)rows, (int)inner, 128, 0, 128);
+      };
+      CU(maps(m.q, w.q, Dq, H));
+      CU(maps(m.k, w.k, Dkv, H));
+      CU(maps(m.v, w.v, Dkv, H));
+      CU(maps(m.o, w.o, H, Dq));
+      CU(make_tensor_map_2d(&m.gate.one, w.gate, (int)I, (int)H, 64));  // dual tile: 64 gate + 64 up rows
+      CU(make_tensor_map_2d(&m.up.one, w.up, (int)I, (int)H, 64));
+      CU(maps(m.down, w.down, H, I));
     }
-    CU(make_tensor_map_2d(&e->lm_head_map, e->lm_head, c.vocab, (int)H, 128));
+    CU(make_tensor_map_2d(&e->lm_head_map.one, e->lm_head, c.vocab, (int)H, 128));
+    CU(make_tensor_map_w3d(&e->lm_head_map.two, e->lm_head, c.vocab, (int)H, 128, 0, 128));
     // what the splits of a step write, as many as have all their CTAs on the chip (attention_decode_most_splits): about 1 MB
     e->attn_ws_rows = (size_t)std::max(FD_MOST, attention_decode_most_splits(1, c.n_kv, c.head_dim, e->num_sms)) * c.n_q;
     CU(cudaMalloc(&e->attn_ws, e->attn_ws_rows * (c.head_dim + 2) * sizeof(float)));

@@ -88,12 +88,12 @@ static cudaError_t gemm_rows(qie_engine* e, int kind, GemmArgs g, int n_rows) {
 }
 
 // tcgen05 GEMM launch (fast numerics, rows > 8). x: [n, K] activations.
-static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K, int nseg, const TensorMap2D* const* w, const bf16* const* wp,
+static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K, int nseg, const qie_engine::WeightMaps* const* w,
                            const int* rows, int epi, bf16* out, int ld_out) {
   TcGemm t{};
   for (int i = 0; i < nseg; ++i) {
-    t.w[i] = w[i];
-    t.wp[i] = wp[i];
+    t.w[i] = &w[i]->one;
+    if (epi != EPI_SILU_MUL) t.w2[i] = &w[i]->two;
     t.rows[i] = rows[i];
   }
   t.x = x;
@@ -149,10 +149,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     QIE_TRY(KK_RMSNORM, rms(e->x, w.in_ln, e->xn, n));
     capture_copy(e, "input_norm", l, e->xn, (size_t)n * H);
     if (tc) {
-      const TensorMap2D* wm[3] = {&e->wmaps[l].q, &e->wmaps[l].k, &e->wmaps[l].v};
-      const bf16* wp[3] = {w.q, w.k, w.v};
+      const qie_engine::WeightMaps* wm[3] = {&e->wmaps[l].q, &e->wmaps[l].k, &e->wmaps[l].v};
       const int rows[3] = {Dq, Dkv, Dkv};
-      cudaError_t r = gemm_tc(e, KK_GEMM_QKV, e->xn, n, H, 3, wm, wp, rows, EPI_STORE, e->qkv, Dq + 2 * Dkv);
+      cudaError_t r = gemm_tc(e, KK_GEMM_QKV, e->xn, n, H, 3, wm, rows, EPI_STORE, e->qkv, Dq + 2 * Dkv);
       if (r != cudaSuccess) return r;
     } else {
       GemmArgs g{};
@@ -265,10 +264,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     }
     capture_copy(e, "attn", l, e->att, (size_t)n * Dq);
     if (tc) {
-      const TensorMap2D* wm[1] = {&e->wmaps[l].o};
-      const bf16* wp[1] = {w.o};
+      const qie_engine::WeightMaps* wm[1] = {&e->wmaps[l].o};
       const int rows[1] = {H};
-      cudaError_t r = gemm_tc(e, KK_GEMM_O, e->att, n, Dq, 1, wm, wp, rows, EPI_RESIDUAL, e->x, H);
+      cudaError_t r = gemm_tc(e, KK_GEMM_O, e->att, n, Dq, 1, wm, rows, EPI_RESIDUAL, e->x, H);
       if (r != cudaSuccess) return r;
     } else {
       GemmArgs g{};
@@ -284,10 +282,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     capture_copy(e, "x_attn", l, e->x, (size_t)n * H);
     QIE_TRY(KK_RMSNORM, rms(e->x, w.post_ln, e->xn, n));
     if (tc) {
-      const TensorMap2D* wm[2] = {&e->wmaps[l].gate, &e->wmaps[l].up};
-      const bf16* wp[2] = {w.gate, w.up};
+      const qie_engine::WeightMaps* wm[2] = {&e->wmaps[l].gate, &e->wmaps[l].up};
       const int rows[2] = {I, I};
-      cudaError_t r = gemm_tc(e, KK_GEMM_GATEUP, e->xn, n, H, 2, wm, wp, rows, EPI_SILU_MUL, e->h, I);
+      cudaError_t r = gemm_tc(e, KK_GEMM_GATEUP, e->xn, n, H, 2, wm, rows, EPI_SILU_MUL, e->h, I);
       if (r != cudaSuccess) return r;
     } else {
       GemmArgs g{};
@@ -302,10 +299,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     }
     capture_copy(e, "mlp_h", l, e->h, (size_t)n * I);
     if (tc) {
-      const TensorMap2D* wm[1] = {&e->wmaps[l].down};
-      const bf16* wp[1] = {w.down};
+      const qie_engine::WeightMaps* wm[1] = {&e->wmaps[l].down};
       const int rows[1] = {H};
-      cudaError_t r = gemm_tc(e, KK_GEMM_DOWN, e->h, n, I, 1, wm, wp, rows, EPI_RESIDUAL, e->x, H);
+      cudaError_t r = gemm_tc(e, KK_GEMM_DOWN, e->h, n, I, 1, wm, rows, EPI_RESIDUAL, e->x, H);
       if (r != cudaSuccess) return r;
     } else {
       GemmArgs g{};
@@ -324,10 +320,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
   // final norm only on the rows that feed lm_head (qwen_main.cu:227-236, :367-372)
   QIE_TRY(KK_RMSNORM, rms(e->x + (size_t)out_row0 * H, e->final_norm, e->xn, n_out));
   if (fast && n_out > 8) {
-    const TensorMap2D* wm[1] = {&e->lm_head_map};
-    const bf16* wp[1] = {e->lm_head};
+    const qie_engine::WeightMaps* wm[1] = {&e->lm_head_map};
     const int rows[1] = {c.vocab};
-    cudaError_t r = gemm_tc(e, KK_LM_HEAD, e->xn, n_out, H, 1, wm, wp, rows, EPI_STORE, e->logits, c.vocab);
+    cudaError_t r = gemm_tc(e, KK_LM_HEAD, e->xn, n_out, H, 1, wm, rows, EPI_STORE, e->logits, c.vocab);
     if (r != cudaSuccess) return r;
   } else {
     GemmArgs g{};

@@ -90,11 +90,14 @@ struct qie_engine {
   int logits_rows = 0;
 
   // fast numerics (opts.numerics == QIE_NUMERICS_FAST)
-  struct LayerMaps {
-    qie::TensorMap2D q, k, v, o, gate, up, down;
+  struct WeightMaps {
+    qie::TensorMap2D one, two;  // boxes of 128 rows x one and two k-blocks of 64 (gate and up: 64 rows, one k-block)
   };
-  std::vector<LayerMaps> wmaps;  // TMA descriptors of the weight matrices (box 128 x 64)
-  qie::TensorMap2D lm_head_map;
+  struct LayerMaps {
+    WeightMaps q, k, v, o, gate, up, down;
+  };
+  std::vector<LayerMaps> wmaps;  // TMA descriptors of the weight matrices
+  WeightMaps lm_head_map;
   qie::bf16* qkv = nullptr;      // fused [rows, Dq + 2*Dkv] projection output
   float* attn_ws = nullptr;      // partial results of a decode step whose keys are split more than FD_CLUSTER ways
   size_t attn_ws_rows = 0;       // (split, row, head) of them

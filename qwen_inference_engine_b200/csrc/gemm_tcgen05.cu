@@ -972,23 +972,35 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
   g.staged = g.splits == 1 && vec;
   g.vec = vec;
+  // the weights' maps, in boxes of one or two k-blocks: those that the caller keeps, else made here
   const CUtensorMap* w[3];
-  for (int i = 0; i < 3; ++i) w[i] = reinterpret_cast<const CUtensorMap*>(t.w[i < t.nseg ? i : 0]);
-  TensorMap2D x;
+  TensorMap2D made[3], x;
+  auto maps = [&](bool two) {
+    for (int i = 0; i < t.nseg; ++i) {
+      const TensorMap2D* m = two ? t.w2[i] : t.w[i];
+      if (!m) {
+        if (!t.wp[i]) return false;
+        const cudaError_t e = two ? make_tensor_map_w3d(&made[i], t.wp[i], t.rows[i], t.K, 2 * BK, 0, BM) : make_tensor_map_2d(&made[i], t.wp[i], t.rows[i], t.K, g.dual ? BM / 2 : BM);
+        if (e != cudaSuccess) return false;
+        m = &made[i];
+      }
+      w[i] = reinterpret_cast<const CUtensorMap*>(m);
+    }
+    for (int i = t.nseg; i < 3; ++i) w[i] = w[0];
+    return true;
+  };
   if (launches) *launches = 1;
   // Two k-blocks a stage where tensor maps can express them (whole k-blocks, and the weights' place is known): half the requests, waits and commits.  Up
   // to 64 tokens: of 128 the ring holds three such stages, too few on the way (8960 x 1536 at 1000 rows 34.8 with stages of one, 37.1).  Gate/up tiles
   // are two boxes a k-block as they are.  Not for 3 or 5 k-blocks: the half of the last stage that is not there is a box of zeros to bring, a quarter of
   // the operands (us with stages of one and of two, 1000 rows: 192 x 130 3.7 4.0, 320 x 130 4.3 4.6, 448 x 130 4.7 4.7, 576 x 130 4.5 4.2).
   const bool whole = g.splits > 1 || g.kb_total % 2 == 0 || g.kb_total > 5;
-  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && t.wp[0]) {
-    TensorMap2D w3[3];
-    bool ok = make_tensor_map_w3d(&x, t.x, t.M, t.K, 2 * BK, 0, tl.bn) == cudaSuccess;
-    for (int i = 0; i < t.nseg; ++i) ok = ok && t.wp[i] && make_tensor_map_w3d(&w3[i], t.wp[i], t.rows[i], t.K, 2 * BK, 0, BM) == cudaSuccess;
-    if (ok) {
-      for (int i = 0; i < 3; ++i) w[i] = reinterpret_cast<const CUtensorMap*>(&w3[i < t.nseg ? i : 0]);
-      return launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
-    }
+  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && maps(true) &&
+      make_tensor_map_w3d(&x, t.x, t.M, t.K, 2 * BK, 0, tl.bn) == cudaSuccess)
+    return launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
+  if (!maps(false)) {
+    if (launches) *launches = 0;
+    return cudaErrorNotSupported;
   }
   cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
   if (e != cudaSuccess) return e;
@@ -1045,17 +1057,15 @@ cudaError_t launch_gemm_ref_rows(const GemmArgs& a, int num_sms, cudaStream_t st
     t.w_static = w_static;
     t.out = a.seg[0].out;
     t.ld_out = a.seg[0].ld_out;
-    TensorMap2D w[3];
-    for (int i = 0; i < t.nseg && tc; ++i) {
+    for (int i = 0; i < t.nseg; ++i) {
       const GemmSeg& sg = a.seg[dual ? 0 : i];
-      tc = make_tensor_map_2d(&w[i], dual && i ? sg.W2 : sg.W, sg.rows, a.K, dual ? BM / 2 : BM) == cudaSuccess;
-      t.w[i] = &w[i];
       t.wp[i] = dual && i ? sg.W2 : sg.W;
       t.rows[i] = sg.rows;
       t.outs[i] = sg.out;
       t.lds[i] = sg.ld_out;
     }
-    if (tc) return launch_gemm_tcgen05(t, num_sms, st, launches);
+    const cudaError_t e = launch_gemm_tcgen05(t, num_sms, st, launches);
+    if (e != cudaErrorNotSupported) return e;  // (no tensor map expresses these weights)
   }
   for (int r0 = 0; r0 < a.M; r0 += 64) {
     GemmArgs c = a;

@@ -166,8 +166,9 @@ cudaError_t make_tensor_map_kv(TensorMap2D* out, const bf16* pool, unsigned long
 // positions of one page, 128-byte swizzle
 cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_elems, int page_size, int n_pages, size_t page_elems, int box_rows);
 struct TcGemm {
-  const TensorMap2D* w[3];  // weight maps, box rows = 128 (EPI_SILU_MUL: 64)
-  const bf16* wp[3];        // the weights themselves (null: stages of one k-block)
+  const TensorMap2D* w[3];   // weight maps, box rows = 128 (EPI_SILU_MUL: 64)
+  const TensorMap2D* w2[3];  // the same of two k-blocks (make_tensor_map_w3d, kc = 128)
+  const bf16* wp[3];         // the weights themselves: maps that are null are made from them, where a launch takes them (null as well: stages of one k-block)
   const bf16* x;            // activations [M, K]
   int rows[3];
   int nseg, M, K, epi;
