@@ -952,8 +952,11 @@ struct TopkSums {
 };
 // Exactly k of a slice of which more than TC_CAP values reach `bound`.  v: the value that the slice's k-th has (the bound itself, unless many large
 // values share few threads); of those that equal it the best by the key's lower half: bit-reversed low byte of the index, largest first, then index.
-// cls: 256 ints (ties by low byte); tie: indices of one low byte, a 2048-th of the row and one more.  Not inlined: beside the kernel's own passes its
-// copies of the loop cost those 15 %.
+// cls: 256 ints (ties by low byte); tie: indices of one low byte (topk_tie_ints).  Not inlined: beside the kernel's own passes its copies of the loop
+// cost those 15 %.
+// What `tie` has to hold: a slice is ceil(vocab / 8 / ctas) pieces side by side, of which every 256 consecutive elements hold one of a low byte, and in the first
+// slice up to 14 elements more in front of the first and behind the last whole piece of the row: two runs, each with at most one more of the byte.
+constexpr size_t topk_tie_ints(size_t vocab, int ctas) { return ((vocab / 8 + ctas - 1) / ctas * 8 + 255) / 256 + 2; }
 template <int TC_THREADS>
 __device__ __noinline__ void topk_slice_ties(const TopkSlice<TC_THREADS> sl, TopkSums sum, uint32_t mx, uint32_t bound, int k, unsigned long long* cand, int* cls,
                                               int* tie, int* s_n, int* s_tot) {
@@ -1006,9 +1009,9 @@ __device__ __noinline__ void topk_slice_ties(const TopkSlice<TC_THREADS> sl, Top
   __syncthreads();
   if (tid < 3) sum.cnt[tid] = 0;
 }
-// STAGED: the slice is copied to shared memory once, its two passes read it there (up to TC_STAGE bytes, 48 KB with the 9.6 KB of the rest, so that four
-// CTAs share an SM; the first CTA's gathered candidates go over it).
-constexpr int TC_STAGE = 38 * 1024;  // bytes in clusters of 8, twice and four times that in clusters of 4 and 2
+// STAGED: the slice is copied to shared memory once, its two passes read it there; the first CTA's gathered candidates go over it.  In clusters of 8 up
+// to TC_STAGE bytes, 48 KB with the 9.6 KB of the rest, so that four CTAs share an SM; in clusters of 4 and 2 twice and four times that, two CTAs and one.
+constexpr int TC_STAGE = 38 * 1024;
 template <int TC_THREADS, bool STAGED, int CTAS>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(TC_THREADS)
     sample_topk_cluster_kernel(const bf16* __restrict__ logits, int* __restrict__ out, size_t vocab, float temperature, int k, uint64_t seed,
@@ -1215,7 +1218,7 @@ template <int TC_THREADS, bool STAGED, int CTAS>
 static cudaError_t launch_topk_cluster(const bf16* logits, int* out_tokens, int n_rows, size_t vocab, float temperature, int k, uint64_t seed, uint64_t seed_stride,
                                        const int* step_ptr, unsigned long long subsequence, cudaStream_t st) {
   constexpr size_t all = (size_t)CTAS * TC_CAP * 8;
-  const size_t slice = (vocab / 8 + CTAS - 1) / CTAS * 16, smem = STAGED ? std::max(slice, all) : all;
+  const size_t slice = (vocab / 8 + CTAS - 1) / CTAS * 16, tie = topk_tie_ints(vocab, CTAS) * sizeof(int), smem = std::max({STAGED ? slice : 0, all, tie});
   if constexpr (STAGED && CTAS < TC_CTAS) {
     static PerDeviceOnce set;
     if (set.need()) {
