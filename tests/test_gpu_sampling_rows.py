@@ -17,7 +17,7 @@ def layers():
     return L
 
 
-def row(kind, vocab, rng):
+def row(kind, vocab, rng, ctas=8):
     x = rng.standard_normal(vocab).astype(np.float32) * 2.5
     if kind == "ties":
         x = np.round(x)
@@ -35,7 +35,7 @@ def row(kind, vocab, rng):
         x[rng.integers(0, vocab, size=3)] = 5.0
     if kind == "few threads":  # more large values than a list holds, in the 16-byte pieces of 30 threads of a slice
         piece = np.arange(vocab) // 8
-        x[piece % max(1, (vocab // 8 + 7) // 8) % 512 < 30] += 25
+        x[piece % max(1, (vocab // 8 + ctas - 1) // ctas) % 512 < 30] += 25
     return f32_to_bf16(x)
 
 
@@ -75,3 +75,17 @@ def test_slices_of_hardly_more_pieces_than_k(layers, oracle, vocab, k, rows, kin
     rng = np.random.default_rng(vocab + rows)
     lg = np.stack([row(kind, vocab, rng) for _ in range(5)])
     some_rows(layers, oracle, np.tile(lg, (rows // 5 + 1, 1))[:rows], vocab, k, 1234, range(5))
+
+
+@pytest.mark.parametrize("k", [1, 2, 50, 128])
+@pytest.mark.parametrize("vocab,rows,ctas", [(151936, 4, 8), (151936, 5, 8), (151936, 8, 8), (151936, 9, 4), (151936, 16, 4), (151936, 17, 4), (151936, 32, 4), (151936, 33, 2),
+                                             (151936, 64, 2), (155655, 9, 4), (155655, 33, 2), (155656, 2, 8), (155656, 17, 8), (262144, 3, 8), (262144, 17, 8), (65536, 16, 4),
+                                             (32001, 12, 4), (32001, 40, 2)])
+def test_every_cluster_size_and_both_sides_of_its_rules(layers, oracle, vocab, rows, ctas, k):
+    """slices of two, four and eight CTAs with and without the copy in shared memory, on and off a 16-byte boundary, lists that overflow, hardly any candidates;
+    greedy rows in 64, 32 and 8 slices (k = 1, whole pieces)"""
+    rng = np.random.default_rng(vocab + rows + k)
+    lg = np.stack([row(kind, vocab, rng, ctas) for kind in ("few threads", "ties", "normal", "equal", "few")])
+    for at in range(0, 5, rows):
+        part = lg[at:at + rows]
+        some_rows(layers, oracle, np.tile(part, (rows // len(part) + 1, 1))[:rows], vocab, k, 77, range(len(part)))
