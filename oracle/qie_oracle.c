@@ -187,7 +187,7 @@ void orc_rope(const float* cos_values, const float* sin_values, orc_bf16* x, int
       }
 }
 
-/* "HF-correct" RoPE (SURVEY 8f rank 1; transformers' rotate_half): element j of a head pairs with j + hd/2,
+/* "HF-correct" RoPE (transformers' rotate_half): element j of a head pairs with j + hd/2,
  *   out[j] = x[j]*c_j - x[j+hd/2]*s_j ;  out[j+hd/2] = x[j+hd/2]*c_j + x[j]*s_j,   c_j, s_j the same table rows.
  * Not in the reference (its RoPE is the interleaved form above); fp32 math, one bf16 rounding, same fma placement. */
 void orc_rope_half(const float* cos_values, const float* sin_values, orc_bf16* x, int n_tok, int head_dim, int row_dim,
