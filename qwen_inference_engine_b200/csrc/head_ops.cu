@@ -237,8 +237,7 @@ cudaError_t launch_qkv_post(const QkvPostArgs& a, cudaStream_t st) {
   if (heads == 0) return cudaSuccess;
   const bool vec = on16({a.q, a.q_in, a.k, a.v, a.q_norm_w, a.k_norm_w, a.cos_t, a.sin_t, a.q_bias, a.k_bias, a.v_bias, a.kv.pool}) && a.q_in_stride % 8 == 0 &&
                    a.kv_stride % 8 == 0;
-  QIE_HEADS(a.kv.hd, vec, (void)(launch_spread<qkv_post_kernel<NP, V>>(dim3(blocks_of(heads, a.kv.hd)), dim3(128), 0, st, a)));
-  return cudaGetLastError();
+  QIE_HEADS(a.kv.hd, vec, return launched(launch_spread<qkv_post_kernel<NP, V>>(dim3(blocks_of(heads, a.kv.hd)), dim3(128), 0, st, a)));
 }
 
 cudaError_t launch_qknorm_ref(bf16* x, const bf16* w, int hd, int n_tok, int row_dim, int n_heads, cudaStream_t st) {

@@ -52,6 +52,12 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
+// What a launcher returns: the launch's own error, or one that an earlier call left; either way none is left for the next.
+inline cudaError_t launched(cudaError_t e) {
+  const cudaError_t last = cudaGetLastError();
+  return e != cudaSuccess ? e : last;
+}
+
 // an attribute of a device, asked for once (0: the runtime does not say)
 template <cudaDeviceAttr A>
 inline int device_attribute(int dev) {

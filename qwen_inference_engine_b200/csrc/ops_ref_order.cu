@@ -48,8 +48,7 @@ __global__ void embedding_kernel(bf16* __restrict__ out, const bf16* __restrict_
 cudaError_t launch_embedding(bf16* out, const bf16* table, const int* ids, size_t hidden, size_t n_tok,
                              cudaStream_t st) {
   if (n_tok == 0) return cudaSuccess;
-  (void)launch_spread<embedding_kernel>(dim3((unsigned)n_tok), dim3(128), 0, st, out, table, ids, hidden);
-  return cudaGetLastError();
+  return launched(launch_spread<embedding_kernel>(dim3((unsigned)n_tok), dim3(128), 0, st, out, table, ids, hidden));
 }
 
 // ------------------------------------------------------------------ a prompt's rows
@@ -196,16 +195,16 @@ cudaError_t launch_rmsnorm_ref(const bf16* x, const bf16* w, bf16* y, size_t hid
   const size_t pitch = rms_pitch(hidden, sizeof(bf16)), sms = device_attribute<cudaDevAttrMultiProcessorCount>(dev);
   const bool vec = hidden % 8 == 0 && x_stride % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   if (vec && n_tok >= (hidden < RMS_WIDE ? 2 : 1) * RMS_MANY * sms && 4 * pitch <= 40 * 1024)
-    return launch_spread<rmsnorm_ref_kernel<4, true>>(dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+    return launched(launch_spread<rmsnorm_ref_kernel<4, true>>(dim3((unsigned)((n_tok + 3) / 4)), dim3(256), 4 * pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps));
   if (vec)
-    return launch_spread<rmsnorm_ref_kernel<1, true>>(dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+    return launched(launch_spread<rmsnorm_ref_kernel<1, true>>(dim3((unsigned)n_tok), dim3(128), pitch, st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps));
   static PerDeviceOnce set;  // (12288 elements are a little more than the 48 KB that need no attribute)
   if (set.need()) {
     e = cudaFuncSetAttribute(rmsnorm_ref_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     if (e != cudaSuccess) return e;
     set.done();
   }
-  return launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), rms_pitch(hidden, sizeof(float)), st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps);
+  return launched(launch_k(rmsnorm_ref_kernel<1, false>, dim3((unsigned)n_tok), dim3(128), rms_pitch(hidden, sizeof(float)), st, x, w, y, (int)hidden, x_stride, (int)n_tok, eps));
 }
 
 // fast-numerics variant: the sum of squares is reduced in parallel (warp shuffles), so it
@@ -279,9 +278,7 @@ cudaError_t launch_rmsnorm_fast(const bf16* x, const bf16* w, bf16* y, size_t hi
   // (every row count takes this kernel when the layout allows: a row's result must not depend on how a prompt is chunked)
   if (hidden % 8 == 0 && x_stride % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
-    (void)launch_spread<rmsnorm_fast_rows_kernel>(dim3((unsigned)((n_tok + 7) / 8)), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps,
-                   (int)n_tok);
-    return cudaGetLastError();
+    return launched(launch_spread<rmsnorm_fast_rows_kernel>(dim3((unsigned)((n_tok + 7) / 8)), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps, (int)n_tok));
   }
   (void)launch_k(rmsnorm_fast_kernel, dim3((unsigned)n_tok), dim3(256), 0, st, x, w, y, (int)hidden, x_stride, eps);
   return cudaGetLastError();
