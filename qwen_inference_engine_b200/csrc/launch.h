@@ -23,16 +23,17 @@ extern bool g_use_pdl;  // engine.cu; set per process from QIE_PDL (default on)
 
 // Function attributes (opt-in dynamic shared memory, cluster size) are per DEVICE: a process that creates engines on
 // several devices must set them on each.  One flag per device ordinal instead of a process-wide `static bool`.
+// Two threads that meet here both set the attributes.
 struct PerDeviceOnce {
-  unsigned long long mask[4] = {0ull, 0ull, 0ull, 0ull};
+  std::atomic<unsigned long long> mask[4] = {};
   bool need() const {
     int d = 0;
     if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= 256) return true;
-    return ((mask[d >> 6] >> (d & 63)) & 1ull) == 0ull;
+    return ((mask[d >> 6].load(std::memory_order_acquire) >> (d & 63)) & 1ull) == 0ull;
   }
   void done() {
     int d = 0;
-    if (cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 256) mask[d >> 6] |= 1ull << (d & 63);
+    if (cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 256) mask[d >> 6].fetch_or(1ull << (d & 63), std::memory_order_release);
   }
 };
 
