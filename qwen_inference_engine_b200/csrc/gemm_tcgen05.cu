@@ -892,9 +892,11 @@ struct TcTile {
   int bn, splits;
   bool persist, half;
 };
-// Tokens of a tile and splits over K.  Measured on B200 in graphs of the same launch, weights in L2 (us):
-//  * One wave of CTAs: the smallest of 16 ... 128 tokens whose tiles all fit on the SMs.  A k-block takes the same time at any width up
-//    to 128, narrower tiles fill and drain faster: 896 x 896, 1000 tokens: 64 7.1, 128 7.8, 256 9.5 (a split over 5 CTAs: 50.8).
+// Tokens of a tile and splits over K.  Measured on B200 in graphs of the same launch, weights in L2 (us), with stages of one k-block, 0.19 us each at any
+// width up to 128.  Stages of two, which came later (up to 64 tokens, launch_gemm_tcgen05), take 0.13 a k-block: the choices between 64 and 128 tokens
+// and between splits are still those of the older figure.
+//  * One wave of CTAs: the smallest of 16 ... 128 tokens whose tiles all fit on the SMs, since narrower tiles fill and drain faster: 896 x 896,
+//    1000 tokens: 64 7.1, 128 7.8, 256 9.5 (a split over 5 CTAs: 50.8).
 //  * More tiles than that: the persistent kernel.  256 tokens, unless a width with fuller waves takes less than 0.9 of waves x width
 //    (1536 outputs at 4096 rows: 107 -> 86 with 176; a few per cent less on paper were none: 8960 outputs 82.7 with 256, 85.5 with
 //    224).  Below 160 tokens the loop, not the tensor core, sets a tile's time, so of those the narrowest wins, whose ring holds most

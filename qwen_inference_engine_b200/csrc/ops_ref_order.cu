@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(256) rmsnorm_fast_rows_kernel(const bf16* __re
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const Quot rms = quot_of(__fsqrt_rn(__fadd_rn(__fdiv_rn(sum, (float)hidden), eps)));
   for (int i = lane; i < nv; i += 32) {
-    const uint4 v = xr[i], wv = wr[i];  // (the row is still in L1)
+    const uint4 v = xr[i], wv = wr[i];  // (from L2 where launch_spread's padding leaves L1 less than the SM's rows)
     const uint32_t u[4] = {v.x, v.y, v.z, v.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
     uint32_t o4[4];
     norm8(u, ww, rms, o4);
