@@ -251,11 +251,12 @@ cudaError_t launch_qknorm_ref(bf16* x, const bf16* w, int hd, int n_tok, int row
 cudaError_t launch_rope_ref(const float* cos_t, const float* sin_t, bf16* x, int n_tok, const int* pos, int pos0, int hd, int row_dim, int n_heads, cudaStream_t st) {
   const long heads = (long)n_tok * n_heads;
   if (heads == 0) return cudaSuccess;
-  // 16 elements a lane from 4096 heads of 64 on, as many elements of wider ones; off a 16-byte boundary from 6144 (256 wide from 40000 heads, since 32 lanes
-  // read whole sectors and 16 do not).  us with 32 lanes and with 16 elements: 17 heads of 64 1.2 1.3, 2800 1.6 1.8, 4000 1.7 1.8, 7168 2.5 1.8; off a
-  // boundary 1 head 1.2 1.4, 4000 1.8 2.0, 7168 2.6 2.2; 14000 of 256 there 4.5 5.5, 42000 11.7 10.9.
+  // 16 elements a lane from 2048 heads of 64 on, as many elements of wider ones; off a 16-byte boundary from 6144 (256 wide from 40000 heads, since 32 lanes
+  // read whole sectors and 16 do not).  us with 32 lanes and with 16 elements, alone: 17 heads of 64 1.2 1.3, 2800 1.6 1.8, 4000 1.7 1.8, 7168 2.5 1.8;
+  // behind a norm and head norms 32 lanes are 1 us slower from about 3500 heads on (1792 of 128, the three operators 7.7 and 6.7) and the same below; off
+  // a boundary 1 head 1.2 1.4, 4000 1.8 2.0, 7168 2.6 2.2; 14000 of 256 there 4.5 5.5, 42000 11.7 10.9.
   const bool vec = on16({x, cos_t, sin_t}) && row_dim % 8 == 0;
-  if (heads * hd > 64L * (vec ? 4096 : hd < 256 ? 6144 : 160000)) {
+  if (heads * hd > 64L * (vec ? 2048 : hd < 256 ? 6144 : 160000)) {
     QIE_HEADS(hd, vec, (void)launch_k(rope_ref_kernel<NP, V>, dim3(blocks_of(heads, hd)), dim3(128), 0, st, cos_t, sin_t, x, n_tok, pos, pos0, row_dim, n_heads));
     return cudaGetLastError();
   }
