@@ -657,7 +657,8 @@ __global__ void __launch_bounds__(1024) sample_topk_kernel(const bf16* __restric
 // 64).  Stage 1: CTA (slice, row) reduces its slice to one candidate; stage 2: one warp per row merges the slices.
 // Eight logits are one packed maximum, looked at further only where it reaches the thread's best, and few long rows are cut into more slices: one row
 // of 151936 behind lm_head 22 us with 8 slices and a comparison in the full order for each, 4.2 now (alone 10.5 and 4.1); 16 rows 12.4 and 5.3, 64 rows 16.7
-// and 9.4.  Below 65536 logits 8 slices hold few pieces a thread as they are (32000: 4.8 and 3.7).
+// and 9.4.  Below 65536 logits 8 slices hold few pieces a thread as they are (32000: 4.8 and 3.7).  Vocabularies of 65536 to 262144, 1 to 256 rows: 0.28 to 0.73
+// of the time of 8 slices read value by value, 17 to 48 rows, which keep 8 slices, 0.44 to 0.71.
 constexpr int GREEDY_SLICES = 8, GREEDY_MOST = 64;
 static int greedy_slices(int n_rows, size_t vocab) { return vocab < 65536 || n_rows > 16 ? GREEDY_SLICES : n_rows > 4 ? 32 : GREEDY_MOST; }
 __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) {  // two bf16 each; a number wins over a NaN
@@ -1273,7 +1274,9 @@ cudaError_t launch_sample_topk(const bf16* logits, int* out_tokens, int n_rows, 
     // 151936, k = 50, 8 4 2 CTAs a row: 1 row 14.0 14.9 16.5, 8 14.2 15.4 17.1, 16 17.3 15.6 17.5, 32 17.9 17.3 17.9, 48 24.4 20.8 19.0, 64 25.2 21.9 19.4).  A
     // slice has to hold an eighth more pieces than k: with hardly more, the k-th of their maxima is a bound that most values reach, and the lists are
     // long or overflow (33 rows of 2064, k = 128: 19.9 with eight CTAs, 25.3 with two; from 2304 on two are quicker).  More than 16 rows that stay
-    // with eight take 256 threads, so that all clusters are on the chip at once (256 rows of 2056, k = 128: 77 us, 132 with 512).
+    // with eight take 256 threads, so that all clusters are on the chip at once (256 rows of 2056, k = 128: 77 us, 132 with 512).  Against eight CTAs for all
+    // (256 threads from 17 rows on, everything read twice from memory), 24 vocabularies of 500 to 262144, 1 to 256 rows, k of 2 to 128: 0.30 to 1.0 of the
+    // time; clusters of two near the staging limit, one CTA an SM, 100 to 256 rows of 128256 to 155648 0.51 to 0.64.
     const bool staged = (vocab / 8 + TC_CTAS - 1) / TC_CTAS * 16 <= (size_t)TC_STAGE;
     auto holds = [&](int ctas) { return vocab <= (size_t)ctas * TC_CAP || vocab / (ctas * 8) >= (size_t)k + k / 8; };
     auto launch = staged && n_rows > 32 && holds(2)  ? launch_topk_cluster<512, true, 2>
