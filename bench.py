@@ -289,7 +289,7 @@ def config4_leg(q, torch, np, rank, world, local, use_dist):
         e1.record()
     eng.sync()
     ms = e0.elapsed_time(e1)
-    mega = bool(eng.uses_mega(n_seq, 32 + 8 + steps + 2))
+    mega = bool(eng.uses_mega(n_seq, 32 + 8 + steps + 2)) and int(eng.launch_count()) < q.make_config(ARCH).layers  # (launches of the last step)
     eng.close()
     if use_dist:
         t = torch.tensor([ms], device="cuda", dtype=torch.float64)
@@ -835,7 +835,7 @@ def main():
     barrier()
 
     # ---------------- per-kernel-class timing of one step (roofline leg) -----------------
-    mega = eng.uses_mega(B, eng.seq_len(seqs[0]) + 2)
+    mega = eng.uses_mega(B, eng.seq_len(seqs[0]) + 2) and int(eng.launch_count()) < cfg.layers  # (launches of the step before)
     mega_phase_us = None
     if mega:
         # ONE kernel per step: its phases are timed by device timestamps taken inside the kernel
@@ -861,8 +861,8 @@ def main():
     ctx_now = eng.seq_len(seqs[0])
     topk_extra = None
     if rank == 0 and world == 1 and not args.no_extra:
-        # the reference's real sampling mode on the same batch: top-k 50, T 0.7, XORWOW (qwen_main.cu:381-388) -- the
-        # persistent kernel leaves the logits, one radix-select + draw kernel follows (the reference does k = 50 scans)
+        # the reference's real sampling mode on the same batch: top-k 50, T 0.7, XORWOW (qwen_main.cu:381-388) -- one
+        # radix-select + draw kernel behind the logits (the reference does k = 50 scans)
         try:
             eng.set_sampling(topk=50, temperature_prefill=1.0, temperature_decode=0.7, seed=1234, add_step=True)
             cur = eng.decode_step(seqs, cur)
@@ -1013,7 +1013,7 @@ def main():
             b1_bytes = q.weight_bytes(cfg) + kvpp * (eng.seq_len(s1) - 60)
             line.setdefault("extra", {})["batch1"] = {
                 "workload": "batch 1, 32-token prompt, greedy decode (qie_decode_run, 120 tokens)",
-                "persistent_kernel": bool(eng.uses_mega(1, 200)),
+                "persistent_kernel": bool(eng.uses_mega(1, 200)) and int(eng.launch_count()) < 120 * cfg.layers,
                 "tokens_per_s": 120 / dt, "us_per_token": 1e6 * dt / 120,
                 "frac_of_hbm_peak": (b1_bytes * 120 / dt / 1e9) / peak}
             eng.free_sequence(s1)

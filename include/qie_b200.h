@@ -394,11 +394,12 @@ const char* qie_kernel_kind_name(int kind);
 int qie_profile_begin(qie_engine* e);
 int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int n_kinds);
 
-/* Persistent decode kernel (decode_mega.cu): reference-order decode steps of <= 8 rows run
- * as ONE cooperative launch.  qie_engine_set_int keys: "mega" (0/1, default 1 unless
- * QIE_MEGA=0), "mega_layers_run" (debug: stop after N layers, 0 = whole step), "mega_prof"
- * (0/1: record a device timestamp at every phase boundary).  qie_decode_uses_mega tells
- * whether a step of n rows at this KV length would take that path.
+/* Persistent decode kernel (decode_mega.cu): a reference-order decode step of up to 64 rows
+ * as ONE cooperative launch.  By default a step runs so only where the operators are not
+ * quicker (the same bits either way).  qie_engine_set_int keys: "mega" (0: never, 1: wherever
+ * the kernel takes the step; QIE_MEGA=0 is the former), "mega_layers_run" (debug: stop after N layers, 0 = whole step), "mega_prof"
+ * (0/1: record a device timestamp at every phase boundary, in the persistent kernel).
+ * qie_decode_uses_mega tells whether the kernel takes a step of n rows at this KV length.
  * qie_mega_prof_read copies the timestamps (ns, globaltimer) of the last profiled step to
  * HOST memory: [0] start, then 16 per layer (QKV: rows loaded, normed, GEMM done, barrier;
  * attention: done, barrier; O: loaded, GEMM, barrier; gate/up: loaded, normed, GEMM, barrier;

@@ -45,29 +45,6 @@ __device__ __forceinline__ uint4 load8(const bf16* p) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-__device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
-  asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tadd.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}"
-      : "+f"(a), "+f"(b) : "f"(x), "f"(y));
-}
-// the low and the high products of two words of bf16 pairs, with c and d added before the one rounding each
-__device__ __forceinline__ void fma16(float& a, float& b, uint32_t x, uint32_t y, float c, float d) {
-  asm("{\n\t.reg .b16 xl, xh, yl, yh;\n\tmov.b32 {xl, xh}, %2;\n\tmov.b32 {yl, yh}, %3;\n\tfma.rn.f32.bf16 %0, xl, yl, %4;\n\tfma.rn.f32.bf16 %1, xh, yh, %5;\n\t}"
-      : "=&f"(a), "=f"(b) : "r"(x), "r"(y), "f"(c), "f"(d));
-}
-// Products of two bf16 numbers between 2^-62 and 2^62 are exact in fp32, so p + q k rounded once is what the product and the sum are; a product
-// alone is -0 + q k.
-// Lowest and highest magnitude of packed pairs, and whether they leave that range (a zero does: its tiles take products and sums).
-struct Magnitudes {
-  uint32_t lo = 0x7fff7fffu, hi = 0u;
-  __device__ __forceinline__ void see(uint32_t w) {
-    w &= 0x7fff7fffu;
-    lo = __vminu2(lo, w), hi = __vmaxu2(hi, w);
-  }
-  __device__ __forceinline__ bool beyond() const {
-    return min(lo & 0xffffu, lo >> 16) < (uint32_t)(127 - 62) << 7 || max(hi & 0xffffu, hi >> 16) > (uint32_t)(127 + 62) << 7;
-  }
-};
-
 // A lane's part of a score's product tree, depth first over the 16-byte pieces of its 64 elements: leaf l is pieces l and l + 4 (stride 32), then strides
 // 16 and 8.
 template <bool FUSED, int STEP, class Q, class G>

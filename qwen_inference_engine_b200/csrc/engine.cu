@@ -260,6 +260,8 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.max_kv_len = max_kv_len;
       a.kv = e->kv;
       a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
+      a.decode = a.early = advance;
+      a.status = e->wait_status;
       QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
     }
     capture_copy(e, "attn", l, e->att, (size_t)n * Dq);
@@ -522,6 +524,26 @@ bool decode_uses_mega(const qie_engine* e, int n, int max_kv_len) {
     return false;
   return decode_mega_supports(c.hidden, c.inter, c.layers, c.n_q, c.n_kv, c.head_dim, nb, max_kv_len, e->num_sms,
                               e->mega_kc[mega_tile_set(e, nb, max_kv_len)], fast, e->kv.page_size);
+}
+
+// Steps in the reference's order that are quicker by operators than in the persistent kernel.  That kernel walks one (row, kv head) per SM through chains that wait for
+// one another and streams every phase's operands by itself; the operators have their products on tcgen05 and attn_ref_decode.cu.  us a step in graphs, persistent
+// kernel and operators: 0.5B, 24 layers, 64 rows at 2000 positions 2894 and 1928, at 500 2087 and 1402; 16 rows at 100 1580 and 1170; 8 at 32 1162 and 1127; 4 at 300
+// (8 layers) 458 and 445, at 60 418 and 421; 1 at 2000 1869 and 1596, at 500 1233 and 1221, at 32 986 and 1087.  1.5B, 8 layers: 1 at 32 606 and 605, 32 at 300
+// 1100 and 679.  7B, 4 layers: 1 at 32 893 and 730, 16 at 2000 1491 and 901.  Rows of 128 to 256: 1 at 16 123 and 113, 126 and 125.
+bool decode_by_operators(const qie_engine* e, int n, int max_kv_len) {
+  const qie_config& c = e->cfg;
+  if (e->mega_always || e->mega_prof_on || e->mega_layers_run > 0 || e->tp.size > 1 || e->opts.numerics == QIE_NUMERICS_FAST) return false;
+  if (n <= 4 && max_kv_len <= 384 && c.hidden > 256 && c.hidden < 1536) return false;
+  AttnArgs a{};
+  a.q = e->q;
+  a.out = e->att;
+  a.n_tok = n;
+  a.n_q = c.n_q;
+  a.max_kv_len = max_kv_len;
+  a.kv = e->kv;
+  int stages = 0;
+  return attention_ref_decode_heads(a, e->num_sms, &stages) > 0;
 }
 
 static cudaError_t forward_decode_mega_rows(qie_engine* e, int row0, int n, int max_kv_len, float temperature);

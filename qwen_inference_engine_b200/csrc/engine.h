@@ -104,6 +104,7 @@ struct qie_engine {
 
   // persistent decode kernel (decode_mega.cu): reference-order decode steps of <= 8 rows
   bool use_mega = true;              // QIE_MEGA=0 disables
+  bool mega_always = false;          // the caller asked for the persistent kernel ("mega" 1): also where the operators are quicker
   qie::MegaLayer* mega_layers_d = nullptr;
   // 7 per layer + lm_head 3-D weight views (box 8 rows x mega_kc[s]); set 1 (larger tiles) serves batches <= 8
   qie::TensorMap2D* mega_wmaps_d[2] = {nullptr, nullptr};
@@ -198,6 +199,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n_rows, int max_kv_len, int out_r
 cudaError_t engine_alloc_shared(qie_engine* e, int n_pages, int context);
 // true if a decode step of n rows / this kv bucket runs through the persistent kernel
 bool decode_uses_mega(const qie_engine* e, int n_rows, int max_kv_len);
+bool decode_by_operators(const qie_engine* e, int n, int max_kv_len);  // a step that the persistent kernel takes too is quicker by operators
 // one decode step (rows described in ids_d/pos_d/slot_d) through the persistent kernel
 cudaError_t forward_decode_mega(qie_engine* e, int n_rows, int max_kv_len, float temperature);
 }  // namespace qie

@@ -495,6 +495,11 @@ cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
+    if (a.decode) {
+      int stages = 0;
+      const int heads = attention_ref_decode_heads(a, sms, &stages);
+      if (heads) return launch_attention_ref_decode(a, heads, stages, st);
+    }
     a.tile_rows = attention_ref_tile_rows(a, sms, &vr);
     if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
       e = launch_attention_ref_rows(a, a.tile_rows, vr, st);
