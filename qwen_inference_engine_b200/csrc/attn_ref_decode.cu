@@ -1,4 +1,4 @@
-// attn_ref_decode.cu -- reference-order attention of rows that each belong to a sequence of their own (decode steps), bit for bit what
+// attn_ref_decode.cu -- reference-order attention of rows on their own (decode steps, few rows of a prompt), bit for bit what
 // attention_ref_kernel (ops_ref_order.cu) and the reference's selfattention (layers/src/self_attension.cu:10-149) compute per row and head.
 //
 // CTA = one row and up to eight query heads of one kv head, whose key and value rows are read once for all of them.
@@ -427,12 +427,16 @@ cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages
   TensorMap2D kvm;
   cudaError_t e = make_tensor_map_kv(&kvm, a.kv.pool, (unsigned long long)a.kv.n_pages * a.kv.n_layers * 2ull * a.kv.n_kv * a.kv.page_size, a.kv.hd, box);
   if (e != cudaSuccess) return e;
-  auto go = [&](auto kernel) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
-    if (e != cudaSuccess) return e;
+  auto go = [&](auto kernel, PerDeviceOnce& set) {
+    if (set.need()) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+      if (e != cudaSuccess) return e;
+      set.done();
+    }
     return launch_k(kernel, dim3(parts * a.kv.n_kv, a.n_tok), dim3(NT), smem, st, a, heads, stages, box, *reinterpret_cast<const CUtensorMap*>(&kvm));
   };
-  return a.kv.hd == 64 ? go(attention_ref_decode_kernel<1>) : go(attention_ref_decode_kernel<2>);
+  static PerDeviceOnce set[2];
+  return a.kv.hd == 64 ? go(attention_ref_decode_kernel<1>, set[0]) : go(attention_ref_decode_kernel<2>, set[1]);
 }
 
 }  // namespace qie

@@ -183,7 +183,9 @@ int qie_attention(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16*
                   const int* block_table, int max_pages, int n_tok, int n_q_heads, qie_stream st) {
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention: bad layer");
   if (!heads_ok(n_q_heads, kv->n_kv_heads)) return fail(QIE_EINVAL, "attention: %d query heads on %d kv heads", n_q_heads, kv->n_kv_heads);
+  OP_STATUS(status);
   AttnArgs a{};
+  a.status = status;
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
   a.pos = pos;
