@@ -38,9 +38,9 @@ namespace qie {
 
 static constexpr int BM = 128;  // weight rows per CTA (UMMA M)
 static constexpr int BK = 64;   // k elements per stage (128 B rows, SWIZZLE_128B)
-template <int BN, bool HALF, int KB>
-struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens); KB: k-blocks of a stage
-  static constexpr int STAGES = (HALF ? 6 : BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : 7) / KB;  // what 227 KiB hold
+template <int BN, bool HALF, int KB, int TM>
+struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens); KB: k-blocks of a stage; TM: weight rows of a tile
+  static constexpr int STAGES = TM == 64 ? 220 / (KB * (8 + BN / 8)) : (HALF ? 6 : BN <= 16 ? 12 : BN <= 32 ? 11 : BN <= 64 ? 9 : 7) / KB;  // what 227 KiB hold
 };
 
 // ------------------------------------------------------------------ PTX wrappers (tc_ptx.cuh has the rest)
@@ -108,7 +108,7 @@ struct TcArgs {
   TcSeg seg[3];
 };
 
-template <int BN, bool HALF, int KB>
+template <int BN, bool HALF, int KB, int TM>
 __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
@@ -118,11 +118,11 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   __shared__ int dead_s;
   volatile int* const dead = &dead_s;
   if (threadIdx.x == 0) dead_s = 0;  // (a barrier follows before any wait)
-  constexpr int A_BLK = BM * BK * 2, A_BYTES = KB * A_BLK;  // 16 KiB a k-block
+  constexpr int A_BLK = TM * BK * 2, A_BYTES = KB * A_BLK;  // 16 KiB a k-block (8 of 64 rows)
   constexpr int B_BLK = BN * BK * 2, B_BYTES = KB * B_BLK;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
-  constexpr int TC_STAGES = TcCfg<BN, HALF, KB>::STAGES;
+  constexpr int TC_STAGES = TcCfg<BN, HALF, KB, TM>::STAGES;
   static_assert(TC_STAGES * STAGE_BYTES >= BN * (BM + 32) * 4, "reduction tile must fit in the pipeline ring");
   // 1024-byte alignment for SWIZZLE_128B (same offset in every CTA of a cluster: the dynamic
   // shared window starts at the same address in all CTAs of a kernel)
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   while (si + 1 < g.nseg && tile >= g.seg[si + 1].tile0) ++si;
   // dual (gate/up): one tile = 64 gate rows + the same 64 up rows; segment 0 = gate map, 1 = up map
   const CUtensorMap* map_w = g.dual ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
-  const int row0 = g.dual ? tile * (BM / 2) : (tile - g.seg[si].tile0) * BM;
+  const int row0 = g.dual ? tile * (BM / 2) : (tile - g.seg[si].tile0) * TM;
   const int seg_rows = g.seg[si].rows, ld = g.seg[si].ld;
   bf16* const out = g.seg[si].out;
   const int kb0 = split * g.kb_per_split;
@@ -185,11 +185,11 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     else tma_load_2d(sb, &map_x, full_bar(s), (kb0 + i) * BK, tok_base);
   };
 
-  // The loops of both roles carry stage, parity and descriptors from step to step, and the MMA loop runs on the whole warp with one
-  // elected lane.  With a division by the stage count, a clock read per wait and descriptors built per product a step took 0.27 us
+  // The loops of both roles carry stage, parity and descriptors from step to step.  With a division by the stage count, a clock read per wait and descriptors built per product a step took 0.27 us
   // whatever the tile's width (76 steps at K = 4864: 22.8 us on an idle chip), then 0.18 us (15.7 us).  The products of a step
   // themselves take 0.025 us at 16 tokens, 0.27 us at 256.  With two k-blocks a stage (KB) a k-block takes 0.13 us: us before and after, in graphs, in the
-  // reference's order: 64 rows of 896 x 896 4.6 4.1, 4864 x 896 15.7 12.3, 8960 x 1536 27.3 20.7, 18944 x 3584 56.2 42.8; 512 rows 4864 x 896 16.6 13.7.
+  // reference's order: 64 rows of 896 x 896 4.6 4.1, 4864 x 896 15.7 12.3, 8960 x 1536 27.3 20.7, 18944 x 3584 56.2 42.8; 512 rows 4864 x 896 16.6 13.7.  Tiles of 64 weight rows and four
+  // k-blocks a stage, the wait for the next stage between the products: 4.1 4.0, 12.6 8.4, 21.2 13.6, 51.9 35; 14.0 11.5 (launch_gemm_tcgen05).
   if (warp == 0) {
     if (elect_tc()) {
       // Weights never depend on the previous kernel: start streaming them BEFORE waiting for
@@ -214,27 +214,51 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     __syncwarp();
   } else if (warp == 1) {
     pdl_wait();  // (a wait's limit counts this kernel's time, not its predecessor's)
-    const uint32_t idesc = idesc_tc(BM, BN, false);
+    const uint32_t idesc = idesc_tc(TM, BN, false);
     const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0;
     uint32_t ph = 0;
-    for (int i = 0; i < nst; ++i) {
-      mbar_wait_tc(full_bar(s), ph, dead);
-      tc_fence_after();
-      const uint64_t step = (uint64_t)(s * (STAGE_BYTES >> 4));
+    auto products = [&](int i, int b, int st) {  // of a k-block of stage i, which lies in slot st
+      if (b == 0 || i * KB + b < nkb)
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) {  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
+          const uint64_t step = (uint64_t)(st * (STAGE_BYTES >> 4));
+          umma_tc(tmem_base, ad0 + step + b * (A_BLK >> 4) + 2 * k, bd0 + step + b * (B_BLK >> 4) + 2 * k, idesc, (i | b | k) != 0);
+        }
+    };
+    if (nst >= (KB > 1 ? 16 : BN == 128 ? 8 : 40)) {
+      // Many stages: the next one is waited for in front of a stage's last products.  The tensor core has about four products ahead (160 cycles at 16 tokens and 128
+      // rows, 39 each; 94 of 64 rows, 23 each), less than a wait behind a commit takes.  us without and with: 64 rows 4864 x 896 8.7 8.4, 8960 x 1536 14.3
+      // 13.6; 1000 rows 15.5 14.6, 35.3 31.3; 1500 of 896 x 896 (14 stages of one k-block, 128 tokens) 7.1 6.8; 4 stages (896 x 896) 3.7 4.0, 16 of one k-block (1000 x 1000) 5.9 6.2.
       if (elect_tc()) {
+        mbar_wait_tc(full_bar(0), 0, dead);
+        for (int i = 0; i < nst; ++i) {
+          tc_fence_after();
+          const int st = s;
+          if (++s == TC_STAGES) s = 0, ph ^= 1;
 #pragma unroll
-        for (int b = 0; b < KB; ++b)
-          if (b == 0 || i * KB + b < nkb)
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k)  // 16 bf16 = 32 bytes along K inside the 128-byte swizzle atom
-              umma_tc(tmem_base, ad0 + step + b * (A_BLK >> 4) + 2 * k, bd0 + step + b * (B_BLK >> 4) + 2 * k, idesc, (i | b | k) != 0);
-        umma_commit_tc(empty_bar(s));  // frees the smem stage once the MMAs have read it
+          for (int b = 0; b < KB; ++b) {
+            if (b == KB - 1 && i + 1 < nst) mbar_wait_tc(full_bar(s), ph, dead);
+            products(i, b, st);
+          }
+          umma_commit_tc(empty_bar(st));  // frees the smem stage once the MMAs have read it
+        }
+        umma_commit_tc(tmem_full_bar);  // accumulator complete
       }
-      __syncwarp();
-      if (++s == TC_STAGES) s = 0, ph ^= 1;
+    } else {
+      for (int i = 0; i < nst; ++i) {
+        mbar_wait_tc(full_bar(s), ph, dead);
+        tc_fence_after();
+        if (elect_tc()) {
+#pragma unroll
+          for (int b = 0; b < KB; ++b) products(i, b, s);
+          umma_commit_tc(empty_bar(s));
+        }
+        __syncwarp();
+        if (++s == TC_STAGES) s = 0, ph ^= 1;
+      }
+      if (elect_tc()) umma_commit_tc(tmem_full_bar);
     }
-    if (elect_tc()) umma_commit_tc(tmem_full_bar);  // accumulator complete
     __syncwarp();
   }
 
@@ -246,7 +270,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     // through shared memory as bf16 [token][128 rows] (the pipeline ring is idle by now), then
     // written -- or read-modified-written -- with independent 16-byte accesses, a 256-byte
     // contiguous run per token.  Rounding points are the reference's (R3 / R8 / R9).
-    constexpr uint32_t PITCH = BM * 2;
+    constexpr uint32_t PITCH = TM * 2;
     const uint32_t stg = smem0;
     if (warp >= 2) {
       const int qd = warp & 3;
@@ -256,7 +280,9 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
         tc_fence_after();
       }
       const bool bad = *dead;
-      const int lane_row = qd * 32 + lane;
+      // (64 rows lie in the lower half of each quarter's lanes)
+      const int lane_row = TM == 64 ? qd * 16 + lane : qd * 32 + lane;
+      const bool has_row = TM == 128 || lane < 16;
 #pragma unroll
       for (int c0 = 0; c0 < BN; c0 += 16) {
         uint32_t r[16];
@@ -270,7 +296,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const unsigned short hb = __bfloat16_as_ushort(f2bf(__uint_as_float(r[j])));
-          asm volatile("st.shared.u16 [%0], %1;" ::"r"(stg + (uint32_t)(c0 + j) * PITCH + (uint32_t)lane_row * 2u), "h"(hb) : "memory");
+          if (has_row) asm volatile("st.shared.u16 [%0], %1;" ::"r"(stg + (uint32_t)(c0 + j) * PITCH + (uint32_t)lane_row * 2u), "h"(hb) : "memory");
         }
       }
       tc_fence_before();
@@ -283,7 +309,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
         return v;
       };
       if (!g.dual) {
-        const int total = n_tok * (BM / 8);
+        const int total = n_tok * (TM / 8);
         for (int c = t; c < total; c += 4 * 128) {
           uint4 y[4], x[4];
           bf16* dst[4];
@@ -291,7 +317,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int cc = c + u * 128;
-            const int tok = cc >> 4, part = cc & 15;
+            const int tok = cc / (TM / 8), part = cc % (TM / 8);
             const int w_row = row0 + part * 8;
             ok[u] = cc < total && w_row < seg_rows;
             dst[u] = out + (size_t)(tok_base + tok) * ld + w_row;
@@ -353,7 +379,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   const bool epi_warp = warp >= 2;
   const int qd = warp & 3;  // TMEM lane quarter of this epilogue warp
   const bool via_smem = g.splits > 1 || g.dual;
-  const int tile_rows = g.dual ? BM / 2 : BM;  // output rows produced by this tile
+  const int tile_rows = g.dual ? BM / 2 : TM;  // output rows produced by this tile
   const int rows_per = ((tile_rows + g.splits - 1) / g.splits + 3) & ~3;
   const uint32_t pitch = (uint32_t)(BM + min(rows_per, 32)) * 4u;
   if (epi_warp) {
@@ -363,7 +389,9 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       tc_fence_after();
     }
     const bool bad = *dead;
-    const int lane_row = qd * 32 + lane;  // TMEM lane = row inside the 128-row tile
+    // TMEM lane = row inside the tile (of 64 rows: the lower half of each quarter's lanes)
+    const int lane_row = TM == 64 ? qd * 16 + lane : qd * 32 + lane;
+    const bool has_row = TM == 128 || lane < 16;
 #pragma unroll
     for (int c0 = 0; c0 < BN; c0 += 16) {
       uint32_t r[16];
@@ -381,7 +409,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
       } else {
         // no split, single accumulator: epilogue straight from registers
         const int w_row = row0 + lane_row;
-        if (w_row < seg_rows) {
+        if (has_row && w_row < seg_rows) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int tok = tok_base + c0 + j;
@@ -840,15 +868,15 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN, bool HALF, int KB>
+template <int BN, bool HALF, int KB, int TM>
 static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
-  constexpr int STAGE_BYTES = KB * (BM * BK * 2 + BN * BK * 2);
-  constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  constexpr int STAGE_BYTES = KB * (TM * BK * 2 + BN * BK * 2);
+  constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB, TM>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     set.done();
   }
@@ -873,17 +901,21 @@ static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], 
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB, TM>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
 }
 
 template <int KB>
 static cudaError_t launch_tile(int bn, bool half, const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
+  constexpr int TM = KB == 4 ? 64 : BM;
   switch (bn) {
-    case 16: return half ? launch_bn<16, true, KB>(g, w, x, token_tiles, st) : launch_bn<16, false, KB>(g, w, x, token_tiles, st);
-    case 32: return launch_bn<32, false, KB>(g, w, x, token_tiles, st);
-    case 64: return launch_bn<64, false, KB>(g, w, x, token_tiles, st);
+    case 16:
+      if constexpr (KB != 4)
+        if (half) return launch_bn<16, true, KB, TM>(g, w, x, token_tiles, st);
+      return launch_bn<16, false, KB, TM>(g, w, x, token_tiles, st);
+    case 32: return launch_bn<32, false, KB, TM>(g, w, x, token_tiles, st);
+    case 64: return launch_bn<64, false, KB, TM>(g, w, x, token_tiles, st);
     default:
-      if constexpr (KB == 1) return launch_bn<128, false, 1>(g, w, x, token_tiles, st);
+      if constexpr (KB == 1) return launch_bn<128, false, 1, TM>(g, w, x, token_tiles, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -949,7 +981,16 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   // for it, and fast numerics keep the reference's.
   g.ref_silu = t.exact || t.M <= 128;
   g.status = t.status;
-  int tiles = 0, cols = 0;
+  int tiles = 0;
+  auto segments = [&](int tm) {  // tiles of tm weight rows
+    int cols = 0;
+    tiles = 0;
+    for (int i = 0; i < t.nseg; ++i) {
+      g.seg[i] = t.outs[i] ? TcSeg{t.rows[i], tiles, t.lds[i], t.outs[i]} : TcSeg{t.rows[i], tiles, t.ld_out, t.out + cols};
+      tiles += (t.rows[i] + tm - 1) / tm;
+      cols += t.rows[i];
+    }
+  };
   if (g.dual) {
     // segments = (gate, up) with equal row counts; the weight maps must have 64-row boxes
     if (t.nseg != 2 || t.rows[0] != t.rows[1]) return cudaErrorInvalidValue;
@@ -957,32 +998,45 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     g.nseg = 1;
     tiles = (t.rows[0] + BM / 2 - 1) / (BM / 2);
   } else {
-    for (int i = 0; i < t.nseg; ++i) {
-      g.seg[i] = t.outs[i] ? TcSeg{t.rows[i], tiles, t.lds[i], t.outs[i]} : TcSeg{t.rows[i], tiles, t.ld_out, t.out + cols};
-      tiles += (t.rows[i] + BM - 1) / BM;
-      cols += t.rows[i];
-    }
+    segments(BM);
   }
-  g.n_tiles = tiles;
   g.kb_total = (t.K + BK - 1) / BK;
   bool vec = true;  // 16-byte stores reach every row of the outputs
   for (int i = 0; i < g.nseg; ++i)
     vec = vec && g.seg[i].rows % 8 == 0 && g.seg[i].ld % 8 == 0 && (reinterpret_cast<uintptr_t>(g.seg[i].out) & 15) == 0;
-  const TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, !t.exact);
+  TcTile tl = pick_tile(t.M, tiles, g.kb_total, num_sms, !t.exact);
+  // Tiles of 64 weight rows where they all fit on the SMs and a CTA brings fewer rows: with few tiles and a long K a CTA takes its operands at 138 GB/s from L2, whatever
+  // the tile (a k-block of 128 rows and 16 tokens 0.13 us, 32 0.15, 64 0.174).  Four k-blocks a stage (two of 64 rows 0.10 us, four 0.07): from eight on, so that at most one of
+  // three stages is short (of 64 tokens, whose ring holds three, from twenty on: 64 rows of 896 x 4864 4.9 5.1), and not where there would be fewer CTAs (1000 rows of 2048
+  // x 300, 96 and 80: 8.6 8.8).  us of 128 and of 64 rows, reference order: 64 rows 4864 x 896 12.6 8.4, 8960 x 1536 21.2 13.6, 896 x 1152 4.5 4.0; 512 rows 4864 x 896
+  // 14.0 11.5; 200 rows 8960 x 1536 22.9 17.5.  Their maps are made here, so the weights' place has to be known.
+  int tm = BM;
+  bool wp = true;
+  for (int i = 0; i < t.nseg; ++i) wp = wp && t.wp[i];
+  if (!tl.persist && !tl.half && tl.splits == 1 && !g.dual && wp && t.K % BK == 0 && g.kb_total >= 8) {
+    long tiles64 = 0;
+    for (int i = 0; i < t.nseg; ++i) tiles64 += (t.rows[i] + 63) / 64;
+    int bn = 16;
+    while (bn < 128 && tiles64 * ((t.M + bn - 1) / bn) > num_sms) bn *= 2;
+    const auto ctas = [&](long n, int b) { return n * ((t.M + b - 1) / b); };
+    if (bn <= (g.kb_total >= 20 ? 64 : 32) && 64 + bn < BM + tl.bn && ctas(tiles64, bn) >= ctas(tiles, tl.bn)) tm = 64, tl.bn = bn, segments(64);
+  }
+  g.n_tiles = tiles;
   const int token_tiles = (t.M + tl.bn - 1) / tl.bn;
   g.kb_per_split = (g.kb_total + tl.splits - 1) / tl.splits;
   g.splits = (g.kb_total + g.kb_per_split - 1) / g.kb_per_split;
   g.staged = g.splits == 1 && vec;
   g.vec = vec;
-  // the weights' maps, in boxes of one or two k-blocks: those that the caller keeps, else made here
+  // the weights' maps, in boxes of one, two or four k-blocks: those that the caller keeps, else made here
   const CUtensorMap* w[3];
   TensorMap2D made[3], x;
+  const int kb = tm == BM ? 2 : 4;  // k-blocks of a stage of more than one
   auto maps = [&](bool two) {
     for (int i = 0; i < t.nseg; ++i) {
-      const TensorMap2D* m = two ? t.w2[i] : t.w[i];
+      const TensorMap2D* m = tm == 64 ? nullptr : two ? t.w2[i] : t.w[i];
       if (!m) {
         if (!t.wp[i]) return false;
-        const cudaError_t e = two ? make_tensor_map_w3d(&made[i], t.wp[i], t.rows[i], t.K, 2 * BK, 0, BM) : make_tensor_map_2d(&made[i], t.wp[i], t.rows[i], t.K, g.dual ? BM / 2 : BM);
+        const cudaError_t e = two ? make_tensor_map_w3d(&made[i], t.wp[i], t.rows[i], t.K, kb * BK, 0, tm) : make_tensor_map_2d(&made[i], t.wp[i], t.rows[i], t.K, g.dual ? BM / 2 : BM);
         if (e != cudaSuccess) return false;
         m = &made[i];
       }
@@ -998,9 +1052,9 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   // the operands (us with stages of one and of two, 1000 rows: 192 x 130 3.7 4.0, 320 x 130 4.3 4.6, 448 x 130 4.7 4.7, 576 x 130 4.5 4.2).
   const bool whole = g.splits > 1 || g.kb_total % 2 == 0 || g.kb_total > 5;
   if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && maps(true) &&
-      make_tensor_map_w3d(&x, t.x, t.M, t.K, 2 * BK, 0, tl.bn) == cudaSuccess)
-    return launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
-  if (!maps(false)) {
+      make_tensor_map_w3d(&x, t.x, t.M, t.K, kb * BK, 0, tl.bn) == cudaSuccess)
+    return tm == 64 ? launch_tile<4>(tl.bn, false, g, w, x, token_tiles, st) : launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
+  if (tm != BM || !maps(false)) {
     if (launches) *launches = 0;
     return cudaErrorNotSupported;
   }
