@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "cluster.cuh"
 #include "common.cuh"
@@ -108,7 +109,7 @@ struct TcArgs {
   TcSeg seg[3];
 };
 
-template <int BN, bool HALF, int KB, int TM>
+template <int BN, bool HALF, int KB, int TM, bool AHEAD>
 __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
@@ -226,19 +227,19 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
           umma_tc(tmem_base, ad0 + step + b * (A_BLK >> 4) + 2 * k, bd0 + step + b * (B_BLK >> 4) + 2 * k, idesc, (i | b | k) != 0);
         }
     };
-    if (nst >= (KB > 1 ? 16 : BN == 128 ? 8 : 40)) {
-      // Many stages: the next one is waited for in front of a stage's last products.  The tensor core has about four products ahead (160 cycles at 16 tokens and 128
-      // rows, 39 each; 94 of 64 rows, 23 each), less than a wait behind a commit takes.  us without and with: 64 rows 4864 x 896 8.7 8.4, 8960 x 1536 14.3
-      // 13.6; 1000 rows 15.5 14.6, 35.3 31.3; 1500 of 896 x 896 (14 stages of one k-block, 128 tokens) 7.1 6.8; 4 stages (896 x 896) 3.7 4.0, 16 of one k-block (1000 x 1000) 5.9 6.2.
+    if constexpr (AHEAD) {
+      // Many stages: whether the next one is there is asked in front of a stage's last products.  The tensor core has about four products ahead (160 cycles at 16 tokens
+      // and 128 rows, 39 each; 94 of 64 rows, 23 each), less than a wait behind a commit takes.
       if (elect_tc()) {
-        mbar_wait_tc(full_bar(0), 0, dead);
+        bool there = false;
         for (int i = 0; i < nst; ++i) {
+          if (!there) mbar_wait_tc(full_bar(s), ph, dead);
           tc_fence_after();
           const int st = s;
           if (++s == TC_STAGES) s = 0, ph ^= 1;
 #pragma unroll
           for (int b = 0; b < KB; ++b) {
-            if (b == KB - 1 && i + 1 < nst) mbar_wait_tc(full_bar(s), ph, dead);
+            if (b == KB - 1) there = mbar_ready_tc(full_bar(s), ph);
             products(i, b, st);
           }
           umma_commit_tc(empty_bar(st));  // frees the smem stage once the MMAs have read it
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int cc = c + u * 128;
-            const int tok = cc / (TM / 8), part = cc % (TM / 8);
+            const int tok = cc >> (TM == 128 ? 4 : 3), part = cc & (TM / 8 - 1);
             const int w_row = row0 + part * 8;
             ok[u] = cc < total && w_row < seg_rows;
             dst[u] = out + (size_t)(tok_base + tok) * ld + w_row;
@@ -868,15 +869,15 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN, bool HALF, int KB, int TM>
+template <int BN, bool HALF, int KB, int TM, bool AHEAD>
 static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int STAGE_BYTES = KB * (TM * BK * 2 + BN * BK * 2);
   constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB, TM>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     set.done();
   }
@@ -901,21 +902,26 @@ static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], 
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB, TM>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
 }
 
 template <int KB>
-static cudaError_t launch_tile(int bn, bool half, const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
+static cudaError_t launch_tile(int bn, bool half, bool ahead, const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int TM = KB == 4 ? 64 : BM;
+  auto go = [&](auto n) {
+    constexpr int BN = decltype(n)::value;
+    if constexpr (KB > 1 || BN == 128)
+      if (ahead) return launch_bn<BN, false, KB, TM, true>(g, w, x, token_tiles, st);
+    return launch_bn<BN, false, KB, TM, false>(g, w, x, token_tiles, st);
+  };
+  if constexpr (KB != 4)
+    if (half) return launch_bn<16, true, KB, TM, false>(g, w, x, token_tiles, st);
   switch (bn) {
-    case 16:
-      if constexpr (KB != 4)
-        if (half) return launch_bn<16, true, KB, TM>(g, w, x, token_tiles, st);
-      return launch_bn<16, false, KB, TM>(g, w, x, token_tiles, st);
-    case 32: return launch_bn<32, false, KB, TM>(g, w, x, token_tiles, st);
-    case 64: return launch_bn<64, false, KB, TM>(g, w, x, token_tiles, st);
+    case 16: return go(std::integral_constant<int, 16>{});
+    case 32: return go(std::integral_constant<int, 32>{});
+    case 64: return go(std::integral_constant<int, 64>{});
     default:
-      if constexpr (KB == 1) return launch_bn<128, false, 1, TM>(g, w, x, token_tiles, st);
+      if constexpr (KB == 1) return go(std::integral_constant<int, 128>{});
   }
   return cudaErrorInvalidValue;
 }
@@ -1046,6 +1052,10 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     return true;
   };
   if (launches) *launches = 1;
+  // The MMA warp asks ahead for the next stage from 16 stages on, eight of 128 tokens (us without and with: 64 rows 4864 x 896 8.7 8.2, 8960 x 1536 14.3 13.6; 1000 rows
+  // 15.5 14.5, 35.3 30.8; 1500 of 896 x 896 7.1 6.8; 4 stages of four k-blocks, 896 x 896, 3.7 4.0).  Not for gate/up (nothing) and clusters (few stages, or weights
+  // from memory: 300 rows of 8960 x 1536 in two 26.2 26.8).
+  auto ahead = [&](int stage) { return g.splits == 1 && !g.dual && (g.kb_total + stage - 1) / stage >= (tl.bn == 128 ? 8 : 16); };
   // Two k-blocks a stage where tensor maps can express them (whole k-blocks, and the weights' place is known): half the requests, waits and commits.  Up
   // to 64 tokens: of 128 the ring holds three such stages, too few on the way (8960 x 1536 at 1000 rows 34.8 with stages of one, 37.1).  Gate/up tiles
   // are two boxes a k-block as they are.  Not for 3 or 5 k-blocks: the half of the last stage that is not there is a box of zeros to bring, a quarter of
@@ -1053,7 +1063,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   const bool whole = g.splits > 1 || g.kb_total % 2 == 0 || g.kb_total > 5;
   if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && maps(true) &&
       make_tensor_map_w3d(&x, t.x, t.M, t.K, kb * BK, 0, tl.bn) == cudaSuccess)
-    return tm == 64 ? launch_tile<4>(tl.bn, false, g, w, x, token_tiles, st) : launch_tile<2>(tl.bn, tl.half, g, w, x, token_tiles, st);
+    return tm == 64 ? launch_tile<4>(tl.bn, false, ahead(4), g, w, x, token_tiles, st) : launch_tile<2>(tl.bn, tl.half, ahead(2), g, w, x, token_tiles, st);
   if (tm != BM || !maps(false)) {
     if (launches) *launches = 0;
     return cudaErrorNotSupported;
@@ -1084,7 +1094,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     cfg.numAttrs = g_use_pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
   }
-  return launch_tile<1>(tl.bn, tl.half, g, w, x, token_tiles, st);
+  return launch_tile<1>(tl.bn, tl.half, ahead(1), g, w, x, token_tiles, st);
 }
 
 // Reference-order products of any number of rows.  The chain of tcgen05.mma over ascending k of 16 into one accumulator gives the bits of

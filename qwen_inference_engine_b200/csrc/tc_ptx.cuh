@@ -31,6 +31,17 @@ __device__ __forceinline__ bool mbar_wait_tc(uint32_t bar, uint32_t parity, vola
   *dead = 1;
   return false;
 }
+__device__ __forceinline__ bool mbar_ready_tc(uint32_t bar, uint32_t parity) {  // without waiting
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
 __device__ __forceinline__ void drain_tc(const volatile int* dead) {
   if (*dead)
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
