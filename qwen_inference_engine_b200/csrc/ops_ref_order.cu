@@ -499,7 +499,8 @@ cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
     // (us, attention_ref_rows_kernel and here, 14 heads of 64 on 2: 1 row at 301 positions 14.3 7.9, at 2001 60 24, 32 rows behind 300 15.6 9.1, 64 behind 2000
     // 63 35; 17 rows of a prompt 5.8 5.4; up to 16 positions one block per row and head, 3.5 4.5).  More rows than that share their keys and values here in tiles of several rows,
     // which is worth more the shorter the context: w waves are quicker above 160 w positions with all of six to eight heads in a CTA (96 rows behind 120 15.6 15.1, behind 50
-    // 12.5 13.5; 200 behind 300 41 33; 300 behind 800 93 90, behind 300 47 55; 16 heads on 1, 300 behind 800 90 93), one above 32 (24 rows of a prompt, 28 heads of 128 on 4 6.7 7.7).  Operator calls with tables beyond attention_ref_rows_kernel's sizes stay with the
+    // 12.5 13.5; 200 behind 300 41 33; 300 behind 800 93 90, behind 300 47 55), above 225 w with a part of them (16 heads on 1, 200 behind 2000 166 108, 300 behind 800
+    // 90 93), one above 32 (24 rows of a prompt, 28 heads of 128 on 4 6.7 7.7).  Operator calls with tables beyond attention_ref_rows_kernel's sizes stay with the
     // kernel below.
     int stages = 0;
     const int heads = attention_ref_decode_heads(a, sms, &stages);
@@ -507,7 +508,7 @@ cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
     if (heads) {
       const int G = a.n_q / a.kv.n_kv;
       const long ctas = (long)a.n_tok * a.kv.n_kv * ((G + heads - 1) / heads), waves = (ctas + sms - 1) / sms;
-      if (a.decode || (a.tile_rows && (waves == 1 ? heads < 6 || a.max_kv_len > 32 : heads >= 6 && heads == G && a.max_kv_len >= 160 * waves))) return launch_attention_ref_decode(a, heads, stages, st);
+      if (a.decode || (a.tile_rows && (waves == 1 ? heads < 6 || a.max_kv_len > 32 : heads >= 6 && a.max_kv_len >= (heads == G ? 160 : 225) * waves))) return launch_attention_ref_decode(a, heads, stages, st);
     }
     if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
       e = launch_attention_ref_rows(a, a.tile_rows, vr, st);
