@@ -26,6 +26,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <type_traits>
 
@@ -48,7 +49,15 @@ struct TcCfg {  // HALF: a ring that leaves room for a second CTA (16 tokens); K
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+template <int CTAS = 1>  // 2: the barrier may be the other CTA's of a pair
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  if constexpr (CTAS == 2) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+    return;
+  }
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1)
@@ -60,11 +69,22 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2)
       : "memory");
 }
+template <int CTAS = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
+  if constexpr (CTAS == 2) {  // a warp of either CTA
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    return;
+  }
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot_smem), "r"(cols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+template <int CTAS = 1>
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
+  if constexpr (CTAS == 2) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
+    return;
+  }
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -103,6 +123,7 @@ struct TcArgs {
   int epi, dual, w_static;
   int ref_silu;    // persistent kernel: SiLU as the reference computes it (expf, IEEE division); the others always do
   int bn, stages;  // persistent kernel: tokens of a tile (a multiple of 16), stages of its ring
+  int tokens_first;  // ... neighbouring CTAs have a weight tile's token tiles, else a token tile's weight tiles
   int* status;     // host word that a wait which ran out sets, or null
   int vec;         // persistent kernel: rows of the output take 16-byte stores
   int staged;  // splits == 1 and 8-element aligned outputs: epilogue through a bf16 tile in shared memory, 16-byte global accesses
@@ -533,6 +554,9 @@ static constexpr int P_EPI = 256;                 // epilogue threads (8 warps)
 static constexpr int P_THREADS = 64 + P_EPI;      // + TMA warp + MMA warp
 static constexpr int P_STAGING = 2 * P_STEP * BM * 2;               // bf16 [2][64 tokens][128 rows] = 32 KiB
 
+// CTAS 2: a pair of CTAs, a cluster, has two neighbouring weight tiles and one token tile; either brings its own weights and half of the tokens, and the
+// first one's MMA warp multiplies both tiles at once (cta_group::2).
+template <int CTAS>
 __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                                    const __grid_constant__ CUtensorMap map_w1,
                                                                    const __grid_constant__ CUtensorMap map_w2,
@@ -546,7 +570,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   constexpr int A_BYTES = BM * BK * 2;
   constexpr uint32_t TMEM_COLS = 512;  // two accumulators
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const int bn = g.bn, stages = g.stages, stage_bytes = A_BYTES + bn * BK * 2;
+  const int bn = g.bn, stages = g.stages, own = bn / CTAS, stage_bytes = A_BYTES + own * BK * 2;
   const uint32_t stg = smem0 + P_RING;
   const uint32_t bars = stg + P_STAGING;  // full[S], empty[S], tmem_full[2], tmem_empty[2], slot
   auto full_bar = [&](int s) { return bars + 8u * s; };
@@ -556,8 +580,15 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
   const uint32_t slot = bars + 8u * (2 * P_MAX_STAGES + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int total = g.n_tiles * token_tiles;
+  const int pairs = (g.n_tiles + CTAS - 1) / CTAS, total = pairs * token_tiles;
   const int nkb = g.kb_total;
+  const int inner = g.tokens_first ? token_tiles : pairs;  // tiles that neighbours walk
+  const int rank = CTAS == 1 ? 0 : blockIdx.x % CTAS, at0 = blockIdx.x / CTAS, step_t = gridDim.x / CTAS;
+  auto leader = [&](uint32_t bar) {  // the barrier of the pair's first CTA
+    uint32_t r = bar;
+    if (CTAS > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(bar), "r"(0));
+    return r;
+  };
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w0) : "memory");
@@ -570,21 +601,23 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init_tc(tfull_bar(b), 1);
-      mbar_init_tc(tempty_bar(b), 1);
+      mbar_init_tc(tempty_bar(b), CTAS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(slot, TMEM_COLS);
+  if (warp == 1) tmem_alloc<CTAS>(slot, TMEM_COLS);
   tc_fence_before();
-  __syncthreads();
+  if (CTAS > 1) cluster_sync_all();
+  else __syncthreads();
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(slot));
 
   // tile -> (weight tile, token tile, segment) ; dual: one tile = 64 gate rows + the same 64 up rows
   auto tile_geom = [&](int t, int& tile, int& ttile, int& si, int& row0) {
-    tile = t % g.n_tiles;
-    ttile = t / g.n_tiles;
+    const int slow = t / inner, fast = t - slow * inner;
+    tile = (g.tokens_first ? slow : fast) * CTAS + rank;
+    ttile = g.tokens_first ? fast : slow;
     si = 0;
     while (si + 1 < g.nseg && tile >= g.seg[si + 1].tile0) ++si;
     row0 = g.dual ? tile * (BM / 2) : (tile - g.seg[si].tile0) * BM;
@@ -598,35 +631,35 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
       auto load_w = [&](int kb, int si, int row0) {
         const uint32_t sa = smem0 + s * stage_bytes;
         if (g.dual) {
-          tma_load_2d(sa, &map_w0, full_bar(s), kb * BK, row0);
-          tma_load_2d(sa + A_BYTES / 2, &map_w1, full_bar(s), kb * BK, row0);
+          tma_load_2d<CTAS>(sa, &map_w0, leader(full_bar(s)), kb * BK, row0);
+          tma_load_2d<CTAS>(sa + A_BYTES / 2, &map_w1, leader(full_bar(s)), kb * BK, row0);
         } else {
-          tma_load_2d(sa, si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2), full_bar(s), kb * BK, row0);
+          tma_load_2d<CTAS>(sa, si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2), leader(full_bar(s)), kb * BK, row0);
         }
       };
       int tile, ttile, si, row0;
       // the first stages' weights in front of the wait for the previous kernel, which wrote the activations
       int pre = 0;
-      if (g.w_static && blockIdx.x < total) {
-        tile_geom(blockIdx.x, tile, ttile, si, row0);
+      if (g.w_static && at0 < total) {
+        tile_geom(at0, tile, ttile, si, row0);
         for (pre = min(nkb, stages); s < pre; ++s) {
-          mbar_expect_tx(full_bar(s), stage_bytes);
+          if (rank == 0) mbar_expect_tx(full_bar(s), CTAS * stage_bytes);
           load_w(s, si, row0);
         }
         s = 0;
       }
       pdl_wait();
-      for (int t = blockIdx.x; t < total && go; t += gridDim.x) {
+      for (int t = at0; t < total && go; t += step_t) {
         tile_geom(t, tile, ttile, si, row0);
         for (int kb = 0; kb < nkb; ++kb) {
           if (pre > 0) {  // (the first stages: nothing to wait for)
             --pre;
           } else {
             if (!(go = mbar_wait_tc(empty_bar(s), ph, dead))) break;
-            mbar_expect_tx(full_bar(s), stage_bytes);
+            if (rank == 0) mbar_expect_tx(full_bar(s), CTAS * stage_bytes);
             load_w(kb, si, row0);
           }
-          tma_load_2d(smem0 + s * stage_bytes + A_BYTES, &map_x, full_bar(s), kb * BK, ttile * bn);
+          tma_load_2d<CTAS>(smem0 + s * stage_bytes + A_BYTES, &map_x, leader(full_bar(s)), kb * BK, ttile * bn + rank * own);
           if (++s == stages) s = 0, ph ^= 1;
         }
       }
@@ -634,11 +667,11 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     __syncwarp();
   } else if (warp == 1) {
     pdl_wait();  // as above
-    const uint32_t idesc = idesc_tc(BM, bn, false);
+    const uint32_t idesc = idesc_tc(BM * CTAS, bn, false);
     const uint64_t ad0 = desc_k_tc(smem0), bd0 = desc_k_tc(smem0 + A_BYTES);
     int s = 0, j = 0;
     uint32_t ph = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+    for (int t = rank == 0 ? at0 : total; t < total; t += step_t, ++j) {
       const int buf = j & 1;
       mbar_wait_tc(tempty_bar(buf), (((uint32_t)j >> 1) & 1) ^ 1, dead);  // epilogue has drained this accumulator
       tc_fence_after();
@@ -649,13 +682,13 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
         const uint64_t step = (uint64_t)(s * (stage_bytes >> 4));
         if (elect_tc()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_tc(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
-          umma_commit_tc(empty_bar(s));
+          for (int k = 0; k < BK / 16; ++k) umma_tc<CTAS>(acc, ad0 + step + 2 * k, bd0 + step + 2 * k, idesc, (kb | k) != 0);
+          umma_commit_tc<CTAS>(empty_bar(s));
         }
         __syncwarp();
         if (++s == stages) s = 0, ph ^= 1;
       }
-      if (elect_tc()) umma_commit_tc(tfull_bar(buf));
+      if (elect_tc()) umma_commit_tc<CTAS>(tfull_bar(buf));
       __syncwarp();
     }
   } else {
@@ -678,7 +711,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     const int copier = lane < P_STEP / 8 ? (warp - 2) * (P_STEP / 8) + lane : P_STEP;  // the token whose copy this thread issues
     pdl_wait();  // `out` may still be read (residual) by the previous kernel
     int j = 0, it = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, ++j) {
+    for (int t = at0; t < total; t += step_t, ++j) {
       int tile, ttile, si, row0;
       tile_geom(t, tile, ttile, si, row0);
       const int seg_rows = g.seg[si].rows, ld = g.seg[si].ld;
@@ -725,9 +758,9 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         asm volatile("bar.sync 2, 256;" ::: "memory");
-        if (h0 + P_STEP >= bn && tq == 0) mbar_arrive_tc(tempty_bar(buf));  // the MMA warp may overwrite this accumulator (tile j+2)
+        if (h0 + P_STEP >= bn && tq == 0) mbar_arrive_tc<CTAS>(leader(tempty_bar(buf)));  // the MMA warp may overwrite this accumulator (tile j+2)
         if (bulk) {
-          if (copier < n_tok) {
+          if (copier < n_tok && row0 < seg_rows) {  // (a pair's second tile may lie behind the last one)
             bf16* dst = out + (size_t)(tok_base + h0 + copier) * ld + row0;
             asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(st0 + (uint32_t)copier * PITCH),
                          "r"(2 * min(BM, seg_rows - row0))
@@ -779,12 +812,13 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
     }
     if (bulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // written, before the CTA gives its shared memory back
   }
-  __syncthreads();
+  if (CTAS > 1) cluster_sync_all();  // (the other one's operands and barriers are read and written to the end)
+  else __syncthreads();
   if (warp == 1) {
     drain_tc(dead);
     if (lane == 0) report_tc(dead, g.status);
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc<CTAS>(tmem_base, TMEM_COLS);
   }
 }
 
@@ -974,6 +1008,96 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool may_split) 
   return best;
 }
 
+// Tokens of a pair's tile, 0 where single CTAs of `bn` tokens stay.  Costs of a wave are in units of about 1 ns a k-block: a single CTA's operands take it 1.0 a row of 128
+// bytes that it brings from L2 (256 tokens: 48 KB, 0.4 us), a pair's CTA 1.22 a row or the products 1.36 a token, whichever is more; a pair's start and end cost
+// 1.2 us more, and few waves have to gain by more.  Below 20 k-blocks a tile the epilogue sets the pace.  us in graphs, single CTAs and pairs: 4096 rows 1536 x 8960 78 72 (256
+// tokens), 8960 x 1536 83 78 (192), 3584 x 3584 79 70 (224), 2048 rows of 1536 x 8960 40 38, 1500 of 3584 x 3584 33.4 31.0 (160); stay: 2048 of 3584 x 3584 36.6 37.6
+// (224), 1000 rows 21.1 23.2 (224), 700 of 3584 x 4608 19.8 20.3 (192), 4096 of 1536 x 1536 18.4 18.4 (192), of 896 x 4864 33.3 32.2 to 36.8.
+static int pick_pair(int M, int tiles, int nkb, int num_sms, int pairs, int bn) {
+  if (pairs <= 0 || nkb < 20) return 0;
+  auto waves = [&](int t, int b, int at) { return ((long)t * ((M + b - 1) / b) + at - 1) / at; };
+  const float single = (float)waves(tiles, bn, num_sms) * (float)(BM + bn);
+  int best = 0;
+  float cost = single;
+  for (int b = 256; b >= 128; b -= 32) {
+    const long n = waves((tiles + 1) / 2, b, pairs);
+    const float c = (float)n * std::max(1.22f * (float)(BM + b / 2), 1.36f * (float)b) + 1200.f / (float)nkb;
+    if (c < (best ? 0.97f * cost : cost) && c < single * (n > 2 ? 0.97f : n == 2 ? 0.93f : 0.9f)) cost = c, best = b;
+  }
+  return best;
+}
+
+static constexpr size_t P_SMEM = (size_t)P_RING + P_STAGING + 1024 /*align*/ + 256 /*barriers*/;
+template <int CTAS>
+static cudaError_t persist_attributes() {
+  static PerDeviceOnce set;
+  if (!set.need()) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_persist_kernel<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM);
+  if (e == cudaSuccess) set.done();
+  return e;
+}
+
+// at: CTAs, or pairs of them, that run at once
+template <int CTAS>
+static cudaError_t launch_persist(TcArgs g, int bn, int at, const CUtensorMap* const (&w)[3], const bf16* xp, int M, int K, cudaStream_t st) {
+  TensorMap2D x;
+  cudaError_t e = make_tensor_map_2d(&x, xp, M, K, bn / CTAS);
+  if (e != cudaSuccess || (e = persist_attributes<CTAS>()) != cudaSuccess) return e;
+  const int token_tiles = (M + bn - 1) / bn;
+  g.bn = bn;
+  long w_rows = 0;  // K elements each, like the tokens
+  for (int i = 0; i < g.nseg; ++i) w_rows += (g.dual ? 2 : 1) * g.seg[i].rows;
+  // A wave's CTAs share a token tile and bring all weights, which the next wave finds in L2 unless they are too many: then the CTAs share weight tiles and bring all
+  // tokens, if those are few.  us of 3584 x 18944 (136 MB): 400 rows 57.7 48.9, 4096 single CTAs 477 363, pairs 423 333; 896 x 151936, 1000 rows 280 241; 18944 x 3584, 1000
+  // rows 161 135, but 2048 (78 MB of tokens) 228 255.
+  g.tokens_first = 2 * w_rows * K > 64l << 20 && 2 * M < w_rows;
+  g.stages = std::min(P_MAX_STAGES, P_RING / (BM * BK * 2 + bn / CTAS * BK * 2));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(CTAS * std::min<long>(at, (long)((g.n_tiles + CTAS - 1) / CTAS) * token_tiles)));
+  cfg.blockDim = dim3(P_THREADS);
+  cfg.dynamicSmemBytes = P_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute at_[2];
+  int na = 0;
+  if (CTAS > 1) {
+    at_[na].id = cudaLaunchAttributeClusterDimension;
+    at_[na].val.clusterDim.x = CTAS;
+    at_[na].val.clusterDim.y = at_[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (g_use_pdl) {
+    at_[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at_[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg.attrs = at_;
+  cfg.numAttrs = na;
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel<CTAS>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
+}
+
+// pairs of CTAs of the persistent kernel that run at once on this device, 0 if there is no telling
+static int pairs_at_once() {
+  static std::atomic<int> known[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = known[dev].load(std::memory_order_relaxed);
+  if (n) return n > 0 ? n : 0;
+  if (persist_attributes<2>() != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(P_THREADS);
+  cfg.dynamicSmemBytes = P_SMEM;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_persist_kernel<2>, &cfg) != cudaSuccess) n = 0, (void)cudaGetLastError();
+  known[dev].store(n > 0 ? n : -1, std::memory_order_relaxed);
+  return n > 0 ? n : 0;
+}
+
 cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, int* launches) {
   if (t.M < 1 || t.K < BK || (t.K % 8) || t.nseg < 1 || t.nseg > 3) return cudaErrorInvalidValue;
   TcArgs g{};
@@ -1068,32 +1192,14 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     if (launches) *launches = 0;
     return cudaErrorNotSupported;
   }
-  cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
-  if (e != cudaSuccess) return e;
   if (tl.persist) {
     // (widths of the residual stream and of the feed-forward are inner dimensions too, so multiples of 8)
     if (!vec && t.epi != EPI_STORE) return cudaErrorInvalidValue;
-    constexpr size_t smem = (size_t)P_RING + P_STAGING + 1024 /*align*/ + 256 /*barriers*/;
-    static PerDeviceOnce set;
-    if (set.need()) {
-      e = cudaFuncSetAttribute(gemm_tcgen05_persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      set.done();
-    }
-    g.bn = tl.bn;
-    g.stages = std::min(P_MAX_STAGES, P_RING / (BM * BK * 2 + tl.bn * BK * 2));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min<long>(num_sms, (long)tiles * token_tiles));
-    cfg.blockDim = dim3(P_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = g_use_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, gemm_tcgen05_persist_kernel, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g, token_tiles);
+    const int pairs = pairs_at_once(), pair_bn = pick_pair(t.M, tiles, g.kb_total, num_sms, pairs, tl.bn);
+    return pair_bn ? launch_persist<2>(g, pair_bn, pairs, w, t.x, t.M, t.K, st) : launch_persist<1>(g, tl.bn, num_sms, w, t.x, t.M, t.K, st);
   }
+  const cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
+  if (e != cudaSuccess) return e;
   return launch_tile<1>(tl.bn, tl.half, ahead(1), g, w, x, token_tiles, st);
 }
 

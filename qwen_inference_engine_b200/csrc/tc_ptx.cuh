@@ -6,7 +6,11 @@
 namespace qie {
 
 __device__ __forceinline__ void mbar_init_tc(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
-__device__ __forceinline__ void mbar_arrive_tc(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+template <int CTAS = 1>  // 2: the barrier may be the other CTA's of a pair
+__device__ __forceinline__ void mbar_arrive_tc(uint32_t bar) {
+  if constexpr (CTAS == 2) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 // Waits for the phase of this parity.  After about two seconds it sets *dead, and from then on no wait of the CTA waits: its kernel stores values
 // that are not numbers, lets copies in flight land (drain_tc), reports (report_tc) and returns.  The clock is read only where a wait is long.
 constexpr long long WAIT_CYCLES_TC = 4000000000ll;
@@ -60,7 +64,17 @@ __device__ __forceinline__ bool elect_tc() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
+template <int CTAS = 1>  // 2: the operands lie in both CTAs of a pair at the same places, as do the accumulators
 __device__ __forceinline__ void umma_tc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+  if constexpr (CTAS == 2) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+    return;
+  }
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
@@ -68,7 +82,12 @@ __device__ __forceinline__ void umma_tc(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
 }
+template <int CTAS = 1>  // 2: arrives at the barrier of that place in both CTAs
 __device__ __forceinline__ void umma_commit_tc(uint32_t bar) {
+  if constexpr (CTAS == 2) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+    return;
+  }
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16_tc(uint32_t taddr, uint32_t (&r)[16]) {
