@@ -738,6 +738,7 @@ static int engine_finish_setup(qie_engine* e) {
       CU(maps(m.o, w.o, H, Dq));
       CU(make_tensor_map_2d(&m.gate.one, w.gate, (int)I, (int)H, 64));  // dual tile: 64 gate + 64 up rows
       CU(make_tensor_map_2d(&m.up.one, w.up, (int)I, (int)H, 64));
+      m.gate.p = w.gate, m.up.p = w.up;
       CU(maps(m.down, w.down, H, I));
     }
     CU(make_tensor_map_2d(&e->lm_head_map.one, e->lm_head, c.vocab, (int)H, 128));

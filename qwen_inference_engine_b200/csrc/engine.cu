@@ -94,6 +94,7 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
   for (int i = 0; i < nseg; ++i) {
     t.w[i] = &w[i]->one;
     if (epi != EPI_SILU_MUL) t.w2[i] = &w[i]->two;
+    else t.wp[i] = w[i]->p;  // (one map of both, made for the launch)
     t.rows[i] = rows[i];
   }
   t.x = x;

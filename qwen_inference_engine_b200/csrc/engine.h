@@ -92,6 +92,7 @@ struct qie_engine {
   // fast numerics (opts.numerics == QIE_NUMERICS_FAST)
   struct WeightMaps {
     qie::TensorMap2D one, two;  // boxes of 128 rows x one and two k-blocks of 64 (gate and up: 64 rows, one k-block)
+    const qie::bf16* p = nullptr;  // gate and up: the weights
   };
   struct LayerMaps {
     WeightMaps q, k, v, o, gate, up, down;

@@ -69,6 +69,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(c2)
       : "memory");
 }
+// gate and up as one matrix (make_tensor_map_gate_up)
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c1, int c3) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(0), "r"(c1), "r"(0), "r"(c3)
+      : "memory");
+}
 template <int CTAS = 1>
 __device__ __forceinline__ void tmem_alloc(uint32_t slot_smem, uint32_t cols) {
   if constexpr (CTAS == 2) {  // a warp of either CTA
@@ -131,7 +138,7 @@ struct TcArgs {
 };
 
 template <int BN, bool HALF, int KB, int TM, bool AHEAD>
-__global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
+__global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
                                                             const __grid_constant__ CUtensorMap map_x, TcArgs g) {
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map_w) : "memory");
-    if (g.dual) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
+    if (g.dual && KB == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init_tc(full_bar(s), 1);
@@ -190,7 +197,8 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
   auto load_w = [&](int i, int s) {
     const uint32_t sa = smem0 + s * STAGE_BYTES;
     if constexpr (KB > 1) {  // one request for the k-blocks of a stage (behind the matrix: zeros, which no product reads)
-      tma_load_3d(sa, map_w, full_bar(s), row0, kb0 + i * KB);
+      if (g.dual) tma_load_4d(sa, &map_w0, full_bar(s), row0, kb0 + i * KB);
+      else tma_load_3d(sa, map_w, full_bar(s), row0, kb0 + i * KB);
       return;
     }
     if (g.dual) {  // two 64-row boxes: gate rows -> lanes 0-63, up rows -> lanes 64-127
@@ -294,7 +302,7 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
     // contiguous run per token.  Rounding points are the reference's (R3 / R8 / R9).
     constexpr uint32_t PITCH = TM * 2;
     const uint32_t stg = smem0;
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 6) {
       const int qd = warp & 3;
       pdl_wait();  // `out` may still be read (residual) by the previous kernel
       if (nkb > 0) {
@@ -322,65 +330,67 @@ __global__ void __launch_bounds__(192) gemm_tcgen05_kernel(const __grid_constant
         }
       }
       tc_fence_before();
-      asm volatile("bar.sync 2, 128;" ::: "memory");  // the four epilogue warps
+    }
+    if (g.dual) __syncthreads();
+    else if (warp >= 2) asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that drain
+    const int n_tok = min(BN, g.M - tok_base);
+    if (g.dual) {
+      // gate rows sit in lanes 0-63, the matching up rows in lanes 64-127.  All eight warps: 64 tokens are 4096 SiLUs of some 40 instructions
+      pdl_wait();
+      const int total = n_tok * (BM / 8);
+      for (int c = threadIdx.x; c < total; c += blockDim.x) {
+        const int tok = c >> 4, part = c & 15;
+        const int w_row = row0 + part * 4;
+        if (w_row >= seg_rows) continue;
+        const uint32_t at = stg + (uint32_t)tok * PITCH + (uint32_t)part * 8u;
+        uint32_t gs[2], us[2], o2[2];
+        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(gs[0]), "=r"(gs[1]) : "r"(at) : "memory");
+        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(us[0]), "=r"(us[1]) : "r"(at + BM) : "memory");
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(silu_ref_f(lo2f(gs[e])))));
+          const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(silu_ref_f(hi2f(gs[e])))));
+          o2[e] = pack2(f2bf(a0), f2bf(a1));
+        }
+        *reinterpret_cast<uint2*>(out + (size_t)(tok_base + tok) * ld + w_row) = make_uint2(o2[0], o2[1]);
+      }
+    } else if (warp >= 2) {
       const int t = threadIdx.x - 64;
-      const int n_tok = min(BN, g.M - tok_base);
       auto lds128 = [](uint32_t addr) {
         uint4 v;
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
         return v;
       };
-      if (!g.dual) {
-        const int total = n_tok * (TM / 8);
-        for (int c = t; c < total; c += 4 * 128) {
-          uint4 y[4], x[4];
-          bf16* dst[4];
-          bool ok[4];
+      const int total = n_tok * (TM / 8);
+      for (int c = t; c < total; c += 4 * 128) {
+        uint4 y[4], x[4];
+        bf16* dst[4];
+        bool ok[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int cc = c + u * 128;
-            const int tok = cc >> (TM == 128 ? 4 : 3), part = cc & (TM / 8 - 1);
-            const int w_row = row0 + part * 8;
-            ok[u] = cc < total && w_row < seg_rows;
-            dst[u] = out + (size_t)(tok_base + tok) * ld + w_row;
-            if (ok[u]) {
-              y[u] = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
-              if (g.epi == EPI_RESIDUAL) x[u] = *reinterpret_cast<const uint4*>(dst[u]);
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (!ok[u]) continue;
-            if (g.epi == EPI_RESIDUAL) {
-              const uint32_t xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, ys[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
-              uint32_t o4[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                o4[e] = pack2(f2bf(__fadd_rn(lo2f(xs[e]), lo2f(ys[e]))), f2bf(__fadd_rn(hi2f(xs[e]), hi2f(ys[e]))));
-              *reinterpret_cast<uint4*>(dst[u]) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
-            } else {
-              *reinterpret_cast<uint4*>(dst[u]) = y[u];
-            }
+        for (int u = 0; u < 4; ++u) {
+          const int cc = c + u * 128;
+          const int tok = cc >> (TM == 128 ? 4 : 3), part = cc & (TM / 8 - 1);
+          const int w_row = row0 + part * 8;
+          ok[u] = cc < total && w_row < seg_rows;
+          dst[u] = out + (size_t)(tok_base + tok) * ld + w_row;
+          if (ok[u]) {
+            y[u] = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
+            if (g.epi == EPI_RESIDUAL) x[u] = *reinterpret_cast<const uint4*>(dst[u]);
           }
         }
-      } else {
-        // gate rows sit in lanes 0-63, the matching up rows in lanes 64-127
-        const int total = n_tok * (BM / 16);
-        for (int c = t; c < total; c += 128) {
-          const int tok = c >> 3, part = c & 7;
-          const int w_row = row0 + part * 8;
-          if (w_row >= seg_rows) continue;
-          const uint4 gt = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)part * 16u);
-          const uint4 up = lds128(stg + (uint32_t)tok * PITCH + (uint32_t)(BM / 2) * 2u + (uint32_t)part * 16u);
-          const uint32_t gs[4] = {gt.x, gt.y, gt.z, gt.w}, us[4] = {up.x, up.y, up.z, up.w};
-          uint32_t o4[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float a0 = __fmul_rn(lo2f(us[e]), bf2f(f2bf(silu_ref_f(lo2f(gs[e])))));
-            const float a1 = __fmul_rn(hi2f(us[e]), bf2f(f2bf(silu_ref_f(hi2f(gs[e])))));
-            o4[e] = pack2(f2bf(a0), f2bf(a1));
+        for (int u = 0; u < 4; ++u) {
+          if (!ok[u]) continue;
+          if (g.epi == EPI_RESIDUAL) {
+            const uint32_t xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, ys[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
+            uint32_t o4[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              o4[e] = pack2(f2bf(__fadd_rn(lo2f(xs[e]), lo2f(ys[e]))), f2bf(__fadd_rn(hi2f(xs[e]), hi2f(ys[e]))));
+            *reinterpret_cast<uint4*>(dst[u]) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+          } else {
+            *reinterpret_cast<uint4*>(dst[u]) = y[u];
           }
-          *reinterpret_cast<uint4*>(out + (size_t)(tok_base + tok) * ld + w_row) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
         }
       }
     }
@@ -871,6 +881,21 @@ cudaError_t make_tensor_map_w3d(TensorMap2D* out, const bf16* base, int rows, in
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// Two matrices of rows x K as one tensor {64 of a k-block, rows, which one, k-blocks}: a box is 64 rows of both, [k-block][which][row][64] in shared memory, so that
+// one request brings a gate/up tile's k-blocks.  Not supported where the second one does not lie behind the first, or 2^40 bytes away.
+static cudaError_t make_tensor_map_gate_up(TensorMap2D* out, const bf16* gate, const bf16* up, int rows, int K, int kb) {
+  EncodeTiledFn enc = get_encode();
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(gate), hi = reinterpret_cast<uintptr_t>(up);
+  if (!enc || K % 64 || (lo | hi) % 16 || hi <= lo || hi - lo >= 1ull << 40) return cudaErrorNotSupported;
+  cuuint64_t dims[4] = {64, (cuuint64_t)rows, 2, (cuuint64_t)(K / 64)};
+  cuuint64_t strides[3] = {(cuuint64_t)K * 2, (cuuint64_t)(hi - lo), 128};
+  cuuint32_t box[4] = {64, 64, 2, (cuuint32_t)kb};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)gate, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorNotSupported;
+}
+
 // KV pool [page][layer][k|v][head][slot][64] bf16 viewed as rows of 128 bytes (one head of one cached position).
 // One TMA request moves box_rows consecutive slots of a (page, layer, K|V, head) chunk into shared memory; the
 // 128-byte swizzle puts 16-byte chunk c of row r at chunk c ^ (r & 7), so that threads reading one row each
@@ -917,7 +942,7 @@ static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], 
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(g.n_tiles, g.splits, token_tiles);
-  cfg.blockDim = dim3(192);
+  cfg.blockDim = dim3(g.dual && g.staged ? 256 : 192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -1175,6 +1200,11 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
     for (int i = t.nseg; i < 3; ++i) w[i] = w[0];
     return true;
   };
+  auto gate_up = [&]() {  // one map of both
+    if (!t.wp[0] || !t.wp[1] || make_tensor_map_gate_up(&made[0], t.wp[0], t.wp[1], t.rows[0], t.K, 2) != cudaSuccess) return false;
+    for (int i = 0; i < 3; ++i) w[i] = reinterpret_cast<const CUtensorMap*>(&made[0]);
+    return true;
+  };
   if (launches) *launches = 1;
   // The MMA warp asks ahead for the next stage from 16 stages on, eight of 128 tokens (us without and with: 64 rows 4864 x 896 8.7 8.2, 8960 x 1536 14.3 13.6; 1000 rows
   // 15.5 14.5, 35.3 30.8; 1500 of 896 x 896 7.1 6.8; 4 stages of four k-blocks, 896 x 896, 3.7 4.0).  Not for gate/up (nothing) and clusters (few stages, or weights
@@ -1182,10 +1212,11 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   auto ahead = [&](int stage) { return g.splits == 1 && !g.dual && (g.kb_total + stage - 1) / stage >= (tl.bn == 128 ? 8 : 16); };
   // Two k-blocks a stage where tensor maps can express them (whole k-blocks, and the weights' place is known): half the requests, waits and commits.  Up
   // to 64 tokens: of 128 the ring holds three such stages, too few on the way (8960 x 1536 at 1000 rows 34.8 with stages of one, 37.1).  Gate/up tiles
-  // are two boxes a k-block as they are.  Not for 3 or 5 k-blocks: the half of the last stage that is not there is a box of zeros to bring, a quarter of
+  // take both matrices by one request (make_tensor_map_gate_up), one for three of stages of one: a request takes its warp 140 to 270 cycles (896 x 2 x 4864 behind a norm, 64 rows
+  // 7.7 -> 6.7 us; 24 layers in fast numerics, 16 rows, 963 -> 939 us a step.  Not for wider and persistent tiles, whose k-blocks take as long: 200 rows 310 312).  Not for 3 or 5 k-blocks: the half of the last stage that is not there is a box of zeros to bring, a quarter of
   // the operands (us with stages of one and of two, 1000 rows: 192 x 130 3.7 4.0, 320 x 130 4.3 4.6, 448 x 130 4.7 4.7, 576 x 130 4.5 4.2).
   const bool whole = g.splits > 1 || g.kb_total % 2 == 0 || g.kb_total > 5;
-  if (!tl.persist && tl.bn <= 64 && !g.dual && t.K % BK == 0 && g.kb_per_split >= 2 && whole && maps(true) &&
+  if (!tl.persist && tl.bn <= 64 && t.K % BK == 0 && g.kb_per_split >= 2 && whole && (g.dual ? gate_up() : maps(true)) &&
       make_tensor_map_w3d(&x, t.x, t.M, t.K, kb * BK, 0, tl.bn) == cudaSuccess)
     return tm == 64 ? launch_tile<4>(tl.bn, false, ahead(4), g, w, x, token_tiles, st) : launch_tile<2>(tl.bn, tl.half, ahead(2), g, w, x, token_tiles, st);
   if (tm != BM || !maps(false)) {
