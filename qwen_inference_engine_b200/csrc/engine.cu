@@ -199,6 +199,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.v_bias = w.v_bias;
       a.eps = e->eps;
       a.rope_half = e->rope_half ? 1 : 0;
+      a.early = 1;  // (the projections start when the norm lets them, which it does behind its own wait)
       QIE_TRY(KK_QKV_POST, launch_qkv_post(a, st));
     }
     capture_copy(e, "q", l, e->q, (size_t)n * Dq);

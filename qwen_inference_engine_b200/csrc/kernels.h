@@ -86,6 +86,7 @@ struct QkvPostArgs {
   const bf16 *q_bias = nullptr, *k_bias = nullptr, *v_bias = nullptr;
   float eps = 1e-04f;
   int rope_half = 0;
+  int early = 0;  // 1: the kernel in front writes nothing that this one reads but q_in, k and v, and starts when what is in front of its own predecessor has ended
 };
 cudaError_t launch_qkv_post(const QkvPostArgs& a, cudaStream_t st);
 
