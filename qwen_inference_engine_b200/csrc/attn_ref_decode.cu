@@ -184,7 +184,6 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
   }
   // Where the kernel in front of this one writes nothing but the queries and the row's own position (a.early), all else is read before it ends.
   if (!a.early) pdl_wait();
-  pdl_trigger();
   const int len = a.pos[b] + 1, ready = a.early ? len - 1 : len;  // positions that are there already
   bf16* const out = a.out + (size_t)b * a.n_q * HD + (size_t)h0 * HD;
   if (len <= 0) {  // no position: zeros, and no page to read
@@ -362,6 +361,7 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
       }
     }
     bar_compute();
+    pdl_trigger();
     // ---- values
     if (warp < units) {
       const int hu = warp / NP * pair, col = warp % NP * 64 + 2 * lane, nh = min(pair, hs - hu);

@@ -142,7 +142,6 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
                                                             const __grid_constant__ CUtensorMap map_x, TcArgs g) {
-  pdl_trigger();  // let the next kernel's CTAs get scheduled; they wait in their own pdl_wait()
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ int dead_s;
   volatile int* const dead = &dead_s;
@@ -240,6 +239,7 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
         load_x(i, s);
         if (++s == TC_STAGES) s = 0, ph ^= 1;
       }
+      pdl_trigger();  // (one thread's counts for the block)
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -572,7 +572,6 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
                                                                    const __grid_constant__ CUtensorMap map_w2,
                                                                    const __grid_constant__ CUtensorMap map_x, TcArgs g,
                                                                    int token_tiles) {
-  pdl_trigger();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ int dead_s;
   volatile int* const dead = &dead_s;
@@ -673,6 +672,7 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
           if (++s == stages) s = 0, ph ^= 1;
         }
       }
+      pdl_trigger();
     }
     __syncwarp();
   } else if (warp == 1) {

@@ -1,10 +1,14 @@
 // launch.h -- kernel launch helper with programmatic dependent launch (PDL).
 // Every kernel of the decode step starts with pdl_wait() (griddepcontrol.wait: all
 // prerequisite grids complete, their writes visible) before it touches global memory, and
-// calls pdl_trigger() (griddepcontrol.launch_dependents) right away so the NEXT kernel's
+// calls pdl_trigger() (griddepcontrol.launch_dependents) behind it so the NEXT kernel's
 // CTAs can be scheduled, set up their barriers/TMEM/tensor-map prefetch and -- for the
 // GEMMs -- start streaming weights while this kernel is still running, where shared memory holds CTAs of both (a GEMM's ring of 192 to 224 KB
-// lets it in beside a kernel of a few KB, or when CTAs of this one have left).  Launched without
+// lets it in beside a kernel of a few KB, or when CTAs of this one have left).  Never ahead of its own wait: then a third kernel comes in while the first one runs,
+// and every start and end of a step's graph takes longer (GEMMs and decode attention that did, us a step of 24 layers of 0.5B widths and now: 64 rows at 2048 positions 1784 -> 1713,
+// 48 at 300 1188 -> 1067, 16 at 500 1120 -> 996, 5 at 100 963 -> 895; 28 layers of 1.5B widths, 32 at 500 1856 -> 1760; fast numerics 1426 -> 1345, 931 -> 913).  A GEMM lets the next
+// one in when its last load is on its way (behind its wait: 16 rows 1021, 1.5B 1782), decode attention when the softmax is done (in front of it 1754 and 1092 with GEMMs as they
+// were, behind the softmax 1753 and 1067, at its end 1800 and 1128).  Launched without
 // the attribute both instructions are no-ops, so the same kernels work eagerly.
 #pragma once
 #include <cuda_runtime.h>
