@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "head_math.cuh"
 #include "kernels.h"
 #include "launch.h"
 #include "ref_math.cuh"
@@ -37,10 +38,10 @@ __host__ __device__ inline int score_pitch(int max_kv_len) { return (max_kv_len 
 struct Layout {
   int q, pages, score, k, v, total;  // byte offsets
 };
-__host__ __device__ inline Layout layout_of(int hd, int hp, int max_kv_len, int page_size, int stages) {
+__host__ __device__ inline Layout layout_of(int hd, int hp, int max_kv_len, int page_size, int stages, bool post) {
   Layout l;
-  l.q = HEADER;
-  l.pages = l.q + hp * hd * 2;
+  l.q = HEADER;  // the queries; behind them the row's own key and value (post)
+  l.pages = l.q + (hp + (post ? 2 : 0)) * hd * 2;
   l.score = l.pages + ((((max_kv_len + page_size - 1) / page_size) * 4 + 15) & ~15);
   l.k = (l.score + hp * score_pitch(max_kv_len) * 4 + 1023) & ~1023;  // (the copies' swizzle counts rows from there)
   l.v = l.k + NW * SLOT;
@@ -157,8 +158,11 @@ struct Weigh {
   }
 };
 
-template <int NP>
-__global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnArgs a, const int hp, const int stages, const int box, const __grid_constant__ CUtensorMap kvm) {
+// POST: the queries, the key and the value of the row come from the projections: bias, head norm and rotary position as in qkv_post_kernel (head_ops.cu), queries back in place,
+// key and value into the pool by the first part of a kv head.  The last position's key and value are read from shared memory, all others from the pool.
+template <int NP, bool POST>
+__global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnArgs a, const int hp, const int stages, const int box, const __grid_constant__ CUtensorMap kvm,
+                                                                     const QkvPostArgs post) {
   constexpr int HD = 64 * NP, RW = 2 / NP, GK = 32 * RW, ROW = HD * 2, WORDS = 32 * NP, TV = VTILE / ROW;
   extern __shared__ __align__(1024) unsigned char smem[];
   volatile int* const dead = reinterpret_cast<volatile int*>(smem + OFF_DEAD);
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
   const int G = a.n_q / a.kv.n_kv, parts = (G + hp - 1) / hp;
   const int kvh = blockIdx.x / parts, part = blockIdx.x - kvh * parts, b = blockIdx.y;
   const int h0 = kvh * G + part * hp, hs = min(hp, G - part * hp);
-  const Layout lay = layout_of(HD, hp, a.max_kv_len, a.kv.page_size, stages);
+  const Layout lay = layout_of(HD, hp, a.max_kv_len, a.kv.page_size, stages, POST);
   const uint32_t bars = smem_u32(smem);  // full and empty of the values' stages, full of the warps' keys
   auto vfull = [&](int s) { return bars + 8 * s; };
   auto vempty = [&](int s) { return bars + 8 * (MAX_STAGES + s); };
@@ -184,7 +188,9 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
   }
   // Where the kernel in front of this one writes nothing but the queries and the row's own position (a.early), all else is read before it ends.
   if (!a.early) pdl_wait();
-  const int len = a.pos[b] + 1, ready = a.early ? len - 1 : len;  // positions that are there already
+  const int len = a.pos[b] + 1, ready = a.early && !POST ? len - 1 : len;  // positions that are there already, or are not read
+  const int kept = POST ? len - 1 : len;                                    // positions whose values come from the pool
+  unsigned char* const own = smem + lay.q + hp * HD * 2;                    // (POST) the row's key, then its value
   bf16* const out = a.out + (size_t)b * a.n_q * HD + (size_t)h0 * HD;
   if (len <= 0) {  // no position: zeros, and no page to read
     if (a.early) pdl_wait();
@@ -206,8 +212,8 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
     int s = 0;
     uint32_t ph = 1;  // (the first pass over the ring waits for nothing)
     bool waits = a.early;
-    for (int k0 = 0; k0 < len; k0 += TV) {
-      const int n = min(TV, len - k0);
+    for (int k0 = 0; k0 < kept; k0 += TV) {
+      const int n = min(TV, kept - k0);
       if (waits && k0 + n > ready) pdl_wait(), waits = false;
       if (!mbar_wait_tc(vempty(s), ph, dead)) break;
       const uint32_t full = vfull(s), dst = smem_u32(smem + lay.v + s * VTILE);
@@ -241,16 +247,58 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
       }
     };
     const bool asked = warp < ng && (warp + 1) * GK <= ready;
-    if (asked) copy(warp);
-    if (a.early) pdl_wait();
-    if (!asked && warp < ng) copy(warp);
+    if (asked || (POST && warp < ng)) copy(warp);
     // queries in the tree's order: quad u is pairs m0, m0 + half, m1, m1 + half of leaves 2 u and 2 u + 1
+    constexpr int BITS = NP == 1 ? 4 : 5;
     Magnitudes mag;
-    for (int i = tid; i < hs * WORDS; i += NW * 32) {
-      const int h = i / WORDS, e = i % WORDS, leaf = e >> 1;
-      const uint32_t w = *reinterpret_cast<const uint32_t*>(a.q + (size_t)b * a.n_q * HD + (size_t)(h0 + h) * HD + 2 * (brev(leaf, NP == 1 ? 4 : 5) + (e & 1) * 16 * NP));
-      mag.see(w);
-      reinterpret_cast<uint32_t*>(smem + lay.q)[i] = w;
+    if constexpr (POST) {
+      using Hd = Head<NP>;
+      const int at = tid / Hd::LH, l = tid % Hd::LH, kind = at < hs ? 0 : at == hs ? 1 : 2;  // a head of the CTA: queries, the key, the value
+      const int ps = len - 1;
+      const bf16 *bias = kind == 0 ? post.q_bias : kind == 1 ? post.k_bias : post.v_bias, *w = kind == 0 ? post.q_norm_w : post.k_norm_w;
+      const float *co = post.cos_t + (size_t)ps * Hd::HALF, *si = post.sin_t + (size_t)ps * Hd::HALF;
+      if (at <= hs) {  // (on their way while the projections run)
+        const int first = post.rope_half ? 8 * l : 4 * l, second = post.rope_half ? 8 * l + 4 : Hd::HALF / 2 + 4 * l;
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(co + first)));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(co + second)));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(si + first)));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(si + second)));
+      }
+      pdl_wait();
+      if (warp * 32 / Hd::LH <= hs + 1) {  // (whole warps: the sum of squares is an exchange)
+        const bf16* src = kind == 0 ? post.q_in + (size_t)b * post.q_in_stride + (size_t)(h0 + at) * HD : (kind == 1 ? post.k : post.v) + (size_t)b * post.kv_stride + (size_t)kvh * HD;
+        const size_t head = kind == 0 ? h0 + at : kvh;
+        Hd x;
+        x.template load<true>(src, l);
+        if (bias) x.template add_bias<true>(bias + head * HD, l);
+        const float sum = x.squares();
+        if (kind != 2) {
+          if (w) x.template norm<true>(sum, w, l, post.eps);
+          if (post.rope_half) x.template rope_half<true>(co, si, l);
+          else x.template rope<true>(co, si, l);
+        }
+        if (kind == 0) {
+          x.template store<true>(post.q + (size_t)b * a.n_q * HD + head * HD, l);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t pair = pack2f(x.x[2 * j], x.x[2 * j + 1]);
+            mag.see(pair);
+            reinterpret_cast<uint32_t*>(smem + lay.q)[at * WORDS + 2 * (int)(__brev(4 * l + j % 4) >> (32 - BITS)) + j / 4] = pair;
+          }
+        } else if (at <= hs + 1) {
+          x.template store<true>(reinterpret_cast<bf16*>(own) + (kind - 1) * HD, l);
+          if (part == 0) x.template store<true>(a.kv.chunk(pages[ps / psz], a.layer, kind - 1, kvh) + (size_t)(ps % psz) * HD, l);
+        }
+      }
+    } else {
+      if (a.early) pdl_wait();
+      if (!asked && warp < ng) copy(warp);
+      for (int i = tid; i < hs * WORDS; i += NW * 32) {
+        const int h = i / WORDS, e = i % WORDS, leaf = e >> 1;
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(a.q + (size_t)b * a.n_q * HD + (size_t)(h0 + h) * HD + 2 * (brev(leaf, BITS) + (e & 1) * 16 * NP));
+        mag.see(w);
+        reinterpret_cast<uint32_t*>(smem + lay.q)[i] = w;
+      }
     }
     const bool q_beyond = bar_or(mag.beyond());
     const Quot den = quot_of(__fsqrt_rn((float)HD));
@@ -266,9 +314,10 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
         uint32_t row = 0xffffffffu;
+        const bool is_own = POST && g * GK + 32 * r + lane == len - 1;
 #pragma unroll
         for (int c = 0; c < 8 * NP; ++c) {
-          const uint4 t = *reinterpret_cast<const uint4*>(slot + c / 8 * GK * 128 + (lane + 32 * r) * 128 + ((c % 8 ^ (lane & 7)) << 4));
+          const uint4 t = *reinterpret_cast<const uint4*>(is_own ? own + 16 * c : slot + c / 8 * GK * 128 + (lane + 32 * r) * 128 + ((c % 8 ^ (lane & 7)) << 4));
           const uint32_t w[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) k[r][4 * c + i] = w[i], row &= w[i] ^ (w[i] << 1);
@@ -373,15 +422,16 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
         uint32_t ph = 0;
         Weigh<decltype(heads)::value, ROW> w;
 #pragma unroll 1
-        for (int k0 = 0; k0 < len; k0 += TV) {
+        for (int k0 = 0; k0 < kept; k0 += TV) {
           if (!mbar_wait_tc(vfull(s), ph, dead)) break;
           const unsigned char* v = smem + lay.v + s * VTILE + col * 2;
-          if (k0 + TV <= len) w.template all<TV>(v, p0 + k0, p1 + k0, o);
-          else w.some(v, p0 + k0, p1 + k0, len - k0, o);
+          if (k0 + TV <= kept) w.template all<TV>(v, p0 + k0, p1 + k0, o);
+          else w.some(v, p0 + k0, p1 + k0, kept - k0, o);
           __syncwarp();
           if (lane == 0) mbar_arrive_tc(vempty(s));
           if (++s == stages) s = 0, ph ^= 1;
         }
+        if constexpr (POST) w.some(own + HD * 2 + col * 2, p0 + kept, p1 + kept, 1, o);
       };
       if (pair == 2) go(std::integral_constant<int, 2>{});
       else go(std::integral_constant<int, 1>{});
@@ -401,8 +451,7 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
 
 }  // namespace
 
-// Heads of a CTA, 0 where this kernel does not take the call.
-int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages) {
+static int heads_of(const AttnArgs& a, int num_sms, int* stages, bool post) {
   const int G = a.n_q / a.kv.n_kv, hd = a.kv.hd;
   auto at16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if ((hd != 64 && hd != 128) || a.k_pages || a.kv.page_size % 8 || !at16(a.kv.pool) || !at16(a.q) || !at16(a.out)) return 0;
@@ -412,16 +461,16 @@ int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages) {
   while (parts < G && (long)tasks * (parts + 1) <= num_sms) ++parts;
   for (int hp = (G + parts - 1) / parts; hp >= 1; --hp)
     for (int st = MAX_STAGES; st >= 2; --st)
-      if (layout_of(hd, hp, a.max_kv_len, a.kv.page_size, st).total <= 226 * 1024) {
+      if (layout_of(hd, hp, a.max_kv_len, a.kv.page_size, st, post).total <= 226 * 1024) {
         *stages = st;
         return hp;
       }
   return 0;
 }
 
-cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages, cudaStream_t st) {
+static cudaError_t launch_decode(const AttnArgs& a, int heads, int stages, const QkvPostArgs* post, cudaStream_t st) {
   const int G = a.n_q / a.kv.n_kv, parts = (G + heads - 1) / heads;
-  const size_t smem = layout_of(a.kv.hd, heads, a.max_kv_len, a.kv.page_size, stages).total;
+  const size_t smem = layout_of(a.kv.hd, heads, a.max_kv_len, a.kv.page_size, stages, post != nullptr).total;
   int box = 8;  // rows of a copy: as many as a page and a group hold
   while (a.kv.page_size % (2 * box) == 0 && 2 * box * a.kv.hd * 2 <= SLOT) box *= 2;
   TensorMap2D kvm;
@@ -433,10 +482,31 @@ cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages
       if (e != cudaSuccess) return e;
       set.done();
     }
-    return launch_k(kernel, dim3(parts * a.kv.n_kv, a.n_tok), dim3(NT), smem, st, a, heads, stages, box, *reinterpret_cast<const CUtensorMap*>(&kvm));
+    return launch_k(kernel, dim3(parts * a.kv.n_kv, a.n_tok), dim3(NT), smem, st, a, heads, stages, box, *reinterpret_cast<const CUtensorMap*>(&kvm), post ? *post : QkvPostArgs{});
   };
-  static PerDeviceOnce set[2];
-  return a.kv.hd == 64 ? go(attention_ref_decode_kernel<1>, set[0]) : go(attention_ref_decode_kernel<2>, set[1]);
+  static PerDeviceOnce set[3];
+  if (post) return go(attention_ref_decode_kernel<1, true>, set[2]);
+  return a.kv.hd == 64 ? go(attention_ref_decode_kernel<1, false>, set[0]) : go(attention_ref_decode_kernel<2, false>, set[1]);
+}
+
+// Heads of a CTA, 0 where this kernel does not take the call.
+int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages) { return heads_of(a, num_sms, stages, false); }
+
+cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages, cudaStream_t st) { return launch_decode(a, heads, stages, nullptr, st); }
+
+// What launch_qkv_post and this kernel do, in one launch: the store and the way back of the queries and a start of a kernel less, and the keys of a step are
+// asked for while the projections run.  us a step of 24 layers, 14 heads of 64 on 2, two launches and one: 64 rows at 2048 positions 1712 1693, 16 at 500 994 971, 5 at 100 892
+// 860.  Heads of 128 keep two: 28 layers, 12 heads on 2, 32 rows at 500 1759 1777, 8 at 100 1457 1488, 16 at 1000 1870 1906 (64 at 300 1834 1821).  Nor where a row or a
+// table is off a 16-byte boundary (*taken false, nothing launched).
+cudaError_t launch_attention_ref_post(const AttnArgs& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st) {
+  uintptr_t at = 0;
+  for (const void* q : {(const void*)p.q, (const void*)p.q_in, (const void*)p.k, (const void*)p.v, (const void*)p.q_norm_w, (const void*)p.k_norm_w, (const void*)p.cos_t,
+                        (const void*)p.sin_t, (const void*)p.q_bias, (const void*)p.k_bias, (const void*)p.v_bias})
+    at |= reinterpret_cast<uintptr_t>(q);
+  int stages = 0, heads = 0;
+  if (a.kv.hd == 64 && a.decode && a.early && a.n_tok > 0 && at % 16 == 0 && p.q_in_stride % 8 == 0 && p.kv_stride % 8 == 0) heads = heads_of(a, num_sms, &stages, true);
+  *taken = heads > 0;
+  return heads ? launch_decode(a, heads, stages, &p, st) : cudaSuccess;
 }
 
 }  // namespace qie

@@ -126,7 +126,7 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
 // Launch order = llm()'s (qwen_main.cu:77-222 prefill / :271-365 decode): per layer
 // rms -> q,k,v -> q/k-norm -> RoPE -> KV store -> attention -> o (+residual) -> rms ->
 // up,gate -> SiLU*up -> down (+residual); then final norm -> lm_head -> sampling.
-// 18 kernels + 2-4 memcpys per layer in the reference become 8 launches here.
+// 18 kernels + 2-4 memcpys per layer in the reference become 8 launches here (7 in a decode step in the reference's order with heads of 64).
 cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int n_out, float temperature,
                          bool advance) {
   if (e->tp.size > 1) return forward_rows_tp(e, n, max_kv_len, out_row0, n_out, temperature, advance);
@@ -167,8 +167,9 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       cudaError_t r = gemm_rows(e, KK_GEMM_QKV, g, n);
       if (r != cudaSuccess) return r;
     }
+    QkvPostArgs post{};
     {
-      QkvPostArgs a{};
+      QkvPostArgs& a = post;
       a.q = e->q;
       if (tc) {
         a.q_in = e->qkv;
@@ -200,8 +201,33 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.eps = e->eps;
       a.rope_half = e->rope_half ? 1 : 0;
       a.early = 1;  // (the projections start when the norm lets them, which it does behind its own wait)
-      QIE_TRY(KK_QKV_POST, launch_qkv_post(a, st));
     }
+    AttnArgs ra{};  // reference-order attention
+    bool posted = false;
+    if (!fast) {
+      AttnArgs& a = ra;
+      a.q = e->q;
+      a.out = e->att;
+      a.pos = e->pos_d;
+      a.slot = e->slot_d;
+      a.block_table = e->block_table_d;
+      a.max_pages = e->max_pages_per_seq;
+      a.n_tok = n;
+      a.n_q = c.n_q;
+      a.layer = l;
+      a.max_kv_len = max_kv_len;
+      a.kv = e->kv;
+      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
+      a.decode = a.early = advance;
+      a.status = e->wait_status;
+      // a decode step's head norms, positions and store belong to the attention kernel, unless somebody looks between the two
+      if (advance && !e->capture && !e->prof_on) {
+        const cudaError_t r = launch_attention_ref_post(a, post, e->num_sms, &posted, st);
+        if (r != cudaSuccess) return r;
+        if (posted) ++e->launches;
+      }
+    }
+    if (!posted) QIE_TRY(KK_QKV_POST, launch_qkv_post(post, st));
     capture_copy(e, "q", l, e->q, (size_t)n * Dq);
     if (!tc) capture_copy(e, "v", l, e->v, (size_t)n * Dkv);
     if (fast_attn) {
@@ -248,23 +274,8 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
         QIE_TRY(KK_ATTN, launch_attention_prefill_tc(a, st));
       else
         QIE_TRY(KK_ATTN, launch_attention_prefill_fast(a, st));
-    } else {
-      AttnArgs a{};
-      a.q = e->q;
-      a.out = e->att;
-      a.pos = e->pos_d;
-      a.slot = e->slot_d;
-      a.block_table = e->block_table_d;
-      a.max_pages = e->max_pages_per_seq;
-      a.n_tok = n;
-      a.n_q = c.n_q;
-      a.layer = l;
-      a.max_kv_len = max_kv_len;
-      a.kv = e->kv;
-      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
-      a.decode = a.early = advance;
-      a.status = e->wait_status;
-      QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
+    } else if (!posted) {
+      QIE_TRY(KK_ATTN, launch_attention_ref(ra, st));
     }
     capture_copy(e, "attn", l, e->att, (size_t)n * Dq);
     if (tc) {
