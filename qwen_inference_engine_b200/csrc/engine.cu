@@ -539,15 +539,14 @@ bool decode_uses_mega(const qie_engine* e, int n, int max_kv_len) {
                               e->mega_kc[mega_tile_set(e, nb, max_kv_len)], fast, e->kv.page_size);
 }
 
-// Steps in the reference's order that are quicker by operators than in the persistent kernel.  That kernel walks one (row, kv head) per SM through chains that wait for
-// one another and streams every phase's operands by itself; the operators have their products on tcgen05 and attn_ref_decode.cu.  us a step in graphs, persistent
-// kernel and operators: 0.5B, 24 layers, 64 rows at 2000 positions 2894 and 1928, at 500 2087 and 1402; 16 rows at 100 1580 and 1170; 8 at 32 1162 and 1127; 4 at 300
-// (8 layers) 458 and 445, at 60 418 and 421; 1 at 2000 1869 and 1596, at 500 1233 and 1221, at 32 986 and 1087.  1.5B, 8 layers: 1 at 32 606 and 605, 32 at 300
-// 1100 and 679.  7B, 4 layers: 1 at 32 893 and 730, 16 at 2000 1491 and 901.  Rows of 128 to 256: 1 at 16 123 and 113, 126 and 125.
+// Steps in the reference's order are quicker by operators than in the persistent kernel wherever attn_ref_decode.cu takes them.  That kernel walks one (row, kv head) per SM through chains
+// that wait for one another and streams every phase's operands by itself; the operators have their products on tcgen05 and that attention.  us a step in graphs,
+// persistent kernel and operators: 0.5B, 24 layers, 64 rows at 2000 positions 2894 and 1690; 8 at 200 1254 and 890, at 30 1163 and 829; 4 at 250 1210 and 907, at 30 1091 and
+// 826; 2 at 100 1069 and 856; 1 at 1000 1463 and 1091, at 300 1139 and 921, at 30 997 and 862.  1.5B, 28 layers: 4 at 300 2271 and 1525, 1 at 30 1855 and 1444.  7B, 4 layers: 1
+// at 32 893 and 730, 16 at 2000 1491 and 901.  Rows of 128 to 256: 1 at 16 123 and 113, 126 and 125.
 bool decode_by_operators(const qie_engine* e, int n, int max_kv_len) {
   const qie_config& c = e->cfg;
   if (e->mega_always || e->mega_prof_on || e->mega_layers_run > 0 || e->tp.size > 1 || e->opts.numerics == QIE_NUMERICS_FAST) return false;
-  if (n <= 4 && max_kv_len <= 384 && c.hidden > 256 && c.hidden < 1536) return false;
   AttnArgs a{};
   a.q = e->q;
   a.out = e->att;
