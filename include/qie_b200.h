@@ -395,8 +395,8 @@ int qie_profile_begin(qie_engine* e);
 int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int n_kinds);
 
 /* Persistent decode kernel (decode_mega.cu): a reference-order decode step of up to 64 rows
- * as ONE cooperative launch.  By default a step runs so only where the operators are not
- * quicker (the same bits either way).  qie_engine_set_int keys: "mega" (0: never, 1: wherever
+ * as ONE cooperative launch.  By default a step runs so only where the operators do not
+ * take it (tensor parallel, very long contexts; the same bits either way).  qie_engine_set_int keys: "mega" (0: never, 1: wherever
  * the kernel takes the step; QIE_MEGA=0 is the former), "mega_layers_run" (debug: stop after N layers, 0 = whole step), "mega_prof"
  * (0/1: record a device timestamp at every phase boundary, in the persistent kernel).
  * qie_decode_uses_mega tells whether the kernel takes a step of n rows at this KV length.
