@@ -137,8 +137,9 @@ struct TcArgs {
   TcSeg seg[3];
 };
 
-template <int BN, bool HALF, int KB, int TM, bool AHEAD>
-__global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
+// DUAL: gate/up tiles (EPI_SILU_MUL), instantiations of their own: with their epilogue in the others' code each product took 0.1 to 0.2 us more (us, 128 rows of 896 x 4864 5.06 4.91, of 1536 x 8960 7.17 6.87, prompts of 300 rows of 1.5B widths, four layers, 457 446).
+template <int BN, bool HALF, int KB, int TM, bool AHEAD, bool DUAL>
+__global__ void __launch_bounds__(DUAL ? 256 : 192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
                                                             const __grid_constant__ CUtensorMap map_x, TcArgs g) {
@@ -166,8 +167,8 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
   int si = 0;
   while (si + 1 < g.nseg && tile >= g.seg[si + 1].tile0) ++si;
   // dual (gate/up): one tile = 64 gate rows + the same 64 up rows; segment 0 = gate map, 1 = up map
-  const CUtensorMap* map_w = g.dual ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
-  const int row0 = g.dual ? tile * (BM / 2) : (tile - g.seg[si].tile0) * TM;
+  const CUtensorMap* map_w = DUAL ? &map_w0 : (si == 0 ? &map_w0 : (si == 1 ? &map_w1 : &map_w2));
+  const int row0 = DUAL ? tile * (BM / 2) : (tile - g.seg[si].tile0) * TM;
   const int seg_rows = g.seg[si].rows, ld = g.seg[si].ld;
   bf16* const out = g.seg[si].out;
   const int kb0 = split * g.kb_per_split;
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
 
   if (warp == 0 && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(map_w) : "memory");
-    if (g.dual && KB == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
+    if (DUAL && KB == 1) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w1) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init_tc(full_bar(s), 1);
@@ -196,11 +197,11 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
   auto load_w = [&](int i, int s) {
     const uint32_t sa = smem0 + s * STAGE_BYTES;
     if constexpr (KB > 1) {  // one request for the k-blocks of a stage (behind the matrix: zeros, which no product reads)
-      if (g.dual) tma_load_4d(sa, &map_w0, full_bar(s), row0, kb0 + i * KB);
+      if constexpr (DUAL) tma_load_4d(sa, &map_w0, full_bar(s), row0, kb0 + i * KB);
       else tma_load_3d(sa, map_w, full_bar(s), row0, kb0 + i * KB);
       return;
     }
-    if (g.dual) {  // two 64-row boxes: gate rows -> lanes 0-63, up rows -> lanes 64-127
+    if (DUAL) {  // two 64-row boxes: gate rows -> lanes 0-63, up rows -> lanes 64-127
       tma_load_2d(sa, &map_w0, full_bar(s), (kb0 + i) * BK, row0);
       tma_load_2d(sa + A_BYTES / 2, &map_w1, full_bar(s), (kb0 + i) * BK, row0);
     } else {
@@ -331,10 +332,10 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
       }
       tc_fence_before();
     }
-    if (g.dual) __syncthreads();
+    if constexpr (DUAL) __syncthreads();
     else if (warp >= 2) asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that drain
     const int n_tok = min(BN, g.M - tok_base);
-    if (g.dual) {
+    if constexpr (DUAL) {
       // gate rows sit in lanes 0-63, the matching up rows in lanes 64-127.  All eight warps: 64 tokens are 4096 SiLUs of some 40 instructions
       pdl_wait();
       const int total = n_tok * (BM / 8);
@@ -410,8 +411,8 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
   const uint32_t red = smem0;
   const bool epi_warp = warp >= 2;
   const int qd = warp & 3;  // TMEM lane quarter of this epilogue warp
-  const bool via_smem = g.splits > 1 || g.dual;
-  const int tile_rows = g.dual ? BM / 2 : TM;  // output rows produced by this tile
+  const bool via_smem = g.splits > 1 || DUAL;
+  const int tile_rows = DUAL ? BM / 2 : TM;  // output rows produced by this tile
   const int rows_per = ((tile_rows + g.splits - 1) / g.splits + 3) & ~3;
   const uint32_t pitch = (uint32_t)(BM + min(rows_per, 32)) * 4u;
   if (epi_warp) {
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
         for (int sp = 0; sp < MAXS; ++sp)
           if (sp < S) {
             ld4(sp, off, v[sp]);
-            if (g.dual) ld4(sp, off + (uint32_t)(BM / 2) * 4u, v2[sp]);  // the up half of the tile
+            if (DUAL) ld4(sp, off + (uint32_t)(BM / 2) * 4u, v2[sp]);  // the up half of the tile
           }
         bf16* dst = out + (size_t)(tok_base + tok) * ld + w_row;
         float old[4] = {0.f, 0.f, 0.f, 0.f};
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(256) gemm_tcgen05_kernel(const __grid_constant
           for (int sp = 0; sp < MAXS; ++sp)
             if (sp < S) {  // rank order
               acc += v[sp][e];
-              if (g.dual) acc2 += v2[sp][e];
+              if (DUAL) acc2 += v2[sp][e];
             }
           if (g.epi == EPI_STORE) {
             y[e] = f2bf(acc);
@@ -928,21 +929,21 @@ cudaError_t make_tensor_map_pages(TensorMap2D* out, const bf16* base, int row_el
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int BN, bool HALF, int KB, int TM, bool AHEAD>
+template <int BN, bool HALF, int KB, int TM, bool AHEAD, bool DUAL = false>
 static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int STAGE_BYTES = KB * (TM * BK * 2 + BN * BK * 2);
   constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB, TM>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
   static PerDeviceOnce set;
   if (set.need()) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD, DUAL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     set.done();
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(g.n_tiles, g.splits, token_tiles);
-  cfg.blockDim = dim3(g.dual && g.staged ? 256 : 192);
+  cfg.blockDim = dim3(DUAL && g.staged ? 256 : 192);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[2];
@@ -961,7 +962,7 @@ static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], 
   }
   cfg.attrs = at;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
+  return cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD, DUAL>, *w[0], *w[1], *w[2], *reinterpret_cast<const CUtensorMap*>(&x), g);
 }
 
 template <int KB>
@@ -969,12 +970,14 @@ static cudaError_t launch_tile(int bn, bool half, bool ahead, const TcArgs& g, c
   constexpr int TM = KB == 4 ? 64 : BM;
   auto go = [&](auto n) {
     constexpr int BN = decltype(n)::value;
+    if constexpr (KB < 4)
+      if (g.dual) return launch_bn<BN, false, KB, TM, false, true>(g, w, x, token_tiles, st);
     if constexpr (KB > 1 || BN == 128)
       if (ahead) return launch_bn<BN, false, KB, TM, true>(g, w, x, token_tiles, st);
     return launch_bn<BN, false, KB, TM, false>(g, w, x, token_tiles, st);
   };
   if constexpr (KB != 4)
-    if (half) return launch_bn<16, true, KB, TM, false>(g, w, x, token_tiles, st);
+    if (half) return g.dual ? launch_bn<16, true, KB, TM, false, true>(g, w, x, token_tiles, st) : launch_bn<16, true, KB, TM, false>(g, w, x, token_tiles, st);
   switch (bn) {
     case 16: return go(std::integral_constant<int, 16>{});
     case 32: return go(std::integral_constant<int, 32>{});
