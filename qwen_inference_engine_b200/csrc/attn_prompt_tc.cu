@@ -431,19 +431,25 @@ cudaError_t launch_hd(const FastAttnArgs& a, int two_term, const TensorMap2D& kv
   return cudaLaunchKernelEx(&cfg, attn_prompt_tc_kernel<HD>, a, two_term, parts, alone, *reinterpret_cast<const CUtensorMap*>(&kvm));
 }
 
-__global__ void wait_selftest_kernel(int* status) {
+// a pair of CTAs: the wait is the first one's, the report the other one's
+__global__ void __cluster_dims__(2) wait_selftest_kernel(int* status) {
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int dead_s;
-  dead_s = 0;
-  mbar_init_tc(smem_u32(&bar), 1);
-  mbar_wait_tc(smem_u32(&bar), 0, &dead_s);
-  report_tc(&dead_s, status);
+  const bool one = threadIdx.x == 0;
+  if (one) dead_s = 0, mbar_init_tc(smem_u32(&bar), 1);
+  cluster_sync_all();
+  if (blockIdx.x == 0 && one) {
+    mbar_wait_tc(smem_u32(&bar), 0, &dead_s);
+    tell_other_tc(&dead_s);
+  }
+  cluster_sync_all();
+  if (blockIdx.x == 1 && one) report_tc(&dead_s, status);
 }
 
 }  // namespace
 
 cudaError_t launch_wait_selftest(int* status, cudaStream_t st) {
-  wait_selftest_kernel<<<1, 1, 0, st>>>(status);
+  wait_selftest_kernel<<<2, 32, 0, st>>>(status);
   return cudaGetLastError();
 }
 

@@ -699,7 +699,10 @@ __global__ void __launch_bounds__(P_THREADS) gemm_tcgen05_persist_kernel(const _
         __syncwarp();
         if (++s == stages) s = 0, ph ^= 1;
       }
-      if (elect_tc()) umma_commit_tc<CTAS>(tfull_bar(buf));
+      if (elect_tc()) {
+        if (CTAS > 1) tell_other_tc(dead);
+        umma_commit_tc<CTAS>(tfull_bar(buf));
+      }
       __syncwarp();
     }
   } else {

@@ -50,6 +50,18 @@ __device__ __forceinline__ void drain_tc(const volatile int* dead) {
   if (*dead)
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
 }
+// For pairs of CTAs that work on one tile: a wait that ran out in this one counts for the other one too, whose results hang on this one's operands.  One thread, ahead of the
+// arrival that lets the other one go on; the word is read back, so it is there before that arrival.
+__device__ __forceinline__ void tell_other_tc(volatile int* dead) {
+  if (!*dead) return;
+  uint32_t rank, there;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(const_cast<int*>(dead))), "r"(rank ^ 1u));
+  asm volatile("st.volatile.shared::cluster.u32 [%0], 1;" ::"r"(there) : "memory");
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  asm volatile("{\n\t.reg .b32 seen;\n\tld.volatile.shared::cluster.u32 seen, [%0];\n\t}" ::"r"(there) : "memory");
+  asm volatile("fence.acq_rel.cluster;" ::: "memory");
+}
 // one thread, behind the CTA's last wait: status is a word that the host reads (mapped memory), or null
 __device__ __forceinline__ void report_tc(const volatile int* dead, int* status) {
   if (*dead && status) {

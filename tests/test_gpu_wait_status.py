@@ -1,5 +1,6 @@
 """A wait inside a kernel that runs out (csrc/tc_ptx.cuh) is an error of the call that learns of it, once, and the context stays usable.  The
-self-test's wait is on a barrier that nothing completes, through the limit and the report that the tcgen05 kernels use."""
+self-test's wait is on a barrier that nothing completes, through the limit and the report that the tcgen05 kernels use.  It is a pair of CTAs as the GEMM's are: the
+first one waits and the other one, which waits for nothing, reports what it was told (tell_other_tc)."""
 import numpy as np
 import pytest
 import torch
