@@ -137,9 +137,12 @@ struct TcArgs {
   TcSeg seg[3];
 };
 
-// DUAL: gate/up tiles (EPI_SILU_MUL), instantiations of their own: with their epilogue in the others' code each product took 0.1 to 0.2 us more (us, 128 rows of 896 x 4864 5.06 4.91, of 1536 x 8960 7.17 6.87, prompts of 300 rows of 1.5B widths, four layers, 457 446).
+// DUAL: gate/up tiles (EPI_SILU_MUL), instantiations of their own: with their epilogue in the others' code each product took 0.1 to 0.2 us more (us, 128 rows of
+// 896 x 4864 5.06 4.91, of 1536 x 8960 7.17 6.87, prompts of 300 rows of 1.5B widths, four layers, 457 446).  The epilogue of the others stays in one branch, and the compiler is told
+// that one CTA an SM is enough: without the two, tiles of 64 tokens took 0.1 us more (us in graphs of twenty alike, without, with: 1000 rows of 896 x 896 5.10 4.97, 128 of 896 x 4864 5.01
+// 4.88, 512 of 1536 x 1536 6.75 6.61; a decode step of 16 sequences at 500 positions 978 971).
 template <int BN, bool HALF, int KB, int TM, bool AHEAD, bool DUAL>
-__global__ void __launch_bounds__(DUAL ? 256 : 192) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
+__global__ void __launch_bounds__(DUAL ? 256 : 192, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w0,
                                                             const __grid_constant__ CUtensorMap map_w1,
                                                             const __grid_constant__ CUtensorMap map_w2,
                                                             const __grid_constant__ CUtensorMap map_x, TcArgs g) {
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(DUAL ? 256 : 192) gemm_tcgen05_kernel(const __
     // contiguous run per token.  Rounding points are the reference's (R3 / R8 / R9).
     constexpr uint32_t PITCH = TM * 2;
     const uint32_t stg = smem0;
-    if (warp >= 2 && warp < 6) {
+    auto drain = [&]() {  // four warps
       const int qd = warp & 3;
       pdl_wait();  // `out` may still be read (residual) by the previous kernel
       if (nkb > 0) {
@@ -331,14 +334,13 @@ __global__ void __launch_bounds__(DUAL ? 256 : 192) gemm_tcgen05_kernel(const __
         }
       }
       tc_fence_before();
-    }
-    if constexpr (DUAL) __syncthreads();
-    else if (warp >= 2) asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that drain
-    const int n_tok = min(BN, g.M - tok_base);
+    };
     if constexpr (DUAL) {
+      if (warp >= 2 && warp < 6) drain();
+      __syncthreads();
       // gate rows sit in lanes 0-63, the matching up rows in lanes 64-127.  All eight warps: 64 tokens are 4096 SiLUs of some 40 instructions
       pdl_wait();
-      const int total = n_tok * (BM / 8);
+      const int total = min(BN, g.M - tok_base) * (BM / 8);
       for (int c = threadIdx.x; c < total; c += blockDim.x) {
         const int tok = c >> 4, part = c & 15;
         const int w_row = row0 + part * 4;
@@ -356,13 +358,15 @@ __global__ void __launch_bounds__(DUAL ? 256 : 192) gemm_tcgen05_kernel(const __
         *reinterpret_cast<uint2*>(out + (size_t)(tok_base + tok) * ld + w_row) = make_uint2(o2[0], o2[1]);
       }
     } else if (warp >= 2) {
+      drain();
+      asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that drain
       const int t = threadIdx.x - 64;
       auto lds128 = [](uint32_t addr) {
         uint4 v;
         asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
         return v;
       };
-      const int total = n_tok * (TM / 8);
+      const int total = min(BN, g.M - tok_base) * (TM / 8);
       for (int c = t; c < total; c += 4 * 128) {
         uint4 y[4], x[4];
         bf16* dst[4];
