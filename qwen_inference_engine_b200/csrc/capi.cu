@@ -11,6 +11,7 @@
 #include <string>
 
 #include "engine.h"
+#include "launch.h"
 #include "model_registry.h"
 
 using namespace qie;
@@ -89,8 +90,10 @@ static int engine_sync(qie_engine* e) {
 
 static cudaError_t sm_count(int* n) {
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  return e == cudaSuccess ? cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev) : e;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  *n = device_attribute<cudaDevAttrMultiProcessorCount>(dev);
+  return *n > 0 ? cudaSuccess : cudaErrorUnknown;
 }
 
 // ---------------------------------------------------------------- operator level

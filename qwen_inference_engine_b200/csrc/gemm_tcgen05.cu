@@ -1045,11 +1045,12 @@ static TcTile pick_tile(int M, int tiles, int nkb, int num_sms, bool may_split) 
 
 // Tokens of a pair's tile, 0 where single CTAs of `bn` tokens stay.  Costs of a wave are in units of about 1 ns a k-block: a single CTA's operands take it 1.0 a row of 128
 // bytes that it brings from L2 (256 tokens: 48 KB, 0.4 us), a pair's CTA 1.22 a row or the products 1.36 a token, whichever is more; a pair's start and end cost
-// 1.2 us more, and few waves have to gain by more.  Below 20 k-blocks a tile the epilogue sets the pace.  us in graphs, single CTAs and pairs: 4096 rows 1536 x 8960 78 72 (256
+// 1.2 us more, and few waves have to gain by more.  Below PAIR_KB k-blocks a tile the epilogue sets the pace.  us in graphs, single CTAs and pairs: 4096 rows 1536 x 8960 78 72 (256
 // tokens), 8960 x 1536 83 78 (192), 3584 x 3584 79 70 (224), 2048 rows of 1536 x 8960 40 38, 1500 of 3584 x 3584 33.4 31.0 (160); stay: 2048 of 3584 x 3584 36.6 37.6
 // (224), 1000 rows 21.1 23.2 (224), 700 of 3584 x 4608 19.8 20.3 (192), 4096 of 1536 x 1536 18.4 18.4 (192), of 896 x 4864 33.3 32.2 to 36.8.
+static constexpr int PAIR_KB = 20;
 static int pick_pair(int M, int tiles, int nkb, int num_sms, int pairs, int bn) {
-  if (pairs <= 0 || nkb < 20) return 0;
+  if (pairs <= 0 || nkb < PAIR_KB) return 0;
   auto waves = [&](int t, int b, int at) { return ((long)t * ((M + b - 1) / b) + at - 1) / at; };
   const float single = (float)waves(tiles, bn, num_sms) * (float)(BM + bn);
   int best = 0;
@@ -1236,7 +1237,7 @@ cudaError_t launch_gemm_tcgen05(const TcGemm& t, int num_sms, cudaStream_t st, i
   if (tl.persist) {
     // (widths of the residual stream and of the feed-forward are inner dimensions too, so multiples of 8)
     if (!vec && t.epi != EPI_STORE) return cudaErrorInvalidValue;
-    const int pairs = pairs_at_once(), pair_bn = pick_pair(t.M, tiles, g.kb_total, num_sms, pairs, tl.bn);
+    const int pairs = g.kb_total < PAIR_KB ? 0 : pairs_at_once(), pair_bn = pick_pair(t.M, tiles, g.kb_total, num_sms, pairs, tl.bn);
     return pair_bn ? launch_persist<2>(g, pair_bn, pairs, w, t.x, t.M, t.K, st) : launch_persist<1>(g, tl.bn, num_sms, w, t.x, t.M, t.K, st);
   }
   const cudaError_t e = make_tensor_map_2d(&x, t.x, t.M, t.K, tl.bn);
