@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(DUAL ? 256 : 192, 1) gemm_tcgen05_kernel(const
   const uint32_t red = smem0;
   const bool epi_warp = warp >= 2;
   const int qd = warp & 3;  // TMEM lane quarter of this epilogue warp
-  const bool via_smem = g.splits > 1 || DUAL;
+  const bool via_smem = TM == BM && (g.splits > 1 || DUAL);  // (the tile below has 128 lanes of rows: 64-row tiles are never split, launch_bn)
   const int tile_rows = DUAL ? BM / 2 : TM;  // output rows produced by this tile
   const int rows_per = ((tile_rows + g.splits - 1) / g.splits + 3) & ~3;
   const uint32_t pitch = (uint32_t)(BM + min(rows_per, 32)) * 4u;
@@ -940,6 +940,8 @@ template <int BN, bool HALF, int KB, int TM, bool AHEAD, bool DUAL = false>
 static cudaError_t launch_bn(const TcArgs& g, const CUtensorMap* const (&w)[3], const TensorMap2D& x, int token_tiles, cudaStream_t st) {
   constexpr int STAGE_BYTES = KB * (TM * BK * 2 + BN * BK * 2);
   constexpr size_t smem = (size_t)TcCfg<BN, HALF, KB, TM>::STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static_assert(TM == BM || !DUAL, "gate/up tiles have 128 rows");
+  if (TM != BM && g.splits > 1) return cudaErrorInvalidValue;
   static PerDeviceOnce set;
   if (set.need()) {
     cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, HALF, KB, TM, AHEAD, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
