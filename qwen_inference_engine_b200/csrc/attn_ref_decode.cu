@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnA
     bool waits = a.early;
     for (int k0 = 0; k0 < kept; k0 += TV) {
       const int n = min(TV, kept - k0);
-      if (waits && k0 + n > ready) pdl_wait(), waits = false;
+      if (waits && (k0 + n > ready || ph == 0)) pdl_wait(), waits = false;  // (a wait's limit counts this kernel's time: stages come free behind the wait only)
       if (!mbar_wait_tc(vempty(s), ph, dead)) break;
       const uint32_t full = vfull(s), dst = smem_u32(smem + lay.v + s * VTILE);
       if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"(n * ROW) : "memory");
