@@ -123,6 +123,25 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
   return cudaSuccess;
 }
 
+// reference-order attention of layer l over this rank's n_q heads: of one prompt's rows, or of one row of each sequence (advance)
+static AttnArgs ref_attention(const qie_engine* e, int n, int n_q, int l, int max_kv_len, bool advance) {
+  AttnArgs a{};
+  a.q = e->q;
+  a.out = e->att;
+  a.pos = e->pos_d;
+  a.slot = e->slot_d;
+  a.block_table = e->block_table_d;
+  a.max_pages = e->max_pages_per_seq;
+  a.n_tok = n;
+  a.n_q = n_q;
+  a.layer = l;
+  a.max_kv_len = max_kv_len;
+  a.kv = e->kv;
+  a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
+  a.status = e->wait_status;
+  return a;
+}
+
 // Launch order = llm()'s (qwen_main.cu:77-222 prefill / :271-365 decode): per layer
 // rms -> q,k,v -> q/k-norm -> RoPE -> KV store -> attention -> o (+residual) -> rms ->
 // up,gate -> SiLU*up -> down (+residual); then final norm -> lm_head -> sampling.
@@ -205,24 +224,11 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
     AttnArgs ra{};  // reference-order attention
     bool posted = false;
     if (!fast) {
-      AttnArgs& a = ra;
-      a.q = e->q;
-      a.out = e->att;
-      a.pos = e->pos_d;
-      a.slot = e->slot_d;
-      a.block_table = e->block_table_d;
-      a.max_pages = e->max_pages_per_seq;
-      a.n_tok = n;
-      a.n_q = c.n_q;
-      a.layer = l;
-      a.max_kv_len = max_kv_len;
-      a.kv = e->kv;
-      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
-      a.decode = a.early = advance;
-      a.status = e->wait_status;
+      ra = ref_attention(e, n, c.n_q, l, max_kv_len, advance);
+      ra.decode = ra.early = advance;
       // a decode step's head norms, positions and store belong to the attention kernel, unless somebody looks between the two
       if (advance && !e->capture && !e->prof_on) {
-        const cudaError_t r = launch_attention_ref_post(a, post, e->num_sms, &posted, st);
+        const cudaError_t r = launch_attention_ref_post(ra, post, e->num_sms, &posted, st);
         if (r != cudaSuccess) return r;
         if (posted) ++e->launches;
       }
@@ -431,19 +437,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       QIE_TRY(KK_QKV_POST, launch_qkv_post(a, st));
     }
     {
-      AttnArgs a{};
-      a.q = e->q;
-      a.out = e->att;
-      a.pos = e->pos_d;
-      a.slot = e->slot_d;
-      a.block_table = e->block_table_d;
-      a.max_pages = e->max_pages_per_seq;
-      a.n_tok = n;
-      a.n_q = pl.n_q;
-      a.layer = l;
-      a.max_kv_len = max_kv_len;
-      a.kv = e->kv;
-      a.one_seq = !advance;  // prefill rows are consecutive positions of one sequence
+      const AttnArgs a = ref_attention(e, n, pl.n_q, l, max_kv_len, advance);
       QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
     }
     {  // o_proj over the local head columns -> partial sums -> all-reduce -> residual
