@@ -289,7 +289,7 @@ def config4_leg(q, torch, np, rank, world, local, use_dist):
         e1.record()
     eng.sync()
     ms = e0.elapsed_time(e1)
-    mega = bool(eng.uses_mega(n_seq, 32 + 8 + steps + 2)) and int(eng.launch_count()) < q.make_config(ARCH).layers  # (launches of the last step)
+    mega = bool(eng.runs_mega(n_seq, 32 + 8 + steps + 2))
     eng.close()
     if use_dist:
         t = torch.tensor([ms], device="cuda", dtype=torch.float64)
@@ -378,7 +378,7 @@ def tp_leg(q, torch, np, rank, world, local):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t.item())
         rec = {"ms_per_step": ms / steps, "tokens_per_s": batch * steps / (ms / 1e3),
-               "persistent_kernel": bool(eng.uses_mega(batch, 32 + 6 + steps + 2)),
+               "persistent_kernel": bool(eng.runs_mega(batch, 32 + 6 + steps + 2)),
                "exchanges_per_token": 2 * cfg7.layers + 1,
                "nvlink_bytes_sent_per_token_per_gpu": int((2 * cfg7.layers) * (world - 1) * batch * cfg7.hidden * 4)}
         if rec["persistent_kernel"]:
@@ -835,7 +835,7 @@ def main():
     barrier()
 
     # ---------------- per-kernel-class timing of one step (roofline leg) -----------------
-    mega = eng.uses_mega(B, eng.seq_len(seqs[0]) + 2) and int(eng.launch_count()) < cfg.layers  # (launches of the step before)
+    mega = eng.runs_mega(B, eng.seq_len(seqs[0]) + 2)
     mega_phase_us = None
     if mega:
         # ONE kernel per step: its phases are timed by device timestamps taken inside the kernel
@@ -1013,7 +1013,7 @@ def main():
             b1_bytes = q.weight_bytes(cfg) + kvpp * (eng.seq_len(s1) - 60)
             line.setdefault("extra", {})["batch1"] = {
                 "workload": "batch 1, 32-token prompt, greedy decode (qie_decode_run, 120 tokens)",
-                "persistent_kernel": bool(eng.uses_mega(1, 200)) and int(eng.launch_count()) < 120 * cfg.layers,
+                "persistent_kernel": bool(eng.runs_mega(1, 200)),
                 "tokens_per_s": 120 / dt, "us_per_token": 1e6 * dt / 120,
                 "frac_of_hbm_peak": (b1_bytes * 120 / dt / 1e9) / peak}
             eng.free_sequence(s1)
@@ -1034,7 +1034,7 @@ def main():
                                 "per token, weight rows streamed by bulk copies, warp-per-row-group FHFMA dot products, "
                                 "split-KV flash decoding, no grid barrier between the phases -- consumers poll per-layer "
                                 "activation buffers; 1e-2 tolerance per layer, tokens not bit-exact)",
-                    "persistent_kernel": bool(eng.uses_mega(1, 200)),
+                    "persistent_kernel": bool(eng.runs_mega(1, 200)),
                     "tokens_per_s": 120 / dtf, "us_per_token": 1e6 * dtf / 120,
                     "frac_of_hbm_peak": (b1_bytes * 120 / dtf / 1e9) / peak}
         except Exception as ex:  # the side measurement must never break the contract line

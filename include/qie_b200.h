@@ -394,12 +394,13 @@ const char* qie_kernel_kind_name(int kind);
 int qie_profile_begin(qie_engine* e);
 int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int n_kinds);
 
-/* Persistent decode kernel (decode_mega.cu): a reference-order decode step of up to 64 rows
- * as ONE cooperative launch.  By default a step runs so only where the operators do not
- * take it (tensor parallel, very long contexts; the same bits either way).  qie_engine_set_int keys: "mega" (0: never, 1: wherever
- * the kernel takes the step; QIE_MEGA=0 is the former), "mega_layers_run" (debug: stop after N layers, 0 = whole step), "mega_prof"
- * (0/1: record a device timestamp at every phase boundary, in the persistent kernel).
- * qie_decode_uses_mega tells whether the kernel takes a step of n rows at this KV length.
+/* Persistent decode kernel (decode_mega.cu): a reference-order decode step of up to 64 rows as ONE cooperative launch, in fast numerics one of up to 8 rows.
+ * By default a step in the reference's order runs so only where the operators' attention (attn_ref_decode.cu) does not take it: tensor parallel, pages that are
+ * no multiple of 8 positions, a pool off a 16-byte boundary or of 2^31 rows; the same bits either way.  A context that is too long for both kernels' shared memory
+ * takes the operators with attention_ref_kernel.  qie_engine_set_int keys: "mega" (0: never, as with QIE_MEGA=0 in the environment; 1: wherever the kernel
+ * takes the step; -1: the default), "mega_layers_run" (debug: stop after N layers, 0 = whole step), "mega_prof" (0/1: record a device timestamp at every phase
+ * boundary, in the persistent kernel).  qie_decode_uses_mega tells whether the kernel takes a step of n rows at this KV length, qie_decode_runs_mega
+ * whether such a step goes that way as the engine is set.
  * qie_mega_prof_read copies the timestamps (ns, globaltimer) of the last profiled step to
  * HOST memory: [0] start, then 16 per layer (QKV: rows loaded, normed, GEMM done, barrier;
  * attention: done, barrier; O: loaded, GEMM, barrier; gate/up: loaded, normed, GEMM, barrier;
@@ -412,6 +413,7 @@ int qie_profile_end(qie_engine* e, float* ms_by_kind, int* launches_by_kind, int
  * memory (names: x qkv att h logits sampled kv); returns the byte count copied. */
 int qie_engine_set_int(qie_engine* e, const char* key, long value);
 int qie_decode_uses_mega(const qie_engine* e, int n_rows, int kv_len);
+int qie_decode_runs_mega(const qie_engine* e, int n_rows, int kv_len);
 long qie_mega_prof_read(qie_engine* e, uint64_t* h_out, size_t max_values);
 long qie_engine_read_activation(qie_engine* e, const char* name, void* h_out, size_t max_bytes);
 /* Layer-isolation parity hook of the per-operator forward: qie_engine_set_int keys "layer_first" / "layer_count"

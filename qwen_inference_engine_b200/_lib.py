@@ -138,6 +138,7 @@ def lib():
         "qie_profile_end": (i32, [vp, vp, vp, i32]),
         "qie_engine_set_int": (i32, [vp, C.c_char_p, C.c_long]),
         "qie_decode_uses_mega": (i32, [vp, i32, i32]),
+        "qie_decode_runs_mega": (i32, [vp, i32, i32]),
         "qie_mega_prof_read": (C.c_long, [vp, vp, sz]),
         "qie_engine_read_activation": (C.c_long, [vp, C.c_char_p, vp, sz]),
         "qie_engine_write_activation": (C.c_long, [vp, C.c_char_p, vp, sz]),

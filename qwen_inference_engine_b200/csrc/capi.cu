@@ -1166,7 +1166,7 @@ int qie_prefill(qie_engine* e, int seq, const int32_t* h_ids, int n, int32_t* h_
 // one decode step for the batch already staged on the device (ids/pos/slot/rowstep)
 static cudaError_t decode_forward(qie_engine* e, int n, int bucket) {
   if (e->fam) return e->fam->forward(e, n, n, n, bucket, e->temp_decode, true);  // one row and one segment per sequence
-  if (decode_uses_mega(e, n, bucket) && !decode_by_operators(e, n, bucket)) {
+  if (decode_runs_mega(e, n, bucket)) {
     cudaError_t r = forward_decode_mega(e, n, bucket, e->temp_decode);
     if (r != cudaErrorNotReady) return r;  // NotReady: the cooperative launch could not be placed, nothing ran yet
   }
@@ -1465,7 +1465,7 @@ int qie_engine_set_int(qie_engine* e, const char* key, long value) {
   if (k == "dump_layers") {
     if (!e->fam) return fail(QIE_EINVAL, "dump_layers: families with an fp32 residual stream only");
     e->fam->dump_layers = value != 0;
-  } else if (k == "mega") e->use_mega = e->mega_always = value != 0;
+  } else if (k == "mega") e->use_mega = value != 0, e->mega_always = value > 0;
   else if (k == "gemv") e->use_gemv = value != 0;
   else if (k == "gemv_dataflow") e->gemv_dataflow = value;
   else if (k == "mega_layers_run") e->mega_layers_run = (int)value;
@@ -1485,6 +1485,11 @@ int qie_engine_set_int(qie_engine* e, const char* key, long value) {
 int qie_decode_uses_mega(const qie_engine* e, int n_rows, int kv_len) {
   if (!e) return 0;
   return decode_uses_mega(e, n_rows, ((kv_len + 127) / 128) * 128) ? 1 : 0;
+}
+
+int qie_decode_runs_mega(const qie_engine* e, int n_rows, int kv_len) {
+  if (!e || e->fam) return 0;
+  return decode_runs_mega(e, n_rows, ((kv_len + 127) / 128) * 128) ? 1 : 0;
 }
 
 long qie_mega_prof_read(qie_engine* e, uint64_t* h_out, size_t max_values) {

@@ -103,9 +103,9 @@ struct qie_engine {
   float* attn_ws = nullptr;      // partial results of a decode step whose keys are split more than FD_CLUSTER ways
   size_t attn_ws_rows = 0;       // (split, row, head) of them
 
-  // persistent decode kernel (decode_mega.cu): reference-order decode steps of <= 8 rows
-  bool use_mega = true;              // QIE_MEGA=0 disables
-  bool mega_always = false;          // the caller asked for the persistent kernel ("mega" 1): also where the operators are quicker
+  // persistent decode kernel (decode_mega.cu)
+  bool use_mega = true;              // QIE_MEGA=0 or "mega" 0: never
+  bool mega_always = false;          // "mega" 1: also where the operators are quicker (-1: only where they are not, the default)
   qie::MegaLayer* mega_layers_d = nullptr;
   // 7 per layer + lm_head 3-D weight views (box 8 rows x mega_kc[s]); set 1 (larger tiles) serves batches <= 8
   qie::TensorMap2D* mega_wmaps_d[2] = {nullptr, nullptr};
@@ -198,9 +198,10 @@ cudaError_t forward_rows_tp(qie_engine* e, int n_rows, int max_kv_len, int out_r
 // what every family needs besides its own buffers: the page free list and sequence slots, block tables (device +
 // pinned mirror), row metadata and the pinned staging buffers; sized by e->opts and n_pages
 cudaError_t engine_alloc_shared(qie_engine* e, int n_pages, int context);
-// true if a decode step of n rows / this kv bucket runs through the persistent kernel
+// true if the persistent kernel takes a decode step of n rows / this kv bucket
 bool decode_uses_mega(const qie_engine* e, int n_rows, int max_kv_len);
-bool decode_by_operators(const qie_engine* e, int n, int max_kv_len);  // a step that the persistent kernel takes too is quicker by operators
+// the kernel takes the step and the operators are not quicker: the way that a step goes
+bool decode_runs_mega(const qie_engine* e, int n, int max_kv_len);
 // one decode step (rows described in ids_d/pos_d/slot_d) through the persistent kernel
 cudaError_t forward_decode_mega(qie_engine* e, int n_rows, int max_kv_len, float temperature);
 }  // namespace qie

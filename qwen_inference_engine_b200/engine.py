@@ -294,7 +294,12 @@ class Engine:
         check(self._L.qie_engine_set_int(self._h, key.encode(), int(value)))
 
     def uses_mega(self, n_rows, kv_len):
+        """whether the persistent kernel takes such a decode step (by default the operators run it where they are quicker: runs_mega)"""
         return bool(self._L.qie_decode_uses_mega(self._h, n_rows, kv_len))
+
+    def runs_mega(self, n_rows, kv_len):
+        """whether such a decode step goes through the persistent kernel"""
+        return bool(self._L.qie_decode_runs_mega(self._h, n_rows, kv_len))
 
     def mega_prof(self):
         """device timestamps (ns) of the last profiled persistent-kernel step"""
