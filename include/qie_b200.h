@@ -378,6 +378,8 @@ long qie_capture_read(qie_engine* e, const char* tag, int layer, qie_bf16* h_out
 
 /* launch statistics of the last forward: kernels launched by this library. */
 long qie_launch_count(const qie_engine* e);
+/* kernels in the CUDA graphs of decode steps that the engine keeps by now (bounded; the graphs least used are given up) */
+long qie_decode_graph_kernels(const qie_engine* e);
 
 /* Measurement helpers (bench.py). qie_seq_fill_synthetic appends n_pos positions of seeded
  * random K/V to a sequence WITHOUT running the model (stand-in for a long prefill when only

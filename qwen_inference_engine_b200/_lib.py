@@ -129,6 +129,7 @@ def lib():
         "qie_capture_enable": (i32, [vp, i32]),
         "qie_capture_read": (C.c_long, [vp, C.c_char_p, i32, vp, sz]),
         "qie_launch_count": (C.c_long, [vp]),
+        "qie_decode_graph_kernels": (C.c_long, [vp]),
         "qie_seq_fill_synthetic": (i32, [vp, i32, i32, u64]),
         "qie_seq_kv_read": (i32, [vp, i32, i32, i32, vp, vp]),
         "qie_seq_kv_write": (i32, [vp, i32, i32, i32, vp, vp]),

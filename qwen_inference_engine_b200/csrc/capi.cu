@@ -495,8 +495,7 @@ static void engine_free(qie_engine* e) {
   if (!e) return;
   cudaSetDevice(e->opts.device);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  for (auto& kvp : e->graphs)
-    if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
+  e->drop_graphs();
   for (auto& kvp : e->cap)
     if (kvp.second.d) cudaFree(kvp.second.d);
   if (e->fam) {
@@ -1033,9 +1032,7 @@ int qie_engine_set_sampling(qie_engine* e, int topk, float temperature_prefill, 
                             uint64_t seed, int add_step) {
   if (!e || topk < 1 || topk > 256) return fail(QIE_EINVAL, "set_sampling: topk must be in [1,256]");
   cudaStreamSynchronize(e->stream);
-  for (auto& kvp : e->graphs)  // sampling parameters are baked into captured graphs
-    if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
-  e->graphs.clear();
+  e->drop_graphs();  // sampling parameters are baked into captured graphs
   e->topk = topk;
   e->temp_prefill = temperature_prefill;
   e->temp_decode = temperature_decode;
@@ -1056,9 +1053,7 @@ int qie_engine_set_repetition_penalty(qie_engine* e, float penalty) {
     CU(cudaMemset(e->hist_d, 0xff, n * sizeof(int)));  // -1: positions never written are ignored by the kernel
   }
   e->rep_penalty = penalty;
-  for (auto& kvp : e->graphs)  // captured graphs bake the launch sequence in
-    if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
-  e->graphs.clear();
+  e->drop_graphs();  // captured graphs bake the launch sequence in
   return QIE_OK;
 }
 
@@ -1173,34 +1168,96 @@ static cudaError_t decode_forward(qie_engine* e, int n, int bucket) {
   return forward_rows(e, n, bucket, 0, n, e->temp_decode, true);
 }
 
+// Graphs of decode steps.  Of a step's kernels only the attention depends on the positions, and a graph of 173 kernels takes 0.1 to 0.2 ms to capture, 0.3 to 1.7 ms to instantiate and
+// 1.5 MB of host memory, while a replay saves 15 to 50 us of a step by launches (0.5B, 24 layers).  So
+//  * a step's first pass is by launches (it sets the kernels' attributes, and a shape that cannot be placed is found there);
+//  * the second one takes over the graph of as many rows and fewer positions by an update (0.04 ms), which is what a batch that grows does every 128 positions.  us of the two steps
+//    behind such a point, a graph each and now: 1 row 1040 1700 to 2300, 1000 1170; 64 rows at 2000 positions 2080 2550, 2050 2000.  A graph that comes back, as with
+//    two batches in turn, gets one of its own;
+//  * else a graph of more than GRAPH_FEW kernels is made in pass GRAPH_PASS: a shape that is seen less often is as quick by launches (a batch of 1 to 64 sequences that changes
+//    every three steps 1414 -> 1179 us a step, every ten 1200 -> 1182);
+//  * at most GRAPH_KERNELS kernels (some 94 such graphs) are kept: the graph whose last use is longest ago is taken over or given up.
+// Families and tensor parallel take over none, and make theirs in the second pass.
+static constexpr long GRAPH_FEW = 16, GRAPH_PASS = 12, GRAPH_KERNELS = 16384;
+
+static cudaError_t drop_graph(qie_engine* e, qie_engine::GraphEntry& g) {
+  const cudaError_t r = cudaStreamSynchronize(e->stream);  // (it may be running)
+  cudaGraphExecDestroy(g.exec);
+  g.exec = nullptr;
+  e->graph_kernels -= g.launches;
+  return r;
+}
+
+// the kept graph whose last use is longest ago: of n rows and fewer positions, or of any (n 0)
+static qie_engine::GraphEntry* oldest_graph(qie_engine* e, int n, int bucket) {
+  qie_engine::GraphEntry* best = nullptr;
+  for (auto& kvp : e->graphs) {
+    qie_engine::GraphEntry& g = kvp.second;
+    if (!g.exec || (n && (kvp.first.first != n || kvp.first.second >= bucket || g.own))) continue;
+    if (!best || g.used < best->used) best = &g;
+  }
+  return best;
+}
+
+// captures the step into g, by an update of `from`'s graph where that can be
+static int make_graph(qie_engine* e, qie_engine::GraphEntry& g, qie_engine::GraphEntry* from, int n, int bucket) {
+  struct Graph {
+    cudaGraph_t h = nullptr;
+    ~Graph() {
+      if (h) cudaGraphDestroy(h);
+    }
+  } graph;
+  CU(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
+  const long before = e->launches;
+  const cudaError_t fe = decode_forward(e, n, bucket);
+  const cudaError_t ce = cudaStreamEndCapture(e->stream, &graph.h);
+  const long launches = e->launches - before;
+  e->launches = before;
+  if (fe != cudaSuccess) return cuda_fail(fe, "forward (capture)");
+  if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
+  g.launches = launches;
+  if (from && from->launches == launches) {  // (launches of that graph by now are not affected)
+    cudaGraphExecUpdateResultInfo info{};
+    if (cudaGraphExecUpdate(from->exec, graph.h, &info) == cudaSuccess) {
+      g.exec = from->exec;
+      from->exec = nullptr, from->own = true;
+      return QIE_OK;
+    }
+    (void)cudaGetLastError();
+    CU(drop_graph(e, *from));  // (a failed update leaves it undefined)
+  }
+  while (e->graph_kernels > 0 && e->graph_kernels + launches > GRAPH_KERNELS) CU(drop_graph(e, *oldest_graph(e, 0, 0)));
+  CU(cudaGraphInstantiate(&g.exec, graph.h, 0));
+  e->graph_kernels += launches;
+  return QIE_OK;
+}
+
 static int decode_launch(qie_engine* e, int n, int max_kv_len) {
   const int bucket = ((max_kv_len + 127) / 128) * 128;
   if (!e->opts.use_graph || e->capture || e->prof_on) {
     CU(decode_forward(e, n, bucket));
     return QIE_OK;
   }
-  auto key = std::make_pair(n, bucket);
-  auto it = e->graphs.find(key);
-  if (it == e->graphs.end()) {
-    e->graphs.emplace(key, qie_engine::GraphEntry());
-    CU(decode_forward(e, n, bucket));
-    return QIE_OK;
+  qie_engine::GraphEntry& g = e->graphs[std::make_pair(n, bucket)];
+  g.used = ++e->graph_clock, ++g.visits;
+  if (!g.exec) {
+    const bool few = g.launches <= GRAPH_FEW || e->fam || e->tp.size > 1;
+    qie_engine::GraphEntry* from = nullptr;
+    if (g.visits > 1 && !few) {
+      from = oldest_graph(e, n, bucket);
+      if (!from && e->graph_kernels + g.launches > GRAPH_KERNELS) from = oldest_graph(e, 0, 0);
+    }
+    if (g.visits < 2 || (!from && !few && g.visits < GRAPH_PASS)) {
+      const long before = e->launches;
+      CU(decode_forward(e, n, bucket));
+      g.launches = e->launches - before;
+      return QIE_OK;
+    }
+    const int rc = make_graph(e, g, from, n, bucket);
+    if (rc) return rc;
   }
-  if (!it->second.exec) {
-    cudaGraph_t graph = nullptr;
-    CU(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-    long before = e->launches;
-    cudaError_t fe = decode_forward(e, n, bucket);
-    cudaError_t ce = cudaStreamEndCapture(e->stream, &graph);
-    if (fe != cudaSuccess) return cuda_fail(fe, "forward (capture)");
-    if (ce != cudaSuccess) return cuda_fail(ce, "cudaStreamEndCapture");
-    it->second.launches = e->launches - before;
-    e->launches = before;
-    CU(cudaGraphInstantiate(&it->second.exec, graph, 0));
-    cudaGraphDestroy(graph);
-  }
-  CU(cudaGraphLaunch(it->second.exec, e->stream));
-  e->launches += it->second.launches;  // the graph replays exactly these kernels
+  CU(cudaGraphLaunch(g.exec, e->stream));
+  e->launches += g.launches;  // the graph replays exactly these kernels
   return QIE_OK;
 }
 
@@ -1337,6 +1394,7 @@ long qie_capture_read(qie_engine* e, const char* tag, int layer, qie_bf16* h_out
 }
 
 long qie_launch_count(const qie_engine* e) { return e ? e->launches : 0; }
+long qie_decode_graph_kernels(const qie_engine* e) { return e ? e->graph_kernels : 0; }
 
 // KV offload (the experiment commented out in the reference's main(), iengine.cu:376-429): the pages of a
 // sequence are copied to pinned host memory and handed back to the pool; swap-in takes fresh pages (any ids) and
@@ -1476,9 +1534,7 @@ int qie_engine_set_int(qie_engine* e, const char* key, long value) {
   else return fail(QIE_EINVAL, "unknown option %s", key);
   // captured graphs bake these choices in
   ENGINE_SYNC(e);
-  for (auto& kvp : e->graphs)
-    if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
-  e->graphs.clear();
+  e->drop_graphs();
   return QIE_OK;
 }
 

@@ -156,13 +156,22 @@ struct qie_engine {
   bool capture = false;
   std::map<std::string, qie::CaptureBuf> cap;
 
-  // CUDA graphs of the decode step keyed by (rows, kv bucket). A shape is run eagerly
-  // the first time it is seen (that also sets kernel attributes) and captured the second.
+  // CUDA graphs of the decode step by rows and positions (multiples of 128); decode_launch says when one is made, taken over or given up.
   struct GraphEntry {
     cudaGraphExec_t exec = nullptr;
-    long launches = 0;
+    long launches = 0;  // kernels of the step
+    long visits = 0, used = 0;
+    bool own = false;  // was taken over by a longer context and came back: not taken over again
   };
   std::map<std::pair<int, int>, GraphEntry> graphs;
+  long graph_clock = 0;    // steps by now, for `used`
+  long graph_kernels = 0;  // kernels in the graphs that are kept
+  void drop_graphs() {     // (the stream is idle)
+    for (auto& kvp : graphs)
+      if (kvp.second.exec) cudaGraphExecDestroy(kvp.second.exec);
+    graphs.clear();
+    graph_kernels = 0;
+  }
 
   long launches = 0;
 

@@ -322,6 +322,10 @@ class Engine:
     def launch_count(self):
         return self._L.qie_launch_count(self._h)
 
+    def decode_graph_kernels(self):
+        """kernels in the CUDA graphs of decode steps that are kept"""
+        return self._L.qie_decode_graph_kernels(self._h)
+
     # -- parity hooks ------------------------------------------------------------
     def capture(self, on=True):
         check(self._L.qie_capture_enable(self._h, int(on)))
