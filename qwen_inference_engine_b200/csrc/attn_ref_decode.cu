@@ -161,7 +161,7 @@ struct Weigh {
 // POST: the queries, the key and the value of the row come from the projections: bias, head norm and rotary position as in qkv_post_kernel (head_ops.cu), queries back in place,
 // key and value into the pool by the first part of a kv head.  The last position's key and value are read from shared memory, all others from the pool.
 template <int NP, bool POST>
-__global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnArgs a, const int hp, const int stages, const int box, const __grid_constant__ CUtensorMap kvm,
+__global__ void __launch_bounds__(NT, 1) attention_ref_decode_kernel(const AttnRefCall a, const int hp, const int stages, const int box, const __grid_constant__ CUtensorMap kvm,
                                                                      const QkvPostArgs post) {
   constexpr int HD = 64 * NP, RW = 2 / NP, GK = 32 * RW, ROW = HD * 2, WORDS = 32 * NP, TV = VTILE / ROW;
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -468,7 +468,7 @@ static int heads_of(const AttnArgs& a, int num_sms, int* stages, bool post) {
   return 0;
 }
 
-static cudaError_t launch_decode(const AttnArgs& a, int heads, int stages, const QkvPostArgs* post, cudaStream_t st) {
+static cudaError_t launch_decode(const AttnRefCall& a, int heads, int stages, const QkvPostArgs* post, cudaStream_t st) {
   const int G = a.n_q / a.kv.n_kv, parts = (G + heads - 1) / heads;
   const size_t smem = layout_of(a.kv.hd, heads, a.max_kv_len, a.kv.page_size, stages, post != nullptr).total;
   int box = 8;  // rows of a copy: as many as a page and a group hold
@@ -492,13 +492,13 @@ static cudaError_t launch_decode(const AttnArgs& a, int heads, int stages, const
 // Heads of a CTA, 0 where this kernel does not take the call.
 int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages) { return heads_of(a, num_sms, stages, false); }
 
-cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages, cudaStream_t st) { return launch_decode(a, heads, stages, nullptr, st); }
+cudaError_t launch_attention_ref_decode(const AttnRefCall& a, int heads, int stages, cudaStream_t st) { return launch_decode(a, heads, stages, nullptr, st); }
 
 // What launch_qkv_post and this kernel do, in one launch: the store and the way back of the queries and a start of a kernel less, and the keys of a step are
 // asked for while the projections run.  us a step of 24 layers, 14 heads of 64 on 2, two launches and one: 64 rows at 2048 positions 1712 1693, 16 at 500 994 971, 5 at 100 892
 // 860.  Heads of 128 keep two: 28 layers, 12 heads on 2, 32 rows at 500 1759 1777, 8 at 100 1457 1488, 16 at 1000 1870 1906 (64 at 300 1834 1821).  Nor where a row or a
 // table is off a 16-byte boundary (*taken false, nothing launched).
-cudaError_t launch_attention_ref_post(const AttnArgs& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st) {
+cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st) {
   uintptr_t at = 0;
   for (const void* q : {(const void*)p.q, (const void*)p.q_in, (const void*)p.k, (const void*)p.v, (const void*)p.q_norm_w, (const void*)p.k_norm_w, (const void*)p.cos_t,
                         (const void*)p.sin_t, (const void*)p.q_bias, (const void*)p.k_bias, (const void*)p.v_bias})

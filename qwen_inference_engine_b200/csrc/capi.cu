@@ -187,7 +187,7 @@ int qie_attention(const qie_kv_view* kv, int layer, const qie_bf16* Q, qie_bf16*
   if (!kv || layer < 0 || layer >= kv->n_layers) return fail(QIE_EINVAL, "attention: bad layer");
   if (!heads_ok(n_q_heads, kv->n_kv_heads)) return fail(QIE_EINVAL, "attention: %d query heads on %d kv heads", n_q_heads, kv->n_kv_heads);
   OP_STATUS(status);
-  AttnArgs a{};
+  AttnRefCall a{};
   a.status = status;
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
@@ -208,7 +208,7 @@ int qie_attention_pagelist(const qie_bf16* const* d_k_pages, const qie_bf16* con
                            int n_tok, int n_q_heads, qie_stream st) {
   if (!d_k_pages || !d_v_pages || n_pages <= 0 || page_size <= 0 || layer < 0 || layer >= n_layers || !heads_ok(n_q_heads, n_kv_heads))
     return fail(QIE_EINVAL, "attention_pagelist: bad geometry");
-  AttnArgs a{};
+  AttnRefCall a{};
   a.q = (const bf16*)Q;
   a.out = (bf16*)out;
   a.pos = pos;

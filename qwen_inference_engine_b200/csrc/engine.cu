@@ -124,8 +124,8 @@ static cudaError_t gemm_tc(qie_engine* e, int kind, const bf16* x, int n, int K,
 }
 
 // reference-order attention of layer l over this rank's n_q heads: of one prompt's rows, or of one row of each sequence (advance)
-static AttnArgs ref_attention(const qie_engine* e, int n, int n_q, int l, int max_kv_len, bool advance) {
-  AttnArgs a{};
+static AttnRefCall ref_attention(const qie_engine* e, int n, int n_q, int l, int max_kv_len, bool advance) {
+  AttnRefCall a{};
   a.q = e->q;
   a.out = e->att;
   a.pos = e->pos_d;
@@ -221,7 +221,7 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       a.rope_half = e->rope_half ? 1 : 0;
       a.early = 1;  // (the projections start when the norm lets them, which it does behind its own wait)
     }
-    AttnArgs ra{};  // reference-order attention
+    AttnRefCall ra{};  // reference-order attention
     bool posted = false;
     if (!fast) {
       ra = ref_attention(e, n, c.n_q, l, max_kv_len, advance);
@@ -437,7 +437,7 @@ cudaError_t forward_rows_tp(qie_engine* e, int n, int max_kv_len, int out_row0, 
       QIE_TRY(KK_QKV_POST, launch_qkv_post(a, st));
     }
     {
-      const AttnArgs a = ref_attention(e, n, pl.n_q, l, max_kv_len, advance);
+      const AttnRefCall a = ref_attention(e, n, pl.n_q, l, max_kv_len, advance);
       QIE_TRY(KK_ATTN, launch_attention_ref(a, st));
     }
     {  // o_proj over the local head columns -> partial sums -> all-reduce -> residual

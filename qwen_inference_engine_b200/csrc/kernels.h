@@ -111,22 +111,26 @@ struct AttnArgs {
   const bf16* const* v_pages = nullptr;
   int pl_layers = 0;
   int one_seq = 0;    // 1: every row is known to belong to one sequence (a prompt, a page list)
+  int tile_rows = 0;  // attention_ref_kernel: leave tiles of this many rows to attention_ref_rows_kernel where they are one sequence's; 0: none
+};
+// a call: what only attn_ref_decode.cu's kernel reads besides.  (Apart from the others' arguments: with 16 bytes more of them the compiler gives attention_ref_rows_kernel other
+// registers: 500 rows behind 300 positions 0.4 % slower.)
+struct AttnRefCall : AttnArgs {
   int decode = 0;     // 1: every row is of a sequence of its own (a decode step)
   int early = 0;      // 1: the kernel in front writes nothing that the attention reads but q and the rows of position pos[t], and waits for its own predecessor before it
                       // lets this one start (qkv_post_kernel): other keys, values and the tables may be read while it runs
   int* status = nullptr;  // host word that a wait which ran out sets, or null
-  int tile_rows = 0;  // attention_ref_kernel: leave tiles of this many rows to attention_ref_rows_kernel where they are one sequence's; 0: none
 };
-cudaError_t launch_attention_ref(const AttnArgs& a, cudaStream_t st);
+cudaError_t launch_attention_ref(const AttnRefCall& a, cudaStream_t st);
 // the same for rows of one sequence (attn_ref_rows.cu): rows a CTA takes and virtual rows (row x query head) of its tile, 0 if it does
 // not take these sizes
 int attention_ref_tile_rows(const AttnArgs& a, int num_sms, int* virtual_rows);
 cudaError_t launch_attention_ref_rows(const AttnArgs& a, int rows, int virtual_rows, cudaStream_t st);
 // the same for rows of sequences of their own (attn_ref_decode.cu): heads that a CTA takes and stages of its ring of values, 0 if it does not take these sizes
 int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages);
-cudaError_t launch_attention_ref_decode(const AttnArgs& a, int heads, int stages, cudaStream_t st);
+cudaError_t launch_attention_ref_decode(const AttnRefCall& a, int heads, int stages, cudaStream_t st);
 // launch_qkv_post and it in one launch, for decode steps (a.decode, a.early; the kernel in front writes nothing but the projections that p names); *taken: whether it did
-cudaError_t launch_attention_ref_post(const AttnArgs& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st);
+cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st);
 // K, V rows [n_tok, kv_dim] -> positions pos0 + t of a page list in the reference's layout (see AttnArgs)
 cudaError_t launch_kv_store_pagelist(bf16* const* k_pages, bf16* const* v_pages, int page_size, int n_layers, int layer, int kv_dim,
                                      const bf16* K, const bf16* V, int pos0, int n_tok, cudaStream_t st);

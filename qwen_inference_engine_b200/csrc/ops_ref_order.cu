@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(256) attention_ref_kernel(AttnArgs a) {
   }
 }
 
-cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
+cudaError_t launch_attention_ref(const AttnRefCall& args, cudaStream_t st) {
   if (args.n_tok == 0) return cudaSuccess;
   AttnArgs a = args;
   if (a.kv.hd == 64 || a.kv.hd == 128 || a.kv.hd == 256) {
@@ -508,7 +508,7 @@ cudaError_t launch_attention_ref(const AttnArgs& args, cudaStream_t st) {
     if (heads) {
       const int G = a.n_q / a.kv.n_kv;
       const long ctas = (long)a.n_tok * a.kv.n_kv * ((G + heads - 1) / heads), waves = (ctas + sms - 1) / sms;
-      if (a.decode || (a.tile_rows && (waves == 1 ? heads < 6 || a.max_kv_len > 32 : heads >= 6 && a.max_kv_len >= (heads == G ? 160 : 225) * waves))) return launch_attention_ref_decode(a, heads, stages, st);
+      if (args.decode || (a.tile_rows && (waves == 1 ? heads < 6 || a.max_kv_len > 32 : heads >= 6 && a.max_kv_len >= (heads == G ? 160 : 225) * waves))) return launch_attention_ref_decode(args, heads, stages, st);
     }
     if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
       e = launch_attention_ref_rows(a, a.tile_rows, vr, st);
