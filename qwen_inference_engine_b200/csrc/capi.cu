@@ -1174,6 +1174,7 @@ static cudaError_t decode_forward(qie_engine* e, int n, int bucket) {
 //  * the second one takes over the graph of as many rows and fewer positions by an update (0.04 ms), which is what a batch that grows does every 128 positions.  us of the two steps
 //    behind such a point, a graph each and now: 1 row 1040 1700 to 2300, 1000 1170; 64 rows at 2000 positions 2080 2550, 2050 2000.  A graph that comes back, as with
 //    two batches in turn, gets one of its own;
+//  * an engine without graphs makes its first one in the second pass too (a program whose batch stays as it is);
 //  * else a graph of more than GRAPH_FEW kernels is made in pass GRAPH_PASS: a shape that is seen less often is as quick by launches (a batch of 1 to 64 sequences that changes
 //    every three steps 1414 -> 1179 us a step, every ten 1200 -> 1182);
 //  * at most GRAPH_KERNELS kernels (some 94 such graphs) are kept: the graph whose last use is longest ago is taken over or given up.
@@ -1247,7 +1248,7 @@ static int decode_launch(qie_engine* e, int n, int max_kv_len) {
       from = oldest_graph(e, n, bucket);
       if (!from && e->graph_kernels + g.launches > GRAPH_KERNELS) from = oldest_graph(e, 0, 0);
     }
-    if (g.visits < 2 || (!from && !few && g.visits < GRAPH_PASS)) {
+    if (g.visits < 2 || (!from && !few && e->graph_kernels > 0 && g.visits < GRAPH_PASS)) {
       const long before = e->launches;
       CU(decode_forward(e, n, bucket));
       g.launches = e->launches - before;
