@@ -204,8 +204,12 @@ def run_reference(args):
     import numpy as np
     import torch
     from oracle.oracle import Ref, RefSeq
+    try:
+        ref = Ref()
+    except ImportError as ex:  # its sources are needed to build it
+        print(json.dumps({"impl": "reference", "unavailable": str(ex)}), flush=True)
+        return 0
     torch.cuda.set_device(0)
-    ref = Ref()
     desc = _ref_model_on_device(ARCH_DIMS)
     rs = RefSeq(ref, desc, page_size=4)  # the reference's main() uses page_size 4 (iengine.cu:334)
     rs.fake_context(CTX)                 # pages for CTX + 64 positions: the timed tokens never take the allocate-on-demand path

@@ -211,3 +211,18 @@ def test_heads_that_make_no_groups_are_refused(n_q, n_kv):
     assert lib.qie_attention_prefill_fast(C.byref(kv), 0, *ptr, 8, 4, n_q, None) == -1
     assert lib.qie_attention_decode_fast(C.byref(kv), 0, *ptr, 8, 4, n_q, 0, None) == -1
     assert lib.qie_attention_pagelist(*ptr[:2], 8, 16, 1, 0, n_kv, 64, *ptr[2:], 4, n_q, None) == -1
+
+
+def test_reference_arm_without_the_reference():
+    """bench.py --impl reference where the reference's kernels are not built: one line that says so, and no error"""
+    import json
+    import os
+    import subprocess
+    import sys
+    from oracle.oracle import REF_SO
+    if os.path.exists(REF_SO):
+        pytest.skip("the reference's kernels are built here")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, os.path.join(root, "bench.py"), "--impl", "reference", "--gpus", "1", "--steps", "2", "--warmup", "3"], cwd=root, capture_output=True, text=True)
+    line = json.loads(r.stdout)
+    assert r.returncode == 0 and line["impl"] == "reference" and line["unavailable"]
