@@ -901,7 +901,7 @@ def main():
     peak, peak_src = measured_peaks()
     H, I, hd = cfg.hidden, cfg.inter, cfg.head_dim
     Dq, Dkv = cfg.n_q * hd, cfg.n_kv * hd
-    alg_bytes = {  # algorithmic bytes of ONE launch of each class
+    alg_bytes = {  # algorithmic bytes of ONE launch of each class (attention of heads of 64: with head norms, positions and store)
         "attention": B * ctx_now * 2 * Dkv * 2 + 2 * B * Dq * 2,
         "gemm_qkv": 2 * H * (Dq + 2 * Dkv) + B * 2 * (H + Dq + 2 * Dkv),
         "gemm_o": 2 * Dq * H + B * 2 * (Dq + 2 * H),

@@ -497,16 +497,24 @@ cudaError_t launch_attention_ref_decode(const AttnRefCall& a, int heads, int sta
 // What launch_qkv_post and this kernel do, in one launch: the store and the way back of the queries and a start of a kernel less, and the keys of a step are
 // asked for while the projections run.  us a step of 24 layers, 14 heads of 64 on 2, two launches and one: 64 rows at 2048 positions 1712 1693, 16 at 500 994 971, 5 at 100 892
 // 860.  Heads of 128 keep two: 28 layers, 12 heads on 2, 32 rows at 500 1759 1777, 8 at 100 1457 1488, 16 at 1000 1870 1906 (64 at 300 1834 1821).  Nor where a row or a
-// table is off a 16-byte boundary (*taken false, nothing launched).
-cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st) {
+// table is off a 16-byte boundary.
+static int post_heads(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, int* stages) {
   uintptr_t at = 0;
   for (const void* q : {(const void*)p.q, (const void*)p.q_in, (const void*)p.k, (const void*)p.v, (const void*)p.q_norm_w, (const void*)p.k_norm_w, (const void*)p.cos_t,
                         (const void*)p.sin_t, (const void*)p.q_bias, (const void*)p.k_bias, (const void*)p.v_bias})
     at |= reinterpret_cast<uintptr_t>(q);
-  int stages = 0, heads = 0;
-  if (a.kv.hd == 64 && a.decode && a.early && a.n_tok > 0 && at % 16 == 0 && p.q_in_stride % 8 == 0 && p.kv_stride % 8 == 0) heads = heads_of(a, num_sms, &stages, true);
-  *taken = heads > 0;
-  return heads ? launch_decode(a, heads, stages, &p, st) : cudaSuccess;
+  return a.kv.hd == 64 && a.decode && a.early && a.n_tok > 0 && at % 16 == 0 && p.q_in_stride % 8 == 0 && p.kv_stride % 8 == 0 ? heads_of(a, num_sms, stages, true) : 0;
+}
+
+bool attention_ref_post_takes(const AttnRefCall& a, const QkvPostArgs& p, int num_sms) {
+  int stages = 0;
+  return post_heads(a, p, num_sms, &stages) > 0;
+}
+
+cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, cudaStream_t st) {
+  int stages = 0;
+  const int heads = post_heads(a, p, num_sms, &stages);
+  return heads ? launch_decode(a, heads, stages, &p, st) : cudaErrorInvalidValue;
 }
 
 }  // namespace qie

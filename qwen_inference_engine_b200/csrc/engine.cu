@@ -227,13 +227,10 @@ cudaError_t forward_rows(qie_engine* e, int n, int max_kv_len, int out_row0, int
       ra = ref_attention(e, n, c.n_q, l, max_kv_len, advance);
       ra.decode = ra.early = advance;
       // a decode step's head norms, positions and store belong to the attention kernel, unless somebody looks between the two
-      if (advance && !e->capture && !e->prof_on) {
-        const cudaError_t r = launch_attention_ref_post(ra, post, e->num_sms, &posted, st);
-        if (r != cudaSuccess) return r;
-        if (posted) ++e->launches;
-      }
+      posted = advance && !e->capture && attention_ref_post_takes(ra, post, e->num_sms);
     }
-    if (!posted) QIE_TRY(KK_QKV_POST, launch_qkv_post(post, st));
+    if (posted) QIE_TRY(KK_ATTN, launch_attention_ref_post(ra, post, e->num_sms, st));
+    else QIE_TRY(KK_QKV_POST, launch_qkv_post(post, st));
     capture_copy(e, "q", l, e->q, (size_t)n * Dq);
     if (!tc) capture_copy(e, "v", l, e->v, (size_t)n * Dkv);
     if (fast_attn) {

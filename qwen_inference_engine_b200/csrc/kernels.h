@@ -129,8 +129,9 @@ cudaError_t launch_attention_ref_rows(const AttnArgs& a, int rows, int virtual_r
 // the same for rows of sequences of their own (attn_ref_decode.cu): heads that a CTA takes and stages of its ring of values, 0 if it does not take these sizes
 int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages);
 cudaError_t launch_attention_ref_decode(const AttnRefCall& a, int heads, int stages, cudaStream_t st);
-// launch_qkv_post and it in one launch, for decode steps (a.decode, a.early; the kernel in front writes nothing but the projections that p names); *taken: whether it did
-cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, bool* taken, cudaStream_t st);
+// launch_qkv_post and it in one launch, for decode steps (a.decode, a.early; the kernel in front writes nothing but the projections that p names)
+bool attention_ref_post_takes(const AttnRefCall& a, const QkvPostArgs& p, int num_sms);
+cudaError_t launch_attention_ref_post(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, cudaStream_t st);
 // K, V rows [n_tok, kv_dim] -> positions pos0 + t of a page list in the reference's layout (see AttnArgs)
 cudaError_t launch_kv_store_pagelist(bf16* const* k_pages, bf16* const* v_pages, int page_size, int n_layers, int layer, int kv_dim,
                                      const bf16* K, const bf16* V, int pos0, int n_tok, cudaStream_t st);

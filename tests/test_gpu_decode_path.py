@@ -33,3 +33,22 @@ def test_ways(page, default, graph):
             e.free_sequence(s)
     e.close()
     assert all(np.array_equal(got[0], g) for g in got)
+
+
+@pytest.mark.parametrize("hd,kinds", [(64, ("attention",)), (128, ("qkv_post", "attention"))])
+def test_a_profile_times_the_launches_of_the_step(hd, kinds):
+    """heads of 64: one launch does the head norms, the positions, the store and the attention, in a profiled step as in others"""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_inference_engine_b200 as q
+    cfg = q.make_config(dict(hidden=256, inter=512, layers=3, n_q=4, n_kv=2, head_dim=hd, vocab=2048), context=256)
+    e = q.Engine(synthetic=cfg, seed=7, context=256, max_batch_tokens=64, max_seqs=4, max_pages=64)
+    seqs = [e.new_sequence() for _ in range(3)]
+    tokens = [e.prefill(s, prompt_ids(5 + i, 2048, seed=i)) for i, s in enumerate(seqs)]
+    tokens = e.decode_step(seqs, tokens)
+    launches = e.launch_count()
+    prof = e.decode_step_profile(seqs, tokens)
+    e.close()
+    assert [k for k in ("qkv_post", "attention") if prof.get(k, (0, 0))[1]] == list(kinds) and prof["attention"][1] == 3
+    assert sum(n for _, n in prof.values()) == launches
