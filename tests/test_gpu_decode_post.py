@@ -1,6 +1,6 @@
 """Decode steps whose attention kernel does the head norms, the positions and the store (csrc/attn_ref_decode.cu) against steps that launch qkv_post_kernel in
 front of it (the engine's captures of q and v): logits and tokens bit for bit, at edges of the groups of keys and of the stages of values, over steps that read
-what earlier ones stored."""
+what earlier ones stored.  Heads of 128 have two launches either way, by graphs and by launches."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,7 @@ def test_against_two_kernels(nq, nkv, hd, batch, page):
         pytest.skip("no CUDA device")
     import qwen_inference_engine_b200 as q
     cfg = q.make_config(dict(hidden=256, inter=512, layers=2, n_q=nq, n_kv=nkv, head_dim=hd, vocab=2048), context=512)
-    got = []
+    got, launches = [], []
     for capture in (False, True):
         e = q.Engine(synthetic=cfg, seed=3, context=512, max_seqs=batch, max_batch_tokens=batch, max_pages=batch * (320 // page + 2), page_size=page)
         e.set_int("mega", 0)
@@ -32,8 +32,10 @@ def test_against_two_kernels(nq, nkv, hd, batch, page):
         for _ in range(4):
             tokens = e.decode_step(seqs, tokens)
             out.append((np.array(tokens), e.read_activation("logits", batch * 2048)))
+        launches.append(e.launch_count())
         e.close()
         got.append(out)
+    assert launches[1] - launches[0] == (2 if hd == 64 else 0)  # a launch a layer
     for (t0, l0), (t1, l1) in zip(*got):
         assert np.array_equal(t0, t1)
         assert np.array_equal(l0.view(np.uint16), l1.view(np.uint16))

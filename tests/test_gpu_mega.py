@@ -127,9 +127,34 @@ def test_mega_qwen05b_batch64_long_context(qie):
     assert np.array_equal(res[1][0], res[0][0])
 
 
-def test_mega_config2_batch64_ctx2048_vs_reference_kernels(qie, ref):
+def test_mega_batch64_ctx2048(qie):
+    """0.5B-arch, 64 sequences with 2048 cached positions each: two steps of ONE persistent kernel equal those by operators (the default), logits, tokens and the new
+    positions of the cache"""
+    cfg = qie.make_config("qwen2.5-0.5b")
+    B, ctx, got = 64, 2048, []
+    for mega in (1, -1):
+        eng = qie.Engine(synthetic="qwen2.5-0.5b", seed=1234, max_seqs=B + 1, max_batch_tokens=64, use_graph=False,
+                         kv_bytes=B * (ctx + 64) * qie.kv_bytes_per_pos(cfg) + (64 << 20))
+        eng.set_int("mega", mega)
+        assert eng.runs_mega(B, ctx + 2) == (mega == 1)
+        seqs = [eng.new_sequence() for _ in range(B)]
+        for i, s in enumerate(seqs):
+            eng.fill_synthetic(s, ctx, seed=i)
+        tok, out = (np.arange(B, dtype=np.int32) * 977 + 5) % cfg.vocab, []
+        for _ in range(2):
+            tok = eng.decode_step(seqs, tok)
+            assert (eng.launch_count() < cfg.layers) == (mega == 1)
+            out += [tok.copy(), eng.read_activation("logits", B * cfg.vocab)]
+        out += [x for s in (seqs[0], seqs[37], seqs[63]) for x in eng.kv_read(s, ctx, 2)]
+        got.append(out)
+        eng.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("mega", [1, -1])
+def test_mega_config2_batch64_ctx2048_vs_reference_kernels(qie, ref, mega):
     """0.5B-arch, 64 sequences with 2048 cached positions each, ONE persistent
-    kernel step -- and for three of the 64 rows the reference's own kernels (oracle/_ref, llm()'s decode branch) run
+    kernel step, and one by operators (the default) -- and for three of the 64 rows the reference's own kernels (oracle/_ref, llm()'s decode branch) run
     on the SAME cache contents and input token: logits and the greedy token must be bit-identical."""
     from oracle.oracle import RefSeq
     cfg = qie.make_config("qwen2.5-0.5b")
@@ -141,7 +166,8 @@ def test_mega_config2_batch64_ctx2048_vs_reference_kernels(qie, ref):
         s = eng.new_sequence()
         eng.fill_synthetic(s, ctx, seed=i)
         seqs.append(s)
-    assert eng.uses_mega(B, ctx + 1)
+    eng.set_int("mega", mega)
+    assert eng.uses_mega(B, ctx + 1) and eng.runs_mega(B, ctx + 1) == (mega == 1)
     tok_in = (np.arange(B, dtype=np.int32) * 977 + 5) % cfg.vocab
     rows = (0, 37, 63)
     cache = {r: eng.kv_read(seqs[r], 0, ctx) for r in rows}  # [ctx, L, Dkv] = the reference's page layout
@@ -164,7 +190,6 @@ def test_mega_config2_batch64_ctx2048_vs_reference_kernels(qie, ref):
         rs.close()
         assert np.array_equal(logits[r], want_logits), f"row {r}: logits differ from the reference kernels"
         assert int(tok_out[r]) == want_tok
-    # the new position's K/V row written by the persistent kernel equals what a per-operator step writes
     eng.close()
 
 
@@ -184,13 +209,15 @@ def test_mega_graph_replay_and_topk(qie):
     eng.close()
 
 
-def test_mega_config1_vs_reference_kernels(qie, ref):
-    """the batch-1 workload through the persistent kernel: 128 greedy tokens identical to the
+@pytest.mark.parametrize("mega", [1, -1])
+def test_mega_config1_vs_reference_kernels(qie, ref, mega):
+    """the batch-1 workload through the persistent kernel and by operators (the default): 128 greedy tokens identical to the
     reference's own kernels."""
     from test_gpu_e2e_vs_reference import _ref_generate
     eng = qie.Engine(synthetic="qwen2.5-0.5b", seed=1234, max_batch_tokens=64, kv_bytes=256 << 20)
     ids = prompt_ids(32, eng.config.vocab)
-    assert eng.uses_mega(1, 160)
+    eng.set_int("mega", mega)
+    assert eng.uses_mega(1, 160) and eng.runs_mega(1, 160) == (mega == 1)
     want, _, _ = _ref_generate(ref, eng, ids, 128)
     assert eng.generate(ids, 128) == want
     eng.close()
