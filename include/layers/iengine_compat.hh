@@ -130,7 +130,7 @@ void load_weight(const tensor& t, std::ifstream&, T*, T*& d, size_t, __nv_bfloat
 }
 // the two kernels llm() / initialize_model_buffers launch directly with <<<>>> (embedding_matrix_func: utills.cu:51-54,
 // qwen_main.cu:259-267; the sampler: qwen_main.cu:388) cannot cross a shared-library boundary as __global__ symbols;
-// a maintainer replaces those three launches with launch_embedding / sample_topk_bf16 (INTEGRATION.md)
+// a maintainer replaces those three launches with launch_embedding / sample_topk_bf16
 void launch_embedding(__nv_bfloat16* out, __nv_bfloat16* table, int* d_token_ids, size_t hidden, size_t n_tok);
 // helpers.cuh:121-129.  Row t of Q attends to cache positions 0 .. min(mkv - 1, causal ? q_abs_base + t : mkv - 1) of the
 // page list (reference layout, see allocate_page_buffers)

@@ -1189,7 +1189,7 @@ __global__ void __launch_bounds__(GV_THREADS, 1) decode_gemv_kernel(const __grid
     if (a.prof && l == 5) xt0 = (long long)globaltimer();
 #endif
     gv_gemv<NB, PH_GATEUP>(a, g, p, smem, smem_base, ring, act, best, A.hh(l));
-#ifdef GV_PROFILE_DETAIL  // start / end of this phase on every CTA (tools/mega_probe.py)
+#ifdef GV_PROFILE_DETAIL  // start / end of this phase on every CTA
     if (a.prof && l == 5 && threadIdx.x == 0 && gridDim.x <= 148) {
       a.prof[a.prof_stride + 8 + blockIdx.x] = globaltimer();
       a.prof[a.prof_stride + 8 + 148 + blockIdx.x] = (unsigned long long)xt0;

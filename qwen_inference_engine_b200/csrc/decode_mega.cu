@@ -424,7 +424,7 @@ struct Best {
 // 8..15 of the MMA tile are register zeros).  MT >= 1: 16*MT token rows by ldmatrix.
 // The accumulation is a dependent HMMA chain per output tile (k ascending: the reference's
 // order); measured on B200 the dependent HMMA.16816 latency is 20.7 cycles and the issue
-// interval 8 cycles per SM sub-partition (tools/ubench/hmma_lat.cu), so the fragment loads
+// interval 8 cycles per SM sub-partition, so the fragment loads
 // (LDSM/LDS, ~33 cycles) are software-pipelined one group of k-steps ahead in registers and
 // never sit on the chain.
 template <int MT, bool DUAL>  // MT here = token tiles handled by ONE warp (0: the <= 8 token path)

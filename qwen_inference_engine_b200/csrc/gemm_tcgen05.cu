@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(DUAL ? 256 : 192, 1) gemm_tcgen05_kernel(const
 // CTAs share a token tile in L2), the accumulator is double buffered in TMEM (2 x 256 columns), and the epilogue of tile j (TMEM ->
 // bf16 staging tile in shared memory -> global memory, 64 tokens at a time) runs on warps 2-9 while warps 0/1 already
 // stream and multiply tile j+1.  ncu on the one-tile-per-CTA kernel showed the tensor pipe 32-47 % active at K = 1536: per tile
-// ~2.5 us of prologue and ~8 us of epilogue sat next to a ~7-9 us mainloop (profiles/r01c_ncu_full_prefill_kernels.csv).
+// ~2.5 us of prologue and ~8 us of epilogue sat next to a ~7-9 us mainloop.
 // A tile has g.bn tokens, any multiple of 16 (pick_tile): with 256 always, 4096 tokens x 1536 outputs were 192 tiles on 148 SMs, two
 // waves filled to 65 %.  The ring takes the stages that fit: 4 of 48 KiB at 256 tokens, 10 of 18 KiB at 16.
 static constexpr int PBN = 256;                   // TMEM columns of an accumulator

@@ -8,7 +8,7 @@
 //   selfattention  src/self_attension.cu:10-149
 //   sampling       src/logit_decode.cu:149-274
 // This file is compiled with -fmad=false; every fused multiply-add that nvcc's default
-// contraction makes of the reference's source expressions is spelled __fmaf_rn here (tools/ubench/fma_contract.cu
+// contraction makes of the reference's source expressions is spelled __fmaf_rn here (oracle/fma_contract.cu
 // finds the placement from outputs), everything else is an explicit _rn intrinsic.
 #include <curand_kernel.h>
 #include <math_constants.h>

@@ -3,7 +3,7 @@
 // (ops_ref_order.cu, gemm_ref_order.cu) and the persistent decode kernel (decode_mega.cu).
 // Translation units including this header are compiled with -fmad=false: every fused
 // multiply-add that nvcc's default contraction makes of the reference's source expressions is
-// spelled __fmaf_rn (which product of a two-product sum it fuses: tools/ubench/fma_contract.cu
+// spelled __fmaf_rn (which product of a two-product sum it fuses: oracle/fma_contract.cu
 // compares outputs), everything else is an explicit _rn intrinsic.
 #pragma once
 #include <math_constants.h>

@@ -5,7 +5,7 @@
 //   initialize_model_buffers (:25-47) -> create_page_list + allocate_page_buffers per page (:334-351) ->
 //   llm(prefill) -> { generated_token / state = decode / step++ ; llm(decode) } (:384-456)
 // -- so that "iengine's main() compiles and runs against the B200 library" is something a test executes
-// (tests/test_gpu_compat_replay.py), not a claim in INTEGRATION.md.  What the reference hard-codes (absolute paths,
+// (tests/test_gpu_compat_replay.py), not a claim.  What the reference hard-codes (absolute paths,
 // the prompt literal, getchar() between tokens) comes from argv / the environment here.
 //   usage: QIE_META=<meta_data.txt> main_callseq <weights.bin> <n_new_tokens> <id> <id> ...
 #include <cstdio>

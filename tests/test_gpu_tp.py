@@ -1,11 +1,10 @@
 """gpu (needs >= 2 GPUs, skipped otherwise): tensor-parallel engine over NCCL, launched the way
-bench.py is (torchrun, one rank per GPU).  tools/tp_probe.py --check compares the TP engine with
+bench.py is (torchrun, one rank per GPU).  tp_probe.py --check compares the TP engine with
 a tp_size 1 engine on rank 0: every rank returns the same tokens and the teacher-forced greedy
 choices agree except at near-ties.  The ranks' o_proj / down_proj partial sums are added in fp32
 and rounded to bf16 once, so a TP forward differs from the unsharded one only by the fp32 sum
 order (a bf16 output moves by one ulp where the sum sits on a rounding boundary).  Random-init
-weights amplify such flips layer by layer (the same growth the fast-numerics probe shows:
-tools/fast_error_probe.py), so the bounds are: logits of ONE forward of the 3-layer model within
+weights amplify such flips layer by layer (the same growth as of fast numerics), so the bounds are: logits of ONE forward of the 3-layer model within
 the 1e-2 bf16 tolerance; for the 24-layer architecture and after 18 decode steps
 of KV history the measured 2-3e-2 is bounded by 6e-2 and the token agreement is asserted."""
 import json
@@ -35,7 +34,7 @@ def test_tp2_matches_single_gpu(arch, batch):
     if torch.cuda.device_count() < 2:
         pytest.skip("needs 2 GPUs")
     cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", "--nproc-per-node", "2", "--master-addr",
-           "127.0.0.1", "--master-port", str(_free_port()), os.path.join(ROOT, "tools", "tp_probe.py"), "--arch", arch,
+           "127.0.0.1", "--master-port", str(_free_port()), os.path.join(ROOT, "tests", "tp_probe.py"), "--arch", arch,
            "--batch", str(batch), "--prompt", "12", "--steps", "16", "--warmup", "2", "--check"]
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=900, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]

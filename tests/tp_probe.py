@@ -1,7 +1,7 @@
 """Tensor-parallel probe: run under torchrun, one rank per GPU.
 
   python -m torch.distributed.run --nnodes=1 --nproc-per-node 2 --master-addr 127.0.0.1 \
-      --master-port 29511 tools/tp_probe.py --arch qwen2.5-7b --steps 64 [--check]
+      --master-port 29511 tests/tp_probe.py --arch qwen2.5-7b --steps 64 [--check]
 
 Every rank builds the same synthetic checkpoint on its GPU, takes its shard by pointer
 arithmetic (qie_tp_plan) and decodes greedily; o_proj / down_proj partial sums are
