@@ -13,6 +13,8 @@
 #include <curand_kernel.h>
 #include <math_constants.h>
 
+#include <climits>
+
 #include <algorithm>
 #include <type_traits>
 #include <map>
@@ -499,8 +501,11 @@ cudaError_t launch_attention_ref(const AttnRefCall& args, cudaStream_t st) {
     // (us, attention_ref_rows_kernel and here, 14 heads of 64 on 2: 1 row at 301 positions 14.3 7.9, at 2001 60 24, 32 rows behind 300 15.6 9.1, 64 behind 2000
     // 63 35; 17 rows of a prompt 5.8 5.4; up to 16 positions one block per row and head, 3.5 4.5).  More rows than that share their keys and values here in tiles of several rows,
     // which is worth more the shorter the context: w waves are quicker above 160 w positions with all of six to eight heads in a CTA (96 rows behind 120 15.6 15.1, behind 50
-    // 12.5 13.5; 200 behind 300 41 33; 300 behind 800 93 90, behind 300 47 55), above 225 w with a part of them (16 heads on 1, 200 behind 2000 166 108, 300 behind 800
-    // 90 93), one above 32 (24 rows of a prompt, 28 heads of 128 on 4 6.7 7.7).  Operator calls with tables beyond attention_ref_rows_kernel's sizes stay with the
+    // 12.5 13.5; 200 behind 300 41 33; 180 behind 300 40 32).  Tiles of several rows with heads of 64: above 250 w (14 heads on 2, 400 rows behind 800 109 115, behind 600 90 97; 8 heads
+    // on 1, 640 behind 400 69 80).  Three and more waves of rows on a single kv head, whose keys and values are few: above 180 w (8 heads, 300 behind 200 28.2 30.0, 360 behind 200
+    // 35.9 34.3).  A part of a kv head's heads in a CTA: above 225 w (16 heads on 1, 200 behind 2000 166 108, 300 behind 800 90 93), four and more waves of such rows that the tiles take at
+    // once above 300 w (240 behind 900 71 80).  One wave above 32 (24 rows of a prompt, 28 heads of 128 on 4 6.7 7.7).  Over 4680 sizes (twelve pairs of head counts, 17 to 700 rows behind 0 to
+    // 1500 positions) what is taken is at most 2.7 % slower so, 16 % with 160 w and 225 w alone.  Operator calls with tables beyond attention_ref_rows_kernel's sizes stay with the
     // kernel below.
     int stages = 0;
     const int heads = attention_ref_decode_heads(a, sms, &stages);
@@ -508,7 +513,14 @@ cudaError_t launch_attention_ref(const AttnRefCall& args, cudaStream_t st) {
     if (heads) {
       const int G = a.n_q / a.kv.n_kv;
       const long ctas = (long)a.n_tok * a.kv.n_kv * ((G + heads - 1) / heads), waves = (ctas + sms - 1) / sms;
-      if (args.decode || (a.tile_rows && (waves == 1 ? heads < 6 || a.max_kv_len > 32 : heads >= 6 && a.max_kv_len >= (heads == G ? 160 : 225) * waves))) return launch_attention_ref_decode(args, heads, stages, st);
+      const auto positions = [&]() -> long {  // from where on rows on their own are quicker than tiles
+        if (waves == 1) return heads < 6 ? 0 : 33;
+        if (heads < 6) return LONG_MAX;
+        if (heads < G) return (waves > 3 && (long)((a.n_tok + a.tile_rows - 1) / a.tile_rows) * a.kv.n_kv <= 2 * sms ? 300 : 225) * waves;
+        if (a.kv.hd == 64 && a.tile_rows > 1) return 250 * waves;
+        return (a.kv.hd == 64 && a.kv.n_kv == 1 && waves > 2 ? 180 : 160) * waves;
+      };
+      if (args.decode || (a.tile_rows && a.max_kv_len >= positions())) return launch_attention_ref_decode(args, heads, stages, st);
     }
     if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
       e = launch_attention_ref_rows(a, a.tile_rows, vr, st);
