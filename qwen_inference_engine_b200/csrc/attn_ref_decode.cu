@@ -489,6 +489,19 @@ static cudaError_t launch_decode(const AttnRefCall& a, int heads, int stages, co
   return a.kv.hd == 64 ? go(attention_ref_decode_kernel<1, false>, set[0]) : go(attention_ref_decode_kernel<2, false>, set[1]);
 }
 
+// A CTA takes 5 to 6 us before its positions count, so several waves of short contexts are quicker by one block per row and head or per row (a kv head's heads side by side).  us a step of
+// four layers, 1024 wide, those kernels and this one: a head a kv head, nine waves and more up to 128 positions (16 heads of 64 on 16, 150 rows at 20 419 615, at 100 of 128 rows and 256 rows
+// 1023 1074; 8 on 8, 256 at 20 452 601, at 60 587 628, at 100 717 660); parts of a kv head's heads, three waves up to 128 positions (16 on 1, 200 at 20 296 314, at 100 315 324), from four waves
+// on up to 512 of 64, 1024 of 128 (256 at 20 314 352, at 200 363 385, at 400 412 424; 16 of 128 on 1 335 369, 426 439, 520 536).  All else is quicker here or within 3 % (256 rows at 20:
+// 14 heads of 64 on 2 340 350, 12 of 128 on 2 353 364).
+bool attention_ref_decode_step(const AttnArgs& a, int num_sms, int heads) {
+  const int G = a.n_q / a.kv.n_kv;
+  const long ctas = (long)a.n_tok * a.kv.n_kv * ((G + heads - 1) / heads), waves = (ctas + num_sms - 1) / num_sms;
+  if (G == 1) return waves < 9 || a.max_kv_len > 128;
+  if (G > 8) return waves < 3 || a.max_kv_len > (waves == 3 ? 128 : 8 * a.kv.hd);
+  return true;
+}
+
 // Heads of a CTA, 0 where this kernel does not take the call.
 int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages) { return heads_of(a, num_sms, stages, false); }
 
@@ -503,7 +516,9 @@ static int post_heads(const AttnRefCall& a, const QkvPostArgs& p, int num_sms, i
   for (const void* q : {(const void*)p.q, (const void*)p.q_in, (const void*)p.k, (const void*)p.v, (const void*)p.q_norm_w, (const void*)p.k_norm_w, (const void*)p.cos_t,
                         (const void*)p.sin_t, (const void*)p.q_bias, (const void*)p.k_bias, (const void*)p.v_bias})
     at |= reinterpret_cast<uintptr_t>(q);
-  return a.kv.hd == 64 && a.decode && a.early && a.n_tok > 0 && at % 16 == 0 && p.q_in_stride % 8 == 0 && p.kv_stride % 8 == 0 ? heads_of(a, num_sms, stages, true) : 0;
+  if (a.kv.hd != 64 || !a.decode || !a.early || a.n_tok < 1 || at % 16 || p.q_in_stride % 8 || p.kv_stride % 8) return 0;
+  const int heads = heads_of(a, num_sms, stages, true);
+  return heads && attention_ref_decode_step(a, num_sms, heads) ? heads : 0;
 }
 
 bool attention_ref_post_takes(const AttnRefCall& a, const QkvPostArgs& p, int num_sms) {

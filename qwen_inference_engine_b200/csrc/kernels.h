@@ -128,6 +128,7 @@ int attention_ref_tile_rows(const AttnArgs& a, int num_sms, int* virtual_rows);
 cudaError_t launch_attention_ref_rows(const AttnArgs& a, int rows, int virtual_rows, cudaStream_t st);
 // the same for rows of sequences of their own (attn_ref_decode.cu): heads that a CTA takes and stages of its ring of values, 0 if it does not take these sizes
 int attention_ref_decode_heads(const AttnArgs& a, int num_sms, int* stages);
+bool attention_ref_decode_step(const AttnArgs& a, int num_sms, int heads);  // whether a decode step is quicker so than with the kernels that launch_attention_ref has besides
 cudaError_t launch_attention_ref_decode(const AttnRefCall& a, int heads, int stages, cudaStream_t st);
 // launch_qkv_post and it in one launch, for decode steps (a.decode, a.early; the kernel in front writes nothing but the projections that p names)
 bool attention_ref_post_takes(const AttnRefCall& a, const QkvPostArgs& p, int num_sms);

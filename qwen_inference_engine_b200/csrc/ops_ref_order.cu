@@ -520,7 +520,7 @@ cudaError_t launch_attention_ref(const AttnRefCall& args, cudaStream_t st) {
         if (a.kv.hd == 64 && a.tile_rows > 1) return 250 * waves;
         return (a.kv.hd == 64 && a.kv.n_kv == 1 && waves > 2 ? 180 : 160) * waves;
       };
-      if (args.decode || (a.tile_rows && a.max_kv_len >= positions())) return launch_attention_ref_decode(args, heads, stages, st);
+      if (args.decode ? attention_ref_decode_step(a, sms, heads) : a.tile_rows && a.max_kv_len >= positions()) return launch_attention_ref_decode(args, heads, stages, st);
     }
     if (a.tile_rows) {  // (a tile of one row is one sequence's whatever the rows are)
       e = launch_attention_ref_rows(a, a.tile_rows, vr, st);

@@ -65,3 +65,32 @@ def test_biases_and_halves(tmp_path, kind):
     for (t0, l0), (t1, l1) in zip(*got):
         assert np.array_equal(t0, t1)
         assert np.array_equal(l0.view(np.uint16), l1.view(np.uint16))
+
+
+@pytest.mark.parametrize("nq,nkv,hd,batch", [(16, 16, 64, 90), (8, 8, 128, 170), (16, 1, 64, 200), (9, 1, 64, 230), (16, 1, 128, 256)])
+@pytest.mark.parametrize("first", [1, 120])
+def test_many_rows_of_short_contexts(nq, nkv, hd, batch, first):
+    """several waves of CTAs at contexts where the steps go to other kernels (attention_ref_decode_step), and over the end of that range, against steps of a few rows: tokens and logits
+    bit for bit"""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_inference_engine_b200 as q
+    cfg = q.make_config(dict(hidden=256, inter=512, layers=2, n_q=nq, n_kv=nkv, head_dim=hd, vocab=2048), context=512)
+    got = []
+    for portion in (batch, 8):
+        e = q.Engine(synthetic=cfg, seed=3, context=512, max_seqs=batch, max_batch_tokens=batch, max_pages=batch * 12)
+        e.set_int("mega", 0)
+        seqs = [e.new_sequence() for _ in range(batch)]
+        for i, s in enumerate(seqs):
+            e.fill_synthetic(s, first + i % 7, seed=100 + i)
+        tokens, out = np.arange(batch, dtype=np.int32) + 7, []
+        for _ in range(8):
+            step = [(np.array(e.decode_step(seqs[b:b + portion], tokens[b:b + portion])), e.read_activation("logits", len(seqs[b:b + portion]) * 2048)) for b in range(0, batch, portion)]
+            tokens = np.concatenate([t for t, _ in step])
+            out.append((tokens, np.concatenate([x for _, x in step])))
+        e.close()
+        got.append(out)
+    for (t0, l0), (t1, l1) in zip(*got):
+        assert np.array_equal(t0, t1)
+        assert np.array_equal(l0.view(np.uint16), l1.view(np.uint16))
