@@ -490,10 +490,10 @@ static cudaError_t launch_decode(const AttnRefCall& a, int heads, int stages, co
 }
 
 // A CTA takes 5 to 6 us before its positions count, so several waves of short contexts are quicker by one block per row and head or per row (a kv head's heads side by side).  us a step of
-// four layers, 1024 wide, those kernels and this one: a head a kv head, nine waves and more up to 128 positions (16 heads of 64 on 16, 150 rows at 20 419 615, at 100 of 128 rows and 256 rows
-// 1023 1074; 8 on 8, 256 at 20 452 601, at 60 587 628, at 100 717 660); parts of a kv head's heads, three waves up to 128 positions (16 on 1, 200 at 20 296 314, at 100 315 324), from four waves
-// on up to 512 of 64, 1024 of 128 (256 at 20 314 352, at 200 363 385, at 400 412 424; 16 of 128 on 1 335 369, 426 439, 520 536).  All else is quicker here or within 3 % (256 rows at 20:
-// 14 heads of 64 on 2 340 350, 12 of 128 on 2 353 364).
+// four layers, 1024 wide, by those kernels and by this one: a head a kv head, nine waves and more up to 128 positions (16 heads of 64 on 16, 150 rows at 20 397 617, 256 at 20 560 961,
+// at 60 773 1022, at 100 995 1070; 8 on 8, 256 at 20 429 601, at 100 676 657); parts of a kv head's heads, three waves up to 128 positions (16 on 1, 200 at 20 276 312, at
+// 100 295 324), from four waves on up to 512 of 64, 1024 of 128 (256 at 20 292 351, at 200 339 384, at 400 386 425; 16 of 128 on 1 314 370, 401 437, 498 535).  All else is quicker
+// here or nearly so (256 rows at 20 against the kernels before: 14 heads of 64 on 2 340 350, 12 of 128 on 2 353 364; 200 of 4 on 4 323 362).
 bool attention_ref_decode_step(const AttnArgs& a, int num_sms, int heads) {
   const int G = a.n_q / a.kv.n_kv;
   const long ctas = (long)a.n_tok * a.kv.n_kv * ((G + heads - 1) / heads), waves = (ctas + num_sms - 1) / num_sms;
