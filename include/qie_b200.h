@@ -343,9 +343,9 @@ int qie_forward_batch(qie_engine* e, int n_entries, const int* h_seqs, const int
 int qie_decode_step_device(qie_engine* e, const int* h_seqs, int n);
 int qie_sync(qie_engine* e);
 /* Kernels whose waits have a limit report one that ran out (their results are then not numbers): engine calls return QIE_ECUDA when they
- * wait for the stream, operators that use such kernels (qie_matmul, qie_matmul_fast, qie_attention_prefill_*) when the next one is called, or this call
+ * wait for the stream, operators that use such kernels (qie_matmul, qie_matmul_fast, qie_attention, qie_attention_prefill_*) when the next one is called, or this call
  * does, behind the caller's own synchronisation.  A report is given once; the context stays usable.  qie_wait_selftest runs a wait that nothing
- * ends (about two seconds) through the same path: on the engine (returns QIE_ECUDA), or with a null engine as an operator on `st`. */
+ * ends (about two seconds, in the first CTA of a pair, of which the other one reports) through the same path: on the engine (returns QIE_ECUDA), or with a null engine as an operator on `st`. */
 int qie_kernel_status(void);
 int qie_wait_selftest(qie_engine* e, qie_stream st);
 

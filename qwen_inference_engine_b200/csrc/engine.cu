@@ -534,7 +534,8 @@ bool decode_uses_mega(const qie_engine* e, int n, int max_kv_len) {
 // that wait for one another and streams every phase's operands by itself; the operators have their products on tcgen05 and that attention.  us a step in graphs,
 // persistent kernel and operators: 0.5B, 24 layers, 64 rows at 2000 positions 2894 and 1690; 8 at 200 1254 and 890, at 30 1163 and 829; 4 at 250 1210 and 907, at 30 1091 and
 // 826; 2 at 100 1069 and 856; 1 at 1000 1463 and 1091, at 300 1139 and 921, at 30 997 and 862.  1.5B, 28 layers: 4 at 300 2271 and 1525, 1 at 30 1855 and 1444.  7B, 4 layers: 1
-// at 32 893 and 730, 16 at 2000 1491 and 901.  Rows of 128 to 256: 1 at 16 123 and 113, 126 and 125.
+// at 32 893 and 730, 16 at 2000 1491 and 901.  Rows of 128 to 256: 1 at 16 123 and 113, 126 and 125.  Without graphs too: 0.5B 1 at 30 1016 and 930, at 1000 1483 and 1169, 8 at 300 1338 and
+// 1009, 64 at 300 1970 and 1132, at 2000 2936 and 1733; 1.5B 1 at 30 1877 and 1534; 64 to 128 wide 92 and 86 to 131 and 116.
 static bool decode_by_operators(const qie_engine* e, int n, int max_kv_len) {
   const qie_config& c = e->cfg;
   if (e->mega_always || e->mega_prof_on || e->mega_layers_run > 0 || e->tp.size > 1 || e->opts.numerics == QIE_NUMERICS_FAST) return false;

@@ -1086,7 +1086,7 @@ static cudaError_t launch_persist(TcArgs g, int bn, int at, const CUtensorMap* c
   long w_rows = 0;  // K elements each, like the tokens
   for (int i = 0; i < g.nseg; ++i) w_rows += (g.dual ? 2 : 1) * g.seg[i].rows;
   // A wave's CTAs share a token tile and bring all weights, which the next wave finds in L2 unless they are too many: then the CTAs share weight tiles and bring all
-  // tokens, if those are few.  us of 3584 x 18944 (136 MB): 400 rows 57.7 48.9, 4096 single CTAs 477 363, pairs 423 333; 896 x 151936, 1000 rows 280 241; 18944 x 3584, 1000
+  // tokens, if those are few.  (64 MB: half of the L2.)  us of 3584 x 18944 (136 MB): 400 rows 57.7 48.9, 4096 single CTAs 477 363, pairs 423 333; 896 x 151936, 1000 rows 280 241; 18944 x 3584, 1000
   // rows 161 135, but 2048 (78 MB of tokens) 228 255.
   g.tokens_first = 2 * w_rows * K > 64l << 20 && 2 * M < w_rows;
   g.stages = std::min(P_MAX_STAGES, P_RING / (BM * BK * 2 + bn / CTAS * BK * 2));
