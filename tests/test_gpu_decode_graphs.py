@@ -68,3 +68,21 @@ def test_a_bounded_number_of_graphs():
         assert not graph or most > MOST // 2
         got.append(out)
     assert all(np.array_equal(t0, t1) for t0, t1 in zip(*got))
+
+
+@pytest.mark.parametrize("batch", [1, 20])
+def test_runs_without_waits_between_steps(batch):
+    """decode_run over several multiples of 128 positions: graphs are taken over while earlier launches of them are on their way"""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import qwen_inference_engine_b200 as q
+    got = []
+    for graph, e in engines(q, "small", batch, 800):
+        seqs = [e.new_sequence() for _ in range(batch)]
+        for i, s in enumerate(seqs):
+            e.fill_synthetic(s, 100 - i, seed=i)
+        got.append(np.array(e.decode_run(seqs, np.arange(batch, dtype=np.int32), 600)))
+        assert graph == (e.decode_graph_kernels() > 0)
+        assert not graph or e.decode_graph_kernels() < 100  # one graph, which five lengths had in turn
+    assert np.array_equal(*got)
